@@ -5,20 +5,28 @@
 // accuracy, the half k-lattice inside the sphere of radius nmax * 2pi/L, the
 // prefactors, the charge list by type, the rigid-pair and self-energy
 // discounts, the Coulomb constants per type pair and layer).
-// Device, FP64, compiled with -fmad=false:
-//   k_ewald_sf     one block per group of charged atoms: the powers
-//                  exp(i 2pi m x_d / L), m = 0..nmax, by the reference's complex
-//                  recursion into shared memory, then per k-vector the
-//                  block's partial type structure factors S(k, t)
-//   k_ewald_sigma  per k-vector: S summed over blocks in block order,
-//                  sigma(k, t) = sum_u S(k, u) lambda(u, t), energy terms
-//                  prefac(k) sum_t Re(S conj-free dot sigma), grid reduction
-//   k_ewald_force  one thread per charged atom: its powers in shared memory,
-//                  F += sum_k vec(k) (Re sigma Im qe - Re qe Im sigma),
-//                  added to the pair forces (no atomics: one thread per atom)
-// Arithmetic order follows the CPU oracle: q exp(i k.r) = ((q G1) G2) G3,
-// structure factors summed in charge-list order (blocks in order), forces
-// summed over k-vectors in order.
+// Device, FP64.  Both sums are bound by the FP64 pipe (2 FMA per clock per SM), so
+// the kernels are built around the fewest FP64 operations per atom and k-vector and
+// an even spread over the SMs.  The k-vectors come in rows (n1, n2) with
+// n3 = -z..z; with a = q exp(i(n1 x + n2 y)) computed once per row and g = exp(i m z),
+// the products Re a Re g, Im a Im g, Re a Im g, Im a Re g serve both n3 = m and
+// n3 = -m: 2 FMAs per k-vector in the structure factors, 4 in the forces (about 16
+// and 22 operations when every k-vector is evaluated by itself).
+//   k_ewald_tables the powers exp(i 2pi m x_d / L), m = 0..nmax, of every charged
+//                  atom, by the reference's complex recursion (charge included in x)
+//   k_ewald_sf     one block per group of tasks (row, 4 values of m) and chunk of
+//                  charged atoms of one type: the chunk's partial structure factors
+//   k_ewald_sigma  per pair of k-vectors (m, -m): S summed over the type's chunks in
+//                  order, sigma(k, t) = sum_u S(k, u) lambda(u, t), energy terms
+//                  prefac(k) sum_t Re(S conj-free dot sigma), grid reduction; the
+//                  four coefficients per (row, m) that the forces need
+//   k_ewald_force  a few atoms per block, the rows spread over 32 threads per atom:
+//                  F += sum_k vec(k) (Re sigma Im qe - Re qe Im sigma), added to the
+//                  pair forces (no atomics: one thread per component)
+// Every sum has a fixed order (atoms of a chunk, chunks, rows of a thread, threads),
+// so results do not depend on scheduling.
+// 3,000 charges, nmax 12 (1000 water molecules, accuracy 1e-6): structure factors 2395
+// -> 77 us, forces 3528 -> 97 us (about 46 and 80 us at the pipe's peak).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -29,152 +37,229 @@
 namespace emdee {
 
 static const double EW_PI = 3.14159265358979324;
-static const int SF_THREADS = 256;
-static const int FORCE_ATOMS = 64;
+// structure factors: tasks per block, values of m per task, charged atoms staged at a time
+static const int SF_THREADS = 192, SF_M = 4, SF_ATOMS = 16;
+// Forces: atoms per block and threads per atom.  Small blocks of equal work: 3,000 atoms
+// give 750 blocks, 4.9 per SM, so that the last round of blocks costs little.
+static const int FORCE_ATOMS = 4, FORCE_SPLIT = 32;
+// Atoms whose power tables a block held when the k-vectors per dimension were limited
+// to what fits: the limit is kept.
+static const int TABLE_LIMIT_ATOMS = 64;
 
 struct EwArgs {
   const double* R;
   double invL;   // 1 / current box length (theta = 2 pi R / L)
-  int nq, nvecs, nmax, ntypes;
+  double unit2;  // 2 * 2 pi / L of the set-up: vec(k) = unit2 prefac(k) n
+  int nq, nvecs, nmax, ntypes, ntasks, nrows, npairs, nchunks;
   const int* item;
   const int* qtype;
   const double* value;
-  const int* first;
-  const int* last;
-  const int4* n;
+  const int4* task;     // n1, n2, first m, row
+  const int4* row;      // n1, n2, z, first pair; rows in descending z
+  const int2* pair;     // per (row, m = 0..z): k-vectors with n3 = m and n3 = -m (-1: none)
+  const int4* chunk;    // first atom, last + 1, type
+  const int* typeChunk;  // per type: its chunks [typeChunk[t], typeChunk[t + 1])
   const double* prefac;
-  const double* vec;
   const double* lambda;   // this layer: [t][u]
-  double2* partial;       // [block][t][v]
-  double2* sigma;         // [t][v]
-  int sfBlocks, qb;
+  double2* table;         // [d][m][atom]
+  double2* partial;       // [chunk][v]
+  double2* coef;          // [t][pair][2]: (U, V), (X, Y)
   double* F;
   double* epart;
   unsigned int* ticket;
   double* result;
+  double* hostResult;
 };
 
-// powers exp(i 2pi m x / L), m = 0..nm, of one coordinate into table rows
-// row(m) = base + m * stride (src/kspace_ewald.f90:205-243: B = Z; G(j) = B; B = B*Z)
-__device__ __forceinline__ void power_table(double x, double invL, int nm, double2* base, int stride) {
-  const double theta = 6.28318530717958648 * (x * invL);
+// powers exp(i 2pi m x / L), m = 0..nm, of every coordinate of the charged atoms
+// (src/kspace_ewald.f90:205-243: B = Z; G(j) = B; B = B*Z); those of x times the charge
+__global__ void __launch_bounds__(128) k_ewald_tables(EwArgs A) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= 3 * A.nq) return;
+  const int d = k / A.nq, j = k - d * A.nq;
+  const double q = d == 0 ? A.value[j] : 1.0;
+  const double theta = 6.28318530717958648 * (A.R[3 * A.item[j] + d] * A.invL);
   double zi, zr;
   sincos(theta, &zi, &zr);
-  base[0] = make_double2(1.0, 0.0);
+  double2* out = A.table + (size_t)d * (A.nmax + 1) * A.nq + j;
+  out[0] = make_double2(q, 0.0);
   double br = zr, bi = zi;
-  for (int m = 1; m <= nm; m++) {
-    base[(size_t)m * stride] = make_double2(br, bi);
+  for (int m = 1; m <= A.nmax; m++) {
+    out[(size_t)m * A.nq] = make_double2(q * br, q * bi);
     const double nr = br * zr - bi * zi, ni = br * zi + bi * zr;
     br = nr;
     bi = ni;
   }
 }
 
-__device__ __forceinline__ double2 table_get(const double2* row0, int stride, int m) {
-  if (m >= 0) return row0[(size_t)m * stride];
-  const double2 g = row0[(size_t)(-m) * stride];
-  return make_double2(g.x, -g.y);
-}
-
-// q exp(i k.r) = ((q G1) G2) G3
-__device__ __forceinline__ double2 qeikr(double q, double2 g1, double2 g2, double2 g3) {
-  const double ar = q * g1.x, ai = q * g1.y;
-  const double br = ar * g2.x - ai * g2.y, bi = ar * g2.y + ai * g2.x;
-  return make_double2(br * g3.x - bi * g3.y, br * g3.y + bi * g3.x);
+// a = G1 G2 (conjugated for negative n2)
+__device__ __forceinline__ double2 row_phase(double2 gx, double2 gy, int n2) {
+  const double gyi = n2 < 0 ? -gy.y : gy.y;
+  return make_double2(fma(gx.x, gy.x, -(gx.y * gyi)), fma(gx.x, gyi, gx.y * gy.x));
 }
 
 __global__ void __launch_bounds__(SF_THREADS) k_ewald_sf(EwArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int QB = A.qb, QS = QB + 1;   // row stride: odd, so rows fall in different banks
-  const int nm = A.nmax, rows = nm + 1;
-  double2* G = (double2*)smem;        // [d][m][a], row (d, m) at (d * rows + m) * QS
-  double* qs = (double*)(G + (size_t)3 * rows * QS);
-  const int a0 = blockIdx.x * QB, na = min(QB, A.nq - a0);
-  for (int a = threadIdx.x; a < na; a += blockDim.x) {
-    const int i = A.item[a0 + a];
-    qs[a] = A.value[a0 + a];
-    for (int d = 0; d < 3; d++) power_table(A.R[3 * i + d], A.invL, nm, G + (size_t)d * rows * QS + a, QS);
-  }
-  __syncthreads();
-  for (int v = threadIdx.x; v < A.nvecs; v += blockDim.x) {
-    const int4 nv = A.n[v];
-    for (int t = 0; t < A.ntypes; t++) {
-      const int s0 = max(A.first[t] - a0, 0), s1 = min(A.last[t] - a0, na);
-      double sr = 0.0, si = 0.0;
-      for (int a = s0; a < s1; a++) {
-        const double2 c = qeikr(qs[a], G[(size_t)nv.x * QS + a], table_get(G + (size_t)rows * QS + a, QS, nv.y),
-                                table_get(G + (size_t)2 * rows * QS + a, QS, nv.z));
-        sr += c.x;
-        si += c.y;
-      }
-      A.partial[((size_t)blockIdx.x * A.ntypes + t) * A.nvecs + v] = make_double2(sr, si);
+  double2* T = (double2*)smem;   // [atom][d][m], an odd number of entries per atom
+  const int rows = A.nmax + 1, W = 3 * rows, S = W | 1;
+  const int ti = blockIdx.x * SF_THREADS + threadIdx.x;
+  const bool active = ti < A.ntasks;
+  const int4 task = active ? A.task[ti] : make_int4(0, 0, 1, 0);
+  const int4 ch = A.chunk[blockIdx.y];
+  const int ox = task.x, oy = rows + abs(task.y);
+  int oz[SF_M];
+#pragma unroll
+  for (int u = 0; u < SF_M; u++) oz[u] = 2 * rows + min(task.z + u, A.nmax);
+  double s0r = 0.0, s0i = 0.0, rr[SF_M], ii[SF_M], ri[SF_M], ir[SF_M];
+#pragma unroll
+  for (int u = 0; u < SF_M; u++) rr[u] = ii[u] = ri[u] = ir[u] = 0.0;
+  for (int a0 = ch.x; a0 < ch.y; a0 += SF_ATOMS) {
+    const int na = min(SF_ATOMS, ch.y - a0);
+    __syncthreads();
+    for (int k = threadIdx.x; k < W * SF_ATOMS; k += SF_THREADS) {
+      const int e = k / SF_ATOMS, a = k % SF_ATOMS;
+      if (a < na) T[a * S + e] = A.table[(size_t)e * A.nq + a0 + a];
     }
+    __syncthreads();
+    if (!active) continue;
+    for (int a = 0; a < na; a++) {
+      const double2* t = T + a * S;
+      const double2 c = row_phase(t[ox], t[oy], task.y);
+      if (task.z == 1) {
+        s0r += c.x;
+        s0i += c.y;
+      }
+#pragma unroll
+      for (int u = 0; u < SF_M; u++) {
+        const double2 g = t[oz[u]];
+        rr[u] = fma(c.x, g.x, rr[u]);
+        ii[u] = fma(c.y, g.y, ii[u]);
+        ri[u] = fma(c.x, g.y, ri[u]);
+        ir[u] = fma(c.y, g.x, ir[u]);
+      }
+    }
+  }
+  if (!active) return;
+  const int4 row = A.row[task.w];
+  double2* out = A.partial + (size_t)blockIdx.y * A.nvecs;
+  if (task.z == 1) {
+    const int v = A.pair[row.w].x;
+    if (v >= 0) out[v] = make_double2(s0r, s0i);
+  }
+#pragma unroll
+  for (int u = 0; u < SF_M; u++) {
+    const int m = task.z + u;
+    if (m > row.z) break;
+    const int2 v = A.pair[row.w + m];
+    if (v.x >= 0) out[v.x] = make_double2(rr[u] - ii[u], ri[u] + ir[u]);
+    if (v.y >= 0) out[v.y] = make_double2(rr[u] + ii[u], ir[u] - ri[u]);
   }
 }
 
 static const int EW_MAXT = 16;   // charged atom types handled by the k-space kernels
+static const int SIGMA_PAIRS = 32, SIGMA_SLICES = 8;
 
-__global__ void __launch_bounds__(256) k_ewald_sigma(EwArgs A) {
-  double e[1] = {0.0};
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v < A.nvecs) {
-    double Sr[EW_MAXT], Si[EW_MAXT];
-    for (int u = 0; u < A.ntypes; u++) {
-      double sr = 0.0, si = 0.0;
-      for (int b = 0; b < A.sfBlocks; b++) {
-        const double2 p = A.partial[((size_t)b * A.ntypes + u) * A.nvecs + v];
-        sr += p.x;
-        si += p.y;
-      }
-      Sr[u] = sr;
-      Si[u] = si;
+__global__ void __launch_bounds__(SIGMA_PAIRS * SIGMA_SLICES) k_ewald_sigma(EwArgs A) {
+  __shared__ double part[SIGMA_SLICES][4][SIGMA_PAIRS];
+  __shared__ double Ss[EW_MAXT][4][SIGMA_PAIRS];
+  const int x = threadIdx.x % SIGMA_PAIRS, y = threadIdx.x / SIGMA_PAIRS;
+  const int p = blockIdx.x * SIGMA_PAIRS + x;
+  const int2 v = p < A.npairs ? A.pair[p] : make_int2(-1, -1);
+  for (int u = 0; u < A.ntypes; u++) {
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    const double2 none = make_double2(0.0, 0.0);
+    for (int c = A.typeChunk[u] + y; c < A.typeChunk[u + 1]; c += SIGMA_SLICES) {
+      const double2* in = A.partial + (size_t)c * A.nvecs;
+      const double2 a = v.x >= 0 ? in[v.x] : none, b = v.y >= 0 ? in[v.y] : none;
+      s[0] += a.x;
+      s[1] += a.y;
+      s[2] += b.x;
+      s[3] += b.y;
     }
-    double d = 0.0;
+    for (int k = 0; k < 4; k++) part[y][k][x] = s[k];
+    __syncthreads();
+    if (y < 4) {
+      double t = 0.0;
+      for (int k = 0; k < SIGMA_SLICES; k++) t += part[k][y][x];
+      Ss[u][y][x] = t;
+    }
+    __syncthreads();
+  }
+  double e[1] = {0.0};
+  if (y == 0 && p < A.npairs) {
+    const double pp = v.x >= 0 ? A.prefac[v.x] : 0.0, pm = v.y >= 0 ? A.prefac[v.y] : 0.0;
+    double dp = 0.0, dm = 0.0;
     for (int t = 0; t < A.ntypes; t++) {
-      double r = 0.0, im = 0.0;
+      double s[4] = {0.0, 0.0, 0.0, 0.0};
       for (int u = 0; u < A.ntypes; u++) {
         const double lam = A.lambda[t * A.ntypes + u];
-        r += Sr[u] * lam;
-        im += Si[u] * lam;
+        for (int k = 0; k < 4; k++) s[k] += Ss[u][k][x] * lam;
       }
-      A.sigma[(size_t)t * A.nvecs + v] = make_double2(r, im);
-      d += Sr[t] * r + Si[t] * im;
+      dp += Ss[t][0][x] * s[0] + Ss[t][1][x] * s[1];
+      dm += Ss[t][2][x] * s[2] + Ss[t][3][x] * s[3];
+      const double wp = A.unit2 * pp, wm = A.unit2 * pm;
+      const double ar = wp * s[0], ai = wp * s[1], br = wm * s[2], bi = wm * s[3];
+      double2* out = A.coef + ((size_t)t * A.npairs + p) * 2;
+      out[0] = make_double2(ar + br, ai - bi);
+      out[1] = make_double2(ar - br, ai + bi);
     }
-    e[0] = A.prefac[v] * d;
+    e[0] = pp * dp + pm * dm;
   }
-  grid_reduce<1, 256>(e, A.epart, A.ticket, A.result);
+  grid_reduce<1, SIGMA_PAIRS * SIGMA_SLICES>(e, A.epart, A.ticket, A.result, A.hostResult);
 }
 
-__global__ void __launch_bounds__(FORCE_ATOMS) k_ewald_force(EwArgs A) {
+// With rho = unit2 prefac sigma, a row adds to (x, y, z) the values n1 Im(a H0),
+// n2 Im(a H0) and Im(a H1), H0 = sum conj(rho) g^n3, H1 = sum n3 conj(rho) g^n3.  Of
+// n3 = m and n3 = -m together, with g = exp(i m z) and the sums and differences
+// U = Re(rho+ + rho-), V = Im(rho+ - rho-), X = Re(rho+ - rho-), Y = Im(rho+ + rho-):
+//   H0 += (U gr + V gi, X gi - Y gr),  H1 += m (X gr + Y gi, U gi - V gr).
+__global__ void __launch_bounds__(FORCE_ATOMS * FORCE_SPLIT) k_ewald_force(EwArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int nm = A.nmax, rows = nm + 1, QS = FORCE_ATOMS;
-  double2* G = (double2*)smem;   // [d][m][a]
-  const int a = threadIdx.x, j = blockIdx.x * FORCE_ATOMS + a;
+  __shared__ double red[3][FORCE_SPLIT][FORCE_ATOMS];
+  const int rows = A.nmax + 1;
+  double2* T = (double2*)smem;   // [d][m][atom], then m times the powers of z
+  double2* Tm = T + 3 * rows * FORCE_ATOMS;
+  const int a = threadIdx.x % FORCE_ATOMS, split = threadIdx.x / FORCE_ATOMS, j = blockIdx.x * FORCE_ATOMS + a;
   const bool active = j < A.nq;
-  int i = 0, t = 0;
-  double q = 0.0;
-  if (active) {
-    i = A.item[j];
-    t = A.qtype[j];
-    q = A.value[j];
-    for (int d = 0; d < 3; d++) power_table(A.R[3 * i + d], A.invL, nm, G + (size_t)d * rows * QS + a, QS);
+  for (int e = split; e < 3 * rows; e += FORCE_SPLIT) {
+    const double2 g = active ? A.table[(size_t)e * A.nq + j] : make_double2(0.0, 0.0);
+    T[e * FORCE_ATOMS + a] = g;
+    if (e >= 2 * rows) {
+      const double m = (double)(e - 2 * rows);
+      Tm[(e - 2 * rows) * FORCE_ATOMS + a] = make_double2(m * g.x, m * g.y);
+    }
   }
-  if (!active) return;
-  const double2* sig = A.sigma + (size_t)t * A.nvecs;
+  __syncthreads();
+  const double2* coef = A.coef + (size_t)(active ? A.qtype[j] : 0) * A.npairs * 2;
   double f0 = 0.0, f1 = 0.0, f2 = 0.0;
-  for (int v = 0; v < A.nvecs; v++) {
-    const int4 nv = __ldg(&A.n[v]);
-    const double2 c = qeikr(q, G[(size_t)nv.x * QS + a], table_get(G + (size_t)rows * QS + a, QS, nv.y),
-                            table_get(G + (size_t)2 * rows * QS + a, QS, nv.z));
-    const double2 s = __ldg(&sig[v]);
-    const double x = s.x * c.y - c.x * s.y;
-    f0 += __ldg(&A.vec[3 * v]) * x;
-    f1 += __ldg(&A.vec[3 * v + 1]) * x;
-    f2 += __ldg(&A.vec[3 * v + 2]) * x;
+  for (int r = split; r < A.nrows; r += FORCE_SPLIT) {
+    const int4 row = __ldg(&A.row[r]);
+    const double2 c = row_phase(T[row.x * FORCE_ATOMS + a], T[(rows + abs(row.y)) * FORCE_ATOMS + a], row.y);
+    const double2* w = coef + 2 * row.w;
+    double h0r = __ldg(&w[0]).x, h0i = -__ldg(&w[1]).y, h1r = 0.0, h1i = 0.0;
+#pragma unroll 2
+    for (int m = 1; m <= row.z; m++) {
+      const double2 g = T[(2 * rows + m) * FORCE_ATOMS + a], gm = Tm[m * FORCE_ATOMS + a];
+      const double2 uv = __ldg(&w[2 * m]), xy = __ldg(&w[2 * m + 1]);
+      h0r = fma(uv.x, g.x, fma(uv.y, g.y, h0r));
+      h0i = fma(xy.x, g.y, fma(-xy.y, g.x, h0i));
+      h1r = fma(xy.x, gm.x, fma(xy.y, gm.y, h1r));
+      h1i = fma(uv.x, gm.y, fma(-uv.y, gm.x, h1i));
+    }
+    const double x = fma(c.x, h0i, c.y * h0r);
+    f0 = fma((double)row.x, x, f0);
+    f1 = fma((double)row.y, x, f1);
+    f2 = fma(c.x, h1i, fma(c.y, h1r, f2));
   }
-  A.F[3 * i] += f0;
-  A.F[3 * i + 1] += f1;
-  A.F[3 * i + 2] += f2;
+  red[0][split][a] = f0;
+  red[1][split][a] = f1;
+  red[2][split][a] = f2;
+  __syncthreads();
+  if (threadIdx.x < 3 * FORCE_ATOMS && active) {   // thread d * FORCE_ATOMS + a: component d of atom a
+    double f = 0.0;
+    for (int k = 0; k < FORCE_SPLIT; k++) f += red[split][k][a];
+    A.F[3 * A.item[j] + split] += f;
+  }
 }
 
 // ---- host -----------------------------------------------------------------------
@@ -215,7 +300,6 @@ static void ewald_update(Ewald& e, double L) {
     }
     e.nvecs = (int)(e.n.size() / 3);
     e.prefac.assign(e.nvecs, 0.0);
-    e.vec.assign((size_t)3 * e.nvecs, 0.0);
     const double B = -0.25 / (e.alpha * e.alpha);
     e.Volume = L * L * L;
     const double fourPiByV = 4.0 * EW_PI / e.Volume;
@@ -223,14 +307,11 @@ static void ewald_update(Ewald& e, double L) {
       const double k[3] = {unit * e.n[3 * v], unit * e.n[3 * v + 1], unit * e.n[3 * v + 2]};
       const double ksq = k[0] * k[0] + k[1] * k[1] + k[2] * k[2];
       e.prefac[v] = fourPiByV * std::exp(ksq * B) / ksq;
-      for (int d = 0; d < 3; d++) e.vec[3 * v + d] = 2.0 * e.prefac[v] * k[d];
     }
+    e.unit = unit;
   } else {
     const double factor = e.Volume / (L * L * L);
-    for (int v = 0; v < e.nvecs; v++) {
-      e.prefac[v] = factor * e.prefac[v];
-      for (int d = 0; d < 3; d++) e.vec[3 * v + d] = factor * e.vec[3 * v + d];
-    }
+    for (int v = 0; v < e.nvecs; v++) e.prefac[v] = factor * e.prefac[v];
     e.Volume = L * L * L;
   }
   e.L = L;
@@ -240,20 +321,23 @@ void ewald_free(System& s) {
   Ewald& e = s.ewald;
   cudaFree(e.dItem);
   cudaFree(e.dQType);
-  cudaFree(e.dFirst);
-  cudaFree(e.dLast);
   cudaFree(e.dValue);
-  cudaFree(e.dN);
+  cudaFree(e.dTask);
+  cudaFree(e.dRow);
+  cudaFree(e.dPair);
+  cudaFree(e.dChunk);
+  cudaFree(e.dTypeChunk);
   cudaFree(e.dPrefac);
-  cudaFree(e.dVec);
   cudaFree(e.dLambda);
+  cudaFree(e.dTable);
   cudaFree(e.dPartial);
-  cudaFree(e.dSigma);
+  cudaFree(e.dCoef);
   cudaFree(e.dEnergyPartial);
-  e.dItem = e.dQType = e.dFirst = e.dLast = nullptr;
-  e.dValue = e.dPrefac = e.dVec = e.dLambda = e.dEnergyPartial = nullptr;
-  e.dN = nullptr;
-  e.dPartial = e.dSigma = nullptr;
+  e.dItem = e.dQType = e.dTypeChunk = nullptr;
+  e.dValue = e.dPrefac = e.dLambda = e.dEnergyPartial = nullptr;
+  e.dTask = e.dRow = e.dChunk = nullptr;
+  e.dPair = nullptr;
+  e.dTable = e.dPartial = e.dCoef = nullptr;
 }
 
 template <typename T>
@@ -264,11 +348,53 @@ static T* upload_vec(const std::vector<T>& h) {
   return d;
 }
 
-static int sf_block_atoms(int nmax) {
-  // shared memory per atom: 3 (nmax + 1) powers of 16 bytes plus the charge
-  const size_t perAtom = (size_t)3 * (nmax + 1) * 16 + 8;
-  int qb = (int)std::min<size_t>(128, (96 * 1024) / perAtom);
-  return std::max(qb, 1);
+// Rows, pairs, tasks and chunks of the k-space sums (see the head of this file).  The
+// k-vectors of a row are consecutive in e.n, n3 ascending.
+static void ewald_plan(Ewald& e) {
+  std::vector<int4> row;
+  std::vector<int2> pair;
+  for (int v = 0; v < e.nvecs;) {
+    int w = v;
+    while (w < e.nvecs && e.n[3 * w] == e.n[3 * v] && e.n[3 * w + 1] == e.n[3 * v + 1]) w++;
+    row.push_back(make_int4(e.n[3 * v], e.n[3 * v + 1], e.n[3 * (w - 1) + 2], v));
+    v = w;
+  }
+  std::stable_sort(row.begin(), row.end(), [](const int4& a, const int4& b) { return a.z > b.z; });
+  int zmax = 0;
+  for (int4& r : row) {
+    const int v0 = r.w, n0 = e.n[3 * v0 + 2];   // first k-vector of the row and its n3 (-z, or 1 in the row 0, 0)
+    r.w = (int)pair.size();
+    for (int m = 0; m <= r.z; m++)
+      pair.push_back(make_int2(m >= n0 ? v0 + m - n0 : -1, m > 0 && -m >= n0 ? v0 - m - n0 : -1));
+    zmax = std::max(zmax, r.z);
+  }
+  std::vector<int4> task;
+  for (int m = 1; m <= std::max(zmax, 1); m += SF_M)
+    for (int r = 0; r < (int)row.size(); r++)
+      if (row[r].z >= m || m == 1) task.push_back(make_int4(row[r].x, row[r].y, m, r));
+  e.nrows = (int)row.size();
+  e.npairs = (int)pair.size();
+  e.ntasks = (int)task.size();
+  // Chunks of atoms of one type: with the task groups about four blocks per SM, at
+  // least 8 atoms in a chunk
+  const int groups = std::max(1, (e.ntasks + SF_THREADS - 1) / SF_THREADS);
+  const int want = std::max(1, std::min(e.nq / 8, 4 * 152 / groups));
+  std::vector<int4> chunk;
+  std::vector<int> typeChunk;
+  for (int t = 0; t < e.ntypes; t++) {
+    typeChunk.push_back((int)chunk.size());
+    const int n = e.last[t] - e.first[t];
+    const int c = std::max(1, std::min(n, (int)((long)want * n / e.nq)));
+    for (int k = 0; k < c; k++)
+      chunk.push_back(make_int4(e.first[t] + (int)((long)n * k / c), e.first[t] + (int)((long)n * (k + 1) / c), t, 0));
+  }
+  typeChunk.push_back((int)chunk.size());
+  e.nchunks = (int)chunk.size();
+  e.dRow = upload_vec(row);
+  e.dPair = upload_vec(pair);
+  e.dTask = upload_vec(task);
+  e.dChunk = upload_vec(chunk);
+  e.dTypeChunk = upload_vec(typeChunk);
 }
 
 // src/modelClass_kspace.f90:111-243 and src/EmDeeData.f90:403-412
@@ -369,18 +495,13 @@ void ewald_initialize(System& s, double kspaceRc) {
   e.dItem = upload_vec(e.item);
   e.dQType = upload_vec(e.qtype);
   e.dValue = upload_vec(e.value);
-  e.dFirst = upload_vec(e.first);
-  e.dLast = upload_vec(e.last);
-  std::vector<int4> n4(e.nvecs);
-  for (int v = 0; v < e.nvecs; v++) n4[v] = make_int4(e.n[3 * v], e.n[3 * v + 1], e.n[3 * v + 2], 0);
-  e.dN = upload_vec(n4);
   e.dPrefac = upload_vec(e.prefac);
-  e.dVec = upload_vec(e.vec);
   e.dLambda = upload_vec(e.lambda);
-  const int qb = sf_block_atoms(e.nmax), blocks = (e.nq + qb - 1) / qb;
-  CK(cudaMalloc(&e.dPartial, sizeof(double2) * std::max<size_t>((size_t)blocks * nt * e.nvecs, 1)));
-  CK(cudaMalloc(&e.dSigma, sizeof(double2) * std::max<size_t>((size_t)nt * e.nvecs, 1)));
-  CK(cudaMalloc(&e.dEnergyPartial, sizeof(double) * std::max(1, (e.nvecs + 255) / 256)));
+  ewald_plan(e);
+  CK(cudaMalloc(&e.dTable, sizeof(double2) * (size_t)3 * (e.nmax + 1) * e.nq));
+  CK(cudaMalloc(&e.dPartial, sizeof(double2) * std::max<size_t>((size_t)e.nchunks * e.nvecs, 1)));
+  CK(cudaMalloc(&e.dCoef, sizeof(double2) * std::max<size_t>((size_t)2 * nt * e.npairs, 1)));
+  CK(cudaMalloc(&e.dEnergyPartial, sizeof(double) * (e.npairs / SIGMA_PAIRS + 1)));
   // coul_long and other models that need the k-space alpha (src/coul_long.f90:55-64,
   // src/modelClass_coul.f90:101-106)
   for (int l = 0; l < nl; l++) {
@@ -400,50 +521,52 @@ double ewald_compute(System& s) {
   EwArgs A;
   A.R = s.dR;
   A.invL = 1.0 / *s.Lbox;
+  A.unit2 = 2.0 * e.unit;
   A.nq = e.nq;
   A.nvecs = e.nvecs;
   A.nmax = e.nmax;
   A.ntypes = e.ntypes;
+  A.ntasks = e.ntasks;
+  A.nrows = e.nrows;
+  A.npairs = e.npairs;
+  A.nchunks = e.nchunks;
   A.item = e.dItem;
   A.qtype = e.dQType;
   A.value = e.dValue;
-  A.first = e.dFirst;
-  A.last = e.dLast;
-  A.n = e.dN;
+  A.task = e.dTask;
+  A.row = e.dRow;
+  A.pair = e.dPair;
+  A.chunk = e.dChunk;
+  A.typeChunk = e.dTypeChunk;
   A.prefac = e.dPrefac;
-  A.vec = e.dVec;
   A.lambda = e.dLambda + (size_t)l * e.ntypes * e.ntypes;
+  A.table = e.dTable;
   A.partial = e.dPartial;
-  A.sigma = e.dSigma;
-  A.qb = sf_block_atoms(e.nmax);
-  A.sfBlocks = (e.nq + A.qb - 1) / A.qb;
+  A.coef = e.dCoef;
   A.F = s.F();
   A.epart = e.dEnergyPartial;
   A.ticket = s.dTicket + 4;
   A.result = s.dResult + 22;
+  A.hostResult = s.hResult + 22;   // pinned: read after the synchronisation
   const int rows = e.nmax + 1;
-  const size_t smemSF = (size_t)3 * rows * (A.qb + 1) * sizeof(double2) + (size_t)A.qb * sizeof(double);
-  const size_t smemF = (size_t)3 * rows * FORCE_ATOMS * sizeof(double2);
-  static size_t setSF = 0, setF = 0;
-  if (smemSF > setSF) {
-    CK(cudaFuncSetAttribute(k_ewald_sf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemSF));
-    setSF = smemSF;
-  }
-  if (smemF > setF) {
-    CK(cudaFuncSetAttribute(k_ewald_force, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemF));
-    setF = smemF;
-  }
-  if (smemSF > 227 * 1024 || smemF > 227 * 1024) fatal("kspace computation", "too many k-vectors per dimension");
-  k_ewald_sf<<<A.sfBlocks, SF_THREADS, smemSF, s.stream>>>(A);
+  if ((size_t)3 * rows * TABLE_LIMIT_ATOMS * sizeof(double2) > 227 * 1024)
+    fatal("kspace computation", "too many k-vectors per dimension");
+  const size_t smemSF = (size_t)((3 * rows) | 1) * SF_ATOMS * sizeof(double2);
+  const size_t smemF = (size_t)4 * rows * FORCE_ATOMS * sizeof(double2);
+  CK(cudaFuncSetAttribute(k_ewald_sf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemSF));
+  CK(cudaFuncSetAttribute(k_ewald_force, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemF));
+  k_ewald_tables<<<(3 * e.nq + 127) / 128, 128, 0, s.stream>>>(A);
   CK(cudaGetLastError());
-  k_ewald_sigma<<<(e.nvecs + 255) / 256, 256, 0, s.stream>>>(A);
+  const dim3 grid((e.ntasks + SF_THREADS - 1) / SF_THREADS, e.nchunks);
+  k_ewald_sf<<<grid, SF_THREADS, smemSF, s.stream>>>(A);
   CK(cudaGetLastError());
-  k_ewald_force<<<(e.nq + FORCE_ATOMS - 1) / FORCE_ATOMS, FORCE_ATOMS, smemF, s.stream>>>(A);
+  k_ewald_sigma<<<(e.npairs + SIGMA_PAIRS - 1) / SIGMA_PAIRS, SIGMA_PAIRS * SIGMA_SLICES, 0, s.stream>>>(A);
   CK(cudaGetLastError());
-  s.prof.total += 3;
-  double Ek = 0.0;
-  CK(cudaMemcpyAsync(&Ek, s.dResult + 22, sizeof(double), cudaMemcpyDeviceToHost, s.stream));
+  k_ewald_force<<<(e.nq + FORCE_ATOMS - 1) / FORCE_ATOMS, FORCE_ATOMS * FORCE_SPLIT, smemF, s.stream>>>(A);
+  CK(cudaGetLastError());
+  s.prof.total += 4;
   CK(cudaStreamSynchronize(s.stream));
+  const double Ek = s.hResult[22];
   // src/modelClass_kspace.f90:247-314, energy part
   double disc = 0.0;
   for (int k = 0; k < e.nTypePairs; k++) disc += e.lambda1D[(size_t)l * e.nTypePairs + k] * e.Erigid[k];

@@ -88,15 +88,17 @@ struct Ewald {
   std::vector<double> Erigid;              // per type pair (symm1D order): rigid-pair and self discounts
   std::vector<double> lambda, lambda1D;    // [layer][t][u] = kCoul(u, t); [layer][k]
   std::vector<int> n;                      // k-vectors (nvecs x 3 integers)
-  std::vector<double> prefac, vec;         // nvecs; 3 x nvecs
+  std::vector<double> prefac;              // nvecs
+  double unit = 0;                         // 2 pi / L of the set-up
+  int nrows = 0, npairs = 0, ntasks = 0, nchunks = 0;   // plan of the sums (ewald.cu)
   // device
-  int *dItem = nullptr, *dQType = nullptr, *dFirst = nullptr, *dLast = nullptr;
+  int *dItem = nullptr, *dQType = nullptr, *dTypeChunk = nullptr;
   double* dValue = nullptr;
-  int4* dN = nullptr;
-  double *dPrefac = nullptr, *dVec = nullptr, *dLambda = nullptr;
-  double2 *dPartial = nullptr, *dSigma = nullptr;
+  int4 *dTask = nullptr, *dRow = nullptr, *dChunk = nullptr;
+  int2* dPair = nullptr;
+  double *dPrefac = nullptr, *dLambda = nullptr;
+  double2 *dTable = nullptr, *dPartial = nullptr, *dCoef = nullptr;
   double* dEnergyPartial = nullptr;
-  size_t partialCap = 0;
 };
 
 // scratch of EmDee_verlet_step (verlet.cu): shadow start values and reduction partials
