@@ -38,6 +38,7 @@ struct BondedArgs {
   int natoms;
   double* partials;
   unsigned int* ticket;
+  double* hostResult;   // pinned
   double* result;       // [0] Ebond, [1] Wbond, [2] Eangle, [3] Wangle, [4] Ecoul discount
 };
 
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(BONDED_THREADS) k_bonded(BondedArgs A) {
       }
     }
   }
-  grid_reduce<5, BONDED_THREADS>(v, A.partials, A.ticket, A.result);
+  grid_reduce<5, BONDED_THREADS>(v, A.partials, A.ticket, A.result, A.hostResult);
 }
 
 // F(a) += the atom's contributions, in list order
@@ -238,12 +239,12 @@ bool device_bonded(System& s, double out[5]) {
   A.partials = B.dPartials;
   A.ticket = s.dTicket + 7;
   A.result = s.dResult + 40;
+  A.hostResult = s.hResult + 40;
   k_bonded<<<(n + BONDED_THREADS - 1) / BONDED_THREADS, BONDED_THREADS, 0, s.stream>>>(A);
   CK(cudaGetLastError());
   k_bonded_gather<<<(s.natoms + BONDED_THREADS - 1) / BONDED_THREADS, BONDED_THREADS, 0, s.stream>>>(A);
   CK(cudaGetLastError());
   s.prof.total += 2;
-  CK(cudaMemcpyAsync(s.hResult + 40, s.dResult + 40, 5 * sizeof(double), cudaMemcpyDeviceToHost, s.stream));
   CK(cudaStreamSynchronize(s.stream));
   for (int q = 0; q < 5; q++) out[q] = s.hResult[40 + q];
   return true;

@@ -29,7 +29,7 @@ template <bool KIN, bool UNITCP, bool UNITM, bool FMA>
 __global__ void __launch_bounds__(MOTION_THREADS) k_boost(double* __restrict__ P, const double* __restrict__ F,
                                                           const double* __restrict__ invMass, int N, double CP,
                                                           double CF, double* partials, unsigned int* ticket,
-                                                          double* twoKE) {
+                                                          double* twoKE, double* hostKE) {
   double k2[3] = {0.0, 0.0, 0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
     double im = (KIN && !UNITM) ? invMass[i] : 1.0;
@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(MOTION_THREADS) k_boost(double* __restrict__ P
       if (KIN) k2[d] += UNITM ? p * p : im * (p * p);
     }
   }
-  if (KIN) grid_reduce<3, MOTION_THREADS>(k2, partials, ticket, twoKE);
+  if (KIN) grid_reduce<3, MOTION_THREADS>(k2, partials, ticket, twoKE, hostKE);
 }
 
 template <bool UNITCR, bool UNITM, bool FMA>
@@ -123,15 +123,14 @@ static void boost_launch(System& s, double CP, double CF, bool kinetic) {
     auto kern = CP == 1.0 ? (s.unitMass ? k_boost<true, true, true, FMA> : k_boost<true, true, false, FMA>)
                           : (s.unitMass ? k_boost<true, false, true, FMA> : k_boost<true, false, false, FMA>);
     kern<<<blocks, MOTION_THREADS, 0, s.stream>>>(s.dP, s.F(), s.dInvMass, N, CP, CF, s.dKE, s.dTicket + 1,
-                                                  s.dResult + 10);
+                                                  s.dResult + 10, s.hResult + 10);
     CK(cudaGetLastError());
     prof_end(s, PK_BOOST);
-    CK(cudaMemcpyAsync(s.hResult + 10, s.dResult + 10, 3 * sizeof(double), cudaMemcpyDeviceToHost, s.stream));
     CK(cudaStreamSynchronize(s.stream));
   } else {
     prof_begin(s, PK_BOOST);
     auto kern = CP == 1.0 ? k_boost<false, true, true, FMA> : k_boost<false, false, true, FMA>;
-    kern<<<blocks, MOTION_THREADS, 0, s.stream>>>(s.dP, s.F(), s.dInvMass, N, CP, CF, nullptr, nullptr, nullptr);
+    kern<<<blocks, MOTION_THREADS, 0, s.stream>>>(s.dP, s.F(), s.dInvMass, N, CP, CF, nullptr, nullptr, nullptr, nullptr);
     CK(cudaGetLastError());
     prof_end(s, PK_BOOST);
   }
@@ -532,7 +531,7 @@ extern "C" int EmDee_boost_noalloc(double* P, const double* F, const double* inv
   auto kern = unitCP ? (unitM ? k_boost<true, true, true, false> : k_boost<true, true, false, false>)
                      : (unitM ? k_boost<true, false, true, false> : k_boost<true, false, false, false>);
   if (e == cudaSuccess) {
-    kern<<<blocks, MOTION_THREADS, 0, st>>>(P, F, invMass, N, CP, CF, scratch, ticket, twoKE);
+    kern<<<blocks, MOTION_THREADS, 0, st>>>(P, F, invMass, N, CP, CF, scratch, ticket, twoKE, nullptr);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {

@@ -49,7 +49,16 @@ __device__ __forceinline__ MaxPrev mp_combine(MaxPrev a, MaxPrev b) {
   return a;
 }
 
-static const int SKIN_THREADS = 256, SKIN_CHUNKS = 8;   // each warp: 8 x 32 consecutive atoms
+// Each warp takes `chunks` x 32 consecutive atoms: SKIN_CHUNKS where the grid fills the
+// SMs, fewer below (the ordered combine of a chunk waits for its loads, so a small
+// system in chunks of 8 pays eight memory latencies in a row; 16,001 atoms: 11.5 -> 6 us
+// with the sums written straight to pinned memory).
+// The value does not depend on it.
+static const int SKIN_THREADS = 256, SKIN_CHUNKS = 8;
+static int skin_chunks(int N, int most) {
+  const int c = N / (152 * 4 * SKIN_THREADS);
+  return c < 1 ? 1 : c < most ? c : most;
+}
 
 __device__ __forceinline__ MaxPrev warp_ordered_combine(MaxPrev acc) {
   // after the loop lane 0 holds the combination of lanes 0..31 in lane order
@@ -63,14 +72,14 @@ __device__ __forceinline__ MaxPrev warp_ordered_combine(MaxPrev acc) {
 }
 
 __global__ void __launch_bounds__(SKIN_THREADS) k_skin(const double* __restrict__ R, const double* __restrict__ R0,
-                                                       int N, double skinSq, longlong2* partial, unsigned int* ticket,
-                                                       double* result) {
+                                                       int N, int chunks, double skinSq, longlong2* partial,
+                                                       unsigned int* ticket, double* result, double* hostResult) {
   __shared__ MaxPrev wsum[SKIN_THREADS / 32];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int base = (blockIdx.x * (SKIN_THREADS / 32) + warp) * 32 * SKIN_CHUNKS;
+  const int base = (blockIdx.x * (SKIN_THREADS / 32) + warp) * 32 * chunks;
   MaxPrev run{-1, -1};
-  for (int c = 0; c < SKIN_CHUNKS; c++) {
+  for (int c = 0; c < chunks; c++) {
     const int i = base + c * 32 + lane;
     MaxPrev v{-1, -1};
     if (i < N) {
@@ -111,8 +120,8 @@ __global__ void __launch_bounds__(SKIN_THREADS) k_skin(const double* __restrict_
     for (int w = 1; w < SKIN_THREADS / 32; w++) b = mp_combine(b, wsum[w]);
     double maximum = __longlong_as_double(b.m), next = __longlong_as_double(b.p < 0 ? b.m : b.p);
     double value = maximum + 2 * sqrt(maximum * next) + next;
-    result[8] = value;
-    result[9] = value > skinSq ? 1.0 : 0.0;
+    result[8] = hostResult[8] = value;   // pinned host memory: read after the synchronisation
+    result[9] = hostResult[9] = value > skinSq ? 1.0 : 0.0;
     *ticket = 0;
   }
 }
@@ -126,15 +135,14 @@ static void ensure_partials(System& s, int n) {
 }
 
 bool device_skin_check(System& s) {
-  int N = s.natoms;
-  int blocks = (N + SKIN_THREADS * SKIN_CHUNKS - 1) / (SKIN_THREADS * SKIN_CHUNKS);
+  const int N = s.natoms, chunks = skin_chunks(N, SKIN_CHUNKS), per = SKIN_THREADS * chunks;
+  const int blocks = (N + per - 1) / per;
   ensure_partials(s, blocks);
   prof_begin(s, PK_SKIN);
-  k_skin<<<blocks, SKIN_THREADS, 0, s.stream>>>(s.dR, s.dR0, N, s.skinSq, (longlong2*)s.dPartials, s.dTicket,
-                                                 s.dResult);
+  k_skin<<<blocks, SKIN_THREADS, 0, s.stream>>>(s.dR, s.dR0, N, chunks, s.skinSq, (longlong2*)s.dPartials,
+                                                 s.dTicket, s.dResult, s.hResult);
   CK(cudaGetLastError());
   prof_end(s, PK_SKIN);
-  CK(cudaMemcpyAsync(s.hResult + 8, s.dResult + 8, 2 * sizeof(double), cudaMemcpyDeviceToHost, s.stream));
   CK(cudaStreamSynchronize(s.stream));
   return s.hResult[9] != 0.0;
 }
@@ -1426,7 +1434,7 @@ void device_rdf_counts(System& s, int bins, double Rc, const std::vector<uint8_t
 // Contiguous atom ranges combined in index order, as in k_skin, so the skin value
 // is the same for any range size.  Each
 // statement rounds as the separate kernels do (this file uses -fmad=false).
-static const int STEP_CHUNKS = 2;   // 64 consecutive atoms per warp: many warps in flight
+static const int STEP_CHUNKS = 2;   // at most 64 consecutive atoms per warp (skin_chunks): many warps in flight
 
 // FMA (mixed precision only): the updates use fused multiply-adds, which halves the
 // work on the FP64 pipe (the limit of this kernel on GB300); FP64 mode keeps the
@@ -1435,7 +1443,7 @@ template <int NK, bool UNITM, bool PACK, bool FMA>
 __global__ void __launch_bounds__(SKIN_THREADS) k_step_fused(double* __restrict__ R, double* __restrict__ P,
                                                              const double* __restrict__ F,
                                                              const double* __restrict__ invMass,
-                                                             const double* __restrict__ R0, int N, double cf0,
+                                                             const double* __restrict__ R0, int N, int chunks, double cf0,
                                                              double cf1, double CP, double skinSq,
                                                              const int* __restrict__ slotOf,
                                                              const float4* __restrict__ pos0, float scale,
@@ -1445,9 +1453,9 @@ __global__ void __launch_bounds__(SKIN_THREADS) k_step_fused(double* __restrict_
   __shared__ MaxPrev wsum[SKIN_THREADS / 32];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int base = (blockIdx.x * (SKIN_THREADS / 32) + warp) * 32 * STEP_CHUNKS;
+  const int base = (blockIdx.x * (SKIN_THREADS / 32) + warp) * 32 * chunks;
   MaxPrev run{-1, -1};
-  for (int c = 0; c < STEP_CHUNKS; c++) {
+  for (int c = 0; c < chunks; c++) {
     const int i = base + c * 32 + lane;
     MaxPrev v{-1, -1};
     if (i < N) {
@@ -1512,14 +1520,14 @@ __global__ void __launch_bounds__(SKIN_THREADS) k_step_fused(double* __restrict_
 }
 
 void device_step_fused(System& s, double CP) {
-  const int N = s.natoms;
-  const int blocks = (N + SKIN_THREADS * STEP_CHUNKS - 1) / (SKIN_THREADS * STEP_CHUNKS);
+  const int N = s.natoms, chunks = skin_chunks(N, STEP_CHUNKS), per = SKIN_THREADS * chunks;
+  const int blocks = (N + per - 1) / per;
   ensure_partials(s, blocks);
   const bool pack = s.precision == 0 && s.r0Valid && *s.Lbox == s.builtL;
   const Grid& g = s.grid;
   const float scale = g.M > 0 ? (float)((double)g.M / *s.Lbox) : 0.0f;
   prof_begin(s, PK_MOVE);
-#define STEP_ARGS s.dR, s.dP, s.F(), s.dInvMass, s.dR0, N, s.pendCF[0], s.pendCF[1], CP, s.skinSq, g.dSlotOf, \
+#define STEP_ARGS s.dR, s.dP, s.F(), s.dInvMass, s.dR0, N, chunks, s.pendCF[0], s.pendCF[1], CP, s.skinSq, g.dSlotOf, \
                   g.dPos0, scale, g.dPos4, (longlong2*)s.dPartials, s.dTicket, s.dResult, s.hResult
 #define STEP_LAUNCH(NK, UM, PK, FM) k_step_fused<NK, UM, PK, FM><<<blocks, SKIN_THREADS, 0, s.stream>>>(STEP_ARGS)
 #define STEP_NK(UM, PK, FM)                 \

@@ -1,120 +1,100 @@
 // reduce.cuh -- deterministic block and grid reductions of FP64 partial sums.
 //
-// THREADS is the largest block size the kernel is launched with.  Each block reduces its per-thread values (warp shuffles, then warps in
-// order) and writes one partial per quantity; the last block to finish (ticket
-// counter) sums the partials in block order with Neumaier compensation.  The
-// result does not depend on block scheduling.
+// THREADS is the largest block size the kernel is launched with.  Each block reduces
+// its per-thread values (warp shuffles, then warps in order) and writes one partial
+// per quantity; the last block to finish (ticket counter) sums the partials in a fixed
+// order with Neumaier compensation.  The result does not depend on block scheduling.
 #pragma once
 
 namespace emdee {
 
-// Variant whose inputs are already warp sums held by lane 0 of each warp.
+// Per-thread FP64 values -> result[q], also into result2 if set (e.g. pinned host
+// memory: no copy back).  partials holds NQ doubles per block.
+//
+// A small system waits for this reduction's latency, a chain of FP64 additions on a
+// pipe that takes 16 clocks per warp instruction, so the chain is kept short: the
+// values of a warp are summed and distributed over the lanes together (NQ/2 + NQ/4 +
+// ... additions, not 5 NQ), the warps' sums are added by one thread per quantity, and
+// the last block's warps take the quantities side by side (5 sums: k_bonded 34 -> 25 us
+// at 512 molecules, k_vv_post_free 13 -> 11 us at 16,001 atoms).
 template <int NQ, int THREADS>
-__device__ __forceinline__ void grid_reduce_lane0(const double (&v)[NQ], double* partials, unsigned int* ticket,
-                                                  double* result, double* result2 = nullptr) {
-  __shared__ double red[NQ][THREADS / 32];
+__device__ __forceinline__ void grid_reduce(const double (&v)[NQ], double* partials, unsigned int* ticket,
+                                            double* result, double* result2 = nullptr) {
+  static_assert(NQ <= 16, "at most 16 quantities");
+  constexpr int P = NQ <= 1 ? 1 : NQ <= 2 ? 2 : NQ <= 4 ? 4 : NQ <= 8 ? 8 : 16;
+  __shared__ double red[P][THREADS / 32];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  if (lane == 0)
+  double w[P];
 #pragma unroll
-    for (int q = 0; q < NQ; q++) red[q][warp] = v[q];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int q = 0; q < NQ; q++) {
-      double x = 0.0;
-      for (int w = 0; w < nw; w++) x += red[q][w];
-      partials[(size_t)blockIdx.x * NQ + q] = x;
+  for (int q = 0; q < P; q++) w[q] = q < NQ ? v[q] : 0.0;
+#pragma unroll
+  for (int l = 0; l < 5; l++) {
+    const int o = 16 >> l, h = P >> (l + 1);   // quantities a lane keeps after this level
+    if (h >= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int k = 0; k < h; k++) {
+        const double keep = up ? w[k + h] : w[k];
+        w[k] = keep + __shfl_xor_sync(0xffffffffu, up ? w[k] : w[k + h], o);
+      }
+    } else {
+      w[0] += __shfl_xor_sync(0xffffffffu, w[0], o);
     }
-    __threadfence();
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  // lane q * (32 / P) holds the warp's sum of quantity q
+  if (lane % (32 / P) == 0) red[lane / (32 / P)][warp] = w[0];
+  __syncthreads();
+  if (warp == 0) {
+    if (lane < NQ) {
+      double x = 0.0;
+      for (int k = 0; k < nw; k++) x += red[lane][k];
+      partials[(size_t)blockIdx.x * NQ + lane] = x;
+      __threadfence();   // the partial is visible before the ticket counts this block
+    }
+    __syncwarp();
+    if (lane == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  // last block: thread t sums partials t, t + blockDim, ... (Neumaier), then the
-  // per-thread sums are combined by a fixed tree; the order never depends on
-  // which block finished last.
+  // last block: a group of warps per quantity sums the partials in a fixed order
+  // (Neumaier), which never depends on which block finished last
+  const int per = nw / NQ > 0 ? nw / NQ : 1, groups = nw / per;
+  for (int q0 = 0; q0 < NQ; q0 += groups) {
+    const int q = q0 + warp / per, part = warp % per;
+    if (q < NQ && warp / per < groups) {
+      double s = 0.0, c = 0.0;
+      constexpr int U = 8;   // partials in flight per thread, added in increasing block order
+      for (unsigned int b0 = part * 32 + lane; b0 < gridDim.x; b0 += U * per * 32) {
+        double xs[U];
 #pragma unroll
-  for (int q = 0; q < NQ; q++) {
-    double s = 0.0, c = 0.0;
-    constexpr int U = 8;   // partials in flight per thread, added in increasing block order
-    for (unsigned int b0 = threadIdx.x; b0 < gridDim.x; b0 += U * blockDim.x) {
-      double xs[U];
+        for (int u = 0; u < U; u++) {
+          const unsigned int b = b0 + u * per * 32;
+          xs[u] = b < gridDim.x ? __ldcg(&partials[(size_t)b * NQ + q]) : 0.0;
+        }
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        const unsigned int b = b0 + u * blockDim.x;
-        xs[u] = b < gridDim.x ? __ldcg(&partials[(size_t)b * NQ + q]) : 0.0;
+        for (int u = 0; u < U; u++) {
+          if (b0 + u * per * 32 >= gridDim.x) break;
+          const double x = xs[u], t = s + x;
+          c += fabs(s) >= fabs(x) ? (s - t) + x : (x - t) + s;
+          s = t;
+        }
       }
+      double x = s + c;
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        if (b0 + u * blockDim.x >= gridDim.x) break;
-        const double x = xs[u], t = s + x;
-        c += fabs(s) >= fabs(x) ? (s - t) + x : (x - t) + s;
-        s = t;
-      }
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+      if (lane == 0) red[q][part] = x;
     }
-    double x = s + c;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) red[q][warp] = x;
   }
   __syncthreads();
   if (threadIdx.x < NQ) {
     double x = 0.0;
-    for (int w = 0; w < nw; w++) x += red[threadIdx.x][w];
+    for (int k = 0; k < per; k++) x += red[threadIdx.x][k];
     result[threadIdx.x] = x;
-    if (result2) result2[threadIdx.x] = x;   // e.g. pinned host memory: no copy back
+    if (result2) result2[threadIdx.x] = x;
   }
   if (threadIdx.x == 0) *ticket = 0;
-}
-
-// FP64 per-thread values: warp shuffle sums, then as above.
-template <int NQ, int THREADS>
-__device__ __forceinline__ void grid_reduce(double (&v)[NQ], double* partials, unsigned int* ticket, double* result,
-                                            double* result2 = nullptr) {
-#pragma unroll
-  for (int q = 0; q < NQ; q++)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
-  grid_reduce_lane0<NQ, THREADS>(v, partials, ticket, result, result2);
-}
-
-// Warp sums of FP32 values with an error-free two-sum at every level; lane 0
-// converts hi + lo to FP64 (other lanes return 0 and touch no FP64 unit).
-template <int NQ>
-__device__ __forceinline__ void warp_sum_f32(const float (&x)[NQ], double (&out)[NQ]) {
-  float hi[NQ], lo[NQ];
-#pragma unroll
-  for (int q = 0; q < NQ; q++) {
-    hi[q] = x[q];
-    lo[q] = 0.f;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      float h2 = __shfl_down_sync(0xffffffffu, hi[q], o), l2 = __shfl_down_sync(0xffffffffu, lo[q], o);
-      float s = hi[q] + h2, bp = s - hi[q], err = (hi[q] - (s - bp)) + (h2 - bp);
-      hi[q] = s;
-      lo[q] = lo[q] + l2 + err;
-    }
-  if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-    for (int q = 0; q < NQ; q++) out[q] = (double)hi[q] + (double)lo[q];
-  } else {
-#pragma unroll
-    for (int q = 0; q < NQ; q++) out[q] = 0.0;
-  }
-}
-
-// grid_reduce for per-thread FP32 partial sums: compensated warp sums in FP32,
-// FP64 from there on.
-template <int NQ, int THREADS>
-__device__ __forceinline__ void grid_reduce_f32(const float (&v)[NQ], double* partials, unsigned int* ticket,
-                                                double* result) {
-  double w[NQ];
-  warp_sum_f32<NQ>(v, w);
-  grid_reduce_lane0<NQ, THREADS>(w, partials, ticket, result);
 }
 
 // ---- float-float (FP32 pair) reductions: every level on the FP32 pipe ----------

@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(VV_THREADS) k_vv_post_free(const double* __res
                                                              const double* __restrict__ invMass, const int* list,
                                                              int n, double dt, double dt_2,
                                                              const double* __restrict__ s0, double* partials,
-                                                             unsigned int* ticket, double* result) {
+                                                             unsigned int* ticket, double* result, double* hostResult) {
   double v[5] = {0, 0, 0, 0, 0};
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     const int j = list ? list[q] : q;
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(VV_THREADS) k_vv_post_free(const double* __res
       v[4] += im * (f[0] * f[0] + f[1] * f[1] + f[2] * f[2]);
     }
   }
-  if (COMPUTE) grid_reduce<5, VV_THREADS>(v, partials, ticket, result);
+  if (COMPUTE) grid_reduce<5, VV_THREADS>(v, partials, ticket, result, hostResult);
 }
 
 // force and torque, then pcm += CF F, pi += C(q) 2 CF tau (boost with both flags on)
@@ -132,7 +132,7 @@ template <bool COMPUTE>
 __global__ void __launch_bounds__(VV_THREADS) k_vv_post_body(BodyArgs A, const double* __restrict__ F, double dt,
                                                              double dt_2, int mode, const double* __restrict__ r0,
                                                              const double* __restrict__ q0, double* partials,
-                                                             unsigned int* ticket, double* result) {
+                                                             unsigned int* ticket, double* result, double* hostResult) {
   double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < A.nb) {
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(VV_THREADS) k_vv_post_body(BodyArgs A, const d
     }
     A.b[i] = b;
   }
-  if (COMPUTE) grid_reduce<9, VV_THREADS>(v, partials, ticket, result);
+  if (COMPUTE) grid_reduce<9, VV_THREADS>(v, partials, ticket, result, hostResult);
 }
 
 // ---- host -----------------------------------------------------------------------
@@ -224,10 +224,11 @@ static void verlet_post(System& s, double dt, bool compute, int mode, double* ou
     ensure(w.partB, w.partBCap, (size_t)9 * blocks);
     if (compute)
       k_vv_post_body<true><<<blocks, VV_BODY_THREADS, 0, s.stream>>>(body_args(s), s.F(), dt, dt_2, mode, w.r0, w.q0,
-                                                                     w.partB, s.dTicket + 5, s.dResult + 24);
+                                                                     w.partB, s.dTicket + 5, s.dResult + 24,
+                                                                     s.hResult + 24);
     else
       k_vv_post_body<false><<<blocks, VV_BODY_THREADS, 0, s.stream>>>(body_args(s), s.F(), dt, dt_2, mode, w.r0,
-                                                                      w.q0, nullptr, nullptr, nullptr);
+                                                                      w.q0, nullptr, nullptr, nullptr, nullptr);
     CK(cudaGetLastError());
     s.prof.total++;
   }
@@ -237,17 +238,18 @@ static void verlet_post(System& s, double dt, bool compute, int mode, double* ou
     const int* list = all ? nullptr : s.dFree;
     if (compute)
       k_vv_post_free<true, FMA><<<blocks, VV_THREADS, 0, s.stream>>>(s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt, dt_2,
-                                                                w.s0, w.partF, s.dTicket + 6, s.dResult + 34);
+                                                                w.s0, w.partF, s.dTicket + 6, s.dResult + 34,
+                                                                s.hResult + 34);
     else
       k_vv_post_free<false, FMA><<<blocks, VV_THREADS, 0, s.stream>>>(s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt, dt_2,
-                                                                 w.s0, nullptr, nullptr, nullptr);
+                                                                 w.s0, nullptr, nullptr, nullptr, nullptr);
     CK(cudaGetLastError());
     s.prof.total++;
   }
   if (compute) {
-    if (s.nbodies > 0) CK(cudaMemcpyAsync(vb, s.dResult + 24, sizeof(vb), cudaMemcpyDeviceToHost, s.stream));
-    if (nf > 0) CK(cudaMemcpyAsync(vf, s.dResult + 34, sizeof(vf), cudaMemcpyDeviceToHost, s.stream));
     CK(cudaStreamSynchronize(s.stream));
+    for (int k = 0; k < 9 && s.nbodies > 0; k++) vb[k] = s.hResult[24 + k];
+    for (int k = 0; k < 5 && nf > 0; k++) vf[k] = s.hResult[34 + k];
   }
   for (int d = 0; d < 3; d++) {
     out[d] = vb[d] + vf[d];
