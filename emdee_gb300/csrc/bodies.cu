@@ -14,66 +14,231 @@
 namespace emdee {
 
 // One warp per block: the per-body work is a long chain of FP64 operations, so bodies
-// are spread over as many SMs as possible (4096 bodies, boost: 12.6 us in blocks of 128
-// threads, which use 32 of the SMs; 11 us so).  The grid reductions write their sums
+// are spread over as many SMs as possible.  The grid reductions write their sums
 // straight into pinned host memory.
 static const int BODY_THREADS = 32;
+// The boost and the exact rotation run on BODY_LANES lanes per body, one per quaternion
+// component: the FP64 unit of an SM quarter takes 64 clocks per warp instruction however
+// many of its lanes are active, so four times the warps with a quarter of the
+// instructions each use all the units (4096 bodies on one lane each are 128 warps on
+// 608 quarters).  4096 molecules: move 75 -> 31 us,
+// boost 11 -> 8.2 us.
+static const int BODY_LANES = 4, BODY_GROUP_THREADS = 128;
 
-// force_and_torque, then pcm and pi updates; 2KE translational (bodies) and
-// rotational partial sums
-__global__ void __launch_bounds__(BODY_THREADS) k_body_boost(BodyArgs A, const double* __restrict__ F, double CP,
-                                                             double CF, int translate, int rotate, int kinetic,
-                                                             double* partials, unsigned int* ticket, double* result,
-                                                             double* hostResult) {
-  double k6[6] = {0, 0, 0, 0, 0, 0};
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < A.nb) {
-    BodyState b = A.b[i];
-    for (int k = 0; k < 3; k++) b.F[k] = b.tau[k] = 0.0;
-    for (int j = 0; j < b.NP; j++) {
-      const double* Fj = &F[3 * A.atom[b.first + j]];
-      double c[3];
-      rb_cross(&A.delta[3 * (b.first + j)], Fj, c);
-      for (int k = 0; k < 3; k++) {
-        b.F[k] += Fj[k];
-        b.tau[k] += c[k];
-      }
-    }
-    if (translate)
-      for (int k = 0; k < 3; k++) b.pcm[k] = CP * b.pcm[k] + CF * b.F[k];
-    if (rotate) {
-      double Ctau = 2.0 * CF, v[3] = {Ctau * b.tau[0], Ctau * b.tau[1], Ctau * b.tau[2]}, c[4], pi[4];
-      rb_C(b.q, v, c);
-      for (int k = 0; k < 4; k++) pi[k] = CP * b.pi[k] + c[k];
-      rb_assign_pi(b, pi);
-    }
-    if (kinetic)
-      for (int k = 0; k < 3; k++) {
-        k6[k] = b.invMass * (b.pcm[k] * b.pcm[k]);
-        k6[3 + k] = b.MoI[k] * (b.omega[k] * b.omega[k]);
-      }
-    A.b[i] = b;
-  }
-  if (kinetic) grid_reduce<6, BODY_THREADS>(k6, partials, ticket, result, hostResult);
+struct BodyLane {
+  int i, c;        // body and lane (quaternion component)
+  unsigned mask;   // the body's lanes
+};
+__device__ __forceinline__ BodyLane body_lane() {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, c = t % BODY_LANES;
+  return BodyLane{t / BODY_LANES, c, 0xFu << ((threadIdx.x & 31) & ~(BODY_LANES - 1))};
+}
+// value x of lane k of the body
+__device__ __forceinline__ double body_get(const BodyLane& g, double x, int k) {
+  return __shfl_sync(g.mask, x, k, BODY_LANES);
+}
+// component c of B(q) v and of C(q) v (rb_B, rb_C): -q_k v in component 0, else q_0 v_c
+// and the cross product with the sign that tells the two apart
+__device__ __forceinline__ double body_BC(const double* q, const double* v, int c, bool isC) {
+  if (c == 0) return -q[1] * v[0] - q[2] * v[1] - q[3] * v[2];
+  const int a = c % 3, b = (c + 1) % 3;   // 0-based indices after c - 1, cyclic
+  const double vc = c == 1 ? v[0] : c == 2 ? v[1] : v[2];
+  const double qa = a == 0 ? q[1] : a == 1 ? q[2] : q[3], qb = b == 0 ? q[1] : b == 1 ? q[2] : q[3];
+  const double va = a == 0 ? v[0] : a == 1 ? v[1] : v[2], vb = b == 0 ? v[0] : b == 1 ? v[1] : v[2];
+  const double s = isC ? -1.0 : 1.0;
+  return q[0] * vc + s * (qa * vb - qb * va);
+}
+// component k (0..2) of B(q)^T p (rb_Bt)
+__device__ __forceinline__ double body_Bt(const double* q, const double* p, int k) {
+  const int a = (k + 1) % 3, b = (k + 2) % 3;
+  const double qk = k == 0 ? q[1] : k == 1 ? q[2] : q[3], pk = k == 0 ? p[1] : k == 1 ? p[2] : p[3];
+  const double qa = a == 0 ? q[1] : a == 1 ? q[2] : q[3], pa = a == 0 ? p[1] : a == 1 ? p[2] : p[3];
+  const double qb = b == 0 ? q[1] : b == 1 ? q[2] : q[3], pb = b == 0 ? p[1] : b == 1 ? p[2] : p[3];
+  return -qk * p[0] + q[0] * pk + qb * pa - qa * pb;
 }
 
-// rcm update, rotation, atom positions rcm + delta (rotation branch only, as the reference)
-__global__ void __launch_bounds__(BODY_THREADS) k_body_move(BodyArgs A, double* __restrict__ R, double CR, double CP,
-                                                            double dt, int translate, int rotate, int mode) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.nb) return;
+// force_and_torque, then pcm and pi updates; 2KE translational (bodies) and
+// rotational partial sums.  Lane c < 3 takes component c of the vectors.
+__global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_boost(BodyArgs A, const double* __restrict__ F, double CP,
+                                                                   double CF, int translate, int rotate, int kinetic,
+                                                                   double* partials, unsigned int* ticket,
+                                                                   double* result, double* hostResult) {
+  double k6[6] = {0, 0, 0, 0, 0, 0};
+  const BodyLane g = body_lane();
+  if (g.i < A.nb) {
+    BodyState& B = A.b[g.i];
+    const int c = g.c, k = c < 3 ? c : 0, k1 = (k + 1) % 3, k2 = (k + 2) % 3;
+    const int first = B.first, NP = B.NP;
+    double f = 0.0, tau = 0.0;
+    for (int j = 0; j < NP; j++) {
+      const double* Fj = &F[3 * A.atom[first + j]];
+      const double* dj = &A.delta[3 * (first + j)];
+      f += Fj[k];
+      tau += dj[k1] * Fj[k2] - dj[k2] * Fj[k1];
+    }
+    double pcm = B.pcm[k], omega = B.omega[k];
+    const double MoI = B.MoI[k], invMoI = B.invMoI[k], invMass = B.invMass;
+    if (translate) pcm = CP * pcm + CF * f;
+    double pi = B.pi[c];
+    if (rotate) {
+      const double q[4] = {B.q[0], B.q[1], B.q[2], B.q[3]}, t = 2.0 * CF * tau;
+      const double v[3] = {body_get(g, t, 0), body_get(g, t, 1), body_get(g, t, 2)};
+      pi = CP * pi + body_BC(q, v, c, true);
+      const double p[4] = {body_get(g, pi, 0), body_get(g, pi, 1), body_get(g, pi, 2), body_get(g, pi, 3)};
+      omega = 0.5 * invMoI * body_Bt(q, p, k);
+    }
+    if (rotate) B.pi[c] = pi;
+    if (c < 3) {
+      B.F[c] = f;
+      B.tau[c] = tau;
+      B.pcm[c] = pcm;
+      B.omega[c] = omega;
+    }
+    if (kinetic) {
+      const double kt = invMass * (pcm * pcm), kr = MoI * (omega * omega);
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        k6[d] = c == d ? kt : 0.0;
+        k6[3 + d] = c == d ? kr : 0.0;
+      }
+    }
+  }
+  if (kinetic) grid_reduce<6, BODY_GROUP_THREADS>(k6, partials, ticket, result, hostResult);
+}
+
+// rb_series_step (rigid.cuh) on the four lanes of a body: lane c sums the coefficients
+// of quaternion component c and, for c < 3, of w_c; the others come by shuffles.
+// Components of w are held in the lane's cyclic order x0 = w_{r+1}, x1 = w_{r+2},
+// x2 = w_r (r = c, or 0 in lane 3), so that w_r' ~ x0 x1 in every lane.
+__device__ __forceinline__ void body_series_step(const BodyLane& g, double kap, double (&w)[3], double (&q)[4]) {
+  constexpr int N = RB_SERIES_ORDER;
+  constexpr double inv[N + 1] = {0.0,       1.0,       1.0 / 2.0, 1.0 / 3.0, 1.0 / 4.0, 1.0 / 5.0,
+                                 1.0 / 6.0, 1.0 / 7.0, 1.0 / 8.0, 1.0 / 9.0, 1.0 / 10.0};
+  const int c = g.c, r = c < 3 ? c : 0, r1 = (r + 1) % 3, r2 = (r + 2) % 3;
+  // component c of B(q) w = sum over k of sign * q_{c xor (k + 1)} w_k
+  auto sgn = [&](int k) {   // rows of rb_B: (-,-,-), (+,-,+), (+,+,-), (-,+,+)
+    return c == 0 ? -1.0 : c == 1 ? (k == 1 ? -1.0 : 1.0) : c == 2 ? (k == 2 ? -1.0 : 1.0) : (k == 0 ? -1.0 : 1.0);
+  };
+  const int p0 = c ^ (r1 + 1), p1 = c ^ (r2 + 1), p2 = c ^ (r + 1);
+  const double s0 = sgn(r1), s1 = sgn(r2), s2 = sgn(r);
+  auto at3 = [](const double (&v)[3], int k) { return k == 0 ? v[0] : k == 1 ? v[1] : v[2]; };
+  auto at4 = [](const double (&v)[4], int k) { return k == 0 ? v[0] : k == 1 ? v[1] : k == 2 ? v[2] : v[3]; };
+  double X0[N + 1], X1[N + 1], X2[N + 1], B0[N + 1], B1[N + 1], B2[N + 1], Q[N + 1];
+  X0[0] = at3(w, r1);
+  X1[0] = at3(w, r2);
+  X2[0] = at3(w, r);
+  B0[0] = s0 * at4(q, p0);
+  B1[0] = s1 * at4(q, p1);
+  B2[0] = s2 * at4(q, p2);
+  Q[0] = at4(q, c);
+#pragma unroll
+  for (int n = 0; n < N; n++) {
+    double a = 0.0, b = 0.0;
+#pragma unroll
+    for (int i = 0; i <= n; i++) {
+      const int j = n - i;
+      a = fma(X0[i], X1[j], a);
+      b = fma(B0[j], X0[i], fma(B1[j], X1[i], fma(B2[j], X2[i], b)));
+    }
+    a *= kap * inv[n + 1];
+    Q[n + 1] = 0.5 * inv[n + 1] * b;
+    X0[n + 1] = body_get(g, a, r1);
+    X1[n + 1] = body_get(g, a, r2);
+    X2[n + 1] = body_get(g, a, r);
+    B0[n + 1] = s0 * body_get(g, Q[n + 1], p0);
+    B1[n + 1] = s1 * body_get(g, Q[n + 1], p1);
+    B2[n + 1] = s2 * body_get(g, Q[n + 1], p2);
+  }
+  double x = X2[N], y = Q[N];   // small terms first
+#pragma unroll
+  for (int n = N - 1; n >= 0; n--) {
+    x += X2[n];
+    y += Q[n];
+  }
+  for (int k = 0; k < 3; k++) w[k] = body_get(g, x, k);
+  for (int k = 0; k < 4; k++) q[k] = body_get(g, y, k);
+}
+
+// rcm update, rotation, atom positions rcm + delta (rotation branch only, as the reference),
+// one lane per body: NO_SQUISH, and the bodies the series does not take
+__device__ __forceinline__ void body_move_one(const BodyArgs& A, int i, double* __restrict__ R, double CR, double CP,
+                                              double dt, int translate, int rotate, int mode) {
   BodyState b = A.b[i];
   if (translate)
     for (int k = 0; k < 3; k++) b.rcm[k] = CR * b.rcm[k] + CP * b.invMass * b.pcm[k];
   if (rotate) {
     const double* d = &A.d[3 * b.first];
     double* delta = &A.delta[3 * b.first];
-    if (mode == 0) rb_rotate_exact(b, dt, d, delta);
+    if (mode == 0) rb_rotate_elliptic(b, dt, d, delta);
     else rb_rotate_no_squish(b, dt, mode, d, delta);
     for (int j = 0; j < b.NP; j++)
       for (int k = 0; k < 3; k++) R[3 * A.atom[b.first + j] + k] = b.rcm[k] + delta[3 * j + k];
   }
   A.b[i] = b;
+}
+
+__global__ void __launch_bounds__(BODY_THREADS) k_body_move(BodyArgs A, double* __restrict__ R, double CR, double CP,
+                                                            double dt, int translate, int rotate, int mode) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < A.nb) body_move_one(A, i, R, CR, CP, dt, translate, rotate, mode);
+}
+
+// The same with the exact rotation by the series (rb_rotate_series, operation by
+// operation) on BODY_LANES lanes per body.
+__global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_move_series(BodyArgs A, double* __restrict__ R, double CR,
+                                                                         double CP, double dt, int translate) {
+  const BodyLane g = body_lane();
+  if (g.i >= A.nb) return;
+  BodyState& B = A.b[g.i];
+  double MoI[3], omega[3], TwoKr = 0.0, Iw1 = 0.0, Iw2 = 0.0, invMoI[3];
+  for (int k = 0; k < 3; k++) {
+    MoI[k] = B.MoI[k];
+    invMoI[k] = B.invMoI[k];
+    omega[k] = B.omega[k];
+    const double Iw = MoI[k] * omega[k];
+    if (k == 1) Iw1 = Iw;
+    if (k == 2) Iw2 = Iw;
+    TwoKr += Iw * omega[k];
+  }
+  int steps;
+  if (!rb_series_steps(TwoKr * invMoI[2] * (dt * dt), MoI[2], Iw1 * Iw1 + Iw2 * Iw2, steps)) {
+    if (g.c == 0) body_move_one(A, g.i, R, CR, CP, dt, translate, 1, 0);
+    return;
+  }
+  const int c = g.c, k = c < 3 ? c : 0, first = B.first, NP = B.NP;
+  double q[4] = {B.q[0], B.q[1], B.q[2], B.q[3]};
+  double rcm = B.rcm[k];
+  if (translate) rcm = CR * rcm + CP * B.invMass * B.pcm[k];
+  const double h = steps == 1 ? dt : dt / steps, back = steps == 1 ? 1.0 / dt : steps / dt;
+  const double kap = k == 0 ? (MoI[1] - MoI[2]) * invMoI[0]
+                            : k == 1 ? (MoI[2] - MoI[0]) * invMoI[1] : (MoI[0] - MoI[1]) * invMoI[2];
+  double w[3] = {h * omega[0], h * omega[1], h * omega[2]};
+  for (int n = 0; n < steps; n++) body_series_step(g, kap, w, q);
+  const double n2 = q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3], f = 1.5 - 0.5 * n2;
+  double v[3];
+  for (int n = 0; n < 4; n++) q[n] *= f;
+  for (int n = 0; n < 3; n++) {
+    omega[n] = w[n] * back;
+    v[n] = 2.0 * MoI[n] * omega[n];
+  }
+  const double r[3] = {body_get(g, rcm, 0), body_get(g, rcm, 1), body_get(g, rcm, 2)};
+  for (int j = c; j < NP; j += BODY_LANES) {   // a lane per atom
+    double t[4], delta[3];
+    rb_B(q, &A.d[3 * (first + j)], t);
+    rb_Ct(q, t, delta);
+    const int a = A.atom[first + j];
+    for (int n = 0; n < 3; n++) {
+      A.delta[3 * (first + j) + n] = delta[n];
+      R[3 * a + n] = r[n] + delta[n];
+    }
+  }
+  __syncwarp(g.mask);   // every lane has read the state
+  B.q[c] = c == 0 ? q[0] : c == 1 ? q[1] : c == 2 ? q[2] : q[3];
+  B.pi[c] = body_BC(q, v, c, false);
+  if (c < 3) {
+    B.rcm[c] = rcm;
+    B.omega[c] = c == 0 ? omega[0] : c == 1 ? omega[1] : omega[2];
+  }
 }
 
 // W = sum over bodies and their atoms of F . delta (the body virial is -W)
@@ -166,6 +331,10 @@ __global__ void __launch_bounds__(BODY_THREADS) k_move_free(double* __restrict__
 
 
 static int body_blocks(int n) { return n > 0 ? (n + BODY_THREADS - 1) / BODY_THREADS : 1; }
+static int body_group_blocks(int n) {
+  const int per = BODY_GROUP_THREADS / BODY_LANES;
+  return n > 0 ? (n + per - 1) / per : 1;
+}
 
 static void ensure_scratch(System& s, int blocks, int nq) {
   int need = blocks * nq;
@@ -220,7 +389,7 @@ void bodies_update(System& s) {
 // (translational) and [13..15] (rotational)
 void bodies_boost(System& s, double CP, double CF, bool translate, bool rotate, bool kinetic) {
   int freeBlocks = std::min(body_blocks(s.nfree), 1184);
-  ensure_scratch(s, freeBlocks * 3 + body_blocks(s.nbodies) * 6, 1);
+  ensure_scratch(s, freeBlocks * 3 + body_group_blocks(s.nbodies) * 6, 1);
   if (translate && s.nfree > 0) {
     int blocks = freeBlocks;
     if (kinetic) {
@@ -234,8 +403,7 @@ void bodies_boost(System& s, double CP, double CF, bool translate, bool rotate, 
     CK(cudaGetLastError());
     s.prof.total++;
   }
-  int blocks = body_blocks(s.nbodies);
-  k_body_boost<<<blocks, BODY_THREADS, 0, s.stream>>>(body_args(s), s.F(), CP, CF, translate, rotate, kinetic,
+  k_body_boost<<<body_group_blocks(s.nbodies), BODY_GROUP_THREADS, 0, s.stream>>>(body_args(s), s.F(), CP, CF, translate, rotate, kinetic,
                                                        s.dBodyScratch + freeBlocks * 3, s.dTicket + 3, s.dResult + 16,
                                                        s.hResult + 16);
   CK(cudaGetLastError());
@@ -257,7 +425,12 @@ void bodies_move(System& s, double CR, double CP, double dt, bool translate, boo
     CK(cudaGetLastError());
     s.prof.total++;
   }
-  k_body_move<<<body_blocks(s.nbodies), BODY_THREADS, 0, s.stream>>>(body_args(s), s.dR, CR, CP, dt, translate, rotate, mode);
+  if (rotate && mode == 0)
+    k_body_move_series<<<body_group_blocks(s.nbodies), BODY_GROUP_THREADS, 0, s.stream>>>(body_args(s), s.dR, CR, CP,
+                                                                                          dt, translate);
+  else
+    k_body_move<<<body_blocks(s.nbodies), BODY_THREADS, 0, s.stream>>>(body_args(s), s.dR, CR, CP, dt, translate,
+                                                                       rotate, mode);
   CK(cudaGetLastError());
   s.prof.total++;
 }

@@ -287,21 +287,27 @@ RB_HD void rb_series_step(const double (&kap)[3], double (&w)[3], double (&q)[4]
   }
 }
 
-// The series rotation if the body takes at most RB_SERIES_MAX steps; false (nothing
-// done) otherwise, for degenerate moments and for bodies turning about their first
-// axis only, which the closed form handles apart.
+// Steps of the series for theta2 = 2K dt^2 / I3; false for more than RB_SERIES_MAX, for
+// degenerate moments and for bodies that turn about their first axis only (perp: the
+// square of the other components of I w), which the closed form handles apart.
+RB_HD bool rb_series_steps(double theta2, double I3, double perp, int& steps) {
+  const double most = RB_SERIES_STEP * RB_SERIES_MAX;
+  if (!(theta2 <= most * most) || !(I3 > 0.0)) return false;   // NaN: the closed form
+  if (perp < 2.220446049250313e-16) return false;
+  steps = 1;
+  while (steps < RB_SERIES_MAX && theta2 > (RB_SERIES_STEP * steps) * (RB_SERIES_STEP * steps)) steps++;
+  return true;
+}
+
+// The series rotation; false (nothing done) where rb_series_steps says no.
 RB_HD bool rb_rotate_series(BodyState& b, double dt, const double* d, double* delta) {
   double Iw[3], TwoKr = 0.0;
   for (int k = 0; k < 3; k++) {
     Iw[k] = b.MoI[k] * b.omega[k];
     TwoKr += Iw[k] * b.omega[k];
   }
-  const double theta2 = TwoKr * b.invMoI[2] * (dt * dt);
-  const double most = RB_SERIES_STEP * RB_SERIES_MAX;
-  if (!(theta2 <= most * most) || !(b.MoI[2] > 0.0)) return false;   // NaN: the closed form
-  if (Iw[1] * Iw[1] + Iw[2] * Iw[2] < 2.220446049250313e-16) return false;
-  int steps = 1;
-  while (steps < RB_SERIES_MAX && theta2 > (RB_SERIES_STEP * steps) * (RB_SERIES_STEP * steps)) steps++;
+  int steps;
+  if (!rb_series_steps(TwoKr * b.invMoI[2] * (dt * dt), b.MoI[2], Iw[1] * Iw[1] + Iw[2] * Iw[2], steps)) return false;
   const double h = steps == 1 ? dt : dt / steps, back = steps == 1 ? 1.0 / dt : steps / dt;
   const double kap[3] = {(b.MoI[1] - b.MoI[2]) * b.invMoI[0], (b.MoI[2] - b.MoI[0]) * b.invMoI[1],
                          (b.MoI[0] - b.MoI[1]) * b.invMoI[2]};
