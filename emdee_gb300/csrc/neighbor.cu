@@ -460,7 +460,9 @@ struct BuildArgs {
   int* nbInner;
   uint16_t* selfIdx;
   int cap, tileStride;
+  float invM;
   int tpa, tpaShift;   // threads per atom of the split build (a power of 2) and its log2
+  int allInteract;     // every type pair interacts
   int* layout;         // out: per tile off[0..haloCells] and cst[0..haloCells-1] (stage_frame_saved)
   int* maxCount;
 };
@@ -481,6 +483,7 @@ __device__ __forceinline__ bool excluded(const BuildArgs& A, int a, int b) {
 static const int BUILD_THREADS = 512;
 static const int BUILD_THREADS_RULE = 256;
 static const int BUILD_THREADS_SPLIT = 1024;  // split build: several threads per tile atom
+static const int BUILD_PAD = 4;               // halo entries past the last one, far away
 
 // List layout: for tile t, chunk c (8 entries) and tile-local atom li, the
 // entries 8c..8c+7 of atom li are 16 contiguous bytes at
@@ -491,30 +494,39 @@ __device__ __forceinline__ size_t nb_index(int t, int capC, int tileStride, int 
   return (((size_t)t * capC + (n >> 3)) * tileStride + li) * 8 + (n & 7);
 }
 
+// Every atom scans the 25 rows of 5 stencil cells around it, each over the run of cells
+// that can hold a neighbor at the row's distance.  Candidates go in segments of up to
+// 32: four loads at a time, the bits of r^2 minus the bits of the lower band limit, whose
+// sign is shifted into the segment's mask (10 instructions a candidate, no branch; the
+// unsigned minimum of the differences tells whether any candidate lies in the band and
+// the segment needs the FP64 test).  The mask's bits are then taken in order, and a
+// thread that owns its atom stores 8 entries at a time.  The kernel is bound by
+// instruction issue.  1M Lennard-Jones atoms: 630 -> 535 us against candidates that went
+// through their tests and a 2-byte store one by one (L2 sectors 122 -> 26 M).
+// The list order is (row, halo index), a function of the coordinates.
+// SPLIT: A.tpa threads per atom, which take consecutive rows: a first sweep counts, the
+// group's prefix sums give each thread its output positions, a second writes (in the
+// same order as one thread).
 // GENERAL: several atom types, bodies, exclusions or layered lists; MINIMG: M = 5.
-// Register budget: the thread-per-atom variants get up to BUILD_MAXNREG registers
-// (blocks of at most BUILD_THREADS threads); the split variant, in blocks of up to
-// 1024 threads, 64.  Under launch bounds alone the compiler held this kernel at 64
-// registers with spills; 80 (71 used) gave the fastest builds on the 1M-atom
-// workload (745 vs 811 us per rebuild with the pair kernel at 72).
+// Register budget: thread-per-atom variants BUILD_MAXNREG, the split one, in blocks of
+// up to 1024 threads, 64.
 #ifndef BUILD_MAXNREG
 #define BUILD_MAXNREG 80
 #endif
-#define BUILD_BOUNDS __maxnreg__(SPLIT ? 64 : BUILD_MAXNREG)
 template <bool GENERAL, bool MINIMG, bool SPLIT>
-__global__ void BUILD_BOUNDS k_build(BuildArgs A) {
+__global__ void __maxnreg__(SPLIT ? 64 : BUILD_MAXNREG) k_build(BuildArgs A) {
   extern __shared__ __align__(16) unsigned char sraw[];
   __shared__ int ws[33];
   const TileGeom g = A.g;
   const int t = blockIdx.x, cells = g.TB * g.TB * g.TB;
-  // shared memory: the staged halo (and a sentinel entry), the halo cell offsets,
-  // then for the general variant the halo atoms' slots, the type filter and the
-  // halo atoms' types
+  // shared memory: the staged halo (and the entries that a segment of four may read
+  // past its end), the halo cell offsets, then for the general variant the halo atoms'
+  // keys (their body, or with exclusions the atom), the type filter and their types
   float4* hpos = (float4*)sraw;
-  int* off = (int*)(hpos + A.haloCap + 1);
-  int* hslot = off + g.haloCells + 1;
-  const bool single = !GENERAL || A.ntypes == 1;
-  uint8_t* sinter = (uint8_t*)(hslot + (GENERAL ? A.haloCap + 1 : 0));
+  int* off = (int*)(hpos + A.haloCap + BUILD_PAD);
+  int* hkey = off + g.haloCells + 1;
+  const bool single = !GENERAL || A.allInteract;
+  uint8_t* sinter = (uint8_t*)(hkey + (GENERAL ? A.haloCap : 0));
   uint8_t* htype = sinter + A.ntypes * A.ntypes;
   for (int k = threadIdx.x; k < A.ntypes * A.ntypes; k += blockDim.x) sinter[k] = A.interact[k];
   // the layout, saved for the force kernels until the next build: first slots
@@ -547,12 +559,17 @@ __global__ void BUILD_BOUNDS k_build(BuildArgs A) {
   for (int h = threadIdx.x; h < g.haloCells; h += blockDim.x)
     mark_halo_cell(hpos, h, off[h], off[h + 1], lay[g.haloCells + 1 + h]);
   __syncthreads();
-  stage_marked(g, haloCount, A.pos4, hpos, GENERAL ? hslot : nullptr, single ? (uint8_t*)nullptr : htype, A.type8);
+  const bool filterByAtom = GENERAL && (A.hasBodies || A.hasEx);
+  stage_marked(g, haloCount, A.pos4, hpos, filterByAtom ? hkey : nullptr, single ? (uint8_t*)nullptr : htype, A.type8);
+  if (threadIdx.x < BUILD_PAD) hpos[haloCount + threadIdx.x] = make_float4(1e9f, 1e9f, 1e9f, 0.f);
+  if (filterByAtom)   // every thread reads back only the slots it wrote itself
+    for (int k = threadIdx.x; k < haloCount; k += blockDim.x) {
+      const int a = A.orig[hkey[k]];
+      hkey[k] = A.hasEx ? a : A.body[a];
+    }
   __syncthreads();
-  // slot of halo index q (the general variant keeps them; the band test of the
-  // plain one, rare, looks its cell up)
+  // slot of halo index q (for the rare band test): its cell is looked up
   auto slot_of = [&](int q) {
-    if (GENERAL) return hslot[q];
     int lo = 0, hi = g.haloCells - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -562,18 +579,15 @@ __global__ void BUILD_BOUNDS k_build(BuildArgs A) {
     return lay[g.haloCells + 1 + lo] + (q - off[lo]);
   };
   const bool none = A.ntypes == 1 && !sinter[0];   // the only type pair does not interact: empty lists
-  const bool filterByAtom = GENERAL && (A.hasBodies || A.hasEx);
   const bool layered = GENERAL && A.layered;
   const int tb = A.start[t * cells], te = A.start[(t + 1) * cells];
   const int HW = g.HW, capC = A.cap >> 3, chunkStride = A.tileStride * 8;
-  // SPLIT: tpa threads share an atom, each scanning the stencil rows r = sub,
-  // sub + tpa, ...; a first sweep counts the accepted entries (inner and outer),
-  // the group's prefix sums give each thread its output positions, and a second
-  // sweep writes them.  The list order is then (thread, row, halo index) -- a
-  // deterministic function of the coordinates, like the single-thread order.
+  const int loBits = __float_as_int(A.lo2);
+  const unsigned band = (unsigned)(__float_as_int(A.hi2) - loBits);
   const int tpa = SPLIT ? A.tpa : 1, sub = SPLIT ? (int)(threadIdx.x & (tpa - 1)) : 0;
   const int tshift = SPLIT ? A.tpaShift : 0;
   const unsigned gmask = (0xFFFFFFFFu >> (32 - tpa)) << ((threadIdx.x & 31) & ~(tpa - 1));
+  int longest = 0;
   for (int li = threadIdx.x >> tshift; li < te - tb; li += blockDim.x >> tshift) {
     const int si = tb + li;
     const int rank = A.K[si].w, lr = rank - t * cells;
@@ -583,109 +597,153 @@ __global__ void BUILD_BOUNDS k_build(BuildArgs A) {
     const float4 pi = hpos[myq];
     const int ai = A.orig[si], ti = single ? 0 : A.type8[si];
     const int bi = filterByAtom && A.hasBodies ? A.body[ai] : -1;
-    const bool hasEx = filterByAtom && A.hasEx && A.exCount[ai] > 0;
-    uint16_t* myList = A.nb + ((size_t)t * capC * A.tileStride + li) * 8;
-    // accepted candidates of stencil row (rz, ry) -> f(q, inner); the 5 cells of a
-    // row (dx = -2..2) are consecutive in the halo
-    auto zdist2 = [&](int rz) {   // squared distance from atom i to the z slab of offset rz
-      const float z0 = (float)(hcz + rz - g.C);
-      const float dz = fmaxf(fmaxf(z0 - pi.z, pi.z - (z0 + 1.0f)) - 1e-3f, 0.0f);
-      return dz * dz;
+    // the first exclusions of the atom (lists are ascending; -1: none)
+    constexpr int EX = 4;
+    int ex[EX], nEx = 0;
+    if (GENERAL) {
+      nEx = filterByAtom && A.hasEx ? A.exCount[ai] : 0;
+#pragma unroll
+      for (int k = 0; k < EX; k++) ex[k] = k < nEx ? A.exItem[A.exFirst[ai] + k] - 1 : -1;
+    }
+    auto allowed = [&](int q) {
+      if (!single && !sinter[ti * A.ntypes + htype[q]]) return false;
+      if (filterByAtom) {
+        const int key = hkey[q];
+        if (A.hasBodies && (A.hasEx ? A.body[key] : key) == bi) return false;
+        if (nEx > 0) {
+#pragma unroll
+          for (int k = 0; k < EX; k++)
+            if (key == ex[k]) return false;
+          if (nEx > EX && excluded(A, ai, key)) return false;
+        }
+      }
+      return true;
     };
-    auto row = [&](int rz, int ry, float dz2, auto&& f) {
-      const int hz = hcz + rz, hy = hcy + ry;
-      const int h0 = (hcx - 2) + HW * (hy + HW * hz);
-      int q = off[h0];
-      const int q1 = off[h0 + 5];
-      float xhi = 3.0e38f;
+    auto dist2 = [&](int q) {
+      const float4 pj = hpos[q];
+      float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+      if (MINIMG) {
+        dx -= A.Mf * rintf(dx * A.invM);
+        dy -= A.Mf * rintf(dy * A.invM);
+        dz -= A.Mf * rintf(dz * A.invM);
+      }
+      return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+    };
+    // window [q0, q1) of halo indices of stencil row (rz, ry) (the 5 cells of a row are
+    // consecutive): with rho the distance from atom i to the row's y-z cross-section, only
+    // cells that reach |x_j - x_i| < sqrt(hi2 - rho^2) can hold a neighbor; a 1e-3 cell
+    // margin covers the FP32 rounding of the frame and the approximate square root (cell
+    // hx spans [hx - C, hx - C + 1] in the frame).
+    auto window = [&](int rz, int ry, int& q0, int& q1) {
+      const int hz = hcz + rz, hy = hcy + ry, h0 = (hcx - 2) + HW * (hy + HW * hz);
+      int c0 = 0, c1 = 4;
       if (!MINIMG) {
-        // Atoms of a row are sorted along x.  With rho the distance from atom i
-        // to the row's y-z cross-section, only |x_j - x_i| < sqrt(hi2 - rho^2)
-        // can be inside; a 1e-3 cell margin covers the FP32 rounding of the frame.
-        const float y0 = (float)(hy - g.C);
+        const float y0 = (float)(hy - g.C), z0 = (float)(hz - g.C);
         const float dy = fmaxf(fmaxf(y0 - pi.y, pi.y - (y0 + 1.0f)) - 1e-3f, 0.0f);
-        const float rem = A.hi2 - (dy * dy + dz2);
-        if (rem <= 0.0f) return;
-        const float w = rem * rsqrtf(rem) + 1e-3f;   // approximate square root: within the margin
-        const float xlo = pi.x - w;
-        xhi = pi.x + w;
-        // atoms of halo cells left of floor(xlo) lie at x <= floor(xlo) <= xlo (cell
-        // hx spans [hx - C, hx - C + 1] in the frame): start at that cell
-        const int cs = min(max((int)floorf(xlo) + g.C, hcx - 2), hcx + 2);
-        q = off[h0 + cs - (hcx - 2)];
-        while (q < q1 && hpos[q].x <= xlo) q++;
+        const float dz = fmaxf(fmaxf(z0 - pi.z, pi.z - (z0 + 1.0f)) - 1e-3f, 0.0f);
+        const float rem = A.hi2 - fmaf(dy, dy, dz * dz);
+        if (rem <= 0.0f) {
+          q0 = q1 = 0;
+          return;
+        }
+        const float w = fmaf(rem, rsqrtf(rem), 1e-3f);
+        const int shift = g.C - (hcx - 2);
+        c0 = min(max((int)floorf(pi.x - w) + shift, 0), 4);
+        c1 = min(max((int)floorf(pi.x + w) + shift, 0), 4);
       }
-      // candidates in groups of CG: the loads and distance tests of a group are
-      // independent (predicated, no branch per candidate), then the accepted ones
-      // are taken in ascending order; a group that reaches the row's end or the
-      // window's end is the last (the row is sorted along x)
-      constexpr int CG = 2;   // pairs: measured faster than single candidates or groups of four
-      for (; q < q1; q += CG) {
-        float4 pj[CG];
+      q0 = off[h0 + c0];
+      q1 = off[h0 + c1 + 1];
+    };
+    // accepted candidates of q, q + 1, ... (at most 32, up to q1): bit 31 - j is q + j
+    auto segment = [&](int q, int q1) {
+      const int len = min(32, q1 - q);
+      unsigned m = 0, near = 0xFFFFFFFFu;
+      for (int u = 0; u < len; u += 4)
 #pragma unroll
-        for (int u = 0; u < CG; u++) pj[u] = hpos[min(q + u, q1 - 1)];
-        float r2s[CG];
-        unsigned cand = 0;
-        bool last = false;
-#pragma unroll
-        for (int u = 0; u < CG; u++) {
-          const bool valid = q + u < q1 && (MINIMG || pj[u].x < xhi);
-          last |= !valid;
-          float ex = pi.x - pj[u].x, ey = pi.y - pj[u].y, ez = pi.z - pj[u].z;
-          if (MINIMG) {
-            ex -= A.Mf * rintf(ex / A.Mf);
-            ey -= A.Mf * rintf(ey / A.Mf);
-            ez -= A.Mf * rintf(ez / A.Mf);
-          }
-          r2s[u] = ex * ex + ey * ey + ez * ez;
-          cand |= (valid && r2s[u] < A.hi2 && q + u != myq) ? 1u << u : 0u;
+        for (int v = 0; v < 4; v++) {
+          const int d = __float_as_int(dist2(q + u + v)) - loBits;
+          m = __funnelshift_l((unsigned)d, m, 1);
+          near = min(near, (unsigned)d);
         }
-#pragma unroll
-        for (int u = 0; u < CG; u++) {
-          if (!((cand >> u) & 1u)) continue;
-          const int qu = q + u;
-          const float r2 = r2s[u];
-          if (!(r2 < A.lo2 || exact_inside(A.R, A.L, ai, A.orig[slot_of(qu)], A.thr))) continue;
-          if (GENERAL && !single && !sinter[ti * A.ntypes + htype[qu]]) continue;
-          if (filterByAtom) {
-            const int aj = A.orig[hslot[qu]];
-            if (A.hasBodies && A.body[aj] == bi) continue;
-            if (hasEx && excluded(A, ai, aj)) continue;
-          }
-          bool inner = true;
-          if (layered)
-            inner = r2 < A.loIn2 || (r2 < A.hiIn2 && exact_inside(A.R, A.L, ai, A.orig[slot_of(qu)], A.thrIn));
-          f(qu, inner);
+      m <<= (32 - ((len + 3) & ~3));
+      if (near < band)   // some candidate lies within the band: the FP64 test decides it
+        for (int j = 0; j < len; j++) {
+          const unsigned d = (unsigned)(__float_as_int(dist2(q + j)) - loBits);
+          if (d < band && exact_inside(A.R, A.L, ai, A.orig[slot_of(q + j)], A.thr)) m |= 0x80000000u >> j;
         }
-        if (last) break;
+      m &= (unsigned)((int)0x80000000 >> (len - 1));                                  // candidates before q1
+      if ((unsigned)(myq - q) < 32u) m &= ~(0x80000000u >> (myq - q));                // not the atom itself
+      return m;
+    };
+    // f(q) of every accepted neighbor of a row; inner / outer entries of layered lists
+    // in the sweep they belong to
+    auto row = [&](int rz, int ry, auto&& f) {
+      int q0, q1;
+      window(rz, ry, q0, q1);
+      for (int q = q0; q < q1; q += 32) {
+        unsigned m = segment(q, q1);
+        while (m) {
+          const int j = __clz(m);
+          m &= 0x7FFFFFFFu >> j;
+          if (GENERAL && !allowed(q + j)) continue;
+          f(q + j);
+        }
       }
     };
-    auto put = [&](int k, int q) {
-      if (k < A.cap) myList[(k >> 3) * chunkStride + (k & 7)] = (uint16_t)q;
+    auto inside = [&](int q) {
+      const float r2 = dist2(q);
+      return r2 < A.loIn2 || (r2 < A.hiIn2 && exact_inside(A.R, A.L, ai, A.orig[slot_of(q)], A.thrIn));
     };
     int n = 0, nIn = 0;
     if (!SPLIT) {
-      // rows in the order dz = -2..2 (outer), dy = -2..2 (inner); layered lists
-      // take the inner entries in a first sweep and the outer ones in a second
-      for (int pass = 0; pass <= (layered ? 1 : 0) && !none; pass++) {
-        for (int rz = -2; rz <= 2; rz++) {
-          const float dz2 = MINIMG ? 0.0f : zdist2(rz);
-          for (int ry = -2; ry <= 2; ry++)
-            row(rz, ry, dz2, [&](int q, bool inner) {
-              if (layered && inner == (pass == 1)) return;
-              put(n++, q);
-            });
+      // rows in the order dz = -2..2 (outer), dy = -2..2 (inner); layered lists take the
+      // inner entries in a first sweep and the outer ones in a second.  The last 8 entries
+      // sit in four registers until they are complete.
+      uint4 w = make_uint4(0u, 0u, 0u, 0u);
+      uint4* out = reinterpret_cast<uint4*>(A.nb) + ((size_t)t * capC * A.tileStride + li);
+      auto push = [&](int q) {
+        w.x = __funnelshift_r(w.x, w.y, 16);
+        w.y = __funnelshift_r(w.y, w.z, 16);
+        w.z = __funnelshift_r(w.z, w.w, 16);
+        w.w = __funnelshift_r(w.w, (unsigned)q, 16);
+        n++;
+        if ((n & 7) == 0) {
+          if (n <= A.cap) *out = w;
+          out += A.tileStride;
         }
+      };
+      for (int pass = 0; pass <= (layered ? 1 : 0) && !none; pass++) {
+        for (int rz = -2; rz <= 2; rz++)
+          for (int ry = -2; ry <= 2; ry++)
+            row(rz, ry, [&](int q) {
+              if (layered && inside(q) == (pass == 1)) return;
+              push(q);
+            });
         if (pass == 0) nIn = n;
       }
+      const int count = n;
+      while (n & 7) push(A.haloCap);   // sentinel padding of the last chunk
+      n = count;
     } else {
+      uint16_t* myList = A.nb + ((size_t)t * capC * A.tileStride + li) * 8;
+      auto put = [&](int k, int q) {
+        if (k < A.cap) myList[(k >> 3) * chunkStride + (k & 7)] = (uint16_t)q;
+      };
+      const int r0 = 25 * sub >> tshift, r1 = 25 * (sub + 1) >> tshift;
       int cIn = 0, cOut = 0;
       if (!none)
-        for (int r = sub; r < 25; r += tpa)
-          row(r / 5 - 2, r % 5 - 2, MINIMG ? 0.0f : zdist2(r / 5 - 2), [&](int, bool inner) {
-            if (inner) cIn++;
-            else cOut++;
-          });
+        for (int r = r0; r < r1; r++) {
+          if (GENERAL) {
+            row(r / 5 - 2, r % 5 - 2, [&](int q) {
+              if (!layered || inside(q)) cIn++;
+              else cOut++;
+            });
+          } else {   // nothing to filter: the masks' bits are the count
+            int q0, q1;
+            window(r / 5 - 2, r % 5 - 2, q0, q1);
+            for (int q = q0; q < q1; q += 32) cIn += __popc(segment(q, q1));
+          }
+        }
       // exclusive prefix sums over the group's threads, in sub order
       int pIn = cIn, pOut = cOut;
       for (int o = 1; o < tpa; o <<= 1) {
@@ -698,22 +756,25 @@ __global__ void BUILD_BOUNDS k_build(BuildArgs A) {
       const int totIn = __shfl_sync(gmask, pIn, tpa - 1, tpa), totOut = __shfl_sync(gmask, pOut, tpa - 1, tpa);
       int kIn = pIn - cIn, kOut = totIn + pOut - cOut;
       if (!none)
-        for (int r = sub; r < 25; r += tpa)
-          row(r / 5 - 2, r % 5 - 2, MINIMG ? 0.0f : zdist2(r / 5 - 2), [&](int q, bool inner) {
-            if (inner) put(kIn++, q);
+        for (int r = r0; r < r1; r++)
+          row(r / 5 - 2, r % 5 - 2, [&](int q) {
+            if (!layered || inside(q)) put(kIn++, q);
             else put(kOut++, q);
           });
       n = totIn + totOut;
       nIn = totIn;
-      __syncwarp(gmask);
+      // sentinel padding of the last chunk
+      if (sub == 0)
+        for (int k = n; (k & 7) && k < A.cap; k++) put(k, A.haloCap);
     }
     if (sub == 0) {
-      for (int k = n; k < A.cap && (k & 7); k++) myList[(k >> 3) * chunkStride + (k & 7)] = (uint16_t)A.haloCap;
       A.nbCount[si] = n;
       A.nbInner[si] = nIn;
-      atomicMax(A.maxCount, n);
     }
+    longest = max(longest, n);
   }
+  longest = __reduce_max_sync(0xffffffffu, longest);
+  if ((threadIdx.x & 31) == 0 && longest > 0) atomicMax(A.maxCount, longest);
 }
 
 template <typename T>
@@ -725,9 +786,30 @@ static void grow(T*& p, size_t& have, size_t need) {
 }
 
 
+double expected_entries(const System& s) {
+  const double L = *s.Lbox;
+  return s.natoms / (L * L * L) * 4.18879020478639 * s.xRcSq * s.xRc;
+}
+
+int split_threads(const System& s, double entries, int maxThreads) {
+  int tpa = 1;
+  while (tpa < 32 && (double)s.natoms * tpa * 2 <= 152.0 * 2048 && s.grid.tileAtoms * tpa * 2 <= maxThreads &&
+         entries / (tpa * 2) >= 8.0)
+    tpa *= 2;
+  return tpa;
+}
+
+// threads per atom of the build (its candidates are about twice the entries)
+static int build_tpa(const System& s) {
+  return s.buildTpa > 0 ? s.buildTpa : split_threads(s, 2.0 * expected_entries(s), BUILD_THREADS_SPLIT);
+}
+
 int build_block_threads(const System& s) {
-  return s.buildThreads > 0 ? std::min(s.buildThreads, BUILD_THREADS)
-                            : tile_threads(s.grid.tileStride, 0, BUILD_THREADS_RULE);
+  const Grid& g = s.grid;
+  const int least = halo_min_threads(make_geom(g.M, g.TB)), tpa = build_tpa(s);
+  if (tpa > 1) return std::max(least, std::min(BUILD_THREADS_SPLIT, (g.tileAtoms * tpa + 31) / 32 * 32));
+  return std::max(least, s.buildThreads > 0 ? std::min(s.buildThreads, BUILD_THREADS)
+                                            : tile_threads(g.tileAtoms, 0, BUILD_THREADS_RULE));
 }
 
 // the general build variant: several types, bodies, exclusions or layered lists
@@ -736,34 +818,41 @@ static bool build_general(const System& s) {
 }
 
 static size_t build_smem(const Grid& g, int ntypes, bool general) {
-  return (size_t)(g.maxHalo + 1) * (sizeof(float4) + (general ? sizeof(int) + 1 : 0)) +
+  return (size_t)(g.maxHalo + BUILD_PAD) * (sizeof(float4) + (general ? sizeof(int) + 1 : 0)) +
          sizeof(int) * (g.haloCells + 1) + (size_t)ntypes * ntypes + 16;
 }
 
-// Tile edge: EMDEE_TILE, else the system's tuned edge (tileOverride), else a rule on
-// the atoms per cell.
-static int rule_tile(int M, double perCell) {
-  const int tb = perCell <= 4.0 ? 4 : perCell <= 9.0 ? 3 : perCell <= 24.0 ? 2 : 1;
-  return std::min(tb, M);
+// Tile edge: EMDEE_TILE, else the system's tuned edge (tileOverride), else a rule: by the
+// atoms per cell, smaller where the tiles would not give every SM two blocks (two-level
+// lists, whose launches have one thread per atom, keep the larger tiles).
+static int rule_tile(System& s, int M, double perCell) {
+  int tb = std::min(perCell <= 4.0 ? 4 : perCell <= 9.0 ? 3 : perCell <= 24.0 ? 2 : 1, M);
+  while (tb > 1 && !two_level_active(s)) {
+    const int nT = (M + tb - 1) / tb;
+    if (nT * nT * nT >= 2 * 152) break;
+    tb--;
+  }
+  return tb;
 }
 
-static int choose_tile(const System& s, int M, double perCell) {
+static int choose_tile(System& s, int M, double perCell) {
   if (const char* e = getenv("EMDEE_TILE")) {
     int tb = atoi(e);
     if (tb >= 1 && tb <= 6) return std::min(tb, M);
   }
   if (s.tileOverride > 0) return std::min(s.tileOverride, M);
-  return rule_tile(M, perCell);
+  return rule_tile(s, M, perCell);
 }
 
-// Tile edge and block sizes tuned on the system itself at its first build (mixed
-// precision, M > 5, EMDEE_TILE unset).  For each edge from min(rule - 1, 3) to 6
-// cells (the rule's edge always among them) a first build sizes the tiles; then the
-// list build and the pair kernel are timed with CUDA events (the faster of two
-// launches, after a warm-up launch of the pair kernel), each after a pass that moves
-// the memory traffic of an integration step, at the rule's block size and at block
-// sizes from 64 to 512 threads (threads loop over the tile's atoms in rounds; the
-// best size balances the rounds of typical tiles against residency).  The cost of an
+// Tile edge, threads per atom and block sizes tuned on the system itself at its first
+// build (mixed precision, EMDEE_TILE unset).  For each edge from min(rule - 1, 3)
+// (from 1 in small systems, where few large tiles leave most SMs idle) to 6 cells (the
+// rule's edge always among them) a first build sizes the tiles; then the list build
+// and the pair kernel are timed with CUDA events (the faster of two launches, after a
+// warm-up launch of the pair kernel), each after a pass that moves the memory traffic
+// of an integration step, at the rule's shape, at block sizes from 64 to 512 threads
+// (threads loop over the tile's atoms in rounds; the best size balances the rounds of
+// typical tiles against residency) and at 2 to 32 threads per atom.  The cost of an
 // edge is its fastest pair launch plus a seventh of its fastest build (a rebuild
 // every ~7 steps, typical of a liquid with the reference's skin).  The rule's edge
 // and block sizes stay unless another choice is more than 5 % cheaper.  The choice
@@ -783,97 +872,116 @@ __global__ void k_touch(double* __restrict__ R, double* __restrict__ P, const do
 }
 
 struct TileChoice {
-  int tb, buildThreads, pairThreads;
+  int tb, buildTpa, buildThreads, pairTpa, pairThreads;
 };
 static std::vector<std::pair<std::vector<long>, TileChoice>> g_tileTuned;
+
+static void use_choice(System& s, const TileChoice& c) {
+  s.tileOverride = c.tb;
+  s.buildTpa = c.buildTpa;
+  s.buildThreads = c.buildThreads;
+  s.pairTpa = c.pairTpa;
+  s.pairThreads = c.pairThreads;
+}
 
 void device_tune_tile(System& s, bool ljOnly, void (*pair)(System&)) {
   if (getenv("EMDEE_TILE") || (getenv("EMDEE_AUTOTUNE") && !strcmp(getenv("EMDEE_AUTOTUNE"), "0"))) return;
   const double L = *s.Lbox;
   const int M = std::max((int)std::floor(NDIV * L / s.xRc), 2 * NDIV + 1);
-  if (M <= 2 * NDIV + 1) return;
   const double perCell = (double)s.natoms / ((double)M * M * M);
   const std::vector<long> key = {M, (long)std::lround(perCell * 8.0), s.ntypes, ljOnly ? 1 : 0, s.nbodies > 0,
                                  s.hasExclusions ? 1 : 0};
   for (const auto& e : g_tileTuned)
     if (e.first == key) {
-      s.tileOverride = e.second.tb;
-      s.buildThreads = e.second.buildThreads;
-      s.pairThreads = e.second.pairThreads;
+      use_choice(s, e.second);
       return;
     }
-  const int rule = rule_tile(M, perCell);
+  const int rule = rule_tile(s, M, perCell);
   const bool chainReq = s.keChainReq;   // no kinetic pass queued behind the timed pair launches
   s.keChainReq = false;
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   auto timed = [&](auto&& f) {
-    if (!s.phaseShared) {   // (shared R and P may belong to another system's stream)
-      k_touch<<<4 * 152, 256, 0, s.stream>>>(s.dR, s.dP, s.F(), 3L * s.natoms, 0LL);
-      CK(cudaGetLastError());
-      s.prof.total++;
+    double best = 1e30;
+    for (int k = 0; k < 2; k++) {
+      if (!s.phaseShared) {   // (shared R and P may belong to another system's stream)
+        k_touch<<<4 * 152, 256, 0, s.stream>>>(s.dR, s.dP, s.F(), 3L * s.natoms, 0LL);
+        CK(cudaGetLastError());
+        s.prof.total++;
+      }
+      CK(cudaEventRecord(e0, s.stream));
+      f();
+      CK(cudaEventRecord(e1, s.stream));
+      CK(cudaEventSynchronize(e1));
+      float ms = 0.f;
+      CK(cudaEventElapsedTime(&ms, e0, e1));
+      best = std::min(best, (double)ms);
     }
-    CK(cudaEventRecord(e0, s.stream));
-    f();
-    CK(cudaEventRecord(e1, s.stream));
-    CK(cudaEventSynchronize(e1));
-    float ms = 0.f;
-    CK(cudaEventElapsedTime(&ms, e0, e1));
-    return (double)ms;
+    return best;
   };
+  const bool log = getenv("EMDEE_TUNE_LOG") != nullptr;
   double best = 1e30, ruleCost = 1e30;
-  TileChoice choice = {rule, 0, 0};
-  for (int tb = std::max(1, std::min(rule - 1, 3)); tb <= std::min(6, M); tb++) {
-    s.tileOverride = tb;
-    s.buildThreads = s.pairThreads = 0;
+  TileChoice choice = {rule, 0, 0, 0, 0};
+  const bool small = s.natoms < 152 * 1024;   // fewer atoms than half the GPU's threads
+  for (int tb = small ? 1 : std::max(1, std::min(rule - 1, 3)); tb <= std::min(6, M); tb++) {
+    use_choice(s, TileChoice{tb, 0, 0, 0, 0});
     device_build_lists(s);   // sizes the tiles of this edge
     if (s.grid.TB != tb) continue;   // did not fit (halo or shared memory): the build shrank the edge
-    // block sizes: 0 (the rule), then 64 to 256 threads in steps of 32 and 320 to 512
-    // in steps of 64, from the least the halo scans need up to the largest tile
-    const int thMin = halo_min_threads(make_geom(s.grid.M, tb)), thMax = (s.grid.tileStride + 31) / 32 * 32;
-    std::vector<int> sizes = {0};
+    // (threads per atom, threads per block): the rule's (0, 0), then with one thread per
+    // atom 64 to 256 threads in steps of 32 and 320 to 512 in steps of 64, from the least the
+    // halo scans need up to the largest tile, and the splits that the GPU has threads for
+    const int thMin = halo_min_threads(make_geom(s.grid.M, tb)), thMax = (s.grid.tileAtoms + 31) / 32 * 32;
+    std::vector<std::pair<int, int>> shapes = {{0, 0}};
     for (int th = 64; th <= 512; th += th < 256 ? 32 : 64)
-      if (th >= thMin && th <= thMax) sizes.push_back(th);
+      if (th >= thMin && th <= std::max(thMax, 64)) shapes.push_back({1, th});
+    for (int tpa = 2; tpa <= 32; tpa *= 2)
+      if ((double)s.natoms * tpa <= 152.0 * 2048 * 2 && s.grid.tileAtoms * tpa <= 1024) shapes.push_back({tpa, 0});
     double msBuild = 1e30, msPair = 1e30, ruleBuild = 0.0, rulePair = 0.0;
-    int rb = 0, rp = 0;
-    for (int r : sizes) {
-      s.buildThreads = r;
-      const double ms = std::min(timed([&] { device_build_lists(s); }), timed([&] { device_build_lists(s); }));
-      if (getenv("EMDEE_TUNE_LOG"))
-        fprintf(stderr, "  edge %d build, %d threads: %.1f us\n", tb, build_block_threads(s), 1e3 * ms);
-      if (r == 0) ruleBuild = ms;
+    TileChoice here = {tb, 0, 0, 0, 0};
+    for (const auto& sh : shapes) {
+      s.buildTpa = sh.first;
+      s.buildThreads = sh.second;
+      const double ms = timed([&] { device_build_lists(s); });
+      if (log)
+        fprintf(stderr, "  edge %d build, %d per atom, %d threads: %.1f us\n", tb, sh.first, build_block_threads(s),
+                1e3 * ms);
+      if (sh.first == 0) ruleBuild = ms;
       if (ms < msBuild) {
         msBuild = ms;
-        rb = r;
+        here.buildTpa = sh.first;
+        here.buildThreads = sh.second;
       }
     }
-    for (int r : sizes) {
-      s.pairThreads = r;
+    for (const auto& sh : shapes) {
+      s.pairTpa = sh.first;
+      s.pairThreads = sh.second;
       pair(s);   // warm-up
-      const double ms = std::min(timed([&] { pair(s); }), timed([&] { pair(s); }));
-      if (getenv("EMDEE_TUNE_LOG")) fprintf(stderr, "  edge %d pair, %d threads: %.1f us\n", tb, pair_block_threads(s), 1e3 * ms);
-      if (r == 0) rulePair = ms;
+      const double ms = timed([&] { pair(s); });
+      if (log)
+        fprintf(stderr, "  edge %d pair, %d per atom, %d threads: %.1f us\n", tb, sh.first, pair_block_threads(s),
+                1e3 * ms);
+      if (sh.first == 0) rulePair = ms;
       if (ms < msPair) {
         msPair = ms;
-        rp = r;
+        here.pairTpa = sh.first;
+        here.pairThreads = sh.second;
       }
     }
     const double cost = msPair + msBuild / 7.0;
     if (tb == rule) ruleCost = rulePair + ruleBuild / 7.0;
-    if (getenv("EMDEE_TUNE_LOG"))
-      fprintf(stderr, "tile edge %d (at most %d atoms per tile): cost %.1f us\n", tb, s.grid.tileStride, 1e3 * cost);
+    if (log)
+      fprintf(stderr, "tile edge %d (at most %d atoms per tile): cost %.1f us, build %d x %d, pair %d x %d\n", tb,
+              s.grid.tileAtoms, 1e3 * cost, here.buildTpa, here.buildThreads, here.pairTpa, here.pairThreads);
     if (cost < best) {
       best = cost;
-      choice = {tb, rb, rp};
+      choice = here;
     }
   }
-  if (ruleCost < 1e30 && best > 0.95 * ruleCost) choice = {rule, 0, 0};
+  if (ruleCost < 1e30 && best > 0.95 * ruleCost) choice = {rule, 0, 0, 0, 0};
   CK(cudaEventDestroy(e0));
   CK(cudaEventDestroy(e1));
-  s.tileOverride = choice.tb;
-  s.buildThreads = choice.buildThreads;
-  s.pairThreads = choice.pairThreads;
+  use_choice(s, choice);
   s.r0Valid = false;   // the system's own first build comes next, with the chosen edge
   s.keChainReq = chainReq;
   g_tileTuned.push_back({key, choice});
@@ -965,7 +1073,8 @@ static bool build_lists(System& s, bool reuse) {
     int hmax[2];
     CK(cudaMemcpyAsync(hmax, dMax, sizeof(int) * 2, cudaMemcpyDeviceToHost, s.stream));
     CK(cudaStreamSynchronize(s.stream));
-    g.tileStride = std::max(32, (hmax[0] + 31) / 32 * 32);
+    g.tileAtoms = hmax[0];
+    g.tileStride = hmax[0] > 24 ? (hmax[0] + 31) / 32 * 32 : std::max(8, (hmax[0] + 7) / 8 * 8);
     g.maxHalo = hmax[1];
     size_t smem = build_smem(g, s.ntypes, build_general(s));
     size_t smem64 = (size_t)(g.maxHalo + 1) * (4 * sizeof(double) + 1) + 2 * sizeof(int) * (g.haloCells + 1) + 64;
@@ -1043,27 +1152,19 @@ static bool build_lists(System& s, bool reuse) {
   A.layout = g.dLayout;
   const bool general = build_general(s);
   size_t smem = build_smem(g, s.ntypes, general);
-  // Threads per atom: a system too small to fill the GPU with one thread per atom and
-  // with long lists (more than 48 entries per thread) splits the stencil rows of each
-  // atom over 2, 4 or 8 threads (blocks of up to 1024 threads).
-  {
-    const double expected = N / (L * L * L) * 4.18879020478639 * xRcSq * xRc;
-    int tpa = 1, shift = 0;
-    while (tpa < 8 && g.tileStride * tpa * 2 <= BUILD_THREADS_SPLIT && (double)N * tpa * 2 <= 152.0 * 2048 &&
-           expected / (tpa * 2) >= 48) {
-      tpa *= 2;
-      shift++;
-    }
-    A.tpa = tpa;
-    A.tpaShift = shift;
-  }
+  A.invM = 1.0f / A.Mf;
+  A.tpa = build_tpa(s);
+  A.tpaShift = 0;
+  while (1 << A.tpaShift < A.tpa) A.tpaShift++;
+  A.allInteract = 1;
+  for (size_t q = 0; q < (size_t)s.ntypes * s.ntypes; q++)
+    if (!s.interact[q]) A.allInteract = 0;
   const bool split = A.tpa > 1;
   auto kb = split ? (general ? (A.minimg ? k_build<true, true, true> : k_build<true, false, true>)
                              : (A.minimg ? k_build<false, true, true> : k_build<false, false, true>))
                   : (general ? (A.minimg ? k_build<true, true, false> : k_build<true, false, false>)
                              : (A.minimg ? k_build<false, true, false> : k_build<false, false, false>));
-  const int buildThreads = std::max(halo_min_threads(geo), split ? std::min(BUILD_THREADS_SPLIT, g.tileStride * A.tpa)
-                                                                 : build_block_threads(s));
+  const int buildThreads = build_block_threads(s);
   CK(cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 #ifdef EMDEE_MAX_CARVEOUT
   CK(cudaFuncSetAttribute(kb, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));

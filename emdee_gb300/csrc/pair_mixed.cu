@@ -26,10 +26,10 @@ namespace emdee {
 // rounds as blocks of PAIR_THREADS_RULE threads allow.
 static const int PAIR_THREADS = 512;
 static const int PAIR_THREADS_RULE = 256;
-// The general variant (VAR 1) may run several threads per atom in blocks of up to
+// The variants with several threads per atom (VAR 1 and 2) run in blocks of up to
 // PAIR_THREADS_GENERAL threads.
 static const int PAIR_THREADS_GENERAL = 1024;
-#define PAIR_MAX_THREADS (VAR == 1 ? PAIR_THREADS_GENERAL : PAIR_THREADS)
+#define PAIR_MAX_THREADS (VAR == 0 ? PAIR_THREADS : PAIR_THREADS_GENERAL)
 // Register budget: the single-type Lennard-Jones variant gets up to PAIR_MAXNREG
 // registers (blocks of at most PAIR_THREADS threads), the general variant, in blocks
 // of up to 1024 threads, 64, the filtering launches 128.  Under launch bounds alone
@@ -38,7 +38,7 @@ static const int PAIR_THREADS_GENERAL = 1024;
 #ifndef PAIR_MAXNREG
 #define PAIR_MAXNREG 72
 #endif
-#define PAIR_BOUNDS __maxnreg__(VAR == 1 ? 64 : REFILTER ? 128 : PAIR_MAXNREG)
+#define PAIR_BOUNDS __maxnreg__(VAR != 0 ? 64 : REFILTER ? 128 : PAIR_MAXNREG)
 
 struct PairArgsF {
   TileGeom g;
@@ -86,7 +86,8 @@ __device__ __noinline__ bool refilter_exact(const PairArgsF& A, const int* lay, 
 }
 
 // VAR 0: one atom type, Lennard-Jones with modifier MOD, no Coulomb term.
-// VAR 1: any types, any pair model and modifier, Coulomb term.
+// VAR 1: any types, any pair model and modifier, Coulomb term; A.tpa threads per atom.
+// VAR 2: as VAR 0 with A.tpa threads per atom, for systems too small to fill the GPU.
 // COUNT: also count the pairs within the cut-off (statistics launches only).
 // REFILTER (VAR 0, M > 5): walk the outer lists and write the filtered lists.
 // Lists are read 8 entries (16 bytes) per lane at a time, one chunk ahead of
@@ -100,7 +101,7 @@ __global__ void PAIR_BOUNDS k_pair_mixed(PairArgsF A) {
 #ifdef EMDEE_SCALAR_PAIR   // tuning define: the scalar loop for every variant
   constexpr bool PACKED = false;
 #else
-  constexpr bool PACKED = VAR == 0 && MOD == NONE && !MINIMG && !COUNT && !REFILTER;
+  constexpr bool PACKED = VAR != 1 && MOD == NONE && !MINIMG && !COUNT && !REFILTER;
 #endif
   // the flag is 0.0 or 1.0: tested on its bits (an FP64 compare in every thread of
   // every block would queue on the slow FP64 pipe)
@@ -124,7 +125,7 @@ __global__ void PAIR_BOUNDS k_pair_mixed(PairArgsF A) {
   __syncthreads();
 
   NBParams<float> m0 = A.table[0].model;
-  if (VAR == 0) m0.modifier = MOD;
+  if (VAR != 1) m0.modifier = MOD;
   const float sigc = m0.sigsq * A.invw2, eps48 = 2.0f * m0.eps24;
   const f32x2 sigc2 = pk2(sigc, sigc), eps48_2 = pk2(eps48, eps48), meps24_2 = pk2(-m0.eps24, -m0.eps24),
               eps4_2 = pk2(m0.eps4, m0.eps4), meps4_2 = pk2(-m0.eps4, -m0.eps4);
@@ -135,7 +136,7 @@ __global__ void PAIR_BOUNDS k_pair_mixed(PairArgsF A) {
   float Ep = 0.f, Ec = 0.f, Wp = 0.f, Wc = 0.f, within = 0.f;
   // tpa consecutive threads share an atom: thread sub takes the chunks sub, sub + tpa, ...
   // and the group's partial forces are summed by shuffles in a fixed order
-  const int tpa = VAR == 1 ? A.tpa : 1, tpaShift = VAR == 1 ? A.tpaShift : 0, sub = threadIdx.x & (tpa - 1);
+  const int tpa = VAR != 0 ? A.tpa : 1, tpaShift = VAR != 0 ? A.tpaShift : 0, sub = threadIdx.x & (tpa - 1);
   const unsigned gmask = (0xFFFFFFFFu >> (32 - tpa)) << ((threadIdx.x & 31) & ~(tpa - 1));
   int longestIn = 0;   // REFILTER: longest filtered list of this thread
   for (int li = threadIdx.x >> tpaShift; li < te - tb; li += blockDim.x >> tpaShift) {
@@ -211,7 +212,7 @@ __global__ void PAIR_BOUNDS k_pair_mixed(PairArgsF A) {
           if (nIn < A.capIn) myIn[(nIn >> 3) * (A.tileStride * 8) + (nIn & 7)] = (uint16_t)qj;
           nIn++;
         }
-        if (VAR == 0) {
+        if (VAR != 1) {
           // branch-free: every entry runs the same code; entries beyond the
           // cut-off (and sentinels) are zeroed by selects, so the 8 entries of
           // a chunk form one straight-line block the compiler can interleave
@@ -308,16 +309,16 @@ static void launch(System& s, PairArgsF& A, size_t smem, int nTiles, int threads
   kern<<<nTiles, threads, smem, s.stream>>>(A);
 }
 
-template <bool COMPUTE, bool MINIMG, bool REFILTER = false>
+template <bool COMPUTE, int VAR, bool MINIMG, bool REFILTER = false>
 static void launch_lj(System& s, PairArgsF& A, size_t smem, int nt, int th, int mod) {
   switch (mod) {
-    case NONE: launch<COMPUTE, 0, NONE, MINIMG, false, REFILTER>(s, A, smem, nt, th); break;
-    case SHIFTED: launch<COMPUTE, 0, SHIFTED, MINIMG, false, REFILTER>(s, A, smem, nt, th); break;
-    case SHIFTED_FORCE: launch<COMPUTE, 0, SHIFTED_FORCE, MINIMG, false, REFILTER>(s, A, smem, nt, th); break;
-    case SMOOTHED: launch<COMPUTE, 0, SMOOTHED, MINIMG, false, REFILTER>(s, A, smem, nt, th); break;
-    case SHIFTED_SMOOTHED: launch<COMPUTE, 0, SHIFTED_SMOOTHED, MINIMG, false, REFILTER>(s, A, smem, nt, th); break;
-    case SQUARE_SMOOTHED: launch<COMPUTE, 0, SQUARE_SMOOTHED, MINIMG, false, REFILTER>(s, A, smem, nt, th); break;
-    default: launch<COMPUTE, 0, SHIFTED_SQUARE_SMOOTHED, MINIMG, false, REFILTER>(s, A, smem, nt, th); break;
+    case NONE: launch<COMPUTE, VAR, NONE, MINIMG, false, REFILTER>(s, A, smem, nt, th); break;
+    case SHIFTED: launch<COMPUTE, VAR, SHIFTED, MINIMG, false, REFILTER>(s, A, smem, nt, th); break;
+    case SHIFTED_FORCE: launch<COMPUTE, VAR, SHIFTED_FORCE, MINIMG, false, REFILTER>(s, A, smem, nt, th); break;
+    case SMOOTHED: launch<COMPUTE, VAR, SMOOTHED, MINIMG, false, REFILTER>(s, A, smem, nt, th); break;
+    case SHIFTED_SMOOTHED: launch<COMPUTE, VAR, SHIFTED_SMOOTHED, MINIMG, false, REFILTER>(s, A, smem, nt, th); break;
+    case SQUARE_SMOOTHED: launch<COMPUTE, VAR, SQUARE_SMOOTHED, MINIMG, false, REFILTER>(s, A, smem, nt, th); break;
+    default: launch<COMPUTE, VAR, SHIFTED_SQUARE_SMOOTHED, MINIMG, false, REFILTER>(s, A, smem, nt, th); break;
   }
 }
 
@@ -364,43 +365,43 @@ static size_t pair_args(System& s, bool useInRc, double rc2scaled, bool general,
   return smem;
 }
 
+// threads per atom
+static int pair_tpa(const System& s) {
+  return s.pairTpa > 0 ? s.pairTpa : split_threads(s, expected_entries(s), PAIR_THREADS_GENERAL);
+}
+
 int pair_block_threads(const System& s) {
-  return s.pairThreads > 0 ? std::min(s.pairThreads, PAIR_THREADS) : tile_threads(s.grid.tileStride, 0, PAIR_THREADS_RULE);
+  const int tpa = pair_tpa(s), least = halo_min_threads(make_geom(s.grid.M, s.grid.TB));
+  if (tpa > 1) return std::max(least, std::min(PAIR_THREADS_GENERAL, (s.grid.tileAtoms * tpa + 31) / 32 * 32));
+  return std::max(least, s.pairThreads > 0 ? std::min(s.pairThreads, PAIR_THREADS)
+                                           : tile_threads(s.grid.tileAtoms, 0, PAIR_THREADS_RULE));
 }
 
 // variant: 0 single-type Lennard-Jones without charges, 1 general, 2 pair count only
 void device_pair_forces_mixed(System& s, bool compute, bool useInRc, double rc2scaled, int variant) {
   Grid& g = s.grid;
-  const double L = *s.Lbox;
   PairArgsF A;
   const size_t smem = pair_args(s, useInRc, rc2scaled, variant != 0, A);
   const bool mi = g.M == 5;
-  // Threads per atom: systems too small to fill the GPU with one thread per atom
-  // (fewer than ~2048 threads per SM) and with long lists (more than 48 entries per
-  // thread) split each list over 2, 4 or 8 threads of a warp (general variant only,
-  // blocks of up to 1024 threads).  Threads per block: the tile's largest atom count
-  // times that, or fewer with several atoms per thread (EMDEE_PAIR_THREADS), the
-  // single-type variant in even rounds (pair_block_threads).
-  const int maxTh = variant == 0 ? PAIR_THREADS : PAIR_THREADS_GENERAL;
-  const double L3 = L * L * L, expected = s.natoms / L3 * 4.18879020478639 * s.xRcSq * s.xRc;
-  int tpa = 1, shift = 0;
-  if (variant != 0)
-    while (tpa < 8 && g.tileStride * tpa * 2 <= maxTh && (double)s.natoms * tpa * 2 <= 152.0 * 2048 &&
-           expected / (tpa * 2) >= 48) {
-      tpa *= 2;
-      shift++;
-    }
-  A.tpa = tpa;
-  A.tpaShift = shift;
+  // Threads per atom: systems too small to fill the GPU with one thread per atom split
+  // each list over 2 to 32 threads of a warp (split_threads, or the tuned count).
+  A.tpa = pair_tpa(s);
+  A.tpaShift = 0;
+  while (1 << A.tpaShift < A.tpa) A.tpaShift++;
   static const int thEnv = getenv("EMDEE_PAIR_THREADS") ? atoi(getenv("EMDEE_PAIR_THREADS")) : 0;
-  const int th = std::max(halo_min_threads(A.g), thEnv >= 32 && thEnv % 32 == 0 ? std::min(thEnv, maxTh)
-                                                 : variant == 0 ? pair_block_threads(s)
-                                                                : std::min(maxTh, std::max(32, g.tileStride * tpa)));
+  const int maxTh = variant == 0 && A.tpa == 1 ? PAIR_THREADS : PAIR_THREADS_GENERAL;
+  const int th = thEnv >= 32 && thEnv % 32 == 0 ? std::max(halo_min_threads(A.g), std::min(thEnv, maxTh))
+                                                : pair_block_threads(s);
   const int nt = g.nTiles;
   if (variant == 0) {
     const int mod = s.P(0, 0, s.layer - 1).model.p.modifier;
-    if (compute) { if (mi) launch_lj<true, true>(s, A, smem, nt, th, mod); else launch_lj<true, false>(s, A, smem, nt, th, mod); }
-    else { if (mi) launch_lj<false, true>(s, A, smem, nt, th, mod); else launch_lj<false, false>(s, A, smem, nt, th, mod); }
+    if (A.tpa == 1) {
+      if (compute) { if (mi) launch_lj<true, 0, true>(s, A, smem, nt, th, mod); else launch_lj<true, 0, false>(s, A, smem, nt, th, mod); }
+      else { if (mi) launch_lj<false, 0, true>(s, A, smem, nt, th, mod); else launch_lj<false, 0, false>(s, A, smem, nt, th, mod); }
+    } else {
+      if (compute) { if (mi) launch_lj<true, 2, true>(s, A, smem, nt, th, mod); else launch_lj<true, 2, false>(s, A, smem, nt, th, mod); }
+      else { if (mi) launch_lj<false, 2, true>(s, A, smem, nt, th, mod); else launch_lj<false, 2, false>(s, A, smem, nt, th, mod); }
+    }
   } else if (variant == 1) {
     if (compute) { if (mi) launch<true, 1, -1, true, false>(s, A, smem, nt, th); else launch<true, 1, -1, false, false>(s, A, smem, nt, th); }
     else { if (mi) launch<false, 1, -1, true, false>(s, A, smem, nt, th); else launch<false, 1, -1, false, false>(s, A, smem, nt, th); }
@@ -434,10 +435,10 @@ void device_pair_refilter(System& s, bool compute, const double* skip) {
   A.hi2In = (float)(A.thrIn * M2 * (1.0 + LIST_BAND));
   A.R = s.dR;
   A.innerMax = g.dTileInfo + 2 * g.nTiles + 4;
-  const int th = std::max(halo_min_threads(A.g), tile_threads(g.tileStride, 0, PAIR_THREADS_RULE));
+  const int th = std::max(halo_min_threads(A.g), tile_threads(g.tileAtoms, 0, PAIR_THREADS_RULE));
   const int mod = s.P(0, 0, s.layer - 1).model.p.modifier;
-  if (compute) launch_lj<true, false, true>(s, A, smem, g.nTiles, th, mod);
-  else launch_lj<false, false, true>(s, A, smem, g.nTiles, th, mod);
+  if (compute) launch_lj<true, 0, false, true>(s, A, smem, g.nTiles, th, mod);
+  else launch_lj<false, 0, false, true>(s, A, smem, g.nTiles, th, mod);
   CK(cudaGetLastError());
 }
 

@@ -129,7 +129,8 @@ struct Grid {
   int nT = 0;           // tiles per dimension
   int nTiles = 0, nRanks = 0, haloCells = 0;
   int cap = 0;          // neighbor capacity per atom
-  int tileStride = 0;   // max atoms per tile, padded to a multiple of 32
+  int tileAtoms = 0;    // max atoms per tile
+  int tileStride = 0;   // the same, padded (nb layout): a multiple of 32, or of 8 below 32
   int maxHalo = 0;      // max halo atoms over tiles
   size_t nbBytes = 0;
   int *dCount = nullptr, *dStart = nullptr, *dScanTmp = nullptr;
@@ -248,6 +249,7 @@ struct System {
   // threads per block of the list build and of the single-type pair kernel, chosen by
   // device_tune_tile with the edge (0: the rule of tile_threads)
   int buildThreads = 0, pairThreads = 0;
+  int buildTpa = 0, pairTpa = 0;   // threads per atom of both, chosen likewise (0: the rule of split_threads)
   bool tileTuned = false;   // device_tune_tile has run for this system
   double keSpecCF = 0.0, keSpec[3] = {0.0, 0.0, 0.0};
   // CF of the last deferred boost with energies: a momenta upload sums 2KE for an
@@ -318,6 +320,12 @@ void device_tune_tile(System& s, bool ljOnly, void (*pair)(System&));
 // kernel on the current lists.
 int build_block_threads(const System& s);
 int pair_block_threads(const System& s);
+// Threads per atom (a power of 2 up to 32) where the atoms alone do not fill the GPU:
+// as many as keep its threads busy and leave each at least 8 of `entries` entries, in
+// blocks of at most maxThreads threads.
+int split_threads(const System& s, double entries, int maxThreads);
+// expected list length
+double expected_entries(const System& s);
 // Two-level lists: the outer skin in effect for the system (0 = single-level lists),
 // and whether the next rebuild goes through them.
 double outer_delta(System& s);
