@@ -483,6 +483,7 @@ __device__ __forceinline__ bool excluded(const BuildArgs& A, int a, int b) {
 static const int BUILD_THREADS = 512;
 static const int BUILD_THREADS_RULE = 256;
 static const int BUILD_THREADS_SPLIT = 1024;  // split build: several threads per tile atom
+enum BuildMode : int { BUILD_ONE = 0, BUILD_SPLIT, BUILD_WARP };
 static const int BUILD_PAD = 4;               // halo entries past the last one, far away
 
 // List layout: for tile t, chunk c (8 entries) and tile-local atom li, the
@@ -504,17 +505,22 @@ __device__ __forceinline__ size_t nb_index(int t, int capC, int tileStride, int 
 // instruction issue.  1M Lennard-Jones atoms: 630 -> 535 us against candidates that went
 // through their tests and a 2-byte store one by one (L2 sectors 122 -> 26 M).
 // The list order is (row, halo index), a function of the coordinates.
-// SPLIT: A.tpa threads per atom, which take consecutive rows: a first sweep counts, the
-// group's prefix sums give each thread its output positions, a second writes (in the
+// BUILD_SPLIT: A.tpa threads per atom, which take consecutive rows: a first sweep counts,
+// the group's prefix sums give each thread its output positions, a second writes (in the
 // same order as one thread).
+// BUILD_WARP: a warp per atom, its lanes side by side over each row's candidates, the
+// accepted ones placed by ballots (the same order again): for dense cells, whose rows
+// fill the lanes (4096 water molecules, 17 atoms per cell: 262
+// us with 8 threads per atom, 130 us so).
 // GENERAL: several atom types, bodies, exclusions or layered lists; MINIMG: M = 5.
 // Register budget: thread-per-atom variants BUILD_MAXNREG, the split one, in blocks of
 // up to 1024 threads, 64.
 #ifndef BUILD_MAXNREG
 #define BUILD_MAXNREG 80
 #endif
-template <bool GENERAL, bool MINIMG, bool SPLIT>
-__global__ void __maxnreg__(SPLIT ? 64 : BUILD_MAXNREG) k_build(BuildArgs A) {
+template <bool GENERAL, bool MINIMG, int MODE>
+__global__ void __maxnreg__(MODE == BUILD_ONE ? BUILD_MAXNREG : 64) k_build(BuildArgs A) {
+  constexpr bool SPLIT = MODE == BUILD_SPLIT;
   extern __shared__ __align__(16) unsigned char sraw[];
   __shared__ int ws[33];
   const TileGeom g = A.g;
@@ -588,12 +594,15 @@ __global__ void __maxnreg__(SPLIT ? 64 : BUILD_MAXNREG) k_build(BuildArgs A) {
   const int tshift = SPLIT ? A.tpaShift : 0;
   const unsigned gmask = (0xFFFFFFFFu >> (32 - tpa)) << ((threadIdx.x & 31) & ~(tpa - 1));
   int longest = 0;
-  for (int li = threadIdx.x >> tshift; li < te - tb; li += blockDim.x >> tshift) {
+  const int li0 = MODE == BUILD_WARP ? threadIdx.x >> 5 : threadIdx.x >> tshift;
+  const int liStep = MODE == BUILD_WARP ? blockDim.x >> 5 : blockDim.x >> tshift;
+  const bool writer = MODE == BUILD_WARP ? (threadIdx.x & 31) == 0 : sub == 0;
+  for (int li = li0; li < te - tb; li += liStep) {
     const int si = tb + li;
     const int rank = A.K[si].w, lr = rank - t * cells;
     const int hcx = lr % g.TB + 2, hcy = (lr / g.TB) % g.TB + 2, hcz = lr / (g.TB * g.TB) + 2;
     const int myq = off[hcx + HW * (hcy + HW * hcz)] + (si - A.start[rank]);
-    if (sub == 0) A.selfIdx[si] = (uint16_t)myq;
+    if (writer) A.selfIdx[si] = (uint16_t)myq;
     const float4 pi = hpos[myq];
     const int ai = A.orig[si], ti = single ? 0 : A.type8[si];
     const int bi = filterByAtom && A.hasBodies ? A.body[ai] : -1;
@@ -695,7 +704,33 @@ __global__ void __maxnreg__(SPLIT ? 64 : BUILD_MAXNREG) k_build(BuildArgs A) {
       return r2 < A.loIn2 || (r2 < A.hiIn2 && exact_inside(A.R, A.L, ai, A.orig[slot_of(q)], A.thrIn));
     };
     int n = 0, nIn = 0;
-    if (!SPLIT) {
+    if (MODE == BUILD_WARP) {
+      constexpr unsigned FULL = 0xffffffffu;
+      const int lane = threadIdx.x & 31;
+      int w0 = 0, w1 = 0;   // window of row `lane`
+      if (lane < 25 && !none) window(lane / 5 - 2, lane % 5 - 2, w0, w1);
+      uint16_t* myList = A.nb + ((size_t)t * capC * A.tileStride + li) * 8;
+      for (int pass = 0; pass <= (layered ? 1 : 0); pass++) {
+        for (int r = 0; r < 25; r++) {
+          const int q1 = __shfl_sync(FULL, w1, r);
+          for (int q = __shfl_sync(FULL, w0, r) + lane; q - lane < q1; q += 32) {
+            const int d = __float_as_int(dist2(min(q, haloCount - 1))) - loBits;
+            bool acc = q < q1 && d < 0 && q != myq;
+            const bool near = q < q1 && (unsigned)d < band;
+            if (__any_sync(FULL, near) && near) acc = exact_inside(A.R, A.L, ai, A.orig[slot_of(q)], A.thr);
+            if (GENERAL && acc) acc = allowed(q) && (!layered || inside(q) == (pass == 0));
+            const unsigned m = __ballot_sync(FULL, acc);
+            const int at = n + __popc(m & ((1u << lane) - 1u));
+            if (acc && at < A.cap) myList[(at >> 3) * chunkStride + (at & 7)] = (uint16_t)q;
+            n += __popc(m);
+          }
+        }
+        if (pass == 0) nIn = n;
+      }
+      // sentinel padding of the last chunk
+      if ((n & 7) && lane < 8 - (n & 7) && n + lane < A.cap)
+        myList[((n + lane) >> 3) * chunkStride + ((n + lane) & 7)] = (uint16_t)A.haloCap;
+    } else if (MODE == BUILD_ONE) {
       // rows in the order dz = -2..2 (outer), dy = -2..2 (inner); layered lists take the
       // inner entries in a first sweep and the outer ones in a second.  The last 8 entries
       // sit in four registers until they are complete.
@@ -767,7 +802,7 @@ __global__ void __maxnreg__(SPLIT ? 64 : BUILD_MAXNREG) k_build(BuildArgs A) {
       if (sub == 0)
         for (int k = n; (k & 7) && k < A.cap; k++) put(k, A.haloCap);
     }
-    if (sub == 0) {
+    if (writer) {
       A.nbCount[si] = n;
       A.nbInner[si] = nIn;
     }
@@ -799,9 +834,13 @@ int split_threads(const System& s, double entries, int maxThreads) {
   return tpa;
 }
 
-// threads per atom of the build (its candidates are about twice the entries)
+// threads per atom of the build (its candidates are about twice the entries); 32 is the
+// warp-per-atom kernel, the rule's choice where a row of 5 cells fills the lanes
 static int build_tpa(const System& s) {
-  return s.buildTpa > 0 ? s.buildTpa : split_threads(s, 2.0 * expected_entries(s), BUILD_THREADS_SPLIT);
+  if (s.buildTpa > 0) return s.buildTpa;
+  const Grid& g = s.grid;
+  if (s.natoms >= 8.0 * g.M * g.M * g.M) return 32;
+  return std::min(16, split_threads(s, 2.0 * expected_entries(s), BUILD_THREADS_SPLIT));
 }
 
 int build_block_threads(const System& s) {
@@ -936,7 +975,7 @@ void device_tune_tile(System& s, bool ljOnly, void (*pair)(System&)) {
     for (int th = 64; th <= 512; th += th < 256 ? 32 : 64)
       if (th >= thMin && th <= std::max(thMax, 64)) shapes.push_back({1, th});
     for (int tpa = 2; tpa <= 32; tpa *= 2)
-      if ((double)s.natoms * tpa <= 152.0 * 2048 * 2 && s.grid.tileAtoms * tpa <= 1024) shapes.push_back({tpa, 0});
+      if ((double)s.natoms * tpa <= 152.0 * 2048 * 2) shapes.push_back({tpa, 0});
     double msBuild = 1e30, msPair = 1e30, ruleBuild = 0.0, rulePair = 0.0;
     TileChoice here = {tb, 0, 0, 0, 0};
     for (const auto& sh : shapes) {
@@ -1159,11 +1198,14 @@ static bool build_lists(System& s, bool reuse) {
   A.allInteract = 1;
   for (size_t q = 0; q < (size_t)s.ntypes * s.ntypes; q++)
     if (!s.interact[q]) A.allInteract = 0;
-  const bool split = A.tpa > 1;
-  auto kb = split ? (general ? (A.minimg ? k_build<true, true, true> : k_build<true, false, true>)
-                             : (A.minimg ? k_build<false, true, true> : k_build<false, false, true>))
-                  : (general ? (A.minimg ? k_build<true, true, false> : k_build<true, false, false>)
-                             : (A.minimg ? k_build<false, true, false> : k_build<false, false, false>));
+  void (*kb)(BuildArgs) = nullptr;
+#define BUILD_KERNEL(MODE)                                                             \
+  kb = general ? (A.minimg ? k_build<true, true, MODE> : k_build<true, false, MODE>)   \
+               : (A.minimg ? k_build<false, true, MODE> : k_build<false, false, MODE>)
+  if (A.tpa == 1) BUILD_KERNEL(BUILD_ONE);
+  else if (A.tpa < 32) BUILD_KERNEL(BUILD_SPLIT);
+  else BUILD_KERNEL(BUILD_WARP);
+#undef BUILD_KERNEL
   const int buildThreads = build_block_threads(s);
   CK(cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 #ifdef EMDEE_MAX_CARVEOUT
@@ -1386,6 +1428,7 @@ long device_neighbor_pairs(System& s, int* pairs, long capacity) {
   CK(cudaMalloc(&dOut, sizeof(int2) * (total + 1)));
   CK(cudaMemcpy(dSt, st.data(), sizeof(long long) * (N + 1), cudaMemcpyHostToDevice));
   TileGeom geo = make_geom(g.M, g.TB);
+  CK(cudaFuncSetAttribute(k_dump_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(int) * g.maxHalo));
   k_dump_pairs<<<g.nTiles, 128, sizeof(int) * g.maxHalo, s.stream>>>(geo, g.dHaloTab, g.dStart, g.dOrig, g.dNb,
                                                                       g.dNbCount, g.cap, g.tileStride, dSt, dOut);
   CK(cudaGetLastError());
