@@ -309,6 +309,196 @@ static void launch(System& s, PairArgsF& A, size_t smem, int nTiles, int threads
   kern<<<nTiles, threads, smem, s.stream>>>(A);
 }
 
+// Several atom types and charges in one branch-free evaluation: every type pair "none"
+// or Lennard-Jones (plain, shifted or force-shifted), the Coulomb model none or damped
+// (plain or force-shifted); k_pair_mixed<VAR 1> takes the rest.  There each entry runs
+// through the models' switches on parameters fetched field by field from its type
+// pair's record, inside a branch on the cut-off: 135 instructions per entry with 22 of
+// 32 lanes active, bound by instruction issue.  Here a type pair is one 16-byte entry
+// (zero for "none") and a Coulomb constant in shared memory, everything in units of the
+// cell edge, entries beyond the cut-off zeroed by selects: 92 -> 41 us
+// (4096 water molecules), 47 -> 24 (1000 in a box of 5 cells), 39 -> 26 (50,021 atoms of
+// two types).
+// COUL: damped Coulomb; LSHIFT / CSHIFT: the pair / Coulomb model carries shifts.
+struct __align__(16) TypePair {
+  float sig;    // sigma^2, cell units^2
+  float eps4;   // 4 epsilon
+  float fsh;    // force shift per cell edge
+  float esh;    // energy shift
+};
+
+static const int PAIR_THREADS_TYPES = 512;
+
+template <bool COMPUTE, bool COUL, bool LSHIFT, bool CSHIFT, bool MINIMG>
+__global__ void __launch_bounds__(PAIR_THREADS_TYPES) k_pair_types(PairArgsF A) {
+  if (A.skip != nullptr && __double_as_longlong(*A.skip) != 0) return;
+  extern __shared__ __align__(16) unsigned char sraw[];
+  const TileGeom g = A.g;
+  const int t = blockIdx.x, cells = g.TB * g.TB * g.TB, nt = A.ntypes, ntab = nt * nt;
+  // shared memory: the staged halo (and its sentinel), the type pairs, their Coulomb
+  // constants, the halo atoms' types
+  float4* hpos = (float4*)sraw;
+  TypePair* tbl = (TypePair*)(hpos + A.haloCap + 1);
+  float* kq = (float*)(tbl + ntab);
+  uint8_t* htype = (uint8_t*)(kq + ntab);
+  const float w = 1.0f / A.invw;
+  for (int k = threadIdx.x; k < ntab; k += blockDim.x) {
+    const PairEntry<float>& pe = A.table[k];
+    const bool lj = pe.model.kind == MK_LJ_CUT;
+    tbl[k] = TypePair{lj ? pe.model.sigsq * A.invw2 : 0.f, lj ? pe.model.eps4 : 0.f,
+                      lj && pe.model.modifier == SHIFTED_FORCE ? pe.model.fshift * w : 0.f,
+                      lj && pe.model.modifier != NONE ? pe.model.eshift : 0.f};
+    kq[k] = pe.coulomb ? pe.kCoul : 0.f;
+  }
+  if (threadIdx.x == 0) {
+    hpos[A.haloCap] = make_float4(1e9f, 1e9f, 1e9f, 0.f);
+    htype[A.haloCap] = 0;
+  }
+  const int* lay = A.layout + (size_t)t * (2 * g.haloCells + 1);
+  stage_frame_saved(g, lay, A.pos4, hpos, htype, A.type8);
+  __syncthreads();
+  float alpha = 0.f, beta = 0.f, cfsh = 0.f, cesh = 0.f;
+  if (COUL) {
+    alpha = A.coul->alpha * w;
+    beta = A.coul->beta;
+    cfsh = A.coul->fshift * w;
+    cesh = A.coul->eshift;
+  }
+  const int tb = A.start[t * cells], te = A.start[(t + 1) * cells];
+  const int capC = A.cap >> 3;
+  float Ep = 0.f, Ec = 0.f, Wp = 0.f, Wc = 0.f;
+  const int tpa = A.tpa, sub = threadIdx.x & (tpa - 1);
+  const unsigned gmask = (0xFFFFFFFFu >> (32 - tpa)) << ((threadIdx.x & 31) & ~(tpa - 1));
+  const float invM = 1.0f / A.Mf;
+  for (int li = threadIdx.x >> A.tpaShift; li < te - tb; li += blockDim.x >> A.tpaShift) {
+    const int si = tb + li;
+    const int qi = A.self[si];
+    const float4 pi = hpos[qi];
+    const TypePair* row = tbl + htype[qi] * nt;
+    const float* krow = kq + htype[qi] * nt;
+    const int n = min(A.count[si], A.cap);
+    const int nch = (n + 7) >> 3;
+    const uint4* lp = reinterpret_cast<const uint4*>(A.nb) + ((size_t)t * capC * A.tileStride + li);
+    float fx = 0.f, fy = 0.f, fz = 0.f;
+    uint4 cur = sub < nch ? __ldcs(lp + (size_t)sub * A.tileStride) : make_uint4(0u, 0u, 0u, 0u);
+    for (int c = sub; c < nch; c += tpa) {
+      const uint4 nxt = (c + tpa < nch) ? __ldcs(lp + (size_t)(c + tpa) * A.tileStride) : cur;
+      const unsigned words[4] = {cur.x, cur.y, cur.z, cur.w};
+#pragma unroll
+      for (int e = 0; e < 8; e++) {
+        const int qj = (words[e >> 1] >> ((e & 1) * 16)) & 0xFFFF;
+        const float4 pj = hpos[qj];
+        const int tj = htype[qj];
+        const TypePair p = row[tj];
+        float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+        if (MINIMG) {
+          dx -= A.Mf * rintf(dx * invM);
+          dy -= A.Mf * rintf(dy * invM);
+          dz -= A.Mf * rintf(dz * invM);
+        }
+        float r2 = dx * dx + dy * dy + dz * dz;
+        if (MINIMG && c * 8 + e >= n) r2 = 1e18f;   // the wrap of M = 5 brings the sentinel back
+        const bool in = r2 < A.rc2;
+        const float inv2 = Ops<float>::rcp(r2);
+        float rs = 0.f, r = 0.f;
+        if (COUL || LSHIFT) {
+          asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(r2));
+          r = r2 * rs;
+        }
+        // E = 4 eps (sr12 - sr6), W = 24 eps (2 sr12 - sr6)
+        const float sr2 = p.sig * inv2, sr6 = sr2 * sr2 * sr2, a = p.eps4 * sr6, a6 = 6.0f * a;
+        float W = fmaf(a6 + a6, sr6, -a6);
+        if (LSHIFT) W = fmaf(-p.fsh, r, W);
+        W = in ? W : 0.f;
+        if (COMPUTE) {
+          float E = fmaf(a, sr6, -a);
+          if (LSHIFT) E += fmaf(p.fsh, r, p.esh);
+          Ep += in ? E : 0.f;
+        }
+        Wp += W;
+        if (COUL) {
+          const float qq = in ? krow[tj] * pi.w * pj.w : 0.f;
+          const float x = alpha * r, ex = Ops<float>::ex(-x * x);
+          float Eq = uerfc(x, ex) * (rs * A.invw), Wq = fmaf(beta, ex, Eq);
+          if (CSHIFT) Wq = fmaf(-cfsh, r, Wq);
+          if (COMPUTE) {
+            if (CSHIFT) Eq += fmaf(cfsh, r, cesh);
+            Ec = fmaf(qq, Eq, Ec);
+          }
+          Wq *= qq;
+          Wc += Wq;
+          W += Wq;
+        }
+        const float s = W * inv2;
+        fx = fmaf(s, dx, fx);
+        fy = fmaf(s, dy, fy);
+        fz = fmaf(s, dz, fz);
+      }
+      cur = nxt;
+    }
+    for (int o = tpa >> 1; o > 0; o >>= 1) {
+      fx += __shfl_xor_sync(gmask, fx, o);
+      fy += __shfl_xor_sync(gmask, fy, o);
+      fz += __shfl_xor_sync(gmask, fz, o);
+    }
+    if (sub == 0) {
+      double* Fa = A.F + 3 * (size_t)A.orig[si];
+      Fa[0] = f2d_exact(fx * A.invw);
+      Fa[1] = f2d_exact(fy * A.invw);
+      Fa[2] = f2d_exact(fz * A.invw);
+    }
+  }
+  const float v[5] = {0.5f * Ep, 0.5f * Ec, 0.5f * Wp, 0.5f * Wc, 0.f};
+  constexpr unsigned MASK = (COMPUTE ? (COUL ? 3u : 1u) : 0u) | (COUL ? 12u : 4u);
+  grid_reduce_ff<5, PAIR_THREADS_TYPES, MASK>(v, reinterpret_cast<float2*>(A.partials), A.ticket, A.result,
+                                              A.hostResult);
+}
+
+template <bool COMPUTE, bool COUL, bool LSHIFT, bool CSHIFT, bool MINIMG>
+static void launch_types(System& s, PairArgsF& A, size_t smem, int nTiles, int threads) {
+  auto kern = k_pair_types<COMPUTE, COUL, LSHIFT, CSHIFT, MINIMG>;
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<nTiles, threads, smem, s.stream>>>(A);
+}
+
+template <bool COMPUTE, bool MINIMG>
+static void launch_types_sel(System& s, PairArgsF& A, size_t smem, int nt, int th, bool coul, bool lshift, bool cshift) {
+  if (!coul) {
+    if (lshift) launch_types<COMPUTE, false, true, false, MINIMG>(s, A, smem, nt, th);
+    else launch_types<COMPUTE, false, false, false, MINIMG>(s, A, smem, nt, th);
+  } else if (lshift) {
+    if (cshift) launch_types<COMPUTE, true, true, true, MINIMG>(s, A, smem, nt, th);
+    else launch_types<COMPUTE, true, true, false, MINIMG>(s, A, smem, nt, th);
+  } else {
+    if (cshift) launch_types<COMPUTE, true, false, true, MINIMG>(s, A, smem, nt, th);
+    else launch_types<COMPUTE, true, false, false, MINIMG>(s, A, smem, nt, th);
+  }
+}
+
+// Whether k_pair_types evaluates the current layer's models, and which shifts they carry.
+static bool types_kernel_applies(System& s, double rc, bool& coul, bool& lshift, bool& cshift) {
+  const int l = s.layer - 1;
+  lshift = false;
+  bool charges = false;
+  for (int j = 0; j < s.ntypes; j++)
+    for (int i = 0; i < s.ntypes; i++) {
+      const PairHost& p = s.P(i, j, l);
+      charges |= p.coulomb != 0;
+      if (p.model.kind == MK_PAIR_NONE) continue;
+      const int mod = p.model.p.modifier;
+      if (p.model.kind != MK_LJ_CUT || !(mod == NONE || mod == SHIFTED || mod == SHIFTED_FORCE)) return false;
+      lshift |= mod != NONE;
+    }
+  const Model& c = s.coul[l];
+  coul = charges && c.kind != MK_COUL_NONE;
+  cshift = coul && c.p.modifier != NONE;
+  if (!coul) return true;
+  // damped_smoothed whose switch begins at the cut-off is the damped model
+  if (!(c.kind == MK_COUL_DAMPED || c.kind == MK_COUL_LONG || (c.kind == MK_COUL_DAMPED_SMOOTHED && c.p.Rm >= rc)))
+    return false;
+  return c.p.modifier == NONE || c.p.modifier == SHIFTED || c.p.modifier == SHIFTED_FORCE;
+}
+
 template <bool COMPUTE, int VAR, bool MINIMG, bool REFILTER = false>
 static void launch_lj(System& s, PairArgsF& A, size_t smem, int nt, int th, int mod) {
   switch (mod) {
@@ -402,6 +592,11 @@ void device_pair_forces_mixed(System& s, bool compute, bool useInRc, double rc2s
       if (compute) { if (mi) launch_lj<true, 2, true>(s, A, smem, nt, th, mod); else launch_lj<true, 2, false>(s, A, smem, nt, th, mod); }
       else { if (mi) launch_lj<false, 2, true>(s, A, smem, nt, th, mod); else launch_lj<false, 2, false>(s, A, smem, nt, th, mod); }
     }
+  } else if (bool coul, lshift, cshift;
+             variant == 1 && types_kernel_applies(s, useInRc ? s.InRc : s.Rc, coul, lshift, cshift)) {
+    const int tt = std::min(th, PAIR_THREADS_TYPES);
+    if (compute) { if (mi) launch_types_sel<true, true>(s, A, smem, nt, tt, coul, lshift, cshift); else launch_types_sel<true, false>(s, A, smem, nt, tt, coul, lshift, cshift); }
+    else { if (mi) launch_types_sel<false, true>(s, A, smem, nt, tt, coul, lshift, cshift); else launch_types_sel<false, false>(s, A, smem, nt, tt, coul, lshift, cshift); }
   } else if (variant == 1) {
     if (compute) { if (mi) launch<true, 1, -1, true, false>(s, A, smem, nt, th); else launch<true, 1, -1, false, false>(s, A, smem, nt, th); }
     else { if (mi) launch<false, 1, -1, true, false>(s, A, smem, nt, th); else launch<false, 1, -1, false, false>(s, A, smem, nt, th); }
