@@ -9,8 +9,9 @@
 //   (32 -> 64 -> 64 -> 1), E = sum_i E_i,  F = -dE/dR.
 // Kernels (one launch each, over all chains at once):
 //   k_sg_pack      FP64 positions -> FP32, wrapped into the box
-//   k_sg_list      Verlet lists within rc + skin from a cell list (per chain)
-//   k_sg_desc      descriptors, Gaussians by the two-term product recurrence
+//   k_sg_list      Verlet lists within rc + skin from a cell list (per chain), a block
+//                  per cell
+//   k_sg_desc      descriptors, a warp per atom, Gaussians by the two-term product recurrence
 //   k_sg_mlp       per-species tiles of 64 atoms: forward and backward through the
 //                  network on the tensor cores (mma.sync m16n8k16, BF16 operands,
 //                  FP32 accumulation): E_i and dE/dG_i
@@ -195,77 +196,128 @@ __global__ void k_sg_scatter(const int* __restrict__ cellOf, Geometry G, const i
   sorted[starts[r] + atomicAdd(&cursor[r], 1)] = q;
 }
 
-// deterministic order inside a cell
+// Deterministic order inside a cell (ascending atom index): a warp per cell, each atom's
+// place is the number of atoms of the cell with a smaller index.  Cells of more than
+// 32 * SORT_REGS atoms are sorted by lane 0.  (8 x 8000 atoms in cells of 64: one thread
+// per cell took 343 us, 8 us so.)
+constexpr int SORT_REGS = 8;
 __global__ void k_sg_sort(const int* __restrict__ starts, int n, int* __restrict__ sorted) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= n) return;
-  const int b = starts[r], e = starts[r + 1];
-  for (int i = b + 1; i < e; i++) {
-    const int v = sorted[i];
-    int j = i - 1;
-    while (j >= b && sorted[j] > v) {
-      sorted[j + 1] = sorted[j];
-      j--;
-    }
-    sorted[j + 1] = v;
+  const int b = starts[r], m = starts[r + 1] - b;
+  if (m <= 1) return;
+  if (m > 32 * SORT_REGS) {
+    if (lane == 0)
+      for (int i = b + 1; i < b + m; i++) {
+        const int v = sorted[i];
+        int j = i - 1;
+        while (j >= b && sorted[j] > v) {
+          sorted[j + 1] = sorted[j];
+          j--;
+        }
+        sorted[j + 1] = v;
+      }
+    return;
   }
+  int v[SORT_REGS], place[SORT_REGS];
+#pragma unroll
+  for (int u = 0; u < SORT_REGS; u++) {
+    v[u] = 32 * u + lane < m ? sorted[b + 32 * u + lane] : 0;
+    place[u] = 0;
+  }
+#pragma unroll
+  for (int w = 0; w < SORT_REGS; w++) {
+    if (32 * w >= m) break;
+    for (int k = 0; k < min(32, m - 32 * w); k++) {
+      const int x = __shfl_sync(0xffffffffu, v[w], k);
+#pragma unroll
+      for (int u = 0; u < SORT_REGS; u++) place[u] += x < v[u] ? 1 : 0;
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < SORT_REGS; u++)
+    if (32 * u + lane < m) sorted[b + place[u]] = v[u];
 }
 
-// Verlet lists (global atom indices), entry k of atom q at list[k * total + q]
-__global__ void k_sg_list(const float4* __restrict__ pos, Geometry G, const int* __restrict__ cellOf,
-                          const int* __restrict__ starts, const int* __restrict__ sorted, int cap,
-                          int* __restrict__ list, int* __restrict__ count, int* __restrict__ overflow) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  const int total = G.chains * G.N;
-  if (q >= total) return;
-  const int c = q / G.N, M = G.M, cell = cellOf[q];
-  const int cx = cell % M, cy = (cell / M) % M, cz = cell / (M * M);
-  const float4 p = pos[q];
-  int n = 0;
-  const int span = M >= 3 ? 1 : 0;   // M < 3: every cell is a neighbor cell once
-  for (int dz = -span; dz <= span; dz++)
-    for (int dy = -span; dy <= span; dy++)
-      for (int dx = -span; dx <= span; dx++) {
-        if (M < 3 && (dx || dy || dz)) continue;
-        const int nc = ((cx + dx + M) % M) + M * (((cy + dy + M) % M) + M * ((cz + dz + M) % M));
-        const int r = c * M * M * M + nc;
-        const int b0 = M < 3 ? c * M * M * M : r, b1 = M < 3 ? (c + 1) * M * M * M : r + 1;
-        for (int k = starts[b0]; k < starts[b1]; k++) {
-          const int j = sorted[k];
-          if (j == q) continue;
-          const float4 pj = pos[j];
-          float ex = p.x - pj.x, ey = p.y - pj.y, ez = p.z - pj.z;
-          ex -= G.L * rintf(ex * G.invL);
-          ey -= G.L * rintf(ey * G.invL);
-          ez -= G.L * rintf(ez * G.invL);
-          if (ex * ex + ey * ey + ez * ez < G.rlist2) {
-            if (n < cap) list[(size_t)n * total + q] = j;
-            n++;
-          }
-        }
+// Verlet lists (global atom indices), entry e of atom q at list[q * cap + e], in the order
+// of the neighbor cells and of their atoms.  A block per cell stages the candidates of
+// its atoms (27 cells, or with M < 3 the whole chain) in shared memory; a warp per atom
+// goes through them side by side and places the accepted ones by ballots.  More than
+// LIST_CAND candidates are taken in several stages.  (One thread per atom, gathering
+// each candidate's index and position: 428 us at 8 x 8000 atoms; 193 us so.)
+constexpr int LIST_CAND = 2048, LIST_THREADS = 256;
+__global__ void __launch_bounds__(LIST_THREADS) k_sg_list(const float4* __restrict__ pos, Geometry G,
+                                                          const int* __restrict__ starts,
+                                                          const int* __restrict__ sorted, int cap,
+                                                          int* __restrict__ list, int* __restrict__ count,
+                                                          int* __restrict__ overflow) {
+  __shared__ float cx[LIST_CAND], cy[LIST_CAND], cz[LIST_CAND];
+  __shared__ int cj[LIST_CAND];
+  __shared__ int first[28], base[28];   // candidates of the neighbor cells: first slot, running count
+  const int M = G.M, cells = M * M * M, chain = blockIdx.x / cells, cell = blockIdx.x % cells;
+  const int x = cell % M, y = (cell / M) % M, z = cell / (M * M);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int own0 = starts[blockIdx.x], own1 = starts[blockIdx.x + 1];
+  if (own0 == own1) return;
+  const int ncell = M >= 3 ? 27 : 1;   // M < 3: every cell of the chain once
+  if (threadIdx.x < ncell) {
+    const int k = threadIdx.x, dx = k % 3 - 1, dy = k / 3 % 3 - 1, dz = k / 9 - 1;
+    const int r = M >= 3 ? chain * cells + (x + dx + M) % M + M * ((y + dy + M) % M + M * ((z + dz + M) % M))
+                         : chain * cells;
+    first[k] = starts[r];
+    base[k + 1] = M >= 3 ? starts[r + 1] - starts[r] : starts[(chain + 1) * cells] - starts[chain * cells];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    base[0] = 0;
+    for (int k = 0; k < ncell; k++) base[k + 1] += base[k];
+  }
+  __syncthreads();
+  const int total = base[ncell];
+  int longest = 0;
+  for (int c0 = 0; c0 < total; c0 += LIST_CAND) {
+    const int nc = min(LIST_CAND, total - c0);
+    if (c0 > 0) __syncthreads();
+    for (int c = threadIdx.x; c < nc; c += LIST_THREADS) {
+      int k = 0;
+      while (base[k + 1] <= c0 + c) k++;
+      const int j = sorted[first[k] + (c0 + c - base[k])];
+      const float4 p = pos[j];
+      cj[c] = j;
+      cx[c] = p.x;
+      cy[c] = p.y;
+      cz[c] = p.z;
+    }
+    __syncthreads();
+    for (int o = own0 + warp; o < own1; o += LIST_THREADS / 32) {
+      const int q = sorted[o];
+      const float4 p = pos[q];
+      int* out = list + (size_t)q * cap;
+      int n = c0 > 0 ? count[q] : 0;
+      for (int c = lane; c - lane < nc; c += 32) {
+        const int cc = min(c, nc - 1), j = cj[cc];
+        float ex = p.x - cx[cc], ey = p.y - cy[cc], ez = p.z - cz[cc];
+        ex -= G.L * rintf(ex * G.invL);
+        ey -= G.L * rintf(ey * G.invL);
+        ez -= G.L * rintf(ez * G.invL);
+        const bool in = c < nc && j != q && ex * ex + ey * ey + ez * ez < G.rlist2;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        const int at = n + __popc(m & ((1u << lane) - 1u));
+        if (in && at < cap) out[at] = j;
+        n += __popc(m);
       }
-  count[q] = n;
-  if (n > cap) atomicMax(overflow, n);
+      if (lane == 0) count[q] = n;
+      __syncwarp();
+      longest = max(longest, n);
+    }
+  }
+  if (lane == 0 && longest > cap) atomicMax(overflow, longest);
 }
 
 struct PairGeom {
   float r, ux, uy, uz;   // distance and unit vector (i - j) / r
 };
-
-__device__ __forceinline__ bool pair_geom(const float4& pi, const float4& pj, const Geometry& G, PairGeom& pg) {
-  float ex = pi.x - pj.x, ey = pi.y - pj.y, ez = pi.z - pj.z;
-  ex -= G.L * rintf(ex * G.invL);
-  ey -= G.L * rintf(ey * G.invL);
-  ez -= G.L * rintf(ez * G.invL);
-  const float r2 = ex * ex + ey * ey + ez * ez;
-  if (!(r2 < G.rc2)) return false;
-  const float r = sqrtf(r2), inv = 1.f / r;
-  pg.r = r;
-  pg.ux = ex * inv;
-  pg.uy = ey * inv;
-  pg.uz = ez * inv;
-  return true;
-}
 
 // h_k = g_k fc and dh_k/dr for the 16 Gaussians (two-term product recurrence:
 // g_{k+1} = g_k q_k, q_{k+1} = q_k c, c = exp(-2 a dmu^2))
@@ -286,115 +338,184 @@ __device__ __forceinline__ void radial(float r, const Geometry& G, float cdecay,
   }
 }
 
-__global__ void k_sg_desc(const float4* __restrict__ pos, Geometry G, const uint8_t* __restrict__ species,
-                          const int* __restrict__ list, const int* __restrict__ count, int cap,
-                          float* __restrict__ Gout) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  const int total = G.chains * G.N;
-  if (q >= total) return;
-  const float cdecay = __expf(-2.f * G.a * G.dmu * G.dmu);
-  float acc[NS][NG];
-#pragma unroll
-  for (int c = 0; c < NS; c++)
-#pragma unroll
-    for (int k = 0; k < NG; k++) acc[c][k] = 0.f;
+// The descriptor and adjoint kernels run a warp per atom.  The entries of the Verlet
+// list (rc + skin) are tested 32 at a time and those within rc (43 % at rc 2.5, skin 0.8)
+// gathered, in list order, in the warp's buffer; each full batch of 32 goes to
+// batch(n, d, j): lane k < n holds neighbor k, d = (displacement, squared distance).  So
+// the costly radial functions run on full warps; one thread per atom ran them for a
+// warp whenever any lane's entry was within rc, on 3 warps per scheduler.
+constexpr int WARP_ATOMS = 8;   // warps (atoms) per block
+struct NeighborBuffer {
+  float4 d[64];
+  int j[64];
+};
+
+template <class F>
+__device__ __forceinline__ void for_neighbors(const float4* __restrict__ pos, const Geometry& G, int q, const int* list,
+                                              int n, NeighborBuffer& B, F&& batch) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
   const float4 pi = pos[q];
-  const int n = min(count[q], cap);
-  for (int e = 0; e < n; e++) {
-    const int j = list[(size_t)e * total + q];
-    PairGeom pg;
-    if (!pair_geom(pi, pos[j], G, pg)) continue;
-    float h[NG], dh[NG];
-    radial(pg.r, G, cdecay, h, dh);
-    if (species[j % G.N] == 0) {
-#pragma unroll
-      for (int k = 0; k < NG; k++) acc[0][k] += h[k];
-    } else {
-#pragma unroll
-      for (int k = 0; k < NG; k++) acc[1][k] += h[k];
+  int have = 0;
+  for (int e = lane; e - lane < n; e += 32) {
+    const int j = e < n ? list[e] : q;
+    const float4 pj = pos[j];
+    float ex = pi.x - pj.x, ey = pi.y - pj.y, ez = pi.z - pj.z;
+    ex -= G.L * rintf(ex * G.invL);
+    ey -= G.L * rintf(ey * G.invL);
+    ez -= G.L * rintf(ez * G.invL);
+    const float r2 = ex * ex + ey * ey + ez * ez;
+    const bool in = e < n && r2 < G.rc2;
+    const unsigned m = __ballot_sync(FULL, in);
+    const int at = have + __popc(m & ((1u << lane) - 1u));
+    if (in) {
+      B.d[at] = make_float4(ex, ey, ez, r2);
+      B.j[at] = j;
+    }
+    have += __popc(m);
+    __syncwarp();
+    if (have >= 32) {
+      batch(32, B.d[lane], B.j[lane]);
+      have -= 32;
+      float4 d;
+      int k = 0;
+      if (lane < have) {
+        d = B.d[32 + lane];
+        k = B.j[32 + lane];
+      }
+      __syncwarp();
+      if (lane < have) {
+        B.d[lane] = d;
+        B.j[lane] = k;
+      }
+      __syncwarp();
     }
   }
-  float4* out = reinterpret_cast<float4*>(Gout + (size_t)q * DIN);
-#pragma unroll
-  for (int c = 0; c < NS; c++)
-#pragma unroll
-    for (int k = 0; k < NG; k += 4) out[(c * NG + k) / 4] = make_float4(acc[c][k], acc[c][k + 1], acc[c][k + 2], acc[c][k + 3]);
+  if (have > 0) batch(have, lane < have ? B.d[lane] : make_float4(1.f, 1.f, 1.f, 3.f), lane < have ? B.j[lane] : q);
 }
 
-// F_i = -sum_j s_ij r_hat_ij, s_ij = sum_k (dEdG_i[s_j, k] + dEdG_j[s_i, k]) dh_k(r_ij)
-__global__ void k_sg_force(const float4* __restrict__ pos, Geometry G, const uint8_t* __restrict__ species,
-                           const int* __restrict__ list, const int* __restrict__ count, int cap,
-                           const float* __restrict__ dEdG, double* __restrict__ F) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  const int total = G.chains * G.N;
-  if (q >= total) return;
+__device__ __forceinline__ PairGeom unit_vector(const float4& d) {
+  const float r = sqrtf(d.w), inv = 1.f / r;
+  return PairGeom{r, d.x * inv, d.y * inv, d.z * inv};
+}
+
+// Sums of the batch's terms per (species, Gaussian): lane 16 c + k adds the terms of the
+// neighbors of species c in list order.  H: row per neighbor, an odd stride.
+constexpr int HROW = NG + 1;
+
+// 8 x 8000 atoms: 195 us with one thread per atom, 86 us so.
+__global__ void __launch_bounds__(32 * WARP_ATOMS) k_sg_desc(const float4* __restrict__ pos, Geometry G,
+                                                             const uint8_t* __restrict__ species,
+                                                             const int* __restrict__ list,
+                                                             const int* __restrict__ count, int cap,
+                                                             float* __restrict__ Gout) {
+  __shared__ NeighborBuffer nbuf[WARP_ATOMS];
+  __shared__ float hbuf[WARP_ATOMS][32 * HROW];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * WARP_ATOMS + warp;
+  if (q >= G.chains * G.N) return;
   const float cdecay = __expf(-2.f * G.a * G.dmu * G.dmu);
-  const int si = species[q % G.N];
-  const float4 pi = pos[q];
+  float* H = hbuf[warp];
+  const int k = lane & (NG - 1), chain0 = q - q % G.N;   // first atom of the chain
+  const unsigned flip = lane < NG ? 0xffffffffu : 0u;   // species 0 in the lower lanes
+  float acc = 0.f;
+  for_neighbors(pos, G, q, list + (size_t)q * cap, min(count[q], cap), nbuf[warp], [&](int n, float4 d, int j) {
+    float h[NG], dh[NG];
+    radial(sqrtf(d.w), G, cdecay, h, dh);
+#pragma unroll
+    for (int u = 0; u < NG; u++) H[lane * HROW + u] = h[u];
+    const unsigned mine = (__ballot_sync(0xffffffffu, species[j - chain0] != 0) ^ flip) & (0xffffffffu >> (32 - n));
+    __syncwarp();
+    for (int b = 0; b < n; b += 8)
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const float x = H[(b + u) * HROW + k];
+        acc += (mine >> (b + u)) & 1u ? x : 0.f;
+      }
+    __syncwarp();
+  });
+  Gout[(size_t)q * DIN + lane] = acc;
+}
+
+// F_i = -sum_j s_ij r_hat_ij, s_ij = sum_k (dEdG_i[s_j, k] + dEdG_j[s_i, k]) dh_k(r_ij).
+// 8 x 8000 atoms: 293 us with one thread per atom, 164 us so.
+__global__ void __launch_bounds__(32 * WARP_ATOMS) k_sg_force(const float4* __restrict__ pos, Geometry G,
+                                                              const uint8_t* __restrict__ species,
+                                                              const int* __restrict__ list,
+                                                              const int* __restrict__ count, int cap,
+                                                              const float* __restrict__ dEdG,
+                                                              double* __restrict__ F) {
+  __shared__ NeighborBuffer nbuf[WARP_ATOMS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * WARP_ATOMS + warp;
+  if (q >= G.chains * G.N) return;
+  const float cdecay = __expf(-2.f * G.a * G.dmu * G.dmu);
+  const int chain0 = q - q % G.N, si = species[q - chain0];   // first atom of the chain
   const float* gi = dEdG + (size_t)q * DIN;
-  const int n = min(count[q], cap);
   float fx = 0.f, fy = 0.f, fz = 0.f;
-  for (int e = 0; e < n; e++) {
-    const int j = list[(size_t)e * total + q];
-    PairGeom pg;
-    if (!pair_geom(pi, pos[j], G, pg)) continue;
-    float h[NG], dh[NG];
-    radial(pg.r, G, cdecay, h, dh);
-    const int sj = species[j % G.N];
-    const float4* a = reinterpret_cast<const float4*>(gi + sj * NG);
-    const float4* b = reinterpret_cast<const float4*>(dEdG + (size_t)j * DIN + si * NG);
-    float s = 0.f;
+  for_neighbors(pos, G, q, list + (size_t)q * cap, min(count[q], cap), nbuf[warp], [&](int n, float4 d, int j) {
+    if (lane < n) {
+      const PairGeom pg = unit_vector(d);
+      float h[NG], dh[NG];
+      radial(pg.r, G, cdecay, h, dh);
+      const float4* a = reinterpret_cast<const float4*>(gi + species[j - chain0] * NG);
+      const float4* b = reinterpret_cast<const float4*>(dEdG + (size_t)j * DIN + si * NG);
+      float s = 0.f;
 #pragma unroll
-    for (int k4 = 0; k4 < NG / 4; k4++) {
-      const float4 x = a[k4], y = __ldg(&b[k4]);
-      s += (x.x + y.x) * dh[4 * k4] + (x.y + y.y) * dh[4 * k4 + 1] + (x.z + y.z) * dh[4 * k4 + 2] +
-           (x.w + y.w) * dh[4 * k4 + 3];
+      for (int k4 = 0; k4 < NG / 4; k4++) {
+        const float4 x = __ldg(&a[k4]), y = __ldg(&b[k4]);
+        s += (x.x + y.x) * dh[4 * k4] + (x.y + y.y) * dh[4 * k4 + 1] + (x.z + y.z) * dh[4 * k4 + 2] +
+             (x.w + y.w) * dh[4 * k4 + 3];
+      }
+      fx -= s * pg.ux;
+      fy -= s * pg.uy;
+      fz -= s * pg.uz;
     }
-    fx -= s * pg.ux;
-    fy -= s * pg.uy;
-    fz -= s * pg.uz;
+    __syncwarp();
+  });
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    fx += __shfl_xor_sync(0xffffffffu, fx, o);
+    fy += __shfl_xor_sync(0xffffffffu, fy, o);
+    fz += __shfl_xor_sync(0xffffffffu, fz, o);
   }
-  F[3 * q] = fx;
-  F[3 * q + 1] = fy;
-  F[3 * q + 2] = fz;
+  if (lane < 3) F[3 * (size_t)q + lane] = lane == 0 ? fx : lane == 1 ? fy : fz;
 }
 
-// u_i[s_j, k] = sum_j dh_k(r_ij) (v_i - v_j) . r_hat_ij (force residual in descriptor space)
-__global__ void k_sg_udesc(const float4* __restrict__ pos, Geometry G, const uint8_t* __restrict__ species,
-                           const int* __restrict__ list, const int* __restrict__ count, int cap,
-                           const float* __restrict__ v, float* __restrict__ U) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  const int total = G.chains * G.N;
-  if (q >= total) return;
+// u_i[s_j, k] = sum_j dh_k(r_ij) (v_i - v_j) . r_hat_ij (force residual in descriptor space).
+// 8 x 8000 atoms: 248 us with one thread per atom, 146 us so.
+__global__ void __launch_bounds__(32 * WARP_ATOMS) k_sg_udesc(const float4* __restrict__ pos, Geometry G,
+                                                              const uint8_t* __restrict__ species,
+                                                              const int* __restrict__ list,
+                                                              const int* __restrict__ count, int cap,
+                                                              const float* __restrict__ v, float* __restrict__ U) {
+  __shared__ NeighborBuffer nbuf[WARP_ATOMS];
+  __shared__ float hbuf[WARP_ATOMS][32 * HROW];
+  __shared__ float wbuf[WARP_ATOMS][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * WARP_ATOMS + warp;
+  if (q >= G.chains * G.N) return;
   const float cdecay = __expf(-2.f * G.a * G.dmu * G.dmu);
-  float acc[NS][NG];
-#pragma unroll
-  for (int c = 0; c < NS; c++)
-#pragma unroll
-    for (int k = 0; k < NG; k++) acc[c][k] = 0.f;
-  const float4 pi = pos[q];
+  float* H = hbuf[warp];
+  const int k = lane & (NG - 1), chain0 = q - q % G.N;   // first atom of the chain
+  const unsigned flip = lane < NG ? 0xffffffffu : 0u;   // species 0 in the lower lanes
   const float vix = v[3 * q], viy = v[3 * q + 1], viz = v[3 * q + 2];
-  const int n = min(count[q], cap);
-  for (int e = 0; e < n; e++) {
-    const int j = list[(size_t)e * total + q];
-    PairGeom pg;
-    if (!pair_geom(pi, pos[j], G, pg)) continue;
+  float acc = 0.f;
+  for_neighbors(pos, G, q, list + (size_t)q * cap, min(count[q], cap), nbuf[warp], [&](int n, float4 d, int j) {
+    const PairGeom pg = unit_vector(d);
     float h[NG], dh[NG];
     radial(pg.r, G, cdecay, h, dh);
-    const float w = (vix - v[3 * j]) * pg.ux + (viy - v[3 * j + 1]) * pg.uy + (viz - v[3 * j + 2]) * pg.uz;
-    if (species[j % G.N] == 0) {
 #pragma unroll
-      for (int k = 0; k < NG; k++) acc[0][k] += dh[k] * w;
-    } else {
+    for (int u = 0; u < NG; u++) H[lane * HROW + u] = dh[u];
+    wbuf[warp][lane] = (vix - v[3 * j]) * pg.ux + (viy - v[3 * j + 1]) * pg.uy + (viz - v[3 * j + 2]) * pg.uz;
+    const unsigned mine = (__ballot_sync(0xffffffffu, species[j - chain0] != 0) ^ flip) & (0xffffffffu >> (32 - n));
+    __syncwarp();
+    for (int b = 0; b < n; b += 8)
 #pragma unroll
-      for (int k = 0; k < NG; k++) acc[1][k] += dh[k] * w;
-    }
-  }
-  float* out = U + (size_t)q * DIN;
-#pragma unroll
-  for (int c = 0; c < NS; c++)
-#pragma unroll
-    for (int k = 0; k < NG; k++) out[c * NG + k] = acc[c][k];
+      for (int u = 0; u < 8; u++) {
+        const float x = fmaf(H[(b + u) * HROW + k], wbuf[warp][b + u], acc);
+        acc = (mine >> (b + u)) & 1u ? x : acc;
+      }
+    __syncwarp();
+  });
+  U[(size_t)q * DIN + lane] = acc;
 }
 
 // ---- network: inference -----------------------------------------------------------
@@ -775,19 +896,39 @@ struct TrainSmem {
   __nv_bfloat16 gz1[2 * TILE][H + 8];        // rows: gz1 (64), gdz1 (64)
   __nv_bfloat16 tA[H][2 * TILE + 8];         // transposed operands of the weight GEMMs
   __nv_bfloat16 tB[H][2 * TILE + 8];
-  float vb1[H], vb2[H], vw3[H], vb3;
+  float vb1[4][H], vb2[4][H], vw3[4][H], vb3[4];   // per warp
 };
 
-// one launch per species; block b processes tiles b, b + gridDim.x, ... of that species and
-// writes its gradient partial (PER_SPECIES floats) to part[b]
-__global__ void __launch_bounds__(128) k_sg_train(TileArgs T, int species, const float* __restrict__ params,
+// Sums over the rows of a warp's fragments (rows g and g + 8 in slots q = 0, 1 and 2, 3):
+// x[n][j] is this lane's sum for column 8 n + 2 t + j; lanes of equal t are added and
+// the total goes to out[column].
+__device__ __forceinline__ void column_sums(float (&x)[8][2], float* out) {
+#pragma unroll
+  for (int n = 0; n < 8; n++)
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) x[n][j] += __shfl_xor_sync(0xffffffffu, x[n][j], o);
+      if ((threadIdx.x & 31) < 4) out[frag_col(n, j)] += x[n][j];
+    }
+}
+
+// Both species in one launch: blocks 0 .. nb0 - 1 process the tiles of species 0 (the
+// first nt0 of T), the others those of species 1; each writes its gradient partial
+// (PER_SPECIES floats) to part[b].  Bias and output-layer gradients are summed by
+// shuffles per warp (shared-memory atomics, eight lanes to an address, were most of
+// 2 x 419 us at 8 x 8000 atoms; 173 us so).
+__global__ void __launch_bounds__(128) k_sg_train(TileArgs T, int nt0, int nb0, const float* __restrict__ params,
                                                   const float* __restrict__ Gin, const float* __restrict__ Uin,
                                                   const float* __restrict__ eAtom, float* __restrict__ part) {
   extern __shared__ __align__(16) unsigned char raw[];
   TrainSmem& S = *reinterpret_cast<TrainSmem*>(raw);
+  const int species = (int)blockIdx.x < nb0 ? 0 : 1;
+  const int t0 = species == 0 ? blockIdx.x : nt0 + blockIdx.x - nb0, t1 = species == 0 ? nt0 : T.ntiles,
+            tstep = species == 0 ? nb0 : gridDim.x - nb0;
   load_weights(S.w, params + species * PER_SPECIES);
-  for (int q = threadIdx.x; q < H; q += blockDim.x) S.vb1[q] = S.vb2[q] = S.vw3[q] = 0.f;
-  if (threadIdx.x == 0) S.vb3 = 0.f;
+  for (int q = threadIdx.x; q < 4 * H; q += blockDim.x) (&S.vb1[0][0])[q] = (&S.vb2[0][0])[q] = (&S.vw3[0][0])[q] = 0.f;
+  if (threadIdx.x < 4) S.vb3[threadIdx.x] = 0.f;
   __syncthreads();
   const WeightsSmem& W = S.w;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -796,9 +937,8 @@ __global__ void __launch_bounds__(128) k_sg_train(TileArgs T, int species, const
   float gW2[8][4], gW1[4][4];
   zero(gW2);
   zero(gW1);
-  for (int ti = blockIdx.x; ti < T.ntiles; ti += gridDim.x) {
+  for (int ti = t0; ti < t1; ti += tstep) {
     const int3 tile = T.tiles[ti];
-    if (tile.z != species) continue;
     const int r0 = warp * 16;   // this warp's rows in the tile
     const int nrow = max(0, min(16, tile.y - r0));
     // inputs: G and U rows (zero rows beyond the tile)
@@ -837,9 +977,10 @@ __global__ void __launch_bounds__(128) k_sg_train(TileArgs T, int species, const
       e[0] = g < nrow ? eAtom[T.atoms[tile.x + r0 + g]] : 0.f;
       e[1] = g + 8 < nrow ? eAtom[T.atoms[tile.x + r0 + g + 8]] : 0.f;
     }
-    float lb3 = 0.f;
+    float lb3 = 0.f, sb2[8][2], sw3[8][2];
 #pragma unroll
-    for (int n = 0; n < 8; n++)
+    for (int n = 0; n < 8; n++) {
+      sb2[n][0] = sb2[n][1] = sw3[n][0] = sw3[n][1] = 0.f;
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         const int r = frag_row(q), c = frag_col(n, q);
@@ -850,20 +991,27 @@ __global__ void __launch_bounds__(128) k_sg_train(TileArgs T, int species, const
         S.gz2[r0 + r][c] = __float2bfloat16(ok ? g2 : 0.f);
         S.gz2[TILE + r0 + r][c] = __float2bfloat16(ok ? gd2 : 0.f);
         if (ok) {
-          atomicAdd(&S.vb2[c], g2);
-          atomicAdd(&S.vw3[c], ec * silu(z) - s1 * dz2[n][q]);
+          sb2[n][q & 1] += g2;
+          sw3[n][q & 1] += ec * silu(z) - s1 * dz2[n][q];
         }
         if (ok && n == 0 && (q & 1) == 0 && (threadIdx.x & 3) == 0) lb3 += ec;
       }
-    if (lb3 != 0.f) atomicAdd(&S.vb3, lb3);
+    }
+    column_sums(sb2, S.vb2[warp]);
+    column_sums(sw3, S.vw3[warp]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) lb3 += __shfl_xor_sync(0xffffffffu, lb3, o);
+    if (lane == 0) S.vb3[warp] += lb3;
     __syncwarp();
     float p1[8][4], p2[8][4];
     zero(p1);
     zero(p2);
     warp_gemm<H, 8>(&S.gz2[r0][0], H + 8, &W.W2[0][0], H + 8, p1);          // gz2 W2^T
     warp_gemm<H, 8>(&S.gz2[TILE + r0][0], H + 8, &W.W2[0][0], H + 8, p2);   // gdz2 W2^T
+    float sb1[8][2];
 #pragma unroll
-    for (int n = 0; n < 8; n++)
+    for (int n = 0; n < 8; n++) {
+      sb1[n][0] = sb1[n][1] = 0.f;
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         const int r = frag_row(q), c = frag_col(n, q);
@@ -872,8 +1020,10 @@ __global__ void __launch_bounds__(128) k_sg_train(TileArgs T, int species, const
         const float g1 = p1[n][q] * s1 + p2[n][q] * dz1[n][q] * s2, gd1 = p2[n][q] * s1;
         S.gz1[r0 + r][c] = __float2bfloat16(ok ? g1 : 0.f);
         S.gz1[TILE + r0 + r][c] = __float2bfloat16(ok ? gd1 : 0.f);
-        if (ok) atomicAdd(&S.vb1[c], g1);
+        if (ok) sb1[n][q & 1] += g1;
       }
+    }
+    column_sums(sb1, S.vb1[warp]);
     __syncthreads();
     // dW2 += [a1; da1]^T [gz2; gdz2]: A = tA (64 units x 128 atoms), B^T = tB (64 units x 128 atoms)
     for (int q = threadIdx.x; q < 2 * TILE * H; q += blockDim.x) {
@@ -907,20 +1057,55 @@ __global__ void __launch_bounds__(128) k_sg_train(TileArgs T, int species, const
       out[OFF_W1 + (16 * (warp & 1) + frag_row(q)) * H + 32 * (warp >> 1) + frag_col(n, q)] = gW1[n][q];
   __syncthreads();
   for (int q = threadIdx.x; q < H; q += blockDim.x) {
-    out[OFF_B1 + q] = S.vb1[q];
-    out[OFF_B2 + q] = S.vb2[q];
-    out[OFF_W3 + q] = S.vw3[q];
+    out[OFF_B1 + q] = S.vb1[0][q] + S.vb1[1][q] + S.vb1[2][q] + S.vb1[3][q];
+    out[OFF_B2 + q] = S.vb2[0][q] + S.vb2[1][q] + S.vb2[2][q] + S.vb2[3][q];
+    out[OFF_W3 + q] = S.vw3[0][q] + S.vw3[1][q] + S.vw3[2][q] + S.vw3[3][q];
   }
-  if (threadIdx.x == 0) out[OFF_B3] = S.vb3;
+  if (threadIdx.x == 0) out[OFF_B3] = S.vb3[0] + S.vb3[1] + S.vb3[2] + S.vb3[3];
 }
 
-// grad[p] = sum over blocks (in order) of part[b][p]
-__global__ void k_sg_reduce(const float* __restrict__ part, int blocks, int n, float scale, float* __restrict__ grad) {
+// grad[species][p] = sum over the species' blocks (in order) of part[b][p]
+__global__ void k_sg_reduce(const float* __restrict__ part, int nb0, int blocks, float* __restrict__ grad) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
+  if (p >= PER_SPECIES) return;
+  const int species = blockIdx.y, b0 = species == 0 ? 0 : nb0, b1 = species == 0 ? nb0 : blocks;
   float s = 0.f;
-  for (int b = 0; b < blocks; b++) s += part[(size_t)b * n + p];
-  grad[p] = scale * s;
+  constexpr int U = 8;   // partials in flight
+  for (int b = b0; b < b1; b += U) {
+    float x[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) x[u] = b + u < b1 ? part[(size_t)(b + u) * PER_SPECIES + p] : 0.f;
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (b + u < b1) s += x[u];
+  }
+  grad[species * PER_SPECIES + p] = s;
+}
+
+// Residuals of the loss: per atom e = wE 2 (E_c - Etrue_c) / (N^2 C) of its chain, per
+// component v = wF 2 / (3 N C) (F - Ftrue); out[0] = sum (E - Etrue)^2, out[1] = sum |F - Ftrue|^2.
+constexpr int RES_THREADS = 256;
+__global__ void __launch_bounds__(RES_THREADS) k_sg_residual(const double* __restrict__ F,
+                                                             const double* __restrict__ Ft,
+                                                             const double* __restrict__ E,
+                                                             const double* __restrict__ Et, int C, int N, double wE,
+                                                             double fscale, float* __restrict__ v,
+                                                             float* __restrict__ eAtom, double* partials,
+                                                             unsigned int* ticket, double* out, double* hostOut) {
+  const int total = C * N;
+  double s[2] = {0.0, 0.0};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * total; i += gridDim.x * blockDim.x) {
+    const double d = __dsub_rn(F[i], Ft[i]);
+    s[1] = __dadd_rn(s[1], __dmul_rn(d, d));
+    v[i] = (float)__dmul_rn(fscale, d);
+    if (i < total) {
+      const int c = i / N;
+      const double x = __dsub_rn(E[c], Et[c]);
+      eAtom[i] = (float)(wE * 2.0 * x / ((double)N * N * C));
+      if (i == c * N) s[0] = __dadd_rn(s[0], __dmul_rn(x, x));
+    }
+  }
+  grid_reduce<2, RES_THREADS>(s, partials, ticket, out, hostOut);
 }
 
 __global__ void k_sg_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
@@ -984,11 +1169,17 @@ struct Surrogate {
   int *dList = nullptr, *dCount = nullptr, *dOverflow = nullptr;
   float *dG = nullptr, *dEatom = nullptr, *dEdG = nullptr, *dU = nullptr, *dV = nullptr, *dEres = nullptr;
   float *dParams = nullptr, *dPart = nullptr, *dGrad = nullptr, *dM = nullptr, *dVar = nullptr;
-  int trainBlocks = 0;
+  int trainBlocks = 0, trainBlocks0 = 0, tiles0 = 0;   // blocks of k_sg_train, those of species 0, tiles of species 0
+  int3* dTrainTiles = nullptr;                          // the tiles of <= 64 atoms, species 0 first
+  double *dF = nullptr, *dE = nullptr;                  // forces and energies of EmDee_surrogate_gradient
+  double *dResPart = nullptr, *hLoss = nullptr;         // partials, then the sums; pinned sums
+  unsigned int* dTicket = nullptr;
   double* dR0 = nullptr;   // positions of the last list build
 };
 
 static int sg_blocks(int n) { return (n + 255) / 256; }
+static int sg_warp_blocks(int n) { return (n + sg::WARP_ATOMS - 1) / sg::WARP_ATOMS; }
+static const int SG_RES_BLOCKS = 2 * 152;
 
 static void sg_build_lists(Surrogate& S, const double* dR, cudaStream_t st) {
   using namespace sg;
@@ -999,9 +1190,8 @@ static void sg_build_lists(Surrogate& S, const double* dR, cudaStream_t st) {
   k_sg_count<<<sg_blocks(S.total), 256, 0, st>>>(S.dPos, S.G, S.dCellOf, S.dCounts);
   k_sg_scan<<<1, 256, 0, st>>>(S.dCounts, cells, S.dStarts);
   k_sg_scatter<<<sg_blocks(S.total), 256, 0, st>>>(S.dCellOf, S.G, S.dStarts, S.dCursor, S.dSorted);
-  k_sg_sort<<<sg_blocks(cells), 256, 0, st>>>(S.dStarts, cells, S.dSorted);
-  k_sg_list<<<sg_blocks(S.total), 256, 0, st>>>(S.dPos, S.G, S.dCellOf, S.dStarts, S.dSorted, S.cap, S.dList,
-                                                 S.dCount, S.dOverflow);
+  k_sg_sort<<<(cells + 7) / 8, 256, 0, st>>>(S.dStarts, cells, S.dSorted);
+  k_sg_list<<<cells, LIST_THREADS, 0, st>>>(S.dPos, S.G, S.dStarts, S.dSorted, S.cap, S.dList, S.dCount, S.dOverflow);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(S.dR0, dR, sizeof(double) * 3 * S.total, cudaMemcpyDeviceToDevice, st));
 }
@@ -1116,8 +1306,29 @@ void* EmDee_surrogate_create(int chains, int N, double L, const int* types, doub
   CK(cudaMalloc(&S->dVar, sizeof(float) * NPARAM));
   CK(cudaMemset(S->dM, 0, sizeof(float) * NPARAM));
   CK(cudaMemset(S->dVar, 0, sizeof(float) * NPARAM));
-  S->trainBlocks = 2 * 152;
+  {
+    // one training block per SM, shared out by the species' tiles
+    std::vector<int3> byType;
+    for (int sp = 0; sp < NS; sp++)
+      for (const int3& t : S->tiles)
+        if (t.z == sp) byType.push_back(t);
+    for (const int3& t : S->tiles) S->tiles0 += t.z == 0;
+    const int nt = (int)byType.size(), nt1 = nt - S->tiles0, blocks = std::min(152, nt);
+    int b0 = (int)std::lround((double)blocks * S->tiles0 / nt);
+    if (S->tiles0 > 0 && b0 < 1) b0 = 1;
+    if (nt1 > 0 && b0 > blocks - 1) b0 = std::max(S->tiles0 > 0 ? 1 : 0, blocks - 1);
+    S->trainBlocks0 = b0;
+    S->trainBlocks = nt1 > 0 ? std::max(blocks, b0 + 1) : b0;
+    CK(cudaMalloc(&S->dTrainTiles, sizeof(int3) * nt));
+    CK(cudaMemcpy(S->dTrainTiles, byType.data(), sizeof(int3) * nt, cudaMemcpyHostToDevice));
+  }
   CK(cudaMalloc(&S->dPart, sizeof(float) * (size_t)S->trainBlocks * PER_SPECIES));
+  CK(cudaMalloc(&S->dF, sizeof(double) * 3 * T));
+  CK(cudaMalloc(&S->dE, sizeof(double) * chains));
+  CK(cudaMalloc(&S->dResPart, sizeof(double) * (2 * SG_RES_BLOCKS + 2)));
+  CK(cudaMallocHost(&S->hLoss, sizeof(double) * 2));
+  CK(cudaMalloc(&S->dTicket, sizeof(unsigned int)));
+  CK(cudaMemset(S->dTicket, 0, sizeof(unsigned int)));
   CK(cudaMalloc(&S->dR0, sizeof(double) * 3 * T));
   CK(cudaFuncSetAttribute(k_sg_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpSmem)));
   CK(cudaFuncSetAttribute(k_sg_mlp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem_bytes()));
@@ -1145,7 +1356,7 @@ void EmDee_surrogate_descriptors(void* h, const double* dR, float* dGout, int re
   cudaStream_t st = (cudaStream_t)stream;
   if (rebuild) sg_build_lists(S, dR, st);
   else k_sg_pack<<<sg_blocks(S.total), 256, 0, st>>>(dR, S.total, S.L, S.dPos);
-  k_sg_desc<<<sg_blocks(S.total), 256, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dList, S.dCount, S.cap, S.dG);
+  k_sg_desc<<<sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dList, S.dCount, S.cap, S.dG);
   CK(cudaGetLastError());
   if (dGout) CK(cudaMemcpyAsync(dGout, S.dG, sizeof(float) * S.total * DIN, cudaMemcpyDeviceToDevice, st));
 }
@@ -1158,7 +1369,7 @@ int EmDee_surrogate_forces(void* h, const double* dR, double* dF, double* dE, in
   cudaStream_t st = (cudaStream_t)stream;
   EmDee_surrogate_descriptors(h, dR, nullptr, rebuild, stream);
   sg_network(S, S.dParams, st);
-  k_sg_force<<<sg_blocks(S.total), 256, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dList, S.dCount, S.cap, S.dEdG, dF);
+  k_sg_force<<<sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dList, S.dCount, S.cap, S.dEdG, dF);
   CK(cudaGetLastError());
   if (dE) k_sg_chain_sum<<<S.G.chains, 256, 0, st>>>(S.dEatom, S.G.N, dE);
   int ov = 0;
@@ -1192,47 +1403,21 @@ void EmDee_surrogate_gradient(void* h, const double* dR, const double* dEtrue, c
   Surrogate& S = *(Surrogate*)h;
   cudaStream_t st = (cudaStream_t)stream;
   const int C = S.G.chains, N = S.G.N;
-  double *dF, *dE;
-  CK(cudaMallocAsync(&dF, sizeof(double) * 3 * S.total, st));
-  CK(cudaMallocAsync(&dE, sizeof(double) * C, st));
-  EmDee_surrogate_forces(h, dR, dF, dE, 1, stream);
-  // residuals on the host side of the loss: small arrays per chain, per atom on the device
-  std::vector<double> E(C), Et(C);
-  CK(cudaMemcpyAsync(E.data(), dE, sizeof(double) * C, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(Et.data(), dEtrue, sizeof(double) * C, cudaMemcpyDeviceToHost, st));
-  std::vector<double> F((size_t)3 * S.total), Ft((size_t)3 * S.total);
-  CK(cudaMemcpyAsync(F.data(), dF, sizeof(double) * F.size(), cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(Ft.data(), dFtrue, sizeof(double) * Ft.size(), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  double lE = 0.0, lF = 0.0;
-  std::vector<float> eAtom(S.total), v((size_t)3 * S.total);
-  for (int c = 0; c < C; c++) {
-    const double d = E[c] - Et[c];
-    lE += d * d;
-    const float ec = (float)(wE * 2.0 * d / ((double)N * N * C));
-    for (int i = 0; i < N; i++) eAtom[(size_t)c * N + i] = ec;
-  }
+  EmDee_surrogate_forces(h, dR, S.dF, S.dE, 1, stream);
   const double fscale = wF * 2.0 / (3.0 * N * C);
-  for (size_t q = 0; q < F.size(); q++) {
-    const double d = F[q] - Ft[q];
-    lF += d * d;
-    v[q] = (float)(fscale * d);
-  }
-  loss[0] = wE * lE / ((double)N * N * C);
-  loss[1] = wF * lF / (3.0 * N * C);
-  CK(cudaMemcpyAsync(S.dEres, eAtom.data(), sizeof(float) * S.total, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(S.dV, v.data(), sizeof(float) * v.size(), cudaMemcpyHostToDevice, st));
-  k_sg_udesc<<<sg_blocks(S.total), 256, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dList, S.dCount, S.cap, S.dV, S.dU);
-  TileArgs T{S.dAtoms, S.dTiles, (int)S.tiles.size()};
-  for (int sp = 0; sp < NS; sp++) {
-    k_sg_train<<<S.trainBlocks, 128, sizeof(TrainSmem), st>>>(T, sp, S.dParams, S.dG, S.dU, S.dEres, S.dPart);
-    k_sg_reduce<<<(PER_SPECIES + 255) / 256, 256, 0, st>>>(S.dPart, S.trainBlocks, PER_SPECIES, 1.f,
-                                                           dGrad + sp * PER_SPECIES);
-  }
+  k_sg_residual<<<std::min(SG_RES_BLOCKS, sg_blocks(3 * S.total)), RES_THREADS, 0, st>>>(
+      S.dF, dFtrue, S.dE, dEtrue, C, N, wE, fscale, S.dV, S.dEres, S.dResPart, S.dTicket,
+      S.dResPart + 2 * SG_RES_BLOCKS, S.hLoss);
+  k_sg_udesc<<<sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dList, S.dCount, S.cap,
+                                                                  S.dV, S.dU);
+  TileArgs T{S.dAtoms, S.dTrainTiles, (int)S.tiles.size()};
+  k_sg_train<<<S.trainBlocks, 128, sizeof(TrainSmem), st>>>(T, S.tiles0, S.trainBlocks0, S.dParams, S.dG, S.dU,
+                                                            S.dEres, S.dPart);
+  k_sg_reduce<<<dim3((PER_SPECIES + 255) / 256, NS), 256, 0, st>>>(S.dPart, S.trainBlocks0, S.trainBlocks, dGrad);
   CK(cudaGetLastError());
-  CK(cudaFreeAsync(dF, st));
-  CK(cudaFreeAsync(dE, st));
   CK(cudaStreamSynchronize(st));
+  loss[0] = wE * S.hLoss[0] / ((double)N * N * C);
+  loss[1] = wF * S.hLoss[1] / (3.0 * N * C);
 }
 
 // One Adam step on the device master parameters with gradient dGrad (device)
@@ -1266,8 +1451,10 @@ void EmDee_surrogate_destroy(void* h) {
   if (!S) return;
   void* ptrs[] = {S->dSpecies, S->dAtoms, S->dTiles, S->dTiles128, S->dTcError, S->dPos, S->dCellOf, S->dCounts, S->dStarts, S->dCursor,
                   S->dSorted, S->dList, S->dCount, S->dOverflow, S->dG, S->dU, S->dEdG, S->dEatom, S->dEres,
-                  S->dV, S->dParams, S->dGrad, S->dM, S->dVar, S->dPart, S->dR0};
+                  S->dV, S->dParams, S->dGrad, S->dM, S->dVar, S->dPart, S->dR0, S->dTrainTiles, S->dF, S->dE, S->dResPart,
+                  S->dTicket};
   for (void* p : ptrs) cudaFree(p);
+  cudaFreeHost(S->hLoss);
   delete S;
 }
 
