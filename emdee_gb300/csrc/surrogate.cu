@@ -74,26 +74,61 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-__device__ __forceinline__ uint32_t ld32(const __nv_bfloat16* p) { return *reinterpret_cast<const uint32_t*>(p); }
+// four 8 x 8 BF16 matrices from shared memory: lane l supplies the address of row l % 8 of
+// matrix l / 8; lane 4 g + t receives elements (g, 2t..2t+1) of each, or with TRANS
+// (2t..2t+1, g)
+template <bool TRANS>
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __nv_bfloat16* p) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  if (TRANS)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
 
 // acc[nt][4] += A(16 x K) * B(K x 8 NT), A row-major (lda), B given as Bt[n][k] (ldb)
 template <int K, int NT>
 __device__ __forceinline__ void warp_gemm(const __nv_bfloat16* A, int lda, const __nv_bfloat16* Bt, int ldb,
                                           float (&acc)[NT][4]) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int lane = threadIdx.x & 31, row = lane & 7, mat = lane >> 3;
+  const __nv_bfloat16* pa = A + (row + 8 * (mat & 1)) * lda + 8 * (mat >> 1);
+  const __nv_bfloat16* pb = Bt + (row + 8 * (mat >> 1)) * ldb + 8 * (mat & 1);
 #pragma unroll
   for (int k0 = 0; k0 < K; k0 += 16) {
     uint32_t a[4];
-    a[0] = ld32(A + g * lda + k0 + 2 * t);
-    a[1] = ld32(A + (g + 8) * lda + k0 + 2 * t);
-    a[2] = ld32(A + g * lda + k0 + 8 + 2 * t);
-    a[3] = ld32(A + (g + 8) * lda + k0 + 8 + 2 * t);
+    ldmatrix4<false>(a, pa + k0);
 #pragma unroll
-    for (int n = 0; n < NT; n++) {
-      uint32_t b[2];
-      b[0] = ld32(Bt + (n * 8 + g) * ldb + k0 + 2 * t);
-      b[1] = ld32(Bt + (n * 8 + g) * ldb + k0 + 8 + 2 * t);
-      mma16816(acc[n], a, b);
+    for (int n = 0; n < NT; n += 2) {   // two column tiles per load
+      uint32_t b[4];
+      ldmatrix4<false>(b, pb + n * 8 * ldb + k0);
+      const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
+      mma16816(acc[n], a, b0);
+      mma16816(acc[n + 1], a, b1);
+    }
+  }
+}
+
+// acc[nt][4] += A^T(16 x K) * B(K x 8 NT) with A and B stored by rows of k: A[k][m] (lda),
+// B[k][n] (ldb), transposed as they are loaded
+template <int K, int NT>
+__device__ __forceinline__ void warp_gemm_t(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb,
+                                            float (&acc)[NT][4]) {
+  const int lane = threadIdx.x & 31, row = lane & 7, mat = lane >> 3;
+  const __nv_bfloat16* pa = A + (row + 8 * (mat >> 1)) * lda + 8 * (mat & 1);
+  const __nv_bfloat16* pb = B + (row + 8 * (mat & 1)) * ldb + 8 * (mat >> 1);
+#pragma unroll
+  for (int k0 = 0; k0 < K; k0 += 16) {
+    uint32_t a[4];
+    ldmatrix4<true>(a, pa + k0 * lda);
+#pragma unroll
+    for (int n = 0; n < NT; n += 2) {
+      uint32_t b[4];
+      ldmatrix4<true>(b, pb + k0 * ldb + n * 8);
+      const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
+      mma16816(acc[n], a, b0);
+      mma16816(acc[n + 1], a, b1);
     }
   }
 }
@@ -109,7 +144,7 @@ __device__ __forceinline__ int frag_row(int q) { return ((threadIdx.x & 31) >> 2
 __device__ __forceinline__ int frag_col(int n, int q) { return n * 8 + 2 * (threadIdx.x & 3) + (q & 1); }
 
 // shared-memory weights of one species, BF16, in both orientations
-struct WeightsSmem {
+struct __align__(16) WeightsSmem {   // rows on 16-byte boundaries, for ldmatrix
   __nv_bfloat16 W1[DIN][H + 8];    // W1[k][n]        (B^T for dE/dG = dz1 W1^T)
   __nv_bfloat16 W1t[H][DIN + 8];   // W1^T[n][k]      (B^T for z1 = G W1)
   __nv_bfloat16 W2[H][H + 8];      // W2[k][n]        (B^T for da1 = dz2 W2^T)
@@ -240,20 +275,23 @@ __global__ void k_sg_sort(const int* __restrict__ starts, int n, int* __restrict
     if (32 * u + lane < m) sorted[b + place[u]] = v[u];
 }
 
+// rintf for |x| < 2^22 on the FP32 adders (the conversion unit runs at a quarter of
+// their rate)
+__device__ __forceinline__ float nearest(float x) { return __fadd_rn(__fadd_rn(x, 12582912.f), -12582912.f); }
+
 // Verlet lists (global atom indices), entry e of atom q at list[q * cap + e], in the order
 // of the neighbor cells and of their atoms.  A block per cell stages the candidates of
 // its atoms (27 cells, or with M < 3 the whole chain) in shared memory; a warp per atom
 // goes through them side by side and places the accepted ones by ballots.  More than
 // LIST_CAND candidates are taken in several stages.  (One thread per atom, gathering
-// each candidate's index and position: 428 us at 8 x 8000 atoms; 193 us so.)
+// each candidate's index and position: 428 us at 8 x 8000 atoms; 142 us so.)
 constexpr int LIST_CAND = 2048, LIST_THREADS = 256;
 __global__ void __launch_bounds__(LIST_THREADS) k_sg_list(const float4* __restrict__ pos, Geometry G,
                                                           const int* __restrict__ starts,
                                                           const int* __restrict__ sorted, int cap,
                                                           int* __restrict__ list, int* __restrict__ count,
                                                           int* __restrict__ overflow) {
-  __shared__ float cx[LIST_CAND], cy[LIST_CAND], cz[LIST_CAND];
-  __shared__ int cj[LIST_CAND];
+  __shared__ float4 cand[LIST_CAND];   // position (M >= 3: the image next to the cell) and index
   __shared__ int first[28], base[28];   // candidates of the neighbor cells: first slot, running count
   const int M = G.M, cells = M * M * M, chain = blockIdx.x / cells, cell = blockIdx.x % cells;
   const int x = cell % M, y = (cell / M) % M, z = cell / (M * M);
@@ -283,11 +321,15 @@ __global__ void __launch_bounds__(LIST_THREADS) k_sg_list(const float4* __restri
       int k = 0;
       while (base[k + 1] <= c0 + c) k++;
       const int j = sorted[first[k] + (c0 + c - base[k])];
-      const float4 p = pos[j];
-      cj[c] = j;
-      cx[c] = p.x;
-      cy[c] = p.y;
-      cz[c] = p.z;
+      float4 p = pos[j];
+      if (M >= 3) {   // cells across the box's faces: the image on this side
+        const int nx = x + k % 3 - 1, ny = y + k / 3 % 3 - 1, nz = z + k / 9 - 1;
+        p.x += nx < 0 ? -G.L : nx >= M ? G.L : 0.f;
+        p.y += ny < 0 ? -G.L : ny >= M ? G.L : 0.f;
+        p.z += nz < 0 ? -G.L : nz >= M ? G.L : 0.f;
+      }
+      p.w = __int_as_float(j);
+      cand[c] = p;
     }
     __syncthreads();
     for (int o = own0 + warp; o < own1; o += LIST_THREADS / 32) {
@@ -296,11 +338,14 @@ __global__ void __launch_bounds__(LIST_THREADS) k_sg_list(const float4* __restri
       int* out = list + (size_t)q * cap;
       int n = c0 > 0 ? count[q] : 0;
       for (int c = lane; c - lane < nc; c += 32) {
-        const int cc = min(c, nc - 1), j = cj[cc];
-        float ex = p.x - cx[cc], ey = p.y - cy[cc], ez = p.z - cz[cc];
-        ex -= G.L * rintf(ex * G.invL);
-        ey -= G.L * rintf(ey * G.invL);
-        ez -= G.L * rintf(ez * G.invL);
+        const float4 pj = cand[min(c, nc - 1)];
+        const int j = __float_as_int(pj.w);
+        float ex = p.x - pj.x, ey = p.y - pj.y, ez = p.z - pj.z;
+        if (M < 4) {   // a neighbor cell may hold a nearer image
+          ex -= G.L * nearest(ex * G.invL);
+          ey -= G.L * nearest(ey * G.invL);
+          ez -= G.L * nearest(ez * G.invL);
+        }
         const bool in = c < nc && j != q && ex * ex + ey * ey + ez * ez < G.rlist2;
         const unsigned m = __ballot_sync(0xffffffffu, in);
         const int at = n + __popc(m & ((1u << lane) - 1u));
@@ -343,7 +388,9 @@ __device__ __forceinline__ void radial(float r, const Geometry& G, float cdecay,
 // gathered, in list order, in the warp's buffer; each full batch of 32 goes to
 // batch(n, d, j): lane k < n holds neighbor k, d = (displacement, squared distance).  So
 // the costly radial functions run on full warps; one thread per atom ran them for a
-// warp whenever any lane's entry was within rc, on 3 warps per scheduler.
+// warp whenever any lane's entry was within rc, on 3 warps per scheduler.  k_sg_desc
+// leaves the neighbors within rc in `near`, from which the adjoint kernels at the same
+// positions start (each_neighbor).
 constexpr int WARP_ATOMS = 8;   // warps (atoms) per block
 struct NeighborBuffer {
   float4 d[64];
@@ -361,9 +408,9 @@ __device__ __forceinline__ void for_neighbors(const float4* __restrict__ pos, co
     const int j = e < n ? list[e] : q;
     const float4 pj = pos[j];
     float ex = pi.x - pj.x, ey = pi.y - pj.y, ez = pi.z - pj.z;
-    ex -= G.L * rintf(ex * G.invL);
-    ey -= G.L * rintf(ey * G.invL);
-    ez -= G.L * rintf(ez * G.invL);
+    ex -= G.L * nearest(ex * G.invL);
+    ey -= G.L * nearest(ey * G.invL);
+    ez -= G.L * nearest(ez * G.invL);
     const float r2 = ex * ex + ey * ey + ez * ez;
     const bool in = e < n && r2 < G.rc2;
     const unsigned m = __ballot_sync(FULL, in);
@@ -394,6 +441,24 @@ __device__ __forceinline__ void for_neighbors(const float4* __restrict__ pos, co
   if (have > 0) batch(have, lane < have ? B.d[lane] : make_float4(1.f, 1.f, 1.f, 3.f), lane < have ? B.j[lane] : q);
 }
 
+// batch(n, d, j) over the neighbors k_sg_desc left in `near`, 32 at a time
+template <class F>
+__device__ __forceinline__ void each_neighbor(const float4* __restrict__ pos, const Geometry& G, int q, const int* near,
+                                              int n, F&& batch) {
+  const int lane = threadIdx.x & 31;
+  const float4 pi = pos[q];
+  for (int e = 0; e < n; e += 32) {
+    const int m = min(32, n - e), j = lane < m ? near[e + lane] : q;
+    const float4 pj = pos[j];
+    float ex = pi.x - pj.x, ey = pi.y - pj.y, ez = pi.z - pj.z;
+    ex -= G.L * nearest(ex * G.invL);
+    ey -= G.L * nearest(ey * G.invL);
+    ez -= G.L * nearest(ez * G.invL);
+    const float r2 = ex * ex + ey * ey + ez * ez;
+    batch(m, lane < m ? make_float4(ex, ey, ez, r2) : make_float4(1.f, 1.f, 1.f, 3.f), j);
+  }
+}
+
 __device__ __forceinline__ PairGeom unit_vector(const float4& d) {
   const float r = sqrtf(d.w), inv = 1.f / r;
   return PairGeom{r, d.x * inv, d.y * inv, d.z * inv};
@@ -403,12 +468,13 @@ __device__ __forceinline__ PairGeom unit_vector(const float4& d) {
 // neighbors of species c in list order.  H: row per neighbor, an odd stride.
 constexpr int HROW = NG + 1;
 
-// 8 x 8000 atoms: 195 us with one thread per atom, 86 us so.
+// 8 x 8000 atoms: 195 us with one thread per atom, 92 us so.
 __global__ void __launch_bounds__(32 * WARP_ATOMS) k_sg_desc(const float4* __restrict__ pos, Geometry G,
                                                              const uint8_t* __restrict__ species,
                                                              const int* __restrict__ list,
                                                              const int* __restrict__ count, int cap,
-                                                             float* __restrict__ Gout) {
+                                                             float* __restrict__ Gout, int* __restrict__ near,
+                                                             int* __restrict__ nearCount) {
   __shared__ NeighborBuffer nbuf[WARP_ATOMS];
   __shared__ float hbuf[WARP_ATOMS][32 * HROW];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * WARP_ATOMS + warp;
@@ -418,7 +484,11 @@ __global__ void __launch_bounds__(32 * WARP_ATOMS) k_sg_desc(const float4* __res
   const int k = lane & (NG - 1), chain0 = q - q % G.N;   // first atom of the chain
   const unsigned flip = lane < NG ? 0xffffffffu : 0u;   // species 0 in the lower lanes
   float acc = 0.f;
+  int* out = near + (size_t)q * cap;
+  int total = 0;
   for_neighbors(pos, G, q, list + (size_t)q * cap, min(count[q], cap), nbuf[warp], [&](int n, float4 d, int j) {
+    if (lane < n) out[total + lane] = j;
+    total += n;
     float h[NG], dh[NG];
     radial(sqrtf(d.w), G, cdecay, h, dh);
 #pragma unroll
@@ -434,60 +504,69 @@ __global__ void __launch_bounds__(32 * WARP_ATOMS) k_sg_desc(const float4* __res
     __syncwarp();
   });
   Gout[(size_t)q * DIN + lane] = acc;
+  if (lane == 0) nearCount[q] = total;
 }
 
 // F_i = -sum_j s_ij r_hat_ij, s_ij = sum_k (dEdG_i[s_j, k] + dEdG_j[s_i, k]) dh_k(r_ij).
-// 8 x 8000 atoms: 293 us with one thread per atom, 164 us so.
-__global__ void __launch_bounds__(32 * WARP_ATOMS) k_sg_force(const float4* __restrict__ pos, Geometry G,
+// A lane per neighbor computes dh and r_hat; then four lanes per neighbor take four
+// Gaussians each, so that a neighbor's 64 bytes of dE/dG are read side by side (eight
+// lines per load instead of 32), and three of them add one force component each.
+// 8 x 8000 atoms: 293 us with one thread per atom, 116 us so.
+constexpr int DROW = NG + 4;   // rows of 16 + 4 floats: 16-byte aligned, in different banks
+__global__ void __launch_bounds__(32 * WARP_ATOMS, 4) k_sg_force(const float4* __restrict__ pos, Geometry G,
                                                               const uint8_t* __restrict__ species,
-                                                              const int* __restrict__ list,
-                                                              const int* __restrict__ count, int cap,
+                                                              const int* __restrict__ near,
+                                                              const int* __restrict__ nearCount, int cap,
                                                               const float* __restrict__ dEdG,
                                                               double* __restrict__ F) {
-  __shared__ NeighborBuffer nbuf[WARP_ATOMS];
+  // per neighbor: dh[16], r_hat[3], index
+  __shared__ __align__(16) float dbuf[WARP_ATOMS][32 * DROW];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * WARP_ATOMS + warp;
   if (q >= G.chains * G.N) return;
   const float cdecay = __expf(-2.f * G.a * G.dmu * G.dmu);
   const int chain0 = q - q % G.N, si = species[q - chain0];   // first atom of the chain
-  const float* gi = dEdG + (size_t)q * DIN;
-  float fx = 0.f, fy = 0.f, fz = 0.f;
-  for_neighbors(pos, G, q, list + (size_t)q * cap, min(count[q], cap), nbuf[warp], [&](int n, float4 d, int j) {
-    if (lane < n) {
+  const int part = lane & 3, comp = part < 3 ? part : 0;
+  float* D = dbuf[warp];
+  const float4* own = reinterpret_cast<const float4*>(dEdG + (size_t)q * DIN) + part;
+  const float4 own0 = __ldg(&own[0]), own1 = __ldg(&own[NG / 4]);   // this lane's Gaussians of both species
+  float f = 0.f;
+  each_neighbor(pos, G, q, near + (size_t)q * cap, nearCount[q], [&](int n, float4 d, int j) {
+    {
       const PairGeom pg = unit_vector(d);
       float h[NG], dh[NG];
       radial(pg.r, G, cdecay, h, dh);
-      const float4* a = reinterpret_cast<const float4*>(gi + species[j - chain0] * NG);
-      const float4* b = reinterpret_cast<const float4*>(dEdG + (size_t)j * DIN + si * NG);
-      float s = 0.f;
+      float4* row = reinterpret_cast<float4*>(D + lane * DROW);
 #pragma unroll
-      for (int k4 = 0; k4 < NG / 4; k4++) {
-        const float4 x = __ldg(&a[k4]), y = __ldg(&b[k4]);
-        s += (x.x + y.x) * dh[4 * k4] + (x.y + y.y) * dh[4 * k4 + 1] + (x.z + y.z) * dh[4 * k4 + 2] +
-             (x.w + y.w) * dh[4 * k4 + 3];
-      }
-      fx -= s * pg.ux;
-      fy -= s * pg.uy;
-      fz -= s * pg.uz;
+      for (int k = 0; k < NG; k += 4) row[k / 4] = make_float4(dh[k], dh[k + 1], dh[k + 2], dh[k + 3]);
+      // the sign bit of the index carries the species
+      row[NG / 4] = make_float4(pg.ux, pg.uy, pg.uz, __int_as_float(species[j - chain0] ? j | (int)0x80000000 : j));
+    }
+    __syncwarp();
+    for (int b = 0; b < n; b += 8) {
+      const int nb = b + (lane >> 2);
+      const float* row = D + nb * DROW;
+      const int code = __float_as_int(row[NG + 3]), jj = code & 0x7FFFFFFF;
+      const float4 x = code < 0 ? own1 : own0, dh = *reinterpret_cast<const float4*>(row + 4 * part);
+      const float4 y = __ldg(reinterpret_cast<const float4*>(dEdG + (size_t)jj * DIN + si * NG) + part);
+      float s = (x.x + y.x) * dh.x + (x.y + y.y) * dh.y + (x.z + y.z) * dh.z + (x.w + y.w) * dh.w;
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      if (nb < n) f -= s * row[NG + comp];
     }
     __syncwarp();
   });
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    fx += __shfl_xor_sync(0xffffffffu, fx, o);
-    fy += __shfl_xor_sync(0xffffffffu, fy, o);
-    fz += __shfl_xor_sync(0xffffffffu, fz, o);
-  }
-  if (lane < 3) F[3 * (size_t)q + lane] = lane == 0 ? fx : lane == 1 ? fy : fz;
+  for (int o = 4; o < 32; o <<= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+  if (lane < 3) F[3 * (size_t)q + lane] = f;
 }
 
 // u_i[s_j, k] = sum_j dh_k(r_ij) (v_i - v_j) . r_hat_ij (force residual in descriptor space).
-// 8 x 8000 atoms: 248 us with one thread per atom, 146 us so.
-__global__ void __launch_bounds__(32 * WARP_ATOMS) k_sg_udesc(const float4* __restrict__ pos, Geometry G,
+// 8 x 8000 atoms: 248 us with one thread per atom, 93 us so.
+__global__ void __launch_bounds__(32 * WARP_ATOMS, 4) k_sg_udesc(const float4* __restrict__ pos, Geometry G,
                                                               const uint8_t* __restrict__ species,
-                                                              const int* __restrict__ list,
-                                                              const int* __restrict__ count, int cap,
-                                                              const float* __restrict__ v, float* __restrict__ U) {
-  __shared__ NeighborBuffer nbuf[WARP_ATOMS];
+                                                              const int* __restrict__ near,
+                                                              const int* __restrict__ nearCount, int cap,
+                                                              const float4* __restrict__ v, float* __restrict__ U) {
   __shared__ float hbuf[WARP_ATOMS][32 * HROW];
   __shared__ float wbuf[WARP_ATOMS][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * WARP_ATOMS + warp;
@@ -496,15 +575,16 @@ __global__ void __launch_bounds__(32 * WARP_ATOMS) k_sg_udesc(const float4* __re
   float* H = hbuf[warp];
   const int k = lane & (NG - 1), chain0 = q - q % G.N;   // first atom of the chain
   const unsigned flip = lane < NG ? 0xffffffffu : 0u;   // species 0 in the lower lanes
-  const float vix = v[3 * q], viy = v[3 * q + 1], viz = v[3 * q + 2];
+  const float4 vi = v[q];
   float acc = 0.f;
-  for_neighbors(pos, G, q, list + (size_t)q * cap, min(count[q], cap), nbuf[warp], [&](int n, float4 d, int j) {
+  each_neighbor(pos, G, q, near + (size_t)q * cap, nearCount[q], [&](int n, float4 d, int j) {
+    const float4 vj = v[j];
     const PairGeom pg = unit_vector(d);
     float h[NG], dh[NG];
     radial(pg.r, G, cdecay, h, dh);
 #pragma unroll
     for (int u = 0; u < NG; u++) H[lane * HROW + u] = dh[u];
-    wbuf[warp][lane] = (vix - v[3 * j]) * pg.ux + (viy - v[3 * j + 1]) * pg.uy + (viz - v[3 * j + 2]) * pg.uz;
+    wbuf[warp][lane] = (vi.x - vj.x) * pg.ux + (vi.y - vj.y) * pg.uy + (vi.z - vj.z) * pg.uz;
     const unsigned mine = (__ballot_sync(0xffffffffu, species[j - chain0] != 0) ^ flip) & (0xffffffffu >> (32 - n));
     __syncwarp();
     for (int b = 0; b < n; b += 8)
@@ -894,8 +974,6 @@ struct TrainSmem {
   __nv_bfloat16 act[2 * TILE][H + 8];        // rows: a1 (64), da1 (64)
   __nv_bfloat16 gz2[2 * TILE][H + 8];        // rows: gz2 (64), gdz2 (64)
   __nv_bfloat16 gz1[2 * TILE][H + 8];        // rows: gz1 (64), gdz1 (64)
-  __nv_bfloat16 tA[H][2 * TILE + 8];         // transposed operands of the weight GEMMs
-  __nv_bfloat16 tB[H][2 * TILE + 8];
   float vb1[4][H], vb2[4][H], vw3[4][H], vb3[4];   // per warp
 };
 
@@ -917,7 +995,8 @@ __device__ __forceinline__ void column_sums(float (&x)[8][2], float* out) {
 // first nt0 of T), the others those of species 1; each writes its gradient partial
 // (PER_SPECIES floats) to part[b].  Bias and output-layer gradients are summed by
 // shuffles per warp (shared-memory atomics, eight lanes to an address, were most of
-// 2 x 419 us at 8 x 8000 atoms; 173 us so).
+// 2 x 419 us at 8 x 8000 atoms; 173 us so); the weight GEMMs take their operands
+// transposed by ldmatrix, so that two blocks fit an SM (91 us).
 __global__ void __launch_bounds__(128) k_sg_train(TileArgs T, int nt0, int nb0, const float* __restrict__ params,
                                                   const float* __restrict__ Gin, const float* __restrict__ Uin,
                                                   const float* __restrict__ eAtom, float* __restrict__ part) {
@@ -1025,23 +1104,10 @@ __global__ void __launch_bounds__(128) k_sg_train(TileArgs T, int nt0, int nb0, 
     }
     column_sums(sb1, S.vb1[warp]);
     __syncthreads();
-    // dW2 += [a1; da1]^T [gz2; gdz2]: A = tA (64 units x 128 atoms), B^T = tB (64 units x 128 atoms)
-    for (int q = threadIdx.x; q < 2 * TILE * H; q += blockDim.x) {
-      const int r = q / H, c = q % H;
-      S.tA[c][r] = S.act[r][c];
-      S.tB[c][r] = S.gz2[r][c];
-    }
-    __syncthreads();
-    warp_gemm<2 * TILE, 8>(&S.tA[16 * warp][0], 2 * TILE + 8, &S.tB[0][0], 2 * TILE + 8, gW2);
-    __syncthreads();
-    // dW1 += [G; U]^T [gz1; gdz1]: A = in^T (32 inputs x 128 atoms), B^T = gz1^T (64 x 128)
-    for (int q = threadIdx.x; q < 2 * TILE * H; q += blockDim.x) {
-      const int r = q / H, c = q % H;
-      if (c < DIN) S.tA[c][r] = S.in[r][c];
-      S.tB[c][r] = S.gz1[r][c];
-    }
-    __syncthreads();
-    warp_gemm<2 * TILE, 4>(&S.tA[16 * (warp & 1)][0], 2 * TILE + 8, &S.tB[32 * (warp >> 1)][0], 2 * TILE + 8, gW1);
+    // dW2 += [a1; da1]^T [gz2; gdz2] (64 x 64 over 128 atoms), dW1 += [G; U]^T [gz1; gdz1]
+    // (32 x 64)
+    warp_gemm_t<2 * TILE, 8>(&S.act[0][16 * warp], H + 8, &S.gz2[0][0], H + 8, gW2);
+    warp_gemm_t<2 * TILE, 4>(&S.in[0][16 * (warp & 1)], DIN + 8, &S.gz1[0][32 * (warp >> 1)], H + 8, gW1);
     __syncthreads();
   }
   // block partial, FP32: layout of the packed parameters of one species
@@ -1064,46 +1130,50 @@ __global__ void __launch_bounds__(128) k_sg_train(TileArgs T, int nt0, int nb0, 
   if (threadIdx.x == 0) out[OFF_B3] = S.vb3[0] + S.vb3[1] + S.vb3[2] + S.vb3[3];
 }
 
-// grad[species][p] = sum over the species' blocks (in order) of part[b][p]
-__global__ void k_sg_reduce(const float* __restrict__ part, int nb0, int blocks, float* __restrict__ grad) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= PER_SPECIES) return;
-  const int species = blockIdx.y, b0 = species == 0 ? 0 : nb0, b1 = species == 0 ? nb0 : blocks;
+// grad[species][p] = sum over the species' blocks of part[b][p]: 8 slices of the blocks
+// per parameter, each in order, then the slices in order
+constexpr int REDUCE_PARAMS = 32, REDUCE_SLICES = 8;
+__global__ void __launch_bounds__(REDUCE_PARAMS * REDUCE_SLICES) k_sg_reduce(const float* __restrict__ part, int nb0,
+                                                                             int blocks, float* __restrict__ grad) {
+  __shared__ float sum[REDUCE_SLICES][REDUCE_PARAMS];
+  const int x = threadIdx.x % REDUCE_PARAMS, y = threadIdx.x / REDUCE_PARAMS;
+  const int p = blockIdx.x * REDUCE_PARAMS + x, species = blockIdx.y;
+  const int b0 = species == 0 ? 0 : nb0, b1 = species == 0 ? nb0 : blocks, per = (b1 - b0 + REDUCE_SLICES - 1) / REDUCE_SLICES;
   float s = 0.f;
-  constexpr int U = 8;   // partials in flight
-  for (int b = b0; b < b1; b += U) {
-    float x[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) x[u] = b + u < b1 ? part[(size_t)(b + u) * PER_SPECIES + p] : 0.f;
-#pragma unroll
-    for (int u = 0; u < U; u++)
-      if (b + u < b1) s += x[u];
-  }
+  if (p < PER_SPECIES)
+#pragma unroll 8
+    for (int b = b0 + y * per; b < min(b1, b0 + (y + 1) * per); b++) s += part[(size_t)b * PER_SPECIES + p];
+  sum[y][x] = s;
+  __syncthreads();
+  if (y != 0 || p >= PER_SPECIES) return;
+  for (int k = 1; k < REDUCE_SLICES; k++) s += sum[k][x];
   grad[species * PER_SPECIES + p] = s;
 }
 
-// Residuals of the loss: per atom e = wE 2 (E_c - Etrue_c) / (N^2 C) of its chain, per
-// component v = wF 2 / (3 N C) (F - Ftrue); out[0] = sum (E - Etrue)^2, out[1] = sum |F - Ftrue|^2.
+// Residuals of the loss: per atom e = wE 2 (E_c - Etrue_c) / (N^2 C) of its chain and the
+// vector v = wF 2 / (3 N C) (F - Ftrue); out[0] = sum (E - Etrue)^2, out[1] = sum |F - Ftrue|^2.
 constexpr int RES_THREADS = 256;
 __global__ void __launch_bounds__(RES_THREADS) k_sg_residual(const double* __restrict__ F,
                                                              const double* __restrict__ Ft,
                                                              const double* __restrict__ E,
                                                              const double* __restrict__ Et, int C, int N, double wE,
-                                                             double fscale, float* __restrict__ v,
+                                                             double fscale, float4* __restrict__ v,
                                                              float* __restrict__ eAtom, double* partials,
                                                              unsigned int* ticket, double* out, double* hostOut) {
   const int total = C * N;
   double s[2] = {0.0, 0.0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * total; i += gridDim.x * blockDim.x) {
-    const double d = __dsub_rn(F[i], Ft[i]);
-    s[1] = __dadd_rn(s[1], __dmul_rn(d, d));
-    v[i] = (float)__dmul_rn(fscale, d);
-    if (i < total) {
-      const int c = i / N;
-      const double x = __dsub_rn(E[c], Et[c]);
-      eAtom[i] = (float)(wE * 2.0 * x / ((double)N * N * C));
-      if (i == c * N) s[0] = __dadd_rn(s[0], __dmul_rn(x, x));
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    float w[3];
+    for (int k = 0; k < 3; k++) {
+      const double d = __dsub_rn(F[3 * (size_t)i + k], Ft[3 * (size_t)i + k]);
+      s[1] = __dadd_rn(s[1], __dmul_rn(d, d));
+      w[k] = (float)__dmul_rn(fscale, d);
     }
+    v[i] = make_float4(w[0], w[1], w[2], 0.f);
+    const int c = i / N;
+    const double x = __dsub_rn(E[c], Et[c]);
+    eAtom[i] = (float)(wE * 2.0 * x / ((double)N * N * C));
+    if (i == c * N) s[0] = __dadd_rn(s[0], __dmul_rn(x, x));
   }
   grid_reduce<2, RES_THREADS>(s, partials, ticket, out, hostOut);
 }
@@ -1119,7 +1189,7 @@ __global__ void k_sg_adam(float* __restrict__ p, const float* __restrict__ g, fl
   p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
-// per-chain sums of per-atom FP32 values, in atom order within each 256-atom block, blocks in order
+// per-chain sums of per-atom FP32 values in a fixed order (a block per chain)
 __global__ void k_sg_chain_sum(const float* __restrict__ x, int N, double* __restrict__ out) {
   const int c = blockIdx.x;
   __shared__ double ws[32];
@@ -1167,7 +1237,9 @@ struct Surrogate {
   float4* dPos = nullptr;
   int *dCellOf = nullptr, *dCounts = nullptr, *dStarts = nullptr, *dCursor = nullptr, *dSorted = nullptr;
   int *dList = nullptr, *dCount = nullptr, *dOverflow = nullptr;
-  float *dG = nullptr, *dEatom = nullptr, *dEdG = nullptr, *dU = nullptr, *dV = nullptr, *dEres = nullptr;
+  int *dNear = nullptr, *dNearCount = nullptr;   // neighbors within rc at the positions of the last k_sg_desc
+  float *dG = nullptr, *dEatom = nullptr, *dEdG = nullptr, *dU = nullptr, *dEres = nullptr;
+  float4* dV = nullptr;
   float *dParams = nullptr, *dPart = nullptr, *dGrad = nullptr, *dM = nullptr, *dVar = nullptr;
   int trainBlocks = 0, trainBlocks0 = 0, tiles0 = 0;   // blocks of k_sg_train, those of species 0, tiles of species 0
   int3* dTrainTiles = nullptr;                          // the tiles of <= 64 atoms, species 0 first
@@ -1298,7 +1370,9 @@ void* EmDee_surrogate_create(int chains, int N, double L, const int* types, doub
   CK(cudaMalloc(&S->dEdG, sizeof(float) * T * DIN));
   CK(cudaMalloc(&S->dEatom, sizeof(float) * T));
   CK(cudaMalloc(&S->dEres, sizeof(float) * T));
-  CK(cudaMalloc(&S->dV, sizeof(float) * 3 * T));
+  CK(cudaMalloc(&S->dV, sizeof(float4) * T));
+  CK(cudaMalloc(&S->dNear, sizeof(int) * T * S->cap));
+  CK(cudaMalloc(&S->dNearCount, sizeof(int) * T));
   CK(cudaMalloc(&S->dParams, sizeof(float) * NPARAM));
   CK(cudaMemset(S->dParams, 0, sizeof(float) * NPARAM));
   CK(cudaMalloc(&S->dGrad, sizeof(float) * NPARAM));
@@ -1307,13 +1381,13 @@ void* EmDee_surrogate_create(int chains, int N, double L, const int* types, doub
   CK(cudaMemset(S->dM, 0, sizeof(float) * NPARAM));
   CK(cudaMemset(S->dVar, 0, sizeof(float) * NPARAM));
   {
-    // one training block per SM, shared out by the species' tiles
+    // two training blocks per SM, shared out by the species' tiles
     std::vector<int3> byType;
     for (int sp = 0; sp < NS; sp++)
       for (const int3& t : S->tiles)
         if (t.z == sp) byType.push_back(t);
     for (const int3& t : S->tiles) S->tiles0 += t.z == 0;
-    const int nt = (int)byType.size(), nt1 = nt - S->tiles0, blocks = std::min(152, nt);
+    const int nt = (int)byType.size(), nt1 = nt - S->tiles0, blocks = std::min(2 * 152, nt);
     int b0 = (int)std::lround((double)blocks * S->tiles0 / nt);
     if (S->tiles0 > 0 && b0 < 1) b0 = 1;
     if (nt1 > 0 && b0 > blocks - 1) b0 = std::max(S->tiles0 > 0 ? 1 : 0, blocks - 1);
@@ -1356,7 +1430,8 @@ void EmDee_surrogate_descriptors(void* h, const double* dR, float* dGout, int re
   cudaStream_t st = (cudaStream_t)stream;
   if (rebuild) sg_build_lists(S, dR, st);
   else k_sg_pack<<<sg_blocks(S.total), 256, 0, st>>>(dR, S.total, S.L, S.dPos);
-  k_sg_desc<<<sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dList, S.dCount, S.cap, S.dG);
+  k_sg_desc<<<sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dList, S.dCount, S.cap, S.dG,
+                                                                 S.dNear, S.dNearCount);
   CK(cudaGetLastError());
   if (dGout) CK(cudaMemcpyAsync(dGout, S.dG, sizeof(float) * S.total * DIN, cudaMemcpyDeviceToDevice, st));
 }
@@ -1369,9 +1444,10 @@ int EmDee_surrogate_forces(void* h, const double* dR, double* dF, double* dE, in
   cudaStream_t st = (cudaStream_t)stream;
   EmDee_surrogate_descriptors(h, dR, nullptr, rebuild, stream);
   sg_network(S, S.dParams, st);
-  k_sg_force<<<sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dList, S.dCount, S.cap, S.dEdG, dF);
+  k_sg_force<<<sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dNear, S.dNearCount, S.cap,
+                                                                  S.dEdG, dF);
   CK(cudaGetLastError());
-  if (dE) k_sg_chain_sum<<<S.G.chains, 256, 0, st>>>(S.dEatom, S.G.N, dE);
+  if (dE) k_sg_chain_sum<<<S.G.chains, 1024, 0, st>>>(S.dEatom, S.G.N, dE);
   int ov = 0;
   if (rebuild) {
     int flags[2];
@@ -1405,15 +1481,16 @@ void EmDee_surrogate_gradient(void* h, const double* dR, const double* dEtrue, c
   const int C = S.G.chains, N = S.G.N;
   EmDee_surrogate_forces(h, dR, S.dF, S.dE, 1, stream);
   const double fscale = wF * 2.0 / (3.0 * N * C);
-  k_sg_residual<<<std::min(SG_RES_BLOCKS, sg_blocks(3 * S.total)), RES_THREADS, 0, st>>>(
+  k_sg_residual<<<std::min(SG_RES_BLOCKS, sg_blocks(S.total)), RES_THREADS, 0, st>>>(
       S.dF, dFtrue, S.dE, dEtrue, C, N, wE, fscale, S.dV, S.dEres, S.dResPart, S.dTicket,
       S.dResPart + 2 * SG_RES_BLOCKS, S.hLoss);
-  k_sg_udesc<<<sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dList, S.dCount, S.cap,
-                                                                  S.dV, S.dU);
+  k_sg_udesc<<<sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dNear, S.dNearCount,
+                                                                  S.cap, S.dV, S.dU);
   TileArgs T{S.dAtoms, S.dTrainTiles, (int)S.tiles.size()};
   k_sg_train<<<S.trainBlocks, 128, sizeof(TrainSmem), st>>>(T, S.tiles0, S.trainBlocks0, S.dParams, S.dG, S.dU,
                                                             S.dEres, S.dPart);
-  k_sg_reduce<<<dim3((PER_SPECIES + 255) / 256, NS), 256, 0, st>>>(S.dPart, S.trainBlocks0, S.trainBlocks, dGrad);
+  k_sg_reduce<<<dim3((PER_SPECIES + REDUCE_PARAMS - 1) / REDUCE_PARAMS, NS), REDUCE_PARAMS * REDUCE_SLICES, 0, st>>>(
+      S.dPart, S.trainBlocks0, S.trainBlocks, dGrad);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(st));
   loss[0] = wE * S.hLoss[0] / ((double)N * N * C);
@@ -1451,7 +1528,7 @@ void EmDee_surrogate_destroy(void* h) {
   if (!S) return;
   void* ptrs[] = {S->dSpecies, S->dAtoms, S->dTiles, S->dTiles128, S->dTcError, S->dPos, S->dCellOf, S->dCounts, S->dStarts, S->dCursor,
                   S->dSorted, S->dList, S->dCount, S->dOverflow, S->dG, S->dU, S->dEdG, S->dEatom, S->dEres,
-                  S->dV, S->dParams, S->dGrad, S->dM, S->dVar, S->dPart, S->dR0, S->dTrainTiles, S->dF, S->dE, S->dResPart,
+                  S->dV, S->dParams, S->dGrad, S->dM, S->dVar, S->dPart, S->dR0, S->dNear, S->dNearCount, S->dTrainTiles, S->dF, S->dE, S->dResPart,
                   S->dTicket};
   for (void* p : ptrs) cudaFree(p);
   cudaFreeHost(S->hLoss);
