@@ -616,6 +616,7 @@ void EmDee_destroy(tEmDee* md) {
   cudaFree(g.dNbOuter); cudaFree(g.dNbCountOuter); cudaFree(g.dROuter);
   cudaFree(s->models.d64); cudaFree(s->models.d32); cudaFree(s->models.coul64); cudaFree(s->models.coul32);
   cudaFree(s->models.interact);
+  cudaFree(s->dRdf);
   cudaFree(s->dPartials);
   cudaFree(s->dKE);
   cudaFree(s->dTicket);

@@ -412,12 +412,9 @@ bool device_pair_forces(System& s, bool compute, bool speculative) {
   const bool chain = s.keChainReq && s.precision == 0 && s.nbodies == 0 && s.bondedTerms.bonds.empty() &&
                      s.bondedTerms.angles.empty() && !s.coul[l2].requires_kspace;
   if (chain) launch_kinetic_two(s, s.keChainCF, speculative ? s.dResult + 9 : nullptr);
-  // Mixed precision: the last block of the pair kernel wrote the sums, and the fused
-  // step the skin value and rebuild flag ([8], [9]), straight into the pinned hResult,
-  // so one synchronisation returns all of them.  FP64 mode copies them back.
-  if (s.precision == 1)
-    CK(cudaMemcpyAsync(s.hResult, s.dResult, (speculative ? 10 : 4) * sizeof(double), cudaMemcpyDeviceToHost,
-                       s.stream));
+  // The last block of the pair kernel wrote the sums, and the fused step the skin value
+  // and rebuild flag ([8], [9]), straight into the pinned hResult, so one synchronisation
+  // returns all of them.
   CK(cudaStreamSynchronize(s.stream));
   if (speculative && s.hResult[9] != 0.0) {
     if (chain) prof_drop_last(s);   // the kinetic pass returned at once as well

@@ -401,14 +401,17 @@ __global__ void k_pack_delta(const double* __restrict__ R, const double* __restr
                        scale);
 }
 
-// scaled FP64 coordinates Rs = R/L (src/EmDeeCode.f90:1228) in slot order
-__global__ void k_pack_fp64(const double* __restrict__ R, const int* orig, int N, double L, double* Rs) {
+// scaled FP64 coordinates Rs = R/L (src/EmDeeCode.f90:1228) in slot order, and their box
+// fractions (the FP64 mode has no FP32 positions between builds: they take that array)
+__global__ void k_pack_fp64(const double* __restrict__ R, const int* orig, int N, double L, double* Rs, int4* frac) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= N) return;
   int a = orig[s];
-  Rs[3 * s] = R[3 * a] / L;
-  Rs[3 * s + 1] = R[3 * a + 1] / L;
-  Rs[3 * s + 2] = R[3 * a + 2] / L;
+  const double x = R[3 * a] / L, y = R[3 * a + 1] / L, z = R[3 * a + 2] / L;
+  Rs[3 * s] = x;
+  Rs[3 * s + 1] = y;
+  Rs[3 * s + 2] = z;
+  frac[s] = make_int4(box_fraction(x), box_fraction(y), box_fraction(z), 0);
 }
 
 void device_pack(System& s) {
@@ -416,7 +419,7 @@ void device_pack(System& s) {
   int N = s.natoms, th = 256, bl = (N + th - 1) / th;
   prof_begin(s, PK_PACK);
   if (s.precision == 1) {
-    k_pack_fp64<<<bl, th, 0, s.stream>>>(s.dR, g.dOrig, N, *s.Lbox, g.dRs64);
+    k_pack_fp64<<<bl, th, 0, s.stream>>>(s.dR, g.dOrig, N, *s.Lbox, g.dRs64, (int4*)g.dPos4);
   } else if (*s.Lbox == s.builtL) {
     k_pack_delta<<<bl, th, 0, s.stream>>>(s.dR, s.dR0, g.dOrig, g.dPos0, N, (float)((double)g.M / *s.Lbox), g.dPos4);
   } else {   // the box changed since the build: from the coordinates
@@ -1116,7 +1119,7 @@ static bool build_lists(System& s, bool reuse) {
     g.tileStride = hmax[0] > 24 ? (hmax[0] + 31) / 32 * 32 : std::max(8, (hmax[0] + 7) / 8 * 8);
     g.maxHalo = hmax[1];
     size_t smem = build_smem(g, s.ntypes, build_general(s));
-    size_t smem64 = (size_t)(g.maxHalo + 1) * (4 * sizeof(double) + 1) + 2 * sizeof(int) * (g.haloCells + 1) + 64;
+    size_t smem64 = (size_t)(g.maxHalo + 1) * (4 * sizeof(double) + sizeof(int4) + 1) + 64;
     if ((g.maxHalo > 65534 || smem > smemLimit || (s.precision == 1 && smem64 > smemLimit)) && TB > 1) {
       TB--;
       continue;
@@ -1457,60 +1460,94 @@ long device_neighbor_pairs(System& s, int* pairs, long capacity) {
 
 struct RdfArgs {
   TileGeom g;
-  const int2* tab;
+  const int* layout;
   const int* start;
   const int* orig;
+  const uint16_t* self;
   const uint16_t* nb;
   const int* count;   // entries to scan per slot (all, or the inner part)
   const uint8_t* type8;
   const double* R;
   int cap, tileStride, bins, ntp;   // ntp: histogram rows (type pairs, symm1D order)
   double invL, Rc2, binsByRc;
+  float limit;   // box_limit(Rc2)
   const uint8_t* hasPair;   // [type] (0-based)
   const uint8_t* pairOn;    // [ti * ntypes + tj]
   int ntypes, haloCap;
-  unsigned long long* hist;   // [pair][bin], every pair counted from both of its atoms
+  unsigned long long* hist;   // [pair][bin]
   int sharedHist;             // histogram fits in shared memory
 };
 
-__global__ void k_rdf(RdfArgs A) {
-  extern __shared__ int dyn[];
-  __shared__ int ws[33];
-  __shared__ int off[1001], cst[1000];
+static const int RDF_THREADS = 128;
+
+// A halo atom as the histogram needs it: scaled coordinates, slot, type; box fractions
+// and slot
+struct __align__(16) RdfAtom {
+  double x, y, z;
+  int slot, type;
+  int4 frac;
+};
+
+// The lists hold every pair twice, at the same distance: it is counted from one of its
+// atoms, the lower slot if the slots' sum is even and the higher one if it is odd (half of
+// every atom's pairs).  The FP64 distance, bound by its pipe, is evaluated for the entries
+// that a mask of FP32 tests leaves, on nearly full warps.  32,003
+// atoms, 100 bins: 330 us with both directions, FP64 rounding and gathers of R, 140 us so.
+// STAGED: the halo atoms are staged as RdfAtom; tiles whose halo does not fit so keep
+// the slots only and gather the rest.
+template <bool STAGED>
+__global__ void __launch_bounds__(RDF_THREADS) k_rdf(RdfArgs A) {
+  extern __shared__ __align__(16) unsigned char sraw[];
   const TileGeom g = A.g;
   const int t = blockIdx.x, cells = g.TB * g.TB * g.TB;
-  int* hslot = dyn;   // halo index -> slot, then the block's histogram
-  halo_layout(g, t, A.tab, A.start, off, cst, (int*)nullptr, ws);
-  unsigned int* sh = (unsigned int*)(hslot + A.haloCap);
-  for (int h = threadIdx.x; h < g.haloCells; h += blockDim.x)
-    for (int k = off[h]; k < off[h + 1]; k++) hslot[k] = cst[h] + (k - off[h]);
+  RdfAtom* halo = (RdfAtom*)sraw;
+  int* hslot = (int*)sraw;
+  unsigned int* sh = STAGED ? (unsigned int*)(halo + A.haloCap) : (unsigned int*)(hslot + A.haloCap);
+  auto slot = [&](int q) { return STAGED ? halo[q].slot : hslot[q]; };
+  auto load = [&](int sj) {
+    const int a = A.orig[sj];
+    const double x = A.invL * A.R[3 * a], y = A.invL * A.R[3 * a + 1], z = A.invL * A.R[3 * a + 2];
+    return RdfAtom{x, y, z, sj, A.type8[sj], make_int4(box_fraction(x), box_fraction(y), box_fraction(z), sj)};
+  };
+  const int* lay = A.layout + (size_t)t * (2 * g.haloCells + 1);
+  for (int h = threadIdx.x; h < g.haloCells; h += blockDim.x) {
+    const int b = lay[h], e = lay[h + 1], s0 = lay[g.haloCells + 1 + h];
+    for (int q = b; q < e; q++) (STAGED ? halo[q].slot : hslot[q]) = s0 + q - b;
+  }
   const int hn = A.bins * A.ntp;
   if (A.sharedHist)
     for (int k = threadIdx.x; k < hn; k += blockDim.x) sh[k] = 0u;
   __syncthreads();
+  if (STAGED) {
+    const int nh = lay[g.haloCells];
+    for (int q = threadIdx.x; q < nh; q += blockDim.x) halo[q] = load(halo[q].slot);
+    __syncthreads();
+  }
   const int tb = A.start[t * cells], te = A.start[(t + 1) * cells];
   for (int li = threadIdx.x; li < te - tb; li += blockDim.x) {
-    const int si = tb + li, ai = A.orig[si], ti = A.type8[si];
-    if (!A.hasPair[ti]) continue;
-    const double xi = A.invL * A.R[3 * ai], yi = A.invL * A.R[3 * ai + 1], zi = A.invL * A.R[3 * ai + 2];
+    const int si = tb + li;
+    const RdfAtom pi = STAGED ? halo[A.self[si]] : load(si);
+    if (!A.hasPair[pi.type]) continue;
     const int n = A.count[si];
-    for (int k = 0; k < n; k++) {
-      const int q = A.nb[nb_index(t, A.cap >> 3, A.tileStride, li, k)];
-      const int sj = hslot[q], aj = A.orig[sj], tj = A.type8[sj];
-      if (!A.pairOn[ti * A.ntypes + tj]) continue;
-      double dx = xi - A.invL * A.R[3 * aj], dy = yi - A.invL * A.R[3 * aj + 1], dz = zi - A.invL * A.R[3 * aj + 2];
-      dx = dx - round(dx);
-      dy = dy - round(dy);
-      dz = dz - round(dz);
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      if (r2 < A.Rc2) {
-        int bin = (int)(sqrt(r2) * A.binsByRc);
-        bin = min(bin, A.bins - 1);
-        const int a = min(ti, tj), b = max(ti, tj), p = a + (b + 1) * b / 2;   // symm1D - 1 (0-based types)
-        if (A.sharedHist) atomicAdd(&sh[p * A.bins + bin], 1u);
-        else atomicAdd(&A.hist[(size_t)p * A.bins + bin], 1ull);
-      }
-    }
+    const uint4* lp = reinterpret_cast<const uint4*>(A.nb) + ((size_t)t * (A.cap >> 3) * A.tileStride + li);
+    masked_entries(
+        lp, A.tileStride, n,
+        [&](int q) {
+          const int sj = slot(q);
+          if (((si ^ sj) & 1) ? si < sj : si > sj) return false;
+          return !STAGED || box_dist2(pi.frac, halo[q].frac) < A.limit;
+        },
+        [&](int q) {
+          const RdfAtom pj = STAGED ? halo[q] : load(hslot[q]);
+          if (!A.pairOn[pi.type * A.ntypes + pj.type]) return;
+          const double dx = wrap_half(pi.x - pj.x), dy = wrap_half(pi.y - pj.y), dz = wrap_half(pi.z - pj.z);
+          const double r2 = dx * dx + dy * dy + dz * dz;
+          if (!(r2 < A.Rc2)) return;
+          const int bin = min((int)(sqrt(r2) * A.binsByRc), A.bins - 1);
+          const int a = min(pi.type, pj.type), b = max(pi.type, pj.type), p = a + (b + 1) * b / 2;   // symm1D - 1 (0-based types)
+          if (A.sharedHist) atomicAdd(&sh[p * A.bins + bin], 1u);
+          else atomicAdd(&A.hist[(size_t)p * A.bins + bin], 1ull);
+        });
   }
   if (A.sharedHist) {
     __syncthreads();
@@ -1526,9 +1563,10 @@ void device_rdf_counts(System& s, int bins, double Rc, const std::vector<uint8_t
   const int nt = s.ntypes;
   RdfArgs A;
   A.g = make_geom(g.M, g.TB);
-  A.tab = g.dHaloTab;
+  A.layout = g.dLayout;
   A.start = g.dStart;
   A.orig = g.dOrig;
+  A.self = g.dSelf;
   A.nb = g.dNb;
   A.count = Rc < 1.0001 * s.InRc ? g.dNbInner : g.dNbCount;
   A.type8 = g.dType8;
@@ -1540,35 +1578,37 @@ void device_rdf_counts(System& s, int bins, double Rc, const std::vector<uint8_t
   const double invL = 1.0 / *s.Lbox;
   A.invL = invL;
   A.Rc2 = Rc * Rc * (invL * invL);
+  A.limit = box_limit(A.Rc2);
   A.binsByRc = bins / (Rc * invL);
   A.ntypes = nt;
   A.haloCap = g.maxHalo;
-  const size_t hn = (size_t)bins * ntp;
-  uint8_t *dHas, *dOn;
-  unsigned long long* dHist;
-  CK(cudaMalloc(&dHas, nt));
-  CK(cudaMalloc(&dOn, (size_t)nt * nt));
-  CK(cudaMalloc(&dHist, sizeof(unsigned long long) * hn));
-  CK(cudaMemcpy(dHas, hasPair.data(), nt, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(dOn, pairOn.data(), (size_t)nt * nt, cudaMemcpyHostToDevice));
-  CK(cudaMemsetAsync(dHist, 0, sizeof(unsigned long long) * hn, s.stream));
+  // histogram, then the two type filters: one buffer kept with the system
+  const size_t hn = (size_t)bins * ntp, bytes = sizeof(unsigned long long) * hn, filters = (size_t)nt + (size_t)nt * nt;
+  if (s.rdfCap < bytes + filters) {
+    CK(cudaFree(s.dRdf));
+    CK(cudaMalloc(&s.dRdf, bytes + filters));
+    s.rdfCap = bytes + filters;
+  }
+  uint8_t* dHas = s.dRdf + bytes;
+  std::vector<uint8_t> host(hasPair);
+  host.insert(host.end(), pairOn.begin(), pairOn.end());
+  CK(cudaMemsetAsync(s.dRdf, 0, bytes, s.stream));
+  CK(cudaMemcpyAsync(dHas, host.data(), filters, cudaMemcpyHostToDevice, s.stream));
   A.hasPair = dHas;
-  A.pairOn = dOn;
-  A.hist = dHist;
-  size_t smem = sizeof(int) * (size_t)g.maxHalo;
+  A.pairOn = dHas + nt;
+  A.hist = (unsigned long long*)s.dRdf;
   A.sharedHist = (hn * sizeof(unsigned int) <= 48 * 1024) ? 1 : 0;
-  if (A.sharedHist) smem += hn * sizeof(unsigned int);
-  CK(cudaFuncSetAttribute(k_rdf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_rdf<<<g.nTiles, 128, smem, s.stream>>>(A);
+  const size_t histBytes = A.sharedHist ? hn * sizeof(unsigned int) : 0;
+  const bool staged = sizeof(RdfAtom) * (size_t)g.maxHalo + histBytes <= 200 * 1024;
+  const size_t smem = (staged ? sizeof(RdfAtom) : sizeof(int)) * (size_t)g.maxHalo + histBytes;
+  auto kern = staged ? k_rdf<true> : k_rdf<false>;
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<g.nTiles, std::min(RDF_THREADS, (g.tileAtoms + 31) / 32 * 32), smem, s.stream>>>(A);
   CK(cudaGetLastError());
   s.prof.total++;
   counts.assign(hn, 0ull);
+  CK(cudaMemcpyAsync(counts.data(), s.dRdf, bytes, cudaMemcpyDeviceToHost, s.stream));
   CK(cudaStreamSynchronize(s.stream));
-  CK(cudaMemcpy(counts.data(), dHist, sizeof(unsigned long long) * hn, cudaMemcpyDeviceToHost));
-  for (auto& c : counts) c /= 2;   // full lists hold every pair twice, at the same distance
-  CK(cudaFree(dHas));
-  CK(cudaFree(dOn));
-  CK(cudaFree(dHist));
 }
 
 // ---------------------------------------------------------------------------------

@@ -273,6 +273,10 @@ struct System {
   int* hFlags = nullptr;       // pinned: [0] largest filtered list of the last filtering launch,
                                // [2..3] largest list and tile-size overflow of the last list build
 
+  // EmDee_rdf: histogram and type filters
+  uint8_t* dRdf = nullptr;
+  size_t rdfCap = 0;
+
   // reduction scratch
   double* dPartials = nullptr;   // per tile: Epair, Ecoul, Wpair, Wcoul, pairs within rc
   int partialCap = 0;

@@ -77,6 +77,64 @@ static __device__ __noinline__ bool exact_inside(const double* R, double L, int 
   return r2 < thr;
 }
 
+// x - round(x), where |x| < 1/2 (tested on the bits) needs no FP64 operation
+__device__ __forceinline__ double wrap_half(double x) {
+  return (__double2hiint(x) & 0x7FFFFFFF) < 0x3FE00000 ? x : __dsub_rn(x, round(x));
+}
+
+// Fraction of the box of a scaled coordinate, in units of 2^-32, modulo 1: the low word
+// of x 2^32 + 1.5 2^52.  Differences of two such numbers are minimum images as they
+// stand (32-bit wrap-around).
+__device__ __forceinline__ int box_fraction(double x) {
+  if ((__double2hiint(x) & 0x7FFFFFFF) >= 0x41200000) x = __dsub_rn(x, floor(x));   // 2^19 boxes away
+  return __double2loint(fma(x, 4294967296.0, 6755399441055744.0));
+}
+// squared distance of two atoms in those units, FP32 (relative error ~3e-7)
+__device__ __forceinline__ float box_dist2(int4 a, int4 b) {
+  const float dx = (float)(a.x - b.x), dy = (float)(a.y - b.y), dz = (float)(a.z - b.z);
+  return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+}
+// Limit below which box_dist2 may belong to a pair with r^2 < r2 (scaled FP64 units)
+inline float box_limit(double r2) { return (float)(r2 * 18446744073709551616.0 * (1.0 + 2e-6)); }
+
+// The entries of an atom's list for which keep(q) holds, visited in order as f(q), 128 at
+// a time: the masks come from cheap tests first, so that the lanes of a warp, whose kept
+// entries differ in place but hardly in number, run f together.  lp: the atom's first
+// chunk, chunk c at lp[c * stride].
+template <class Keep, class F>
+__device__ __forceinline__ void masked_entries(const uint4* __restrict__ lp, int stride, int n, Keep&& keep, F&& f) {
+  for (int k0 = 0; k0 < n; k0 += 128) {
+    unsigned m[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int w = 0; w < 4; w++)
+      for (int c = 0; c < 4 && k0 + 32 * w + 8 * c < n; c++) {
+        const uint4 x = lp[(size_t)((k0 >> 3) + 4 * w + c) * stride];
+        const unsigned words[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int e = 0; e < 8; e++)
+          if (k0 + 32 * w + 8 * c + e < n && keep((int)((words[e >> 1] >> ((e & 1) * 16)) & 0xFFFF)))
+            m[w] |= 1u << (8 * c + e);
+      }
+    auto next = [&] {   // halo index of the next kept entry, -1 after the last
+      const int w = m[0] ? 0 : m[1] ? 1 : m[2] ? 2 : 3;
+      const unsigned x = m[0] ? m[0] : m[1] ? m[1] : m[2] ? m[2] : m[3];
+      if (x == 0) return -1;
+      const int e = __ffs(x) - 1;
+      if (m[0]) m[0] &= m[0] - 1;
+      else if (m[1]) m[1] &= m[1] - 1;
+      else if (m[2]) m[2] &= m[2] - 1;
+      else m[3] &= m[3] - 1;
+      const int k = k0 + 32 * w + e;
+      return (int)reinterpret_cast<const uint16_t*>(lp + (size_t)(k >> 3) * stride)[k & 7];
+    };
+    for (int q = next(); q >= 0;) {
+      const int after = next();   // its load is in flight during f
+      f(q);
+      q = after;
+    }
+  }
+}
+
 // Exclusive scan over n <= blockDim.x * ITEMS ints held in shared memory
 // (in place); returns the total.  All threads of the block must call it.
 template <int ITEMS>
