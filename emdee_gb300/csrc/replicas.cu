@@ -8,12 +8,12 @@
 // it fires, the pair forces, boost(dt/2) -- so a whole trajectory of hundreds of
 // replicas is one launch (captured once in a CUDA graph and replayed).
 //
-// Per replica, in shared memory: the FP32 positions of its atoms in cell units
-// relative to each atom's cell at the last build (slot order), the cell starts
-// and the 125 stencil offsets.  In global memory: R, P, F, R0 of the system
-// (FP64, API order) and the replica's own cell-sorted order, build-time cells
-// and full neighbor lists (column-major, 32-bit entries: slot | stencil code).
-// Blocks are issued largest replica first.
+// Per replica, in shared memory: the positions of its atoms as 32-bit fractions of the
+// box (slot order), whose differences are minimum images without image arithmetic and
+// finer than FP32 coordinates, and the cell starts.  In global memory: R, P, F, R0 of
+// the system (FP64, API order) and the replica's own cell-sorted order and full neighbor
+// lists (8 slots of 16 bits per 16-byte chunk, chunk-major).  Blocks are issued largest
+// replica first.
 //
 // Scope: up to 8 atom types (pair models with their modifiers), no charges, no
 // rigid bodies, no exclusions, one model layer, FP32 pair arithmetic (the mixed
@@ -36,17 +36,19 @@ struct RepDesc {
   const double* invMass;
   int unitMass;
   int N, M, minimg, cap;
-  double L, scale, skinSq, thr;   // scale = M / L; thr = (rc+skin)^2 / L^2
-  float lo2, hi2, rc2, invw2, invw, Mf;
+  double L, frac, skinSq, thr;   // frac = 2^32 / L; thr = (rc+skin)^2 / L^2
+  float lo2, hi2, Mf;            // list band, cell units^2
+  float rc2, unit, unit2;        // cut-off^2 in box fractions^2; 2^32 / L and its square
   PairEntry<float> model;          // type pair (1, 1)
   int ntypes;
   int ljAll;                       // every type pair is lj_cut without modifier
   const PairEntry<float>* table;   // the system's layer-1 pair table, [jtype][itype]
   const int* type;                 // atom types (1-based, API order)
   int* orig;        // slot -> atom
-  int4* K;          // per slot: build-time unwrapped cell (x, y, z), cell rank (w)
-  int4* atomK;      // per atom scratch of the same
-  uint32_t* list;   // entries 4c..4c+3 of slot i: the 16 bytes at list[(c * N + i) * 4]
+  uint16_t* slotOf; // atom -> slot
+  int4* frac4;      // per atom: box fractions and cell during a build
+  double* Rb;       // coordinates of the build that made the lists below
+  uint4* list;      // entries 8c..8c+7 of slot i: list[c * N + i]
   int* count;       // per slot
   double* out;      // [0] Epair [1] Wpair [2..4] 2KE per dim [5] builds [6] overflow [7] steps done
   int computeLast;  // unused by the kernel (host bookkeeping)
@@ -82,63 +84,64 @@ __device__ __forceinline__ RepMP rep_warp_ordered(RepMP acc) {
   return acc;
 }
 
-// cell and unwrapped cell of an atom (src/neighbor_lists.f90:126-127, index clamped to M-1)
-__device__ __forceinline__ int4 rep_cell(const double* R, int a, double L, int M) {
-  int c[3], K[3];
-  for (int d = 0; d < 3; d++) {
-    double rs = R[3 * a + d] / L, fl = floor(rs);
-    int ci = (int)(M * (rs - fl));
-    ci = ci < 0 ? 0 : (ci >= M ? M - 1 : ci);
-    c[d] = ci;
-    K[d] = (int)fl * M + ci;
-  }
-  return make_int4(K[0], K[1], K[2], c[0] + M * (c[1] + M * c[2]));
-}
-
 struct RepShared {
   RepDesc d;
   int rebuild, overflow;
+  int scan[33];
   RepMP wmp[32];
   float2 wff[2][32];
   double wke[3][32];
 };
 
+// box fraction of a coordinate: low word of R 2^32 / L + 1.5 2^52
+__device__ __forceinline__ int rep_fraction(double r, const RepDesc& D) {
+  const double t = fma(r, D.frac, 6755399441055744.0);
+  if ((__double2hiint(t) & 0xFFF00000) == 0x43300000) return __double2loint(t);
+  return __double2loint(fma(r / D.L - floor(r / D.L), 4294967296.0, 6755399441055744.0));   // 2^19 boxes away
+}
+
+static const int REP_PAD = 4;   // positions a segment of four may read past the last one
+
+// Cells, cell-sorted order and full lists from the coordinates Rb.  The cell of an atom is
+// the product of its box fraction and M (a cell index that differs from the reference's
+// int(M Rs) by rounding changes only the order of candidates).  Lists as k_build makes
+// them: 25 rows of up to 5 cells (one or two runs of slots where a row wraps around the
+// box), only cells in reach of the row's distance, candidates tested into a mask four at
+// a time, 8 entries stored at once.  (8000 atoms on one SM: 1.35 ms when every atom went
+// through all 125 cells one candidate at a time with FP64 cell indices, about
+// 0.75 ms so.)
 template <int THREADS>
-__device__ void rep_build(RepShared& S, const double* Rb, float4* pos, int* cellStart, int* cursor,
-                          const float4* offTab, bool copyR0, uint8_t* stype) {
+__device__ __noinline__ void rep_build(RepShared& S, const double* Rb, float4* pos, int* cellStart, int* cursor,
+                                       bool copyR0) {
   const RepDesc& D = S.d;
   const int N = D.N, M = D.M, cells = M * M * M;
-  for (int c = threadIdx.x; c < cells; c += THREADS) cursor[c] = 0;
+  for (int c = threadIdx.x; c < cells; c += THREADS) cellStart[c] = 0;
   __syncthreads();
   for (int a = threadIdx.x; a < N; a += THREADS) {
-    const int4 k = rep_cell(Rb, a, D.L, M);
-    D.atomK[a] = k;
-    atomicAdd(&cursor[k.w], 1);
-  }
-  __syncthreads();
-  // exclusive scan of the cell counts into cellStart (a single warp walks the cells)
-  if (threadIdx.x < 32) {
-    int carry = 0;
-    for (int base = 0; base < cells; base += 32) {
-      const int c = base + threadIdx.x;
-      const int v = c < cells ? cursor[c] : 0;
-      int incl = v;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if ((int)threadIdx.x >= o) incl += y;
-      }
-      if (c < cells) cellStart[c] = carry + incl - v;
-      carry += __shfl_sync(0xffffffffu, incl, 31);
+    int f[3], cell = 0;
+    for (int d = 2; d >= 0; d--) {
+      const double r = Rb[3 * a + d];
+      f[d] = rep_fraction(r, D);
+      cell = (int)__umulhi((unsigned)f[d], (unsigned)M) + M * cell;
+      D.Rb[3 * a + d] = r;
+      if (copyR0) D.R0[3 * a + d] = r;
     }
-    if (threadIdx.x == 0) cellStart[cells] = carry;
+    D.frac4[a] = make_int4(f[0], f[1], f[2], cell);
+    atomicAdd(&cellStart[cell], 1);
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < cells; c += THREADS) cursor[c] = 0;
-  __syncthreads();
-  for (int a = threadIdx.x; a < N; a += THREADS) {
-    const int r = D.atomK[a].w;
-    D.orig[cellStart[r] + atomicAdd(&cursor[r], 1)] = a;
+  constexpr int ITEMS = 8192 / THREADS;
+  int carry = 0;
+  for (int base = 0; base < cells; base += THREADS * ITEMS) {
+    const int n = min(THREADS * ITEMS, cells - base);
+    const int total = block_exclusive_scan<ITEMS>(cellStart + base, n, S.scan);
+    for (int c = threadIdx.x; c < n; c += THREADS) cursor[base + c] = cellStart[base + c] += carry;
+    carry += total;
+    __syncthreads();
   }
+  if (threadIdx.x == 0) cellStart[cells] = N;
+  __syncthreads();
+  for (int a = threadIdx.x; a < N; a += THREADS) D.orig[atomicAdd(&cursor[D.frac4[a].w], 1)] = a;
   __syncthreads();
   // deterministic order inside a cell: ascending atom index
   for (int c = threadIdx.x; c < cells; c += THREADS) {
@@ -154,129 +157,193 @@ __device__ void rep_build(RepShared& S, const double* Rb, float4* pos, int* cell
     }
   }
   __syncthreads();
+  // positions in cell edges (FP32), with the cell
   for (int s = threadIdx.x; s < N; s += THREADS) {
     const int a = D.orig[s];
-    const int4 k = D.atomK[a];
-    D.K[s] = k;
-    pos[s] = make_float4((float)(Rb[3 * a] * D.scale - (double)k.x), (float)(Rb[3 * a + 1] * D.scale - (double)k.y),
-                         (float)(Rb[3 * a + 2] * D.scale - (double)k.z), 0.f);
-    stype[s] = (uint8_t)(D.ntypes > 1 ? D.type[a] - 1 : 0);
+    const int4 f = D.frac4[a];
+    const float u = 2.3283064365386963e-10f;   // 2^-32
+    const int cx = f.w % M, cy = f.w / M % M, cz = f.w / (M * M);
+    pos[s] = make_float4((float)cx + u * (float)((unsigned)f.x * (unsigned)M), (float)cy + u * (float)((unsigned)f.y * (unsigned)M),
+                         (float)cz + u * (float)((unsigned)f.z * (unsigned)M), __int_as_float(f.w));
+    D.slotOf[a] = (uint16_t)s;
   }
+  if (threadIdx.x < REP_PAD) pos[N + threadIdx.x] = make_float4(1e9f, 1e9f, 1e9f, 0.f);
   __syncthreads();
-  // full lists: 125 stencil cells, candidate order (z, y, x, slot).  M >= 5, so
-  // a neighbour coordinate c + s (|s| <= 2) wraps by at most one period.
+  const int loBits = __float_as_int(D.lo2);
+  const unsigned band = (unsigned)(__float_as_int(D.hi2) - loBits);
+  const float Mf = D.Mf, invM = 1.0f / Mf, hi2 = D.hi2;
+  const bool minimg = D.minimg;
+  const int cap = D.cap;
   for (int i = threadIdx.x; i < N; i += THREADS) {
-    const int4 ki = D.K[i];
-    const int cx = ki.w % M, cy = (ki.w / M) % M, cz = ki.w / (M * M);
     const float4 pi = pos[i];
+    const int cell = __float_as_int(pi.w), cx = cell % M, cy = cell / M % M, cz = cell / (M * M);
     const int ai = D.orig[i];
+    uint4 w = make_uint4(0u, 0u, 0u, 0u);
+    uint4* out = D.list + i;
     int n = 0;
-    for (int code = 0; code < 125; code++) {
-      const int sx = code % 5 - 2, sy = (code / 5) % 5 - 2, sz = code / 25 - 2;
-      int nx = cx + sx, ny = cy + sy, nz = cz + sz;
-      nx += nx < 0 ? M : (nx >= M ? -M : 0);
-      ny += ny < 0 ? M : (ny >= M ? -M : 0);
-      nz += nz < 0 ? M : (nz >= M ? -M : 0);
-      const int nc = nx + M * (ny + M * nz);
-      const float4 o = offTab[code];
-      for (int j = cellStart[nc]; j < cellStart[nc + 1]; j++) {
-        if (j == i) continue;
-        const float4 pj = pos[j];
-        float dx = (pi.x - pj.x) - o.x, dy = (pi.y - pj.y) - o.y, dz = (pi.z - pj.z) - o.z;
-        if (D.minimg) {
-          dx -= D.Mf * rintf(dx / D.Mf);
-          dy -= D.Mf * rintf(dy / D.Mf);
-          dz -= D.Mf * rintf(dz / D.Mf);
+    auto push = [&](int q) {
+      w.x = __funnelshift_r(w.x, w.y, 16);
+      w.y = __funnelshift_r(w.y, w.z, 16);
+      w.z = __funnelshift_r(w.z, w.w, 16);
+      w.w = __funnelshift_r(w.w, (unsigned)q, 16);
+      n++;
+      if ((n & 7) == 0) {
+        if (n <= cap) *out = w;
+        out += N;
+      }
+    };
+    for (int r = 0; r < 25; r++) {
+      const int sy = r % 5 - 2, sz = r / 5 - 2;
+      int ny = cy + sy, nz = cz + sz, c0 = cx - 2, c1 = cx + 2;
+      if (!minimg) {
+        const float dy = fmaxf(fmaxf((float)ny - pi.y, pi.y - (float)(ny + 1)) - 1e-3f, 0.0f);
+        const float dz = fmaxf(fmaxf((float)nz - pi.z, pi.z - (float)(nz + 1)) - 1e-3f, 0.0f);
+        const float rem = hi2 - fmaf(dy, dy, dz * dz);
+        if (rem <= 0.0f) continue;
+        const float reach = fmaf(rem, rsqrtf(rem), 1e-3f);
+        c0 = max(c0, (int)floorf(pi.x - reach));
+        c1 = min(c1, (int)floorf(pi.x + reach));
+      }
+      const float py = pi.y - (ny < 0 ? -Mf : ny >= M ? Mf : 0.f), pz = pi.z - (nz < 0 ? -Mf : nz >= M ? Mf : 0.f);
+      ny += ny < 0 ? M : ny >= M ? -M : 0;
+      nz += nz < 0 ? M : nz >= M ? -M : 0;
+      const int* row = cellStart + M * (ny + M * nz);
+      // the run of slots inside the box, and the one across its face if the row wraps
+      for (int part = 0; part < 2; part++) {
+        int a0 = max(c0, 0), a1 = min(c1, M - 1);
+        float px = pi.x;
+        if (part == 1) {
+          if (c0 < 0) {
+            a0 = c0 + M;
+            a1 = M - 1;
+            px += Mf;
+          } else if (c1 >= M) {
+            a0 = 0;
+            a1 = c1 - M;
+            px -= Mf;
+          } else {
+            break;
+          }
         }
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        if (r2 >= D.hi2) continue;
-        if (!(r2 < D.lo2) && !rep_exact_inside(Rb, D.L, ai, D.orig[j], D.thr)) continue;
-        if (n < D.cap) D.list[((size_t)(n >> 2) * N + i) * 4 + (n & 3)] = (uint32_t)j | ((uint32_t)code << 16);
-        n++;
+        const int q1 = row[a1 + 1];
+        for (int q = row[a0]; q < q1; q += 32) {
+          const int len = min(32, q1 - q);
+          unsigned m = 0, near = 0xFFFFFFFFu;
+          auto bits = [&](int j) {
+            const float4 pj = pos[j];
+            float dx = px - pj.x, dy = py - pj.y, dz = pz - pj.z;
+            if (minimg) {
+              dx -= Mf * rintf(dx * invM);
+              dy -= Mf * rintf(dy * invM);
+              dz -= Mf * rintf(dz * invM);
+            }
+            return __float_as_int(fmaf(dz, dz, fmaf(dy, dy, dx * dx))) - loBits;
+          };
+          for (int u = 0; u < len; u += 4)
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+              const int d = bits(q + u + v);
+              m = __funnelshift_l((unsigned)d, m, 1);
+              near = min(near, (unsigned)d);
+            }
+          m <<= (32 - ((len + 3) & ~3));
+          if (near < band)   // some candidate lies within the band: the FP64 test decides it
+            for (int j = 0; j < len; j++)
+              if ((unsigned)bits(q + j) < band && rep_exact_inside(Rb, D.L, ai, D.orig[q + j], D.thr))
+                m |= 0x80000000u >> j;
+          m &= (unsigned)((int)0x80000000 >> (len - 1));
+          if ((unsigned)(i - q) < 32u) m &= ~(0x80000000u >> (i - q));
+          while (m) {
+            const int j = __clz(m);
+            m &= 0x7FFFFFFFu >> j;
+            push(q + j);
+          }
+        }
       }
     }
     D.count[i] = n;
-    if (n > D.cap) atomicMax(&S.overflow, n);
+    if (n > cap) atomicMax(&S.overflow, n);
+    while (n & 7) push(i);   // the pair loop masks the entries past the count
   }
-  if (copyR0)
-    for (int q = threadIdx.x; q < 3 * N; q += THREADS) D.R0[q] = D.R[q];
   __syncthreads();
 }
 
-// Pair forces of one replica (full lists, one thread per slot, no atomics).  LJ:
-// every type pair lj_cut without modifier, with the Lennard-Jones arithmetic in cell
-// units (E = 4 eps sr6 (sr6 - 1), W = 24 eps sr6 (2 sr6 - 1)); otherwise the
-// general model code.  COMPUTE: energies too (the virial is always summed).
-// TPA threads per atom (1 or 2): with 2, the two threads of a pair take alternate
-// 4-entry chunks of the atom's list and add their partial forces at the end.
+// slot-order box fractions and types from the coordinates R
+template <int THREADS>
+__device__ __forceinline__ void rep_pack(const RepDesc& D, int4* pos) {
+  for (int s = threadIdx.x; s < D.N; s += THREADS) {
+    const int a = D.orig[s];
+    pos[s] = make_int4(rep_fraction(D.R[3 * a], D), rep_fraction(D.R[3 * a + 1], D), rep_fraction(D.R[3 * a + 2], D),
+                       D.ntypes > 1 ? D.type[a] - 1 : 0);
+  }
+}
+
+// Pair forces of one replica (full lists, one thread per slot, no atomics) in units of
+// the box fractions.  LJ: every type pair lj_cut without modifier (E = 4 eps sr6 (sr6 -
+// 1), W = 24 eps sr6 (2 sr6 - 1)); otherwise the general model code.  COMPUTE: energies
+// too (the virial is always summed).  TPA threads per atom (1 or 2): with 2, the two
+// threads of a pair take alternate chunks of the atom's list and add their partial
+// forces at the end.
 template <bool LJ, bool COMPUTE, int TPA>
-__device__ __forceinline__ void rep_pairs(const RepDesc& D, const float4* pos, const float4* offTab,
-                                          const NBParams<float>* ptab, const uint8_t* stype, float& Ep, float& Wp) {
+__device__ __forceinline__ void rep_pairs(const RepDesc& D, const int4* pos, const NBParams<float>* ptab, float& Ep,
+                                          float& Wp) {
   const NBParams<float> mdl = D.model.model;
   const int nt = D.ntypes, N = D.N;
-  const float rc2 = D.rc2, invw2 = D.invw2, invw = D.invw, Mf = D.Mf;
-  const float sigc = mdl.sigsq * invw2, eps48 = 2.0f * mdl.eps24;
-  const bool minimg = D.minimg;
+  const float rc2 = D.rc2, unit2 = D.unit2, unit = D.unit;
+  const float sigc = mdl.sigsq * unit2, eps48 = 2.0f * mdl.eps24;
   const int cap = D.cap;
-  const uint4* __restrict__ list = reinterpret_cast<const uint4*>(D.list);
+  const uint4* __restrict__ list = D.list;
   const int* __restrict__ count = D.count;
   const int* __restrict__ orig = D.orig;
   double* __restrict__ F = D.F;
   const int sub = TPA == 1 ? 0 : (int)(threadIdx.x & (TPA - 1));
   const unsigned pmask = TPA == 1 ? 0xffffffffu : (3u << ((threadIdx.x & 31) & ~1u));
   for (int i = threadIdx.x / TPA; i < N; i += blockDim.x / TPA) {
-    const float4 pi = pos[i];
+    const int4 pi = pos[i];
     const int n = min(count[i], cap);
-    const NBParams<float>* row = ptab + (nt > 1 ? stype[i] * nt : 0);
+    const NBParams<float>* row = ptab + pi.w * nt;
     float fx = 0.f, fy = 0.f, fz = 0.f;
-    const int nch = (n + 3) >> 2;
-    // 4 entries per 16-byte load, the next chunk requested before this one is used
+    const int nch = (n + 7) >> 3;
+    // 8 entries per 16-byte load, the next chunk requested before this one is used
     uint4 cur = sub < nch ? __ldg(&list[(size_t)sub * N + i]) : make_uint4(0u, 0u, 0u, 0u);
     for (int c = sub; c < nch; c += TPA) {
       const uint4 nxt = c + TPA < nch ? __ldg(&list[(size_t)(c + TPA) * N + i]) : cur;
-      const uint32_t w[4] = {cur.x, cur.y, cur.z, cur.w};
+      const unsigned words[4] = {cur.x, cur.y, cur.z, cur.w};
+      const int left = n - 8 * c;   // entries of this chunk, if fewer than 8
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        if (4 * c + u >= n) break;
-        const uint32_t e = w[u];
-        const int j = e & 0xFFFFu;
-        const float4 pj = pos[j];
-        const float4 o = offTab[e >> 16];
-        float dx = (pi.x - pj.x) - o.x, dy = (pi.y - pj.y) - o.y, dz = (pi.z - pj.z) - o.z;
-        if (minimg) {
-          dx -= Mf * rintf(dx / Mf);
-          dy -= Mf * rintf(dy / Mf);
-          dz -= Mf * rintf(dz / Mf);
-        }
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        const bool in = r2 < rc2;
-        const float invR2c = Ops<float>::rcp(r2);
+      for (int u = 0; u < 8; u++) {
+        const int4 pj = pos[(words[u >> 1] >> ((u & 1) * 16)) & 0xFFFF];
+        const float dx = (float)(pi.x - pj.x), dy = (float)(pi.y - pj.y), dz = (float)(pi.z - pj.z);
+        const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+        const bool in = r2 < rc2 && u < left;
+        const float inv2 = in ? Ops<float>::rcp(r2) : 0.f;   // zeroes every term of the others
         float E = 0.f, W;
         if (LJ) {
           float sg = sigc, e48 = eps48, e24 = mdl.eps24, e4 = mdl.eps4;
           if (nt > 1) {
-            const NBParams<float>& m = row[stype[j]];
-            sg = m.sigsq * invw2;
+            const NBParams<float>& m = row[pj.w];
+            sg = m.sigsq * unit2;
             e24 = m.eps24;
             e48 = 2.0f * e24;
             e4 = m.eps4;
           }
-          const float sr2 = sg * invR2c, sr6 = sr2 * sr2 * sr2;
+          const float sr2 = sg * inv2, sr6 = sr2 * sr2 * sr2;
           W = sr6 * fmaf(e48, sr6, -e24);
           if (COMPUTE) E = sr6 * fmaf(e4, sr6, -e4);
         } else {
-          const float invR2 = invR2c * invw2, invR = sqrtf(invR2);
-          const NBParams<float>& m = nt == 1 ? mdl : row[stype[j]];
+          const float invR2 = (in ? inv2 : 1.f) * unit2, invR = sqrtf(invR2);
+          const NBParams<float>& m = nt == 1 ? mdl : row[pj.w];
           nb_compute(m, E, W, invR, invR2);
           modifier_compute(m, E, W, invR, invR2);
+          W = in ? W : 0.f;
+          E = in ? E : 0.f;
         }
-        W = in ? W : 0.f;
-        if (COMPUTE) Ep += in ? E : 0.f;
+        if (COMPUTE) Ep += E;
         Wp += W;
-        const float sc = W * invR2c;
-        fx += sc * dx;
-        fy += sc * dy;
-        fz += sc * dz;
+        const float sc = W * inv2;
+        fx = fmaf(sc, dx, fx);
+        fy = fmaf(sc, dy, fy);
+        fz = fmaf(sc, dz, fz);
       }
       cur = nxt;
     }
@@ -287,11 +354,79 @@ __device__ __forceinline__ void rep_pairs(const RepDesc& D, const float4* pos, c
     }
     if (sub == 0) {
       const int a = orig[i];
-      F[3 * a] = f2d_exact(fx * invw);
-      F[3 * a + 1] = f2d_exact(fy * invw);
-      F[3 * a + 2] = f2d_exact(fz * invw);
+      F[3 * a] = f2d_exact(fx * unit);
+      F[3 * a + 1] = f2d_exact(fy * unit);
+      F[3 * a + 2] = f2d_exact(fz * unit);
     }
   }
+}
+
+// One pass over the atoms between two force evaluations (the boost(dt/2) that ends a step,
+// the boost(dt/2) and displace(dt) that begin the next, FP64 with the fused multiply-adds
+// of the single-system mixed path, the skin displacement, and the new positions' box
+// fractions at their slots).  Without END the first kick is left out, without BEGIN the
+// rest.  Each warp takes a contiguous range of atoms, as the skin check's combine needs.
+template <int THREADS, bool END, bool BEGIN>
+__device__ __forceinline__ void rep_advance(RepShared& S, int4* pos, double dt, bool kinetic) {
+  const RepDesc& D = S.d;
+  const int N = D.N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = THREADS / 32;
+  const double dt_2 = 0.5 * dt;
+  const int per = (N + nw - 1) / nw, a0 = warp * per, a1 = min(N, a0 + per);
+  double ke[3] = {0.0, 0.0, 0.0};
+  RepMP run{-1, -1};
+  for (int base = a0; base < a1; base += 32) {
+    const int a = base + lane;
+    RepMP v{-1, -1};
+    if (a < a1) {
+      const double im = D.unitMass ? 1.0 : D.invMass[a];
+      double dr[3];
+      int x[3];
+      for (int d = 0; d < 3; d++) {
+        const double f = D.F[3 * a + d];
+        double p = D.P[3 * a + d];
+        if (END) {
+          p = fma(dt_2, f, p);
+          if (kinetic) ke[d] += im * (p * p);
+        }
+        if (BEGIN) {
+          p = fma(dt_2, f, p);
+          const double r = D.unitMass ? fma(dt, p, D.R[3 * a + d]) : fma(dt * p, im, D.R[3 * a + d]);
+          D.R[3 * a + d] = r;
+          dr[d] = r - D.R0[3 * a + d];
+          x[d] = rep_fraction(r, D);
+        }
+        D.P[3 * a + d] = p;
+      }
+      if (BEGIN) {
+        v.m = __double_as_longlong(fma(dr[2], dr[2], fma(dr[1], dr[1], dr[0] * dr[0])));
+        int4* q = &pos[D.slotOf[a]];
+        q->x = x[0];
+        q->y = x[1];
+        q->z = x[2];
+      }
+    }
+    if (BEGIN) run = rep_combine(run, rep_warp_ordered(v));
+  }
+  if (END && kinetic) {
+    for (int d = 0; d < 3; d++)
+      for (int o = 16; o > 0; o >>= 1) ke[d] += __shfl_down_sync(0xffffffffu, ke[d], o);
+    if (lane == 0)
+      for (int d = 0; d < 3; d++) S.wke[d][warp] = ke[d];
+  }
+  if (BEGIN && lane == 0) S.wmp[warp] = run;
+  __syncthreads();
+  if (END && kinetic && threadIdx.x < 3) {
+    double x = 0.0;
+    for (int w = 0; w < nw; w++) x += S.wke[threadIdx.x][w];
+    D.out[2 + threadIdx.x] = x;
+  }
+  if (BEGIN && threadIdx.x == 32) {
+    RepMP b = S.wmp[0];
+    for (int w = 1; w < nw; w++) b = rep_combine(b, S.wmp[w]);
+    const double mx = __longlong_as_double(b.m), nx = __longlong_as_double(b.p < 0 ? b.m : b.p);
+    S.rebuild = mx + 2 * sqrt(mx * nx) + nx > D.skinSq;
+  }
+  __syncthreads();
 }
 
 template <int THREADS, int TPA>
@@ -299,18 +434,14 @@ __global__ void __launch_bounds__(THREADS) k_replicas(const RepDesc* __restrict_
                                                       int steps, double dt, int nprop, int Nmax, int cellsMax) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ RepShared S;
-  float4* pos = (float4*)smem;
-  float4* offTab = pos + Nmax;
-  NBParams<float>* ptab = (NBParams<float>*)(offTab + 125);   // [ti * ntypes + tj]
+  int4* pos = (int4*)smem;   // box fractions and type; during a build cell units and cell
+  NBParams<float>* ptab = (NBParams<float>*)(pos + Nmax + REP_PAD);   // [ti * ntypes + tj]
   int* cellStart = (int*)(ptab + REP_MAXT * REP_MAXT);
   int* cursor = cellStart + cellsMax + 1;
-  uint8_t* stype = (uint8_t*)(cursor + cellsMax);
   if (threadIdx.x == 0) {
     S.d = descs[order[blockIdx.x]];
     S.overflow = 0;
   }
-  for (int c = threadIdx.x; c < 125; c += THREADS)
-    offTab[c] = make_float4((float)(c % 5 - 2), (float)((c / 5) % 5 - 2), (float)(c / 25 - 2), 0.f);
   __syncthreads();
   {
     const int nt = S.d.ntypes;
@@ -319,76 +450,42 @@ __global__ void __launch_bounds__(THREADS) k_replicas(const RepDesc* __restrict_
       ptab[q] = S.d.table[ti * nt + tj].model;   // pair(jtype, itype) for an atom of type ti
     }
   }
-  __syncthreads();
   const RepDesc& D = S.d;
-  const int N = D.N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = THREADS / 32;
-  const double dt_2 = 0.5 * dt;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = THREADS / 32;
   int done = (int)D.out[7];
-  // lists as the system's were built: from the positions of the last build (R0)
-  rep_build<THREADS>(S, D.R0, pos, cellStart, cursor, offTab, false, stype);
+  // Lists as the system's were built, from the positions of the last build (R0): those of
+  // an earlier run serve if they were made from the same positions, bit for bit.
+  bool same = true;
+  for (int q = threadIdx.x; q < 3 * D.N; q += THREADS)
+    same = same && __double_as_longlong(D.Rb[q]) == __double_as_longlong(D.R0[q]);
+  if (!__syncthreads_and(same)) rep_build<THREADS>(S, D.R0, (float4*)pos, cellStart, cursor, false);
   double builds = D.out[5];
   // steps < 0: forces, energy and virial at the current positions only
   const bool evaluate = steps < 0;
   const int nsteps = evaluate ? 1 : steps;
+  rep_pack<THREADS>(D, pos);
+  __syncthreads();
+  bool compute = false;
   for (int k = 0; k < nsteps; k++) {
-    const bool compute = evaluate || (k + 1) % nprop == 0;   // every nprop-th step of this call
+    const bool kinetic = compute;   // of the step that the pass below ends
+    compute = evaluate || (k + 1) % nprop == 0;   // every nprop-th step of this call
     if (!evaluate) {
-    // boost(dt/2) and displace(dt), FP64 (src/EmDeeData.f90:823-896)
-    for (int a = threadIdx.x; a < N; a += THREADS) {
-      const double im = D.unitMass ? 1.0 : D.invMass[a];
-      for (int d = 0; d < 3; d++) {   // fused multiply-adds, as the single-system mixed path
-        const double p = fma(dt_2, D.F[3 * a + d], D.P[3 * a + d]);
-        D.P[3 * a + d] = p;
-        D.R[3 * a + d] = D.unitMass ? fma(dt, p, D.R[3 * a + d]) : fma(dt * p, im, D.R[3 * a + d]);
+      if (k == 0) rep_advance<THREADS, false, true>(S, pos, dt, false);
+      else rep_advance<THREADS, true, true>(S, pos, dt, kinetic);
+      if (S.rebuild) {
+        rep_build<THREADS>(S, D.R, (float4*)pos, cellStart, cursor, true);
+        rep_pack<THREADS>(D, pos);
+        builds += 1.0;
+        __syncthreads();
       }
     }
-    __syncthreads();
-    // skin check over atoms in index order: warp w takes a contiguous range
-    {
-      const int per = (N + nw - 1) / nw, a0 = warp * per, a1 = min(N, a0 + per);
-      RepMP run{-1, -1};
-      for (int base = a0; base < a1; base += 32) {
-        const int a = base + lane;
-        RepMP v{-1, -1};
-        if (a < a1) {
-          const double d0 = D.R[3 * a] - D.R0[3 * a], d1 = D.R[3 * a + 1] - D.R0[3 * a + 1],
-                       d2 = D.R[3 * a + 2] - D.R0[3 * a + 2];
-          v.m = __double_as_longlong(d0 * d0 + d1 * d1 + d2 * d2);
-        }
-        v = rep_warp_ordered(v);
-        run = rep_combine(run, v);
-      }
-      if (lane == 0) S.wmp[warp] = run;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        RepMP b = S.wmp[0];
-        for (int w = 1; w < nw; w++) b = rep_combine(b, S.wmp[w]);
-        const double mx = __longlong_as_double(b.m), nx = __longlong_as_double(b.p < 0 ? b.m : b.p);
-        S.rebuild = mx + 2 * sqrt(mx * nx) + nx > D.skinSq;
-      }
-      __syncthreads();
-    }
-    if (S.rebuild) {
-      rep_build<THREADS>(S, D.R, pos, cellStart, cursor, offTab, true, stype);
-      builds += 1.0;
-    }
-    }   // !evaluate
-    // positions in cell units relative to the build-time cells
-    for (int s = threadIdx.x; s < N; s += THREADS) {
-      const int a = D.orig[s];
-      const int4 kk = D.K[s];
-      pos[s] = make_float4((float)fma(D.R[3 * a], D.scale, -(double)kk.x), (float)fma(D.R[3 * a + 1], D.scale, -(double)kk.y),
-                           (float)fma(D.R[3 * a + 2], D.scale, -(double)kk.z), 0.f);
-    }
-    __syncthreads();
     // pair forces (full lists, no atomics); energies on compute steps, virial every step
     float Ep = 0.f, Wp = 0.f;
-    const bool lj = D.ljAll != 0;
-    if (lj) {
-      if (compute) rep_pairs<true, true, TPA>(D, pos, offTab, ptab, stype, Ep, Wp);
-      else rep_pairs<true, false, TPA>(D, pos, offTab, ptab, stype, Ep, Wp);
+    if (D.ljAll) {
+      if (compute) rep_pairs<true, true, TPA>(D, pos, ptab, Ep, Wp);
+      else rep_pairs<true, false, TPA>(D, pos, ptab, Ep, Wp);
     } else {
-      rep_pairs<false, true, TPA>(D, pos, offTab, ptab, stype, Ep, Wp);
+      rep_pairs<false, true, TPA>(D, pos, ptab, Ep, Wp);
     }
     {
       float hi[2] = {0.5f * Ep, 0.5f * Wp}, lo[2] = {0.f, 0.f};
@@ -404,30 +501,9 @@ __global__ void __launch_bounds__(THREADS) k_replicas(const RepDesc* __restrict_
       for (int w = 0; w < nw; w++) ff_add(h, l, S.wff[threadIdx.x][w].x, S.wff[threadIdx.x][w].y);
       if (threadIdx.x == 1 || compute) D.out[threadIdx.x] = (double)h + (double)l;
     }
-    if (evaluate) break;
-    // boost(dt/2) with the new forces; kinetic energies on compute steps
-    double ke[3] = {0.0, 0.0, 0.0};
-    for (int a = threadIdx.x; a < N; a += THREADS) {
-      const double im = D.unitMass ? 1.0 : D.invMass[a];
-      for (int d = 0; d < 3; d++) {
-        const double p = fma(dt_2, D.F[3 * a + d], D.P[3 * a + d]);
-        D.P[3 * a + d] = p;
-        if (compute) ke[d] += im * (p * p);
-      }
-    }
-    if (compute) {
-      for (int d = 0; d < 3; d++)
-        for (int o = 16; o > 0; o >>= 1) ke[d] += __shfl_down_sync(0xffffffffu, ke[d], o);
-      if (lane == 0)
-        for (int d = 0; d < 3; d++) S.wke[d][warp] = ke[d];
-    }
-    __syncthreads();
-    if (compute && threadIdx.x < 3) {
-      double x = 0.0;
-      for (int w = 0; w < nw; w++) x += S.wke[threadIdx.x][w];
-      D.out[2 + threadIdx.x] = x;
-    }
   }
+  // the boost that ends the last step
+  if (!evaluate && nsteps > 0) rep_advance<THREADS, true, false>(S, pos, dt, compute);
   __syncthreads();
   if (threadIdx.x == 0) {
     D.out[5] = builds;
@@ -610,18 +686,19 @@ void* EmDee_replicas_create(int n, tEmDee** systems) {
     d.N = s.natoms;
     const double L = *s.Lbox;
     d.M = std::max((int)std::floor(2.0 * L / s.xRc), 5);
+    // a cell edge of exactly (rc + skin) / 2 leaves no room for the fractions' rounding
+    if (d.M > 5 && L / d.M < 0.5 * s.xRc * (1.0 + 1e-8)) d.M--;
     d.minimg = d.M == 5;
     d.L = L;
-    d.scale = d.M / L;
+    d.frac = 4294967296.0 / L;
     d.skinSq = s.skinSq;
     d.thr = s.xRcSq / (L * L);
     const double M2 = (double)d.M * d.M;
     d.lo2 = (float)(d.thr * M2 * (1.0 - REP_BAND));
     d.hi2 = (float)(d.thr * M2 * (1.0 + REP_BAND));
-    d.rc2 = (float)(s.RcSq / (L * L) * M2);
-    const double w = L / d.M;
-    d.invw2 = (float)(1.0 / (w * w));
-    d.invw = (float)(1.0 / w);
+    d.rc2 = (float)(s.RcSq * d.frac * d.frac);
+    d.unit2 = (float)(d.frac * d.frac);
+    d.unit = (float)d.frac;
     d.Mf = (float)d.M;
     CK(cudaMemcpy(&d.model, s.models.d32, sizeof(PairEntry<float>), cudaMemcpyDeviceToHost));
     d.ntypes = s.ntypes;
@@ -635,13 +712,15 @@ void* EmDee_replicas_create(int n, tEmDee** systems) {
     d.type = s.dType;
     // list capacity: twice the ideal-gas count within rc+skin, at least 64
     const double expect = 4.0 / 3.0 * 3.14159265358979 * std::pow(s.xRc, 3) * s.natoms / (L * L * L);
-    d.cap = std::max(64, ((int)(2.0 * expect) + 7) / 8 * 8);   // a multiple of the 4-entry chunk
+    d.cap = std::max(64, ((int)(2.0 * expect) + 7) / 8 * 8);   // a multiple of the 8-entry chunk
     CK(cudaMalloc(&d.orig, sizeof(int) * d.N));
-    CK(cudaMalloc(&d.K, sizeof(int4) * d.N));
-    CK(cudaMalloc(&d.atomK, sizeof(int4) * d.N));
-    CK(cudaMalloc(&d.list, sizeof(uint32_t) * (size_t)d.cap * d.N));
+    CK(cudaMalloc(&d.slotOf, sizeof(uint16_t) * d.N));
+    CK(cudaMalloc(&d.frac4, sizeof(int4) * d.N));
+    CK(cudaMalloc(&d.Rb, sizeof(double) * 3 * d.N));
+    CK(cudaMemset(d.Rb, 0xFF, sizeof(double) * 3 * d.N));   // no lists yet (NaN)
+    CK(cudaMalloc(&d.list, sizeof(uint16_t) * (size_t)d.cap * d.N));
     CK(cudaMalloc(&d.count, sizeof(int) * d.N));
-    B->owned.insert(B->owned.end(), {d.orig, d.K, d.atomK, d.list, d.count});
+    B->owned.insert(B->owned.end(), {d.orig, d.slotOf, d.frac4, d.Rb, d.list, d.count});
     d.out = B->dOut + 8 * r;
     B->desc.push_back(d);
     B->md.push_back(md);
@@ -651,9 +730,10 @@ void* EmDee_replicas_create(int n, tEmDee** systems) {
     order[r] = r;
   }
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return B->desc[a].N > B->desc[b].N; });
-  B->smem = sizeof(float4) * ((size_t)B->Nmax + 125) + sizeof(NBParams<float>) * REP_MAXT * REP_MAXT +
-            sizeof(int) * (2 * (size_t)B->cellsMax + 1) + (size_t)B->Nmax;
-  if (B->smem > 227 * 1024) fatal(task, "the largest replica does not fit in one block's shared memory");
+  B->smem = sizeof(int4) * ((size_t)B->Nmax + REP_PAD) + sizeof(NBParams<float>) * REP_MAXT * REP_MAXT +
+            sizeof(int) * (2 * (size_t)B->cellsMax + 1);
+  // the limit of 125 stencil offsets and a type byte per atom besides is kept
+  if (B->smem + sizeof(float4) * (125 - REP_PAD) + (size_t)B->Nmax > 227 * 1024) fatal(task, "the largest replica does not fit in one block's shared memory");
   CK(cudaMalloc(&B->dDesc, sizeof(RepDesc) * n));
   CK(cudaMemcpy(B->dDesc, B->desc.data(), sizeof(RepDesc) * n, cudaMemcpyHostToDevice));
   CK(cudaMalloc(&B->dOrder, sizeof(int) * n));
