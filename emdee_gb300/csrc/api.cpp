@@ -301,10 +301,15 @@ static void compute_forces_impl(tEmDee* md) {
     device_tune_tile(s, pair_lj_only(s), [](System& sys) { device_pair_forces(sys, true); });
   }
   bool rebuild = !s.r0Valid, forcesDone = false;
-  if (!rebuild && s.skinReady && s.packReady && s.precision == 0 && s.pairs_exist[s.layer - 1]) {
-    // the fused step left the skin decision and the packed positions on the device:
-    // the pair kernel runs unless a rebuild is due, and one synchronisation returns
-    // both the decision and the sums
+  s.queueExtras = true;
+  s.extrasQueued = false;
+  if (!rebuild && s.precision == 0 && s.pairs_exist[s.layer - 1]) {
+    // the skin decision (left by the fused step, or queued here) stays on the device with
+    // the packed positions: the pair kernel and what follows it run unless a rebuild is
+    // due, and one synchronisation returns both the decision and the sums
+    if (!s.skinReady) device_skin_launch(s);
+    if (!s.packReady) device_pack(s);
+    s.packReady = true;
     forcesDone = device_pair_forces(s, compute, true);
     rebuild = !forcesDone;
   } else if (!rebuild) {
@@ -329,21 +334,32 @@ static void compute_forces_impl(tEmDee* md) {
     if (!((rebuild || s.packReady) && s.precision == 0)) device_pack(s);
     device_pair_forces(s, compute);
   }
+  s.queueExtras = false;
   s.skinReady = s.packReady = false;
+  const int l = s.layer - 1;
+  const bool kspace = s.coul[l].requires_kspace != 0;
+  const bool haveBonded = !s.bondedTerms.bonds.empty() || !s.bondedTerms.angles.empty();
+  if (!s.extrasQueued && (haveBonded || kspace || s.nbodies != 0)) {   // no pair launch to follow
+    bonded_launch(s, nullptr);
+    if (kspace) ewald_launch(s, nullptr);
+    if (s.nbodies != 0) bodies_virial_launch(s, nullptr);
+    CK(cudaStreamSynchronize(s.stream));
+  }
   const double* r = s.hResult;   // Epair, Ecoul, Wpair, Wcoul
-  double bonded[5];   // Ebond, Wbond, Eangle, Wangle, Coulomb discounts of bonds and angles
-  device_bonded(s, bonded);
+  // Ebond, Wbond, Eangle, Wangle, Coulomb discounts of bonds and angles
+  const double none[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  const double* bonded = haveBonded && (s.bonded[l] != 0 || kspace) ? r + 40 : none;
   const double Ecoul = r[1] + bonded[4];
   double Elong = 0.0, Wlong = 0.0;
-  if (s.coul[s.layer - 1].requires_kspace) {   // src/EmDeeCode.f90:1249-1252
-    Elong = ewald_compute(s);
+  if (kspace) {   // src/EmDeeCode.f90:1249-1252
+    Elong = ewald_energy(s);
     Wlong = Ecoul + Elong - r[3];
   }
   s.forcesF32 = s.precision == 0 && !s.coul[s.layer - 1].requires_kspace && s.bondedTerms.uploaded == 0;
   md->Virial.Total = r[2] + r[3] + Wlong + bonded[1] + bonded[3];
   md->Virial.Body = 0.0;
   if (s.nbodies != 0) {   // src/EmDeeData.f90:926-953
-    md->Virial.Body = bodies_virial(s);
+    md->Virial.Body = -r[6];
     md->Virial.Total = md->Virial.Total + md->Virial.Body;
   }
   if (compute) {
@@ -1359,7 +1375,13 @@ void EmDee_verlet_step(tEmDee* md, double dt) {
   double t0 = wtime();
   device_verlet_pre(s, dt, compute, mode);
   md->Time.Motion += wtime() - t0;
+  // free atoms: the closing half-step is queued behind the forces
+  s.vvReq = s.nbodies == 0;
+  s.vvQueued = false;
+  s.vvDt = dt;
+  s.vvCompute = compute;
   compute_forces_impl(md);   // unconditional; other layers keep their flags, as in the reference
+  s.vvReq = false;
   double v[9];
   device_verlet_post(s, dt, compute, mode, v);
   if (compute) {

@@ -244,7 +244,8 @@ __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_move_series(BodyArg
 // W = sum over bodies and their atoms of F . delta (the body virial is -W)
 __global__ void __launch_bounds__(BODY_THREADS) k_body_virial(BodyArgs A, const double* __restrict__ F,
                                                               double* partials, unsigned int* ticket, double* result,
-                                                              double* hostResult) {
+                                                              double* hostResult, const double* skip) {
+  if (skip != nullptr && __double_as_longlong(*skip) != 0) return;   // a rebuild is due
   double w[1] = {0.0};
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < A.nb) {
@@ -435,15 +436,13 @@ void bodies_move(System& s, double CR, double CP, double dt, bool translate, boo
   s.prof.total++;
 }
 
-double bodies_virial(System& s) {
+void bodies_virial_launch(System& s, const double* skip) {
   int blocks = body_blocks(s.nbodies);
   ensure_scratch(s, blocks, 1);
   k_body_virial<<<blocks, BODY_THREADS, 0, s.stream>>>(body_args(s), s.F(), s.dBodyScratch, s.dTicket + 3,
-                                                        s.dResult + 6, s.hResult + 6);
+                                                        s.dResult + 6, s.hResult + 6, skip);
   CK(cudaGetLastError());
   s.prof.total++;
-  CK(cudaStreamSynchronize(s.stream));
-  return -s.hResult[6];
 }
 
 // bodies take their momenta from the particle momenta in dP; 2KE of bodies into k6

@@ -39,6 +39,7 @@ struct BondedArgs {
   double* partials;
   unsigned int* ticket;
   double* hostResult;   // pinned
+  const double* skip;   // if set and *skip != 0 (a rebuild is due), the launches do nothing
   double* result;       // [0] Ebond, [1] Wbond, [2] Eangle, [3] Wangle, [4] Ecoul discount
 };
 
@@ -53,6 +54,7 @@ __device__ __forceinline__ void kspace_discount(double alpha, double beta, doubl
 }
 
 __global__ void __launch_bounds__(BONDED_THREADS) k_bonded(BondedArgs A) {
+  if (A.skip != nullptr && __double_as_longlong(*A.skip) != 0) return;
   double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m < A.nitems) {
@@ -139,6 +141,7 @@ __global__ void __launch_bounds__(BONDED_THREADS) k_bonded(BondedArgs A) {
 
 // F(a) += the atom's contributions, in list order
 __global__ void __launch_bounds__(BONDED_THREADS) k_bonded_gather(BondedArgs A) {
+  if (A.skip != nullptr && __double_as_longlong(*A.skip) != 0) return;
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= A.natoms) return;
   const int e0 = A.first[a], e1 = A.first[a + 1];
@@ -210,9 +213,8 @@ static void bonded_upload(System& s) {
   B.uploaded = n;
 }
 
-bool device_bonded(System& s, double out[5]) {
+bool bonded_launch(System& s, const double* skip) {
   BondedTerms& B = s.bondedTerms;
-  for (int q = 0; q < 5; q++) out[q] = 0.0;
   const int n = (int)(B.bonds.size() + B.angles.size());
   const int l = s.layer - 1;
   const bool bonded = s.bonded[l] != 0, kspace = s.coul[l].requires_kspace != 0;
@@ -240,13 +242,12 @@ bool device_bonded(System& s, double out[5]) {
   A.ticket = s.dTicket + 7;
   A.result = s.dResult + 40;
   A.hostResult = s.hResult + 40;
+  A.skip = skip;
   k_bonded<<<(n + BONDED_THREADS - 1) / BONDED_THREADS, BONDED_THREADS, 0, s.stream>>>(A);
   CK(cudaGetLastError());
   k_bonded_gather<<<(s.natoms + BONDED_THREADS - 1) / BONDED_THREADS, BONDED_THREADS, 0, s.stream>>>(A);
   CK(cudaGetLastError());
   s.prof.total += 2;
-  CK(cudaStreamSynchronize(s.stream));
-  for (int q = 0; q < 5; q++) out[q] = s.hResult[40 + q];
   return true;
 }
 

@@ -69,11 +69,17 @@ struct EwArgs {
   unsigned int* ticket;
   double* result;
   double* hostResult;
+  const double* skip;   // if set and *skip != 0 (a rebuild is due), the launches do nothing
 };
+
+__device__ __forceinline__ bool skipped(const EwArgs& A) {
+  return A.skip != nullptr && __double_as_longlong(*A.skip) != 0;
+}
 
 // powers exp(i 2pi m x / L), m = 0..nm, of every coordinate of the charged atoms
 // (src/kspace_ewald.f90:205-243: B = Z; G(j) = B; B = B*Z); those of x times the charge
 __global__ void __launch_bounds__(128) k_ewald_tables(EwArgs A) {
+  if (skipped(A)) return;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= 3 * A.nq) return;
   const int d = k / A.nq, j = k - d * A.nq;
@@ -99,6 +105,7 @@ __device__ __forceinline__ double2 row_phase(double2 gx, double2 gy, int n2) {
 }
 
 __global__ void __launch_bounds__(SF_THREADS) k_ewald_sf(EwArgs A) {
+  if (skipped(A)) return;
   extern __shared__ __align__(16) unsigned char smem[];
   double2* T = (double2*)smem;   // [atom][d][m], an odd number of entries per atom
   const int rows = A.nmax + 1, W = 3 * rows, S = W | 1;
@@ -160,6 +167,7 @@ static const int EW_MAXT = 16;   // charged atom types handled by the k-space ke
 static const int SIGMA_PAIRS = 32, SIGMA_SLICES = 8;
 
 __global__ void __launch_bounds__(SIGMA_PAIRS * SIGMA_SLICES) k_ewald_sigma(EwArgs A) {
+  if (skipped(A)) return;
   __shared__ double part[SIGMA_SLICES][4][SIGMA_PAIRS];
   __shared__ double Ss[EW_MAXT][4][SIGMA_PAIRS];
   const int x = threadIdx.x % SIGMA_PAIRS, y = threadIdx.x / SIGMA_PAIRS;
@@ -214,6 +222,7 @@ __global__ void __launch_bounds__(SIGMA_PAIRS * SIGMA_SLICES) k_ewald_sigma(EwAr
 // U = Re(rho+ + rho-), V = Im(rho+ - rho-), X = Re(rho+ - rho-), Y = Im(rho+ + rho-):
 //   H0 += (U gr + V gi, X gi - Y gr),  H1 += m (X gr + Y gi, U gi - V gr).
 __global__ void __launch_bounds__(FORCE_ATOMS * FORCE_SPLIT) k_ewald_force(EwArgs A) {
+  if (skipped(A)) return;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[3][FORCE_SPLIT][FORCE_ATOMS];
   const int rows = A.nmax + 1;
@@ -515,7 +524,7 @@ void ewald_initialize(System& s, double kspaceRc) {
 
 // k-space energy of the current layer (plus the rigid-pair and self discounts);
 // forces added to the current layer's force array
-double ewald_compute(System& s) {
+void ewald_launch(System& s, const double* skip) {
   Ewald& e = s.ewald;
   const int l = s.layer - 1;
   EwArgs A;
@@ -548,6 +557,7 @@ double ewald_compute(System& s) {
   A.ticket = s.dTicket + 4;
   A.result = s.dResult + 22;
   A.hostResult = s.hResult + 22;   // pinned: read after the synchronisation
+  A.skip = skip;
   const int rows = e.nmax + 1;
   if ((size_t)3 * rows * TABLE_LIMIT_ATOMS * sizeof(double2) > 227 * 1024)
     fatal("kspace computation", "too many k-vectors per dimension");
@@ -565,7 +575,11 @@ double ewald_compute(System& s) {
   k_ewald_force<<<(e.nq + FORCE_ATOMS - 1) / FORCE_ATOMS, FORCE_ATOMS * FORCE_SPLIT, smemF, s.stream>>>(A);
   CK(cudaGetLastError());
   s.prof.total += 4;
-  CK(cudaStreamSynchronize(s.stream));
+}
+
+double ewald_energy(System& s) {
+  const Ewald& e = s.ewald;
+  const int l = s.layer - 1;
   const double Ek = s.hResult[22];
   // src/modelClass_kspace.f90:247-314, energy part
   double disc = 0.0;

@@ -411,7 +411,14 @@ bool device_pair_forces(System& s, bool compute, bool speculative) {
   const int l2 = s.layer - 1;
   const bool chain = s.keChainReq && s.precision == 0 && s.nbodies == 0 && s.bondedTerms.bonds.empty() &&
                      s.bondedTerms.angles.empty() && !s.coul[l2].requires_kspace;
-  if (chain) launch_kinetic_two(s, s.keChainCF, speculative ? s.dResult + 9 : nullptr);
+  const double* skip = speculative ? s.dResult + 9 : nullptr;
+  if (chain) launch_kinetic_two(s, s.keChainCF, skip);
+  if (s.queueExtras) {
+    bonded_launch(s, skip);
+    if (s.coul[l2].requires_kspace) ewald_launch(s, skip);
+    if (s.nbodies > 0) bodies_virial_launch(s, skip);
+    if (s.vvReq) verlet_post_launch(s, s.vvDt, s.vvCompute, skip);
+  }
   // The last block of the pair kernel wrote the sums, and the fused step the skin value
   // and rebuild flag ([8], [9]), straight into the pinned hResult, so one synchronisation
   // returns all of them.
@@ -422,6 +429,10 @@ bool device_pair_forces(System& s, bool compute, bool speculative) {
     return false;
   }
   if (chain) s.keChained = true;
+  if (s.queueExtras) {
+    s.extrasQueued = true;
+    s.vvQueued = s.vvReq;
+  }
   return true;
 }
 

@@ -134,7 +134,7 @@ static void ensure_partials(System& s, int n) {
   }
 }
 
-bool device_skin_check(System& s) {
+void device_skin_launch(System& s) {
   const int N = s.natoms, chunks = skin_chunks(N, SKIN_CHUNKS), per = SKIN_THREADS * chunks;
   const int blocks = (N + per - 1) / per;
   ensure_partials(s, blocks);
@@ -143,6 +143,10 @@ bool device_skin_check(System& s) {
                                                  s.dTicket, s.dResult, s.hResult);
   CK(cudaGetLastError());
   prof_end(s, PK_SKIN);
+}
+
+bool device_skin_check(System& s) {
+  device_skin_launch(s);
   CK(cudaStreamSynchronize(s.stream));
   return s.hResult[9] != 0.0;
 }
@@ -1623,7 +1627,9 @@ static const int STEP_CHUNKS = 2;   // at most 64 consecutive atoms per warp (sk
 // FMA (mixed precision only): the updates use fused multiply-adds, which halves the
 // work on the FP64 pipe (the limit of this kernel on GB300); FP64 mode keeps the
 // reference's separately rounded statements.
-template <int NK, bool UNITM, bool PACK, bool FMA>
+// VV: the opening half of EmDee_verlet_step (src/EmDeeCode.f90:1107-1211), with the shadow
+// start values in s0 if it is set; each statement as in k_vv_pre_free.
+template <int NK, bool UNITM, bool PACK, bool FMA, bool VV>
 __global__ void __launch_bounds__(SKIN_THREADS) k_step_fused(double* __restrict__ R, double* __restrict__ P,
                                                              const double* __restrict__ F,
                                                              const double* __restrict__ invMass,
@@ -1633,7 +1639,7 @@ __global__ void __launch_bounds__(SKIN_THREADS) k_step_fused(double* __restrict_
                                                              const float4* __restrict__ pos0, float scale,
                                                              float4* __restrict__ pos4, longlong2* partial,
                                                              unsigned int* ticket, double* result,
-                                                             double* hostResult) {
+                                                             double* hostResult, double* __restrict__ s0) {
   __shared__ MaxPrev wsum[SKIN_THREADS / 32];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1647,6 +1653,10 @@ __global__ void __launch_bounds__(SKIN_THREADS) k_step_fused(double* __restrict_
       double r[3];
       for (int d = 0; d < 3; d++) {
         double p = P[3 * i + d];
+        if (VV && s0 != nullptr) {
+          const double f = F[3 * i + d];
+          s0[3 * i + d] = 2.5 * R[3 * i + d] + cf0 * im * (p - cf0 * f);
+        }
         if (FMA) {
           if (NK >= 1) p = fma(cf0, F[3 * i + d], p);
           if (NK >= 2) p = fma(cf1, F[3 * i + d], p);
@@ -1655,7 +1665,7 @@ __global__ void __launch_bounds__(SKIN_THREADS) k_step_fused(double* __restrict_
           if (NK >= 2) p = p + cf1 * F[3 * i + d];
         }
         if (NK >= 1) P[3 * i + d] = p;
-        if (FMA) r[d] = UNITM ? fma(CP, p, R[3 * i + d]) : fma(CP * p, im, R[3 * i + d]);
+        if (FMA) r[d] = UNITM || (VV && im == 1.0) ? fma(CP, p, R[3 * i + d]) : fma(CP * p, im, R[3 * i + d]);
         else r[d] = R[3 * i + d] + (UNITM ? CP * p : CP * p * im);
         R[3 * i + d] = r[d];
       }
@@ -1703,21 +1713,26 @@ __global__ void __launch_bounds__(SKIN_THREADS) k_step_fused(double* __restrict_
   }
 }
 
-void device_step_fused(System& s, double CP) {
+void device_step_fused(System& s, double CP, bool vv, double* s0) {
   const int N = s.natoms, chunks = skin_chunks(N, STEP_CHUNKS), per = SKIN_THREADS * chunks;
   const int blocks = (N + per - 1) / per;
   ensure_partials(s, blocks);
   const bool pack = s.precision == 0 && s.r0Valid && *s.Lbox == s.builtL;
   const Grid& g = s.grid;
   const float scale = g.M > 0 ? (float)((double)g.M / *s.Lbox) : 0.0f;
+  if (vv) {   // no kick is pending: the half-step's own
+    s.pendCF[0] = 0.5 * CP;
+    s.npend = 1;
+  }
   prof_begin(s, PK_MOVE);
 #define STEP_ARGS s.dR, s.dP, s.F(), s.dInvMass, s.dR0, N, chunks, s.pendCF[0], s.pendCF[1], CP, s.skinSq, g.dSlotOf, \
-                  g.dPos0, scale, g.dPos4, (longlong2*)s.dPartials, s.dTicket, s.dResult, s.hResult
-#define STEP_LAUNCH(NK, UM, PK, FM) k_step_fused<NK, UM, PK, FM><<<blocks, SKIN_THREADS, 0, s.stream>>>(STEP_ARGS)
-#define STEP_NK(UM, PK, FM)                 \
-  if (s.npend == 0) STEP_LAUNCH(0, UM, PK, FM); \
-  else if (s.npend == 1) STEP_LAUNCH(1, UM, PK, FM); \
-  else STEP_LAUNCH(2, UM, PK, FM);
+                  g.dPos0, scale, g.dPos4, (longlong2*)s.dPartials, s.dTicket, s.dResult, s.hResult, s0
+#define STEP_LAUNCH(NK, UM, PK, FM, VV) k_step_fused<NK, UM, PK, FM, VV><<<blocks, SKIN_THREADS, 0, s.stream>>>(STEP_ARGS)
+#define STEP_NK(UM, PK, FM)                            \
+  if (vv) STEP_LAUNCH(1, UM, PK, FM, true);            \
+  else if (s.npend == 0) STEP_LAUNCH(0, UM, PK, FM, false); \
+  else if (s.npend == 1) STEP_LAUNCH(1, UM, PK, FM, false); \
+  else STEP_LAUNCH(2, UM, PK, FM, false);
   if (pack) {   // mixed precision: fused multiply-adds
     if (s.unitMass) { STEP_NK(true, true, true) } else { STEP_NK(false, true, true) }
   } else if (s.precision == 0) {

@@ -262,6 +262,13 @@ struct System {
   bool keChainReq = false, keChained = false;
   double keChainCF = 0.0;
   bool skinReady = false, packReady = false;
+  // What a force computation queues behind its pair launch (compute_forces_impl): bonded
+  // terms, k-space, the rigid-body virial and, for EmDee_verlet_step of free atoms
+  // (vvReq), the closing half-step.  All of it is skipped with a speculative launch
+  // that finds a rebuild due, and one synchronisation returns every result.
+  bool queueExtras = false, extrasQueued = false;
+  bool vvReq = false, vvQueued = false, vvCompute = false;
+  double vvDt = 0.0;
   bool phaseShared = false;   // R/P aliased with another system (no deferral then)
   const double* pairSkip = nullptr;   // device rebuild flag the mixed pair kernel checks first
   double builtL = 0;           // box length at the last build
@@ -314,6 +321,9 @@ void prof_drop_last(System& s);
 // Skin-displacement check of src/neighbor_lists.f90:41-59,184; returns true when
 // the lists must be rebuilt.  Synchronizes the stream.
 bool device_skin_check(System& s);
+// The same check queued only: the rebuild flag stays in dResult[9] (and hResult[9] after
+// the next synchronisation).
+void device_skin_launch(System& s);
 // Cell binning, tile sort and neighbor-list build (src/neighbor_lists.f90:63-300).
 // With two-level lists active it builds the outer lists (radius rc + skin + outer skin).
 void device_build_lists(System& s);
@@ -370,14 +380,16 @@ bool device_kinetic(System& s, double* twoKE, const double* src = nullptr, const
 // applies the pending kicks (1 or 2) and writes the momenta to P and to out (a
 // device-accessible pointer to the caller's pinned buffer); synchronizes
 void device_kick_out(System& s, double* out);
-// bonds and angles of the current layer: adds their forces to F and returns
-// Ebond, Wbond, Eangle, Wangle and the Coulomb discount energy; false if none ran
-bool device_bonded(System& s, double out[5]);
+// bonds and angles of the current layer: adds their forces to F; results in
+// hResult[40..44] (Ebond, Wbond, Eangle, Wangle, Coulomb discount energy) after a
+// synchronisation; false if there are none.  skip: the launches do nothing if it is set
+bool bonded_launch(System& s, const double* skip);
 void bonded_free(System& s);
 // R <- CR R + CP P / m (free atoms).
 void device_move(System& s, double CR, double CP);
 // pending boosts + move (CR = 1) + skin displacement + FP32 packing in one pass
-void device_step_fused(System& s, double CP);
+// (vv: with the shadow start values s0 of EmDee_verlet_step if compute; one kick of CP / 2)
+void device_step_fused(System& s, double CP, bool vv = false, double* s0 = nullptr);
 // applies pending boosts (before anything reads P or replaces F)
 void flush_pending(System& s);
 bool device_skin_from_step(System& s);
@@ -386,7 +398,8 @@ void device_pair_statistics(System& s, long* listed, long* within);
 void bodies_update(System& s);
 void bodies_boost(System& s, double CP, double CF, bool translate, bool rotate, bool kinetic);
 void bodies_move(System& s, double CR, double CP, double dt, bool translate, bool rotate, int mode);
-double bodies_virial(System& s);
+// result in hResult[6] (the virial is its negative) after a synchronisation
+void bodies_virial_launch(System& s, const double* skip);
 void bodies_assign(System& s, double* k6);
 void bodies_particle_momenta(System& s, double* dOut);
 void bodies_download(System& s);
@@ -395,13 +408,17 @@ void bodies_upload(System& s);
 long device_neighbor_pairs(System& s, int* pairs, long capacity);
 // Ewald k-space (ewald.cu): set-up at initialization, energy + forces per call
 void ewald_initialize(System& s, double kspaceRc);
-double ewald_compute(System& s);
+// (energy: ewald_energy after a synchronisation; skip as above)
+void ewald_launch(System& s, const double* skip);
+double ewald_energy(System& s);
 void ewald_free(System& s);
 // EmDee_rdf histograms over the current lists (neighbor.cu)
 void device_rdf_counts(System& s, int bins, double Rc, const std::vector<uint8_t>& hasPair,
                        const std::vector<uint8_t>& pairOn, int ntp, std::vector<unsigned long long>& counts);
 // EmDee_verlet_step halves (verlet.cu)
 void device_verlet_pre(System& s, double dt, bool compute, int mode);
+// the closing half of free atoms (results in hResult[34..38])
+void verlet_post_launch(System& s, double dt, bool compute, const double* skip);
 void device_verlet_post(System& s, double dt, bool compute, int mode, double* out);
 
 }  // namespace emdee

@@ -46,7 +46,9 @@ __global__ void __launch_bounds__(VV_THREADS) k_vv_post_free(const double* __res
                                                              const double* __restrict__ invMass, const int* list,
                                                              int n, double dt, double dt_2,
                                                              const double* __restrict__ s0, double* partials,
-                                                             unsigned int* ticket, double* result, double* hostResult) {
+                                                             unsigned int* ticket, double* result, double* hostResult,
+                                                             const double* skip) {
+  if (skip != nullptr && __double_as_longlong(*skip) != 0) return;   // a rebuild is due
   double v[5] = {0, 0, 0, 0, 0};
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     const int j = list ? list[q] : q;
@@ -185,8 +187,10 @@ static void verlet_pre(System& s, double dt, bool compute, int mode) {
   const bool all = s.nbodies == 0;
   const int nf = all ? s.natoms : s.nfree;
   ensure(w.s0, w.s0Cap, (size_t)3 * nf);
-  if (nf > 0) {
-    const int* list = all ? nullptr : s.dFree;
+  if (all) {   // with the skin check and the packing of the new positions in the same pass
+    device_step_fused(s, dt, true, compute ? w.s0 : nullptr);
+  } else if (nf > 0) {
+    const int* list = s.dFree;
     if (compute)
       k_vv_pre_free<true, FMA><<<vv_blocks(nf), VV_THREADS, 0, s.stream>>>(s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt,
                                                                       dt_2, w.s0);
@@ -210,14 +214,38 @@ static void verlet_pre(System& s, double dt, bool compute, int mode) {
   }
 }
 
-// out[0..2] 2KE_t, [3..5] 2KE_r, [6] Ks_t, [7] Ks_r, [8] Us (bodies first, then free atoms,
-// as each thread of the reference sums them)
 template <bool FMA>
-static void verlet_post(System& s, double dt, bool compute, int mode, double* out) {
+static void post_free(System& s, double dt, bool compute, const double* skip) {
   VerletScratch& w = s.verlet;
   const double dt_2 = 0.5 * dt;
   const bool all = s.nbodies == 0;
   const int nf = all ? s.natoms : s.nfree;
+  const int blocks = std::min(vv_blocks(nf), 1184);
+  ensure(w.partF, w.partFCap, (size_t)5 * blocks);
+  const int* list = all ? nullptr : s.dFree;
+  if (compute)
+    k_vv_post_free<true, FMA><<<blocks, VV_THREADS, 0, s.stream>>>(s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt, dt_2,
+                                                              w.s0, w.partF, s.dTicket + 6, s.dResult + 34,
+                                                              s.hResult + 34, skip);
+  else
+    k_vv_post_free<false, FMA><<<blocks, VV_THREADS, 0, s.stream>>>(s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt, dt_2,
+                                                               w.s0, nullptr, nullptr, nullptr, nullptr, skip);
+  CK(cudaGetLastError());
+  s.prof.total++;
+}
+
+void verlet_post_launch(System& s, double dt, bool compute, const double* skip) {
+  if (s.precision == 0) post_free<true>(s, dt, compute, skip);
+  else post_free<false>(s, dt, compute, skip);
+}
+
+// out[0..2] 2KE_t, [3..5] 2KE_r, [6] Ks_t, [7] Ks_r, [8] Us (bodies first, then free atoms,
+// as each thread of the reference sums them).  The free atoms' half may have been queued
+// behind the pair launch (vvQueued): its results are in place then.
+static void verlet_post(System& s, double dt, bool compute, int mode, double* out) {
+  VerletScratch& w = s.verlet;
+  const double dt_2 = 0.5 * dt;
+  const int nf = s.nbodies == 0 ? s.natoms : s.nfree;
   double vb[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, vf[5] = {0, 0, 0, 0, 0};
   if (s.nbodies > 0) {
     const int blocks = vv_body_blocks(s.nbodies);
@@ -232,22 +260,11 @@ static void verlet_post(System& s, double dt, bool compute, int mode, double* ou
     CK(cudaGetLastError());
     s.prof.total++;
   }
-  if (nf > 0) {
-    const int blocks = std::min(vv_blocks(nf), 1184);
-    ensure(w.partF, w.partFCap, (size_t)5 * blocks);
-    const int* list = all ? nullptr : s.dFree;
-    if (compute)
-      k_vv_post_free<true, FMA><<<blocks, VV_THREADS, 0, s.stream>>>(s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt, dt_2,
-                                                                w.s0, w.partF, s.dTicket + 6, s.dResult + 34,
-                                                                s.hResult + 34);
-    else
-      k_vv_post_free<false, FMA><<<blocks, VV_THREADS, 0, s.stream>>>(s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt, dt_2,
-                                                                 w.s0, nullptr, nullptr, nullptr, nullptr);
-    CK(cudaGetLastError());
-    s.prof.total++;
-  }
+  const bool queued = s.vvQueued;
+  s.vvQueued = false;
+  if (nf > 0 && !queued) verlet_post_launch(s, dt, compute, nullptr);
   if (compute) {
-    CK(cudaStreamSynchronize(s.stream));
+    if (!queued) CK(cudaStreamSynchronize(s.stream));
     for (int k = 0; k < 9 && s.nbodies > 0; k++) vb[k] = s.hResult[24 + k];
     for (int k = 0; k < 5 && nf > 0; k++) vf[k] = s.hResult[34 + k];
   }
@@ -266,8 +283,7 @@ void device_verlet_pre(System& s, double dt, bool compute, int mode) {
 }
 
 void device_verlet_post(System& s, double dt, bool compute, int mode, double* out) {
-  if (s.precision == 0) verlet_post<true>(s, dt, compute, mode, out);
-  else verlet_post<false>(s, dt, compute, mode, out);
+  verlet_post(s, dt, compute, mode, out);
 }
 
 }  // namespace emdee
