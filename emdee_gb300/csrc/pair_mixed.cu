@@ -52,7 +52,7 @@ struct PairArgsF {
   const uint16_t* nb;
   const int* count;
   int cap, tileStride, haloCap;
-  int tpa, tpaShift;   // threads per atom (a power of 2, at most 8) and its log2
+  int tpa, tpaShift;   // threads per atom (a power of 2, at most 32) and its log2
   const PairEntry<float>* table;   // this layer: [itype][jtype] -> pair(jtype, itype)
   const NBParams<float>* coul;
   int ntypes;
@@ -96,12 +96,15 @@ __device__ __noinline__ bool refilter_exact(const PairArgsF& A, const int* lay, 
 // wrap would bring the sentinel back).
 template <bool COMPUTE, int VAR, int MOD, bool MINIMG, bool COUNT, bool REFILTER>
 __global__ void PAIR_BOUNDS k_pair_mixed(PairArgsF A) {
-  // plain Lennard-Jones (the benchmark's model): two list entries per step of the
-  // inner loop in packed FP32 arithmetic
+  // plain, shifted and force-shifted Lennard-Jones: two list entries per step of the
+  // inner loop in packed FP32 arithmetic, which halves the issued instructions (force-
+  // shifted, 100,003 atoms: 13.2 M warp instructions per launch one entry at a time,
+  // 10 steps 892 -> 810 us with two)
 #ifdef EMDEE_SCALAR_PAIR   // tuning define: the scalar loop for every variant
   constexpr bool PACKED = false;
 #else
-  constexpr bool PACKED = VAR != 1 && MOD == NONE && !MINIMG && !COUNT && !REFILTER;
+  constexpr bool PACKED = VAR != 1 && (MOD == NONE || MOD == SHIFTED || MOD == SHIFTED_FORCE) && !MINIMG && !COUNT &&
+                          !REFILTER;
 #endif
   // the flag is 0.0 or 1.0: tested on its bits (an FP64 compare in every thread of
   // every block would queue on the slow FP64 pipe)
@@ -129,6 +132,8 @@ __global__ void PAIR_BOUNDS k_pair_mixed(PairArgsF A) {
   const float sigc = m0.sigsq * A.invw2, eps48 = 2.0f * m0.eps24;
   const f32x2 sigc2 = pk2(sigc, sigc), eps48_2 = pk2(eps48, eps48), meps24_2 = pk2(-m0.eps24, -m0.eps24),
               eps4_2 = pk2(m0.eps4, m0.eps4), meps4_2 = pk2(-m0.eps4, -m0.eps4);
+  const float fsh = m0.fshift / A.invw;   // force shift per cell edge
+  const f32x2 fsh2 = pk2(fsh, fsh), mfsh2 = pk2(-fsh, -fsh);
   NBParams<float> coul;
   if (VAR == 1) coul = *A.coul;
   const int tb = A.start[t * cells], te = A.start[(t + 1) * cells];
@@ -149,9 +154,6 @@ __global__ void PAIR_BOUNDS k_pair_mixed(PairArgsF A) {
     const int ti = VAR == 1 ? htype[qi] : 0;
     float fx = 0.f, fy = 0.f, fz = 0.f;
     f32x2 fx2 = 0ull, fy2 = 0ull, fz2 = 0ull, ep2 = 0ull, wp2 = 0ull;   // PACKED accumulators
-#ifdef PAIR_KAHAN
-    f32x2 ec2 = 0ull, wc2 = 0ull;   // compensations
-#endif
     int nIn = 0;
     uint16_t* myIn = REFILTER ? A.nbIn + ((size_t)t * (A.capIn >> 3) * A.tileStride + li) * 8 : nullptr;
     const int ai = REFILTER ? A.orig[si] : 0;
@@ -168,26 +170,23 @@ __global__ void PAIR_BOUNDS k_pair_mixed(PairArgsF A) {
           const float4 pa = hpos[w[k] & 0xFFFF], pb = hpos[w[k] >> 16];
           const f32x2 dx = pk2(pi.x - pa.x, pi.x - pb.x), dy = pk2(pi.y - pa.y, pi.y - pb.y),
                       dz = pk2(pi.z - pa.z, pi.z - pb.z);
-          const float2 r2 = up2(fma2(dz, dz, fma2(dy, dy, mul2(dx, dx))));
-          const f32x2 inv = pk2(r2.x < A.rc2 ? Ops<float>::rcp(r2.x) : 0.f, r2.y < A.rc2 ? Ops<float>::rcp(r2.y) : 0.f);
+          const f32x2 r22 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+          const float2 r2 = up2(r22);
+          const bool ina = r2.x < A.rc2, inb = r2.y < A.rc2;
+          const f32x2 inv = pk2(ina ? Ops<float>::rcp(r2.x) : 0.f, inb ? Ops<float>::rcp(r2.y) : 0.f);
           const f32x2 sr2 = mul2(sigc2, inv), sr6 = mul2(mul2(sr2, sr2), sr2);
-          const f32x2 W = mul2(sr6, fma2(eps48_2, sr6, meps24_2));
-#ifdef PAIR_KAHAN   // tuning define: per-thread compensated (Kahan) energy and virial sums
-          {
-            const f32x2 mone = pk2(-1.f, -1.f);
-            if (COMPUTE) {
-              const f32x2 y = fma2(mone, ec2, mul2(sr6, fma2(eps4_2, sr6, meps4_2))), t = add2(ep2, y);
-              ec2 = fma2(mone, y, fma2(mone, ep2, t));
-              ep2 = t;
-            }
-            const f32x2 y = fma2(mone, wc2, W), t = add2(wp2, y);
-            wc2 = fma2(mone, y, fma2(mone, wp2, t));
-            wp2 = t;
+          f32x2 W = mul2(sr6, fma2(eps48_2, sr6, meps24_2)), r = 0ull;
+          if (MOD == SHIFTED_FORCE) {   // the distance, zero beyond the cut-off
+            r = mul2(r22, pk2(ina ? Ops<float>::rsqrt(r2.x) : 0.f, inb ? Ops<float>::rsqrt(r2.y) : 0.f));
+            W = fma2(mfsh2, r, W);
           }
-#else
-          if (COMPUTE) ep2 = fma2(sr6, fma2(eps4_2, sr6, meps4_2), ep2);
+          if (COMPUTE && MOD == NONE) ep2 = fma2(sr6, fma2(eps4_2, sr6, meps4_2), ep2);
+          if (COMPUTE && MOD != NONE) {
+            f32x2 sh = pk2(ina ? m0.eshift : 0.f, inb ? m0.eshift : 0.f);
+            if (MOD == SHIFTED_FORCE) sh = fma2(fsh2, r, sh);
+            ep2 = add2(ep2, fma2(sr6, fma2(eps4_2, sr6, meps4_2), sh));
+          }
           wp2 = add2(wp2, W);
-#endif
           const f32x2 sc = mul2(W, inv);
           fx2 = fma2(sc, dx, fx2);
           fy2 = fma2(sc, dy, fy2);
@@ -261,14 +260,8 @@ __global__ void PAIR_BOUNDS k_pair_mixed(PairArgsF A) {
       fx = a.x + a.y;
       fy = b.x + b.y;
       fz = c.x + c.y;
-#ifdef PAIR_KAHAN
-      const float2 ce = up2(ec2), cw = up2(wc2);
-      if (COMPUTE) Ep += (ee.x - ce.x) + (ee.y - ce.y);
-      Wp += (ww.x - cw.x) + (ww.y - cw.y);
-#else
       if (COMPUTE) Ep += ee.x + ee.y;
       Wp += ww.x + ww.y;
-#endif
     }
     for (int o = tpa >> 1; o > 0; o >>= 1) {
       fx += __shfl_xor_sync(gmask, fx, o);
@@ -402,7 +395,7 @@ __global__ void __launch_bounds__(PAIR_THREADS_TYPES) k_pair_types(PairArgsF A) 
         const float inv2 = Ops<float>::rcp(r2);
         float rs = 0.f, r = 0.f;
         if (COUL || LSHIFT) {
-          asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(r2));
+          rs = Ops<float>::rsqrt(r2);
           r = r2 * rs;
         }
         // E = 4 eps (sr12 - sr6), W = 24 eps (2 sr12 - sr6)

@@ -70,11 +70,17 @@ template <> struct Ops<float> {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
     return r;
   }
+  static __device__ __forceinline__ float rsqrt(float a) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+  }
   static __device__ __forceinline__ float ex(float a) { return __expf(a); }
   static __device__ __forceinline__ float sq(float a) { return sqrtf(a); }
 #else
   static inline float div(float a, float b) { return a / b; }
   static inline float rcp(float a) { return 1.0f / a; }
+  static inline float rsqrt(float a) { return 1.0f / sqrtf(a); }
   static inline float ex(float a) { return expf(a); }
   static inline float sq(float a) { return sqrtf(a); }
 #endif
