@@ -21,7 +21,19 @@
 
 namespace emdee {
 
-static const int BONDED_THREADS = 256;
+// Threads per block.  A bond or angle is a chain of some 300 FP64 operations and a warp
+// instruction holds its quarter's FP64 unit for 64 cycles, so few terms go in blocks of
+// one warp, spread over all SMs; from BONDED_FEW terms on (one warp for each of the
+// 152 SMs) larger blocks leave fewer partial sums to the last one.  A whole force
+// computation of bonds and angles alone, blocks of 256 threads and the scaled
+// differences -> blocks by the rule and DIFF: 1500 terms 63.4 -> 58.5 us (blocks of 32;
+// 9000 terms: 69.0 with 32, 57.9 with 128, hence the line), 30,000 terms 67.7 -> 61.6 and
+// 90,000 terms 98.8 -> 87 us (of 128), 300,000 terms 171 -> 143 us (of 256; 174 with 128).
+static const int BONDED_THREADS = 256, BONDED_THREADS_MID = 128, BONDED_THREADS_FEW = 32;
+static const int BONDED_FEW = 152 * 32, BONDED_MID = 152 * 1024;
+static int bonded_threads(int n) {
+  return n < BONDED_FEW ? BONDED_THREADS_FEW : n < BONDED_MID ? BONDED_THREADS_MID : BONDED_THREADS;
+}
 
 struct BondedArgs {
   const double* R;
@@ -32,7 +44,7 @@ struct BondedArgs {
   double* vec;          // contribution vectors, 3 doubles each
   int nbonds, nitems;
   int bonded, kspace;
-  double L, invL2, alpha, beta;
+  double L, invL, invL2, alpha, beta;
   const int* first;     // per atom: [first[a], first[a+1]) entries
   const int* entry;     // vector index << 1 | negate
   int natoms;
@@ -46,6 +58,8 @@ struct BondedArgs {
 enum BondedKind : int { BK_NONE = 0, BK_HARMONIC = 1 };
 
 // cKspaceModel_discount (src/modelClass_kspace.f90:321-334)
+__device__ __forceinline__ double nearest(const BondedArgs& A, double x) { return x - A.L * round(x * A.invL); }
+
 __device__ __forceinline__ void kspace_discount(double alpha, double beta, double rsq, double QiQj, double& E,
                                                 double& W) {
   const double r = sqrt(rsq), x = alpha * r, expmx2 = exp(-x * x);
@@ -53,7 +67,11 @@ __device__ __forceinline__ void kspace_discount(double alpha, double beta, doubl
   W = E + QiQj * beta * expmx2;
 }
 
-__global__ void __launch_bounds__(BONDED_THREADS) k_bonded(BondedArgs A) {
+// DIFF (mixed precision): separations as x - L round(x / L) of the difference x, rounded
+// once, instead of the difference of two scaled coordinates (a division each, rounded on
+// the scale of the box).  FP64 mode keeps the reference's statements.
+template <int THREADS, bool DIFF>
+__global__ void __launch_bounds__(THREADS) k_bonded(BondedArgs A) {
   if (A.skip != nullptr && __double_as_longlong(*A.skip) != 0) return;
   double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
@@ -64,10 +82,14 @@ __global__ void __launch_bounds__(BONDED_THREADS) k_bonded(BondedArgs A) {
     if (m < A.nbonds) {   // compute_bonds, src/EmDeeData.f90:443-487
       double Rij[3];
       for (int d = 0; d < 3; d++) {
-        double x = A.R[3 * it.x + d] / A.L - A.R[3 * it.y + d] / A.L;
-        Rij[d] = x - round(x);
+        if (DIFF) {
+          Rij[d] = nearest(A, A.R[3 * it.x + d] - A.R[3 * it.y + d]);
+        } else {
+          double x = A.R[3 * it.x + d] / A.L - A.R[3 * it.y + d] / A.L;
+          Rij[d] = x - round(x);
+        }
       }
-      const double invR2 = A.invL2 / (Rij[0] * Rij[0] + Rij[1] * Rij[1] + Rij[2] * Rij[2]);
+      const double invR2 = (DIFF ? 1.0 : A.invL2) / (Rij[0] * Rij[0] + Rij[1] * Rij[1] + Rij[2] * Rij[2]);
       double W = 0.0;
       if (A.bonded) {
         double E = 0.0;
@@ -86,10 +108,16 @@ __global__ void __launch_bounds__(BONDED_THREADS) k_bonded(BondedArgs A) {
         W = W + WL;
       }
       double* out = A.vec + 3 * (size_t)m;
-      for (int d = 0; d < 3; d++) out[d] = W * invR2 * A.L * Rij[d];
+      for (int d = 0; d < 3; d++) out[d] = DIFF ? W * invR2 * Rij[d] : W * invR2 * A.L * Rij[d];
     } else {              // compute_angles, src/EmDeeData.f90:491-550
       double a[3], b[3];
       for (int d = 0; d < 3; d++) {
+        if (DIFF) {
+          const double rj = A.R[3 * it.y + d];
+          a[d] = nearest(A, A.R[3 * it.x + d] - rj);
+          b[d] = nearest(A, A.R[3 * it.z + d] - rj);
+          continue;
+        }
         const double rj = A.R[3 * it.y + d] / A.L;
         double x = A.R[3 * it.x + d] / A.L - rj, y = A.R[3 * it.z + d] / A.L - rj;
         a[d] = A.L * (x - round(x));
@@ -136,11 +164,12 @@ __global__ void __launch_bounds__(BONDED_THREADS) k_bonded(BondedArgs A) {
       }
     }
   }
-  grid_reduce<5, BONDED_THREADS>(v, A.partials, A.ticket, A.result, A.hostResult);
+  grid_reduce<5, THREADS>(v, A.partials, A.ticket, A.result, A.hostResult);
 }
 
 // F(a) += the atom's contributions, in list order
-__global__ void __launch_bounds__(BONDED_THREADS) k_bonded_gather(BondedArgs A) {
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) k_bonded_gather(BondedArgs A) {
   if (A.skip != nullptr && __double_as_longlong(*A.skip) != 0) return;
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= A.natoms) return;
@@ -201,7 +230,7 @@ static void bonded_upload(System& s) {
   CK(cudaMalloc(&B.dVec, sizeof(double) * 3 * nvec));
   CK(cudaMalloc(&B.dFirst, sizeof(int) * (N + 1)));
   CK(cudaMalloc(&B.dEntry, sizeof(int) * std::max<size_t>(entry.size(), 1)));
-  const int blocks = (n + BONDED_THREADS - 1) / BONDED_THREADS;
+  const int th = bonded_threads(n), blocks = (n + th - 1) / th;
   CK(cudaMalloc(&B.dPartials, sizeof(double) * 5 * blocks));
   CK(cudaMemcpyAsync(B.dItem, item.data(), sizeof(int4) * n, cudaMemcpyHostToDevice, s.stream));
   CK(cudaMemcpyAsync(B.dParam, param.data(), sizeof(double2) * n, cudaMemcpyHostToDevice, s.stream));
@@ -211,6 +240,17 @@ static void bonded_upload(System& s) {
     CK(cudaMemcpyAsync(B.dEntry, entry.data(), sizeof(int) * entry.size(), cudaMemcpyHostToDevice, s.stream));
   CK(cudaStreamSynchronize(s.stream));   // the host vectors above go out of scope
   B.uploaded = n;
+}
+
+template <int THREADS>
+static void launch(System& s, const BondedArgs& A) {
+  const int blocks = (A.nitems + THREADS - 1) / THREADS;
+  if (s.precision == 0) k_bonded<THREADS, true><<<blocks, THREADS, 0, s.stream>>>(A);
+  else k_bonded<THREADS, false><<<blocks, THREADS, 0, s.stream>>>(A);
+  CK(cudaGetLastError());
+  k_bonded_gather<THREADS><<<(A.natoms + THREADS - 1) / THREADS, THREADS, 0, s.stream>>>(A);
+  CK(cudaGetLastError());
+  s.prof.total += 2;
 }
 
 bool bonded_launch(System& s, const double* skip) {
@@ -232,6 +272,7 @@ bool bonded_launch(System& s, const double* skip) {
   A.bonded = bonded;
   A.kspace = kspace;
   A.L = *s.Lbox;
+  A.invL = 1.0 / A.L;
   A.invL2 = 1.0 / (A.L * A.L);
   A.alpha = s.ewald.alpha;
   A.beta = s.ewald.beta;
@@ -243,11 +284,11 @@ bool bonded_launch(System& s, const double* skip) {
   A.result = s.dResult + 40;
   A.hostResult = s.hResult + 40;
   A.skip = skip;
-  k_bonded<<<(n + BONDED_THREADS - 1) / BONDED_THREADS, BONDED_THREADS, 0, s.stream>>>(A);
-  CK(cudaGetLastError());
-  k_bonded_gather<<<(s.natoms + BONDED_THREADS - 1) / BONDED_THREADS, BONDED_THREADS, 0, s.stream>>>(A);
-  CK(cudaGetLastError());
-  s.prof.total += 2;
+  switch (bonded_threads(n)) {
+    case BONDED_THREADS_FEW: launch<BONDED_THREADS_FEW>(s, A); break;
+    case BONDED_THREADS_MID: launch<BONDED_THREADS_MID>(s, A); break;
+    default: launch<BONDED_THREADS>(s, A);
+  }
   return true;
 }
 
