@@ -338,17 +338,23 @@ static void compute_forces_impl(tEmDee* md) {
   s.skinReady = s.packReady = false;
   const int l = s.layer - 1;
   const bool kspace = s.coul[l].requires_kspace != 0;
-  const bool haveBonded = !s.bondedTerms.bonds.empty() || !s.bondedTerms.angles.empty();
+  const bool haveBonded = bonded_active(s);
   if (!s.extrasQueued && (haveBonded || kspace || s.nbodies != 0)) {   // no pair launch to follow
-    bonded_launch(s, nullptr);
-    if (kspace) ewald_launch(s, nullptr);
+    if (haveBonded) {
+      bonded_launch(s, nullptr, s.stream);
+      bonded_add(s, nullptr);
+    }
+    if (kspace) {
+      ewald_launch(s, nullptr, s.stream);
+      ewald_add(s, nullptr);
+    }
     if (s.nbodies != 0) bodies_virial_launch(s, nullptr);
     CK(cudaStreamSynchronize(s.stream));
   }
   const double* r = s.hResult;   // Epair, Ecoul, Wpair, Wcoul
   // Ebond, Wbond, Eangle, Wangle, Coulomb discounts of bonds and angles
   const double none[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  const double* bonded = haveBonded && (s.bonded[l] != 0 || kspace) ? r + 40 : none;
+  const double* bonded = haveBonded ? r + 40 : none;
   const double Ecoul = r[1] + bonded[4];
   double Elong = 0.0, Wlong = 0.0;
   if (kspace) {   // src/EmDeeCode.f90:1249-1252
@@ -526,6 +532,9 @@ tEmDee EmDee_system(int threads, int layers, double rc, double skin, int N, int*
 
   // device state
   CK(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
+  CK(cudaStreamCreateWithFlags(&s->sideStream, cudaStreamNonBlocking));
+  CK(cudaEventCreateWithFlags(&s->forkEvent, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&s->joinEvent, cudaEventDisableTiming));
   size_t b3 = sizeof(double) * 3 * N;
   CK(cudaMalloc(&s->dR, b3));
   CK(cudaMalloc(&s->dP, b3));
@@ -641,6 +650,9 @@ void EmDee_destroy(tEmDee* md) {
   cudaFreeHost(s->hFlags);
   cudaFreeHost(s->hMirrorR); cudaFreeHost(s->hMirrorP); cudaFreeHost(s->hMirrorF); cudaFreeHost(s->hMirrorLayerF);
   if (s->ownsLbox) delete s->Lbox;
+  cudaEventDestroy(s->forkEvent);
+  cudaEventDestroy(s->joinEvent);
+  cudaStreamDestroy(s->sideStream);
   cudaStreamDestroy(s->stream);
   delete s;
   md->Data = nullptr;

@@ -168,8 +168,9 @@ __global__ void __launch_bounds__(THREADS) k_bonded(BondedArgs A) {
 }
 
 // F(a) += the atom's contributions, in list order
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS) k_bonded_gather(BondedArgs A) {
+static const int GATHER_THREADS = 64;
+
+__global__ void __launch_bounds__(GATHER_THREADS) k_bonded_gather(BondedArgs A) {
   if (A.skip != nullptr && __double_as_longlong(*A.skip) != 0) return;
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= A.natoms) return;
@@ -242,24 +243,15 @@ static void bonded_upload(System& s) {
   B.uploaded = n;
 }
 
-template <int THREADS>
-static void launch(System& s, const BondedArgs& A) {
-  const int blocks = (A.nitems + THREADS - 1) / THREADS;
-  if (s.precision == 0) k_bonded<THREADS, true><<<blocks, THREADS, 0, s.stream>>>(A);
-  else k_bonded<THREADS, false><<<blocks, THREADS, 0, s.stream>>>(A);
-  CK(cudaGetLastError());
-  k_bonded_gather<THREADS><<<(A.natoms + THREADS - 1) / THREADS, THREADS, 0, s.stream>>>(A);
-  CK(cudaGetLastError());
-  s.prof.total += 2;
+bool bonded_active(const System& s) {
+  const int l = s.layer - 1;
+  return !(s.bondedTerms.bonds.empty() && s.bondedTerms.angles.empty()) &&
+         (s.bonded[l] != 0 || s.coul[l].requires_kspace != 0);
 }
 
-bool bonded_launch(System& s, const double* skip) {
+static BondedArgs bonded_args(System& s, const double* skip) {
   BondedTerms& B = s.bondedTerms;
-  const int n = (int)(B.bonds.size() + B.angles.size());
-  const int l = s.layer - 1;
-  const bool bonded = s.bonded[l] != 0, kspace = s.coul[l].requires_kspace != 0;
-  if (n == 0 || !(bonded || kspace)) return false;
-  if (B.uploaded != n) bonded_upload(s);
+  const int l = s.layer - 1, n = B.uploaded;
   BondedArgs A;
   A.R = s.dR;
   A.F = s.F();
@@ -269,8 +261,8 @@ bool bonded_launch(System& s, const double* skip) {
   A.vec = B.dVec;
   A.nbonds = (int)B.bonds.size();
   A.nitems = n;
-  A.bonded = bonded;
-  A.kspace = kspace;
+  A.bonded = s.bonded[l] != 0;
+  A.kspace = s.coul[l].requires_kspace != 0;
   A.L = *s.Lbox;
   A.invL = 1.0 / A.L;
   A.invL2 = 1.0 / (A.L * A.L);
@@ -284,12 +276,35 @@ bool bonded_launch(System& s, const double* skip) {
   A.result = s.dResult + 40;
   A.hostResult = s.hResult + 40;
   A.skip = skip;
+  return A;
+}
+
+template <int THREADS>
+static void launch(System& s, const BondedArgs& A, cudaStream_t stream) {
+  const int blocks = (A.nitems + THREADS - 1) / THREADS;
+  if (s.precision == 0) k_bonded<THREADS, true><<<blocks, THREADS, 0, stream>>>(A);
+  else k_bonded<THREADS, false><<<blocks, THREADS, 0, stream>>>(A);
+  CK(cudaGetLastError());
+  s.prof.total++;
+}
+
+void bonded_launch(System& s, const double* skip, cudaStream_t stream) {
+  BondedTerms& B = s.bondedTerms;
+  const int n = (int)(B.bonds.size() + B.angles.size());
+  if (B.uploaded != n) bonded_upload(s);
+  const BondedArgs A = bonded_args(s, skip);
   switch (bonded_threads(n)) {
-    case BONDED_THREADS_FEW: launch<BONDED_THREADS_FEW>(s, A); break;
-    case BONDED_THREADS_MID: launch<BONDED_THREADS_MID>(s, A); break;
-    default: launch<BONDED_THREADS>(s, A);
+    case BONDED_THREADS_FEW: launch<BONDED_THREADS_FEW>(s, A, stream); break;
+    case BONDED_THREADS_MID: launch<BONDED_THREADS_MID>(s, A, stream); break;
+    default: launch<BONDED_THREADS>(s, A, stream);
   }
-  return true;
+}
+
+void bonded_add(System& s, const double* skip) {
+  const BondedArgs A = bonded_args(s, skip);
+  k_bonded_gather<<<(A.natoms + GATHER_THREADS - 1) / GATHER_THREADS, GATHER_THREADS, 0, s.stream>>>(A);
+  CK(cudaGetLastError());
+  s.prof.total++;
 }
 
 void bonded_free(System& s) {

@@ -524,7 +524,7 @@ void ewald_initialize(System& s, double kspaceRc) {
 
 // k-space energy of the current layer (plus the rigid-pair and self discounts);
 // forces added to the current layer's force array
-void ewald_launch(System& s, const double* skip) {
+static EwArgs ewald_args(System& s, const double* skip) {
   Ewald& e = s.ewald;
   const int l = s.layer - 1;
   EwArgs A;
@@ -558,23 +558,35 @@ void ewald_launch(System& s, const double* skip) {
   A.result = s.dResult + 22;
   A.hostResult = s.hResult + 22;   // pinned: read after the synchronisation
   A.skip = skip;
+  return A;
+}
+
+void ewald_launch(System& s, const double* skip, cudaStream_t stream) {
+  Ewald& e = s.ewald;
+  const EwArgs A = ewald_args(s, skip);
   const int rows = e.nmax + 1;
   if ((size_t)3 * rows * TABLE_LIMIT_ATOMS * sizeof(double2) > 227 * 1024)
     fatal("kspace computation", "too many k-vectors per dimension");
   const size_t smemSF = (size_t)((3 * rows) | 1) * SF_ATOMS * sizeof(double2);
-  const size_t smemF = (size_t)4 * rows * FORCE_ATOMS * sizeof(double2);
   CK(cudaFuncSetAttribute(k_ewald_sf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemSF));
-  CK(cudaFuncSetAttribute(k_ewald_force, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemF));
-  k_ewald_tables<<<(3 * e.nq + 127) / 128, 128, 0, s.stream>>>(A);
+  k_ewald_tables<<<(3 * e.nq + 127) / 128, 128, 0, stream>>>(A);
   CK(cudaGetLastError());
   const dim3 grid((e.ntasks + SF_THREADS - 1) / SF_THREADS, e.nchunks);
-  k_ewald_sf<<<grid, SF_THREADS, smemSF, s.stream>>>(A);
+  k_ewald_sf<<<grid, SF_THREADS, smemSF, stream>>>(A);
   CK(cudaGetLastError());
-  k_ewald_sigma<<<(e.npairs + SIGMA_PAIRS - 1) / SIGMA_PAIRS, SIGMA_PAIRS * SIGMA_SLICES, 0, s.stream>>>(A);
+  k_ewald_sigma<<<(e.npairs + SIGMA_PAIRS - 1) / SIGMA_PAIRS, SIGMA_PAIRS * SIGMA_SLICES, 0, stream>>>(A);
   CK(cudaGetLastError());
+  s.prof.total += 3;
+}
+
+void ewald_add(System& s, const double* skip) {
+  Ewald& e = s.ewald;
+  const EwArgs A = ewald_args(s, skip);
+  const size_t smemF = (size_t)4 * (e.nmax + 1) * FORCE_ATOMS * sizeof(double2);
+  CK(cudaFuncSetAttribute(k_ewald_force, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemF));
   k_ewald_force<<<(e.nq + FORCE_ATOMS - 1) / FORCE_ATOMS, FORCE_ATOMS * FORCE_SPLIT, smemF, s.stream>>>(A);
   CK(cudaGetLastError());
-  s.prof.total += 4;
+  s.prof.total++;
 }
 
 double ewald_energy(System& s) {

@@ -224,6 +224,10 @@ struct System {
 
   // device state
   cudaStream_t stream = nullptr;
+  // terms that do not read the pair forces (bonds and angles, the k-space sums) run here
+  // beside the pair kernel, between two events on the system's stream
+  cudaStream_t sideStream = nullptr;
+  cudaEvent_t forkEvent = nullptr, joinEvent = nullptr;
   double *dR = nullptr, *dP = nullptr, *dR0 = nullptr, *dLayerF = nullptr;
   bool ownsRP = true;
   double *dInvMass = nullptr, *dCharge = nullptr;
@@ -380,10 +384,12 @@ bool device_kinetic(System& s, double* twoKE, const double* src = nullptr, const
 // applies the pending kicks (1 or 2) and writes the momenta to P and to out (a
 // device-accessible pointer to the caller's pinned buffer); synchronizes
 void device_kick_out(System& s, double* out);
-// bonds and angles of the current layer: adds their forces to F; results in
-// hResult[40..44] (Ebond, Wbond, Eangle, Wangle, Coulomb discount energy) after a
-// synchronisation; false if there are none.  skip: the launches do nothing if it is set
-bool bonded_launch(System& s, const double* skip);
+// bonds and angles of the current layer, on the given stream: results in hResult[40..44]
+// (Ebond, Wbond, Eangle, Wangle, Coulomb discount energy) after a synchronisation.
+// skip: the launch does nothing if it is set.  bonded_add adds their forces to F.
+bool bonded_active(const System& s);
+void bonded_launch(System& s, const double* skip, cudaStream_t stream);
+void bonded_add(System& s, const double* skip);
 void bonded_free(System& s);
 // R <- CR R + CP P / m (free atoms).
 void device_move(System& s, double CR, double CP);
@@ -408,8 +414,10 @@ void bodies_upload(System& s);
 long device_neighbor_pairs(System& s, int* pairs, long capacity);
 // Ewald k-space (ewald.cu): set-up at initialization, energy + forces per call
 void ewald_initialize(System& s, double kspaceRc);
-// (energy: ewald_energy after a synchronisation; skip as above)
-void ewald_launch(System& s, const double* skip);
+// (the sums over atoms on the given stream, then ewald_add for the forces; energy:
+// ewald_energy after a synchronisation; skip as above)
+void ewald_launch(System& s, const double* skip, cudaStream_t stream);
+void ewald_add(System& s, const double* skip);
 double ewald_energy(System& s);
 void ewald_free(System& s);
 // EmDee_rdf histograms over the current lists (neighbor.cu)
