@@ -1297,7 +1297,14 @@ void EmDee_boost(tEmDee* md, double lambda, double alpha, double dt) {
     return;
   }
   s.keSpecValid = false;
-  if (lambda != 0.0 && !s.forcesUpToDate[s.layer - 1]) compute_forces_impl(md);
+  const System::BodyBoost bb = {CP, CF, translate, rotate, compute};
+  s.boostQueued = false;
+  if (lambda != 0.0 && !s.forcesUpToDate[s.layer - 1]) {
+    s.boost = bb;
+    s.boostReq = s.nbodies > 0 && compute;   // queued behind the forces: one wait for both sums
+    compute_forces_impl(md);
+    s.boostReq = false;
+  }
   // Without energies, a plain kick (CP = 1, free atoms) is deferred to the next
   // kernel that touches P: the fused step of EmDee_displace, or a flush.  The
   // arithmetic and its order are unchanged.
@@ -1308,8 +1315,14 @@ void EmDee_boost(tEmDee* md, double lambda, double alpha, double dt) {
     return;
   }
   flush_pending(s);
-  if (s.nbodies > 0) bodies_boost(s, CP, CF, translate, rotate, compute);
-  else if (translate) device_boost(s, CP, CF, compute);
+  if (s.nbodies > 0) {
+    if (!s.boostQueued) {
+      bodies_boost_launch(s, bb, nullptr);
+      if (compute) CK(cudaStreamSynchronize(s.stream));
+    }
+    if (compute) bodies_boost_sums(s, bb);
+    s.boostQueued = false;
+  } else if (translate) device_boost(s, CP, CF, compute);
   if (compute) {
     if (translate)
       for (int d = 0; d < 3; d++) md->Kinetic.TransPart[d] = 0.5 * s.hResult[10 + d];

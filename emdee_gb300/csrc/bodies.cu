@@ -62,7 +62,9 @@ __device__ __forceinline__ double body_Bt(const double* q, const double* p, int 
 __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_boost(BodyArgs A, const double* __restrict__ F, double CP,
                                                                    double CF, int translate, int rotate, int kinetic,
                                                                    double* partials, unsigned int* ticket,
-                                                                   double* result, double* hostResult) {
+                                                                   double* result, double* hostResult,
+                                                                   const double* skip) {
+  if (skip != nullptr && __double_as_longlong(*skip) != 0) return;   // a rebuild is due
   double k6[6] = {0, 0, 0, 0, 0, 0};
   const BodyLane g = body_lane();
   if (g.i < A.nb) {
@@ -306,7 +308,9 @@ template <bool KIN>
 __global__ void __launch_bounds__(BODY_THREADS) k_boost_free(double* __restrict__ P, const double* __restrict__ F,
                                                              const double* __restrict__ invMass, const int* freeList,
                                                              int nfree, double CP, double CF, double* partials,
-                                                             unsigned int* ticket, double* result, double* hostResult) {
+                                                             unsigned int* ticket, double* result, double* hostResult,
+                                                             const double* skip) {
+  if (skip != nullptr && __double_as_longlong(*skip) != 0) return;   // a rebuild is due
   double k2[3] = {0.0, 0.0, 0.0};
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nfree; q += gridDim.x * blockDim.x) {
     int i = freeList[q];
@@ -386,36 +390,35 @@ void bodies_update(System& s) {
   CK(cudaMemcpy(s.dR, R.data(), sizeof(double) * 3 * N, cudaMemcpyHostToDevice));
 }
 
-// boost of free atoms (through the list) and bodies; 2KE into hResult[10..12]
-// (translational) and [13..15] (rotational)
-void bodies_boost(System& s, double CP, double CF, bool translate, bool rotate, bool kinetic) {
+// boost of free atoms (through the list) and bodies
+void bodies_boost_launch(System& s, const System::BodyBoost& b, const double* skip) {
   int freeBlocks = std::min(body_blocks(s.nfree), 1184);
   ensure_scratch(s, freeBlocks * 3 + body_group_blocks(s.nbodies) * 6, 1);
-  if (translate && s.nfree > 0) {
+  if (b.translate && s.nfree > 0) {
     int blocks = freeBlocks;
-    if (kinetic) {
-      k_boost_free<true><<<blocks, BODY_THREADS, 0, s.stream>>>(s.dP, s.F(), s.dInvMass, s.dFree, s.nfree, CP, CF,
+    if (b.kinetic) {
+      k_boost_free<true><<<blocks, BODY_THREADS, 0, s.stream>>>(s.dP, s.F(), s.dInvMass, s.dFree, s.nfree, b.CP, b.CF,
                                                                 s.dBodyScratch, s.dTicket + 2, s.dResult + 10,
-                                                                s.hResult + 10);
+                                                                s.hResult + 10, skip);
     } else {
-      k_boost_free<false><<<blocks, BODY_THREADS, 0, s.stream>>>(s.dP, s.F(), s.dInvMass, s.dFree, s.nfree, CP, CF,
-                                                                 nullptr, nullptr, nullptr, nullptr);
+      k_boost_free<false><<<blocks, BODY_THREADS, 0, s.stream>>>(s.dP, s.F(), s.dInvMass, s.dFree, s.nfree, b.CP, b.CF,
+                                                                 nullptr, nullptr, nullptr, nullptr, skip);
     }
     CK(cudaGetLastError());
     s.prof.total++;
   }
-  k_body_boost<<<body_group_blocks(s.nbodies), BODY_GROUP_THREADS, 0, s.stream>>>(body_args(s), s.F(), CP, CF, translate, rotate, kinetic,
-                                                       s.dBodyScratch + freeBlocks * 3, s.dTicket + 3, s.dResult + 16,
-                                                       s.hResult + 16);
+  k_body_boost<<<body_group_blocks(s.nbodies), BODY_GROUP_THREADS, 0, s.stream>>>(
+      body_args(s), s.F(), b.CP, b.CF, b.translate, b.rotate, b.kinetic, s.dBodyScratch + freeBlocks * 3,
+      s.dTicket + 3, s.dResult + 16, s.hResult + 16, skip);
   CK(cudaGetLastError());
   s.prof.total++;
-  if (kinetic) {
-    CK(cudaStreamSynchronize(s.stream));
-    const double* k6 = s.hResult + 16;
-    for (int k = 0; k < 3; k++) {
-      s.hResult[10 + k] = (translate && s.nfree > 0 ? s.hResult[10 + k] : 0.0) + k6[k];
-      s.hResult[13 + k] = k6[3 + k];
-    }
+}
+
+void bodies_boost_sums(System& s, const System::BodyBoost& b) {
+  const double* k6 = s.hResult + 16;
+  for (int k = 0; k < 3; k++) {
+    s.hResult[10 + k] = (b.translate && s.nfree > 0 ? s.hResult[10 + k] : 0.0) + k6[k];
+    s.hResult[13 + k] = k6[3 + k];
   }
 }
 

@@ -430,6 +430,7 @@ bool device_pair_forces(System& s, bool compute, bool speculative) {
       if (kspace) ewald_add(s, skip);
     }
     if (s.nbodies > 0) bodies_virial_launch(s, skip);
+    if (s.boostReq) bodies_boost_launch(s, s.boost, skip);
     if (s.vvReq) verlet_post_launch(s, s.vvDt, s.vvCompute, skip);
   }
   // The last block of the pair kernel wrote the sums, and the fused step the skin value
@@ -445,6 +446,7 @@ bool device_pair_forces(System& s, bool compute, bool speculative) {
   if (s.queueExtras) {
     s.extrasQueued = true;
     s.vvQueued = s.vvReq;
+    s.boostQueued = s.boostReq;
   }
   return true;
 }

@@ -273,6 +273,12 @@ struct System {
   bool queueExtras = false, extrasQueued = false;
   bool vvReq = false, vvQueued = false, vvCompute = false;
   double vvDt = 0.0;
+  // EmDee_boost of a system with rigid bodies that waits for new forces: queued the same way
+  struct BodyBoost {
+    double CP, CF;
+    bool translate, rotate, kinetic;
+  } boost = {};
+  bool boostReq = false, boostQueued = false;
   bool phaseShared = false;   // R/P aliased with another system (no deferral then)
   const double* pairSkip = nullptr;   // device rebuild flag the mixed pair kernel checks first
   double builtL = 0;           // box length at the last build
@@ -402,7 +408,10 @@ bool device_skin_from_step(System& s);
 void device_pair_statistics(System& s, long* listed, long* within);
 // Rigid bodies (bodies.cu).
 void bodies_update(System& s);
-void bodies_boost(System& s, double CP, double CF, bool translate, bool rotate, bool kinetic);
+// boost of free atoms and bodies; after a synchronisation, bodies_boost_sums leaves 2KE in
+// hResult[10..12] (translational) and [13..15] (rotational)
+void bodies_boost_launch(System& s, const System::BodyBoost& b, const double* skip);
+void bodies_boost_sums(System& s, const System::BodyBoost& b);
 void bodies_move(System& s, double CR, double CP, double dt, bool translate, bool rotate, int mode);
 // result in hResult[6] (the virial is its negative) after a synchronisation
 void bodies_virial_launch(System& s, const double* skip);
