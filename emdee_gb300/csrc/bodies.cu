@@ -6,6 +6,7 @@
 // variants of the boost and move kernels.
 #include <vector>
 
+#include "chain.cuh"
 #include "reduce.cuh"
 #include "bodies.cuh"
 #include "rigid.cuh"
@@ -64,6 +65,7 @@ __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_boost(BodyArgs A, c
                                                                    double* partials, unsigned int* ticket,
                                                                    double* result, double* hostResult,
                                                                    const double* skip) {
+  chain_wait();
   if (skip != nullptr && __double_as_longlong(*skip) != 0) return;   // a rebuild is due
   double k6[6] = {0, 0, 0, 0, 0, 0};
   const BodyLane g = body_lane();
@@ -181,6 +183,7 @@ __device__ __forceinline__ void body_move_one(const BodyArgs& A, int i, double* 
 
 __global__ void __launch_bounds__(BODY_THREADS) k_body_move(BodyArgs A, double* __restrict__ R, double CR, double CP,
                                                             double dt, int translate, int rotate, int mode) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < A.nb) body_move_one(A, i, R, CR, CP, dt, translate, rotate, mode);
 }
@@ -189,6 +192,7 @@ __global__ void __launch_bounds__(BODY_THREADS) k_body_move(BodyArgs A, double* 
 // operation) on BODY_LANES lanes per body.
 __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_move_series(BodyArgs A, double* __restrict__ R, double CR,
                                                                          double CP, double dt, int translate) {
+  chain_wait();
   const BodyLane g = body_lane();
   if (g.i >= A.nb) return;
   BodyState& B = A.b[g.i];
@@ -247,6 +251,7 @@ __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_move_series(BodyArg
 __global__ void __launch_bounds__(BODY_THREADS) k_body_virial(BodyArgs A, const double* __restrict__ F,
                                                               double* partials, unsigned int* ticket, double* result,
                                                               double* hostResult, const double* skip) {
+  chain_wait();
   if (skip != nullptr && __double_as_longlong(*skip) != 0) return;   // a rebuild is due
   double w[1] = {0.0};
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -310,6 +315,7 @@ __global__ void __launch_bounds__(BODY_THREADS) k_boost_free(double* __restrict_
                                                              int nfree, double CP, double CF, double* partials,
                                                              unsigned int* ticket, double* result, double* hostResult,
                                                              const double* skip) {
+  chain_wait();
   if (skip != nullptr && __double_as_longlong(*skip) != 0) return;   // a rebuild is due
   double k2[3] = {0.0, 0.0, 0.0};
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nfree; q += gridDim.x * blockDim.x) {
@@ -326,6 +332,7 @@ __global__ void __launch_bounds__(BODY_THREADS) k_boost_free(double* __restrict_
 __global__ void __launch_bounds__(BODY_THREADS) k_move_free(double* __restrict__ R, const double* __restrict__ P,
                                                             const double* __restrict__ invMass, const int* freeList,
                                                             int nfree, double CR, double CP) {
+  chain_wait();
   int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nfree) return;
   int i = freeList[q];
@@ -397,17 +404,17 @@ void bodies_boost_launch(System& s, const System::BodyBoost& b, const double* sk
   if (b.translate && s.nfree > 0) {
     int blocks = freeBlocks;
     if (b.kinetic) {
-      k_boost_free<true><<<blocks, BODY_THREADS, 0, s.stream>>>(s.dP, s.F(), s.dInvMass, s.dFree, s.nfree, b.CP, b.CF,
+      launch_chained(k_boost_free<true>, blocks, BODY_THREADS, 0, s.stream, s.dP, s.F(), s.dInvMass, s.dFree, s.nfree, b.CP, b.CF,
                                                                 s.dBodyScratch, s.dTicket + 2, s.dResult + 10,
                                                                 s.hResult + 10, skip);
     } else {
-      k_boost_free<false><<<blocks, BODY_THREADS, 0, s.stream>>>(s.dP, s.F(), s.dInvMass, s.dFree, s.nfree, b.CP, b.CF,
+      launch_chained(k_boost_free<false>, blocks, BODY_THREADS, 0, s.stream, s.dP, s.F(), s.dInvMass, s.dFree, s.nfree, b.CP, b.CF,
                                                                  nullptr, nullptr, nullptr, nullptr, skip);
     }
     CK(cudaGetLastError());
     s.prof.total++;
   }
-  k_body_boost<<<body_group_blocks(s.nbodies), BODY_GROUP_THREADS, 0, s.stream>>>(
+  launch_chained(k_body_boost, body_group_blocks(s.nbodies), BODY_GROUP_THREADS, 0, s.stream,
       body_args(s), s.F(), b.CP, b.CF, b.translate, b.rotate, b.kinetic, s.dBodyScratch + freeBlocks * 3,
       s.dTicket + 3, s.dResult + 16, s.hResult + 16, skip);
   CK(cudaGetLastError());
@@ -424,16 +431,16 @@ void bodies_boost_sums(System& s, const System::BodyBoost& b) {
 
 void bodies_move(System& s, double CR, double CP, double dt, bool translate, bool rotate, int mode) {
   if (translate && s.nfree > 0) {
-    k_move_free<<<body_blocks(s.nfree), BODY_THREADS, 0, s.stream>>>(s.dR, s.dP, s.dInvMass, s.dFree, s.nfree, CR,
+    launch_chained(k_move_free, body_blocks(s.nfree), BODY_THREADS, 0, s.stream, s.dR, s.dP, s.dInvMass, s.dFree, s.nfree, CR,
                                                                       CP);
     CK(cudaGetLastError());
     s.prof.total++;
   }
   if (rotate && mode == 0)
-    k_body_move_series<<<body_group_blocks(s.nbodies), BODY_GROUP_THREADS, 0, s.stream>>>(body_args(s), s.dR, CR, CP,
+    launch_chained(k_body_move_series, body_group_blocks(s.nbodies), BODY_GROUP_THREADS, 0, s.stream, body_args(s), s.dR, CR, CP,
                                                                                           dt, translate);
   else
-    k_body_move<<<body_blocks(s.nbodies), BODY_THREADS, 0, s.stream>>>(body_args(s), s.dR, CR, CP, dt, translate,
+    launch_chained(k_body_move, body_blocks(s.nbodies), BODY_THREADS, 0, s.stream, body_args(s), s.dR, CR, CP, dt, translate,
                                                                        rotate, mode);
   CK(cudaGetLastError());
   s.prof.total++;
@@ -442,7 +449,7 @@ void bodies_move(System& s, double CR, double CP, double dt, bool translate, boo
 void bodies_virial_launch(System& s, const double* skip) {
   int blocks = body_blocks(s.nbodies);
   ensure_scratch(s, blocks, 1);
-  k_body_virial<<<blocks, BODY_THREADS, 0, s.stream>>>(body_args(s), s.F(), s.dBodyScratch, s.dTicket + 3,
+  launch_chained(k_body_virial, blocks, BODY_THREADS, 0, s.stream, body_args(s), s.F(), s.dBodyScratch, s.dTicket + 3,
                                                         s.dResult + 6, s.hResult + 6, skip);
   CK(cudaGetLastError());
   s.prof.total++;

@@ -6,6 +6,7 @@
 // move:   R <- CR R + CP P/m (src/EmDeeData.f90:823-860).
 // FP64 throughout; compiled with -fmad=false so each update rounds exactly like
 // the reference's statement.
+#include "chain.cuh"
 #include "ffkick.cuh"
 #include "fpconv.h"
 #include "reduce.cuh"
@@ -30,6 +31,7 @@ __global__ void __launch_bounds__(MOTION_THREADS) k_boost(double* __restrict__ P
                                                           const double* __restrict__ invMass, int N, double CP,
                                                           double CF, double* partials, unsigned int* ticket,
                                                           double* twoKE, double* hostKE) {
+  chain_wait();
   double k2[3] = {0.0, 0.0, 0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
     double im = (KIN && !UNITM) ? invMass[i] : 1.0;
@@ -47,6 +49,7 @@ template <bool UNITCR, bool UNITM, bool FMA>
 __global__ void __launch_bounds__(MOTION_THREADS) k_move(double* __restrict__ R, const double* __restrict__ P,
                                                          const double* __restrict__ invMass, int N, double CR,
                                                          double CP) {
+  chain_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   double im = UNITM ? 1.0 : invMass[i];
@@ -122,7 +125,7 @@ static void boost_launch(System& s, double CP, double CF, bool kinetic) {
     prof_begin(s, PK_BOOST);
     auto kern = CP == 1.0 ? (s.unitMass ? k_boost<true, true, true, FMA> : k_boost<true, true, false, FMA>)
                           : (s.unitMass ? k_boost<true, false, true, FMA> : k_boost<true, false, false, FMA>);
-    kern<<<blocks, MOTION_THREADS, 0, s.stream>>>(s.dP, s.F(), s.dInvMass, N, CP, CF, s.dKE, s.dTicket + 1,
+    launch_chained(kern, blocks, MOTION_THREADS, 0, s.stream, s.dP, s.F(), s.dInvMass, N, CP, CF, s.dKE, s.dTicket + 1,
                                                   s.dResult + 10, s.hResult + 10);
     CK(cudaGetLastError());
     prof_end(s, PK_BOOST);
@@ -130,7 +133,7 @@ static void boost_launch(System& s, double CP, double CF, bool kinetic) {
   } else {
     prof_begin(s, PK_BOOST);
     auto kern = CP == 1.0 ? k_boost<false, true, true, FMA> : k_boost<false, false, true, FMA>;
-    kern<<<blocks, MOTION_THREADS, 0, s.stream>>>(s.dP, s.F(), s.dInvMass, N, CP, CF, nullptr, nullptr, nullptr, nullptr);
+    launch_chained(kern, blocks, MOTION_THREADS, 0, s.stream, s.dP, s.F(), s.dInvMass, N, CP, CF, nullptr, nullptr, nullptr, nullptr);
     CK(cudaGetLastError());
     prof_end(s, PK_BOOST);
   }
@@ -147,7 +150,7 @@ static void move_launch(System& s, double CR, double CP) {
   prof_begin(s, PK_MOVE);
   auto kern = CR == 1.0 ? (s.unitMass ? k_move<true, true, FMA> : k_move<true, false, FMA>)
                         : (s.unitMass ? k_move<false, true, FMA> : k_move<false, false, FMA>);
-  kern<<<(N + MOTION_THREADS - 1) / MOTION_THREADS, MOTION_THREADS, 0, s.stream>>>(s.dR, s.dP, s.dInvMass, N, CR, CP);
+  launch_chained(kern, (N + MOTION_THREADS - 1) / MOTION_THREADS, MOTION_THREADS, 0, s.stream, s.dR, s.dP, s.dInvMass, N, CR, CP);
   CK(cudaGetLastError());
   prof_end(s, PK_MOVE);
 }
@@ -226,6 +229,7 @@ __global__ void __launch_bounds__(MOTION_THREADS) k_kinetic_pending(const double
                                                                     double cf0, double cf1, double cf2,
                                                                     double* partials, unsigned int* ticket,
                                                                     double* result, double* hostResult) {
+  chain_wait();
   const size_t n3 = 3 * (size_t)N, stride = (size_t)gridDim.x * blockDim.x;
   const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   double k = 0.0;
@@ -255,8 +259,7 @@ void device_kinetic_pending(System& s, double CF) {
   c[s.npend] = CF;
   prof_begin(s, PK_BOOST);
 #define KP_LAUNCH(NK)                                                                                          \
-  (s.unitMass ? k_kinetic_pending<NK, true> : k_kinetic_pending<NK, false>)<<<blocks, MOTION_THREADS, 0,       \
-                                                                              s.stream>>>(                     \
+  launch_chained((s.unitMass ? k_kinetic_pending<NK, true> : k_kinetic_pending<NK, false>), blocks, MOTION_THREADS, 0, s.stream,                      \
       s.dP, s.F(), s.dInvMass, N, c[0], c[1], c[2], s.dKE, s.dTicket + 1, s.dResult, s.hResult)
   if (s.npend == 0) KP_LAUNCH(0);
   else if (s.npend == 1) KP_LAUNCH(1);
@@ -275,6 +278,7 @@ __global__ void __launch_bounds__(MOTION_THREADS) k_kinetic_two(const double* __
                                                                 const double* __restrict__ invMass, int N, double cf,
                                                                 double* partials, unsigned int* ticket, double* result,
                                                                 double* hostResult, const double* skip) {
+  chain_wait();
   if (skip != nullptr && __double_as_longlong(*skip) != 0) return;   // a rebuild is due: nothing to sum
   const size_t n3 = 3 * (size_t)N, stride = (size_t)gridDim.x * blockDim.x;
   const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -305,6 +309,7 @@ __global__ void __launch_bounds__(MOTION_THREADS) k_kinetic_two_ff(const double*
                                                                    float cfl, float2* partials, unsigned int* ticket,
                                                                    double* result, double* hostResult,
                                                                    const double* skip) {
+  chain_wait();
   if (skip != nullptr && __double_as_longlong(*skip) != 0) return;   // a rebuild is due: nothing to sum
   const size_t n3 = 3 * (size_t)N, stride = (size_t)gridDim.x * blockDim.x;
   const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -351,10 +356,10 @@ static void launch_kinetic_two(System& s, double CF, const double* skip) {
   static const bool fp64Only = getenv("EMDEE_KE_FP64") != nullptr;   // tuning switch: the FP64 pass
   if (s.unitMass && s.forcesF32 && !fp64Only) {
     const float ch = (float)CF, cl = (float)(CF - (double)ch);
-    k_kinetic_two_ff<<<ffBlocks, MOTION_THREADS, 0, s.stream>>>(s.dP, s.F(), N, ch, cl, (float2*)s.dKE,
+    launch_chained(k_kinetic_two_ff, ffBlocks, MOTION_THREADS, 0, s.stream, s.dP, s.F(), N, ch, cl, (float2*)s.dKE,
                                                              s.dTicket + 1, s.dResult, s.hResult, skip);
   } else {
-    (s.unitMass ? k_kinetic_two<true> : k_kinetic_two<false>)<<<blocks, MOTION_THREADS, 0, s.stream>>>(
+    launch_chained((s.unitMass ? k_kinetic_two<true> : k_kinetic_two<false>), blocks, MOTION_THREADS, 0, s.stream,
         s.dP, s.F(), s.dInvMass, N, CF, s.dKE, s.dTicket + 1, s.dResult, s.hResult, skip);
   }
   CK(cudaGetLastError());

@@ -18,6 +18,7 @@
 #include <cmath>
 #include <vector>
 
+#include "chain.cuh"
 #include "system.hpp"
 #include "tile.cuh"
 
@@ -74,6 +75,7 @@ __device__ __forceinline__ MaxPrev warp_ordered_combine(MaxPrev acc) {
 __global__ void __launch_bounds__(SKIN_THREADS) k_skin(const double* __restrict__ R, const double* __restrict__ R0,
                                                        int N, int chunks, double skinSq, longlong2* partial,
                                                        unsigned int* ticket, double* result, double* hostResult) {
+  chain_wait();
   __shared__ MaxPrev wsum[SKIN_THREADS / 32];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -139,7 +141,7 @@ void device_skin_launch(System& s) {
   const int blocks = (N + per - 1) / per;
   ensure_partials(s, blocks);
   prof_begin(s, PK_SKIN);
-  k_skin<<<blocks, SKIN_THREADS, 0, s.stream>>>(s.dR, s.dR0, N, chunks, s.skinSq, (longlong2*)s.dPartials,
+  launch_chained(k_skin, blocks, SKIN_THREADS, 0, s.stream, s.dR, s.dR0, N, chunks, s.skinSq, (longlong2*)s.dPartials,
                                                  s.dTicket, s.dResult, s.hResult);
   CK(cudaGetLastError());
   prof_end(s, PK_SKIN);
@@ -189,6 +191,7 @@ __device__ __forceinline__ float charge_f32(double q) {
 // only the order of candidates, not the pair set.
 __global__ void k_assign(const double* __restrict__ R, const double* __restrict__ charge, int N, double scale,
                          TileGeom g, int4* atomK, int* count, int* inCell, float4* pos0, double* __restrict__ R0) {
+  chain_wait();
   int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= N) return;
   int c[3], K[3];
@@ -219,6 +222,7 @@ __global__ void k_assign(const double* __restrict__ R, const double* __restrict_
 static const int SCAN_THREADS = 256, SCAN_ITEMS = 8, SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
 __global__ void k_scan_local(const int* in, int* out, int n, int* blockSums) {
+  chain_wait();
   __shared__ int buf[SCAN_TILE];
   __shared__ int ws[33];
   int base = blockIdx.x * SCAN_TILE;
@@ -231,6 +235,7 @@ __global__ void k_scan_local(const int* in, int* out, int n, int* blockSums) {
 }
 
 __global__ void k_scan_sums(int* blockSums, int nb, int* out, int n) {
+  chain_wait();
   __shared__ int ws[33];
   __shared__ int carry;
   if (threadIdx.x == 0) carry = 0;
@@ -250,6 +255,7 @@ __global__ void k_scan_sums(int* blockSums, int nb, int* out, int n) {
 }
 
 __global__ void k_scan_add(int* out, int n, const int* blockSums) {
+  chain_wait();
   int base = blockIdx.x * SCAN_TILE, add = blockSums[blockIdx.x];
   for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS)
     if (base + k < n) out[base + k] += add;
@@ -257,13 +263,14 @@ __global__ void k_scan_add(int* out, int n, const int* blockSums) {
 
 static void device_scan(System& s, const int* in, int* out, int n) {
   int nb = (n + SCAN_TILE - 1) / SCAN_TILE;
-  k_scan_local<<<nb, SCAN_THREADS, 0, s.stream>>>(in, out, n, s.grid.dScanTmp);
-  k_scan_sums<<<1, SCAN_THREADS, 0, s.stream>>>(s.grid.dScanTmp, nb, out, n);
-  k_scan_add<<<nb, SCAN_THREADS, 0, s.stream>>>(out, n, s.grid.dScanTmp);
+  launch_chained(k_scan_local, nb, SCAN_THREADS, 0, s.stream, in, out, n, s.grid.dScanTmp);
+  launch_chained(k_scan_sums, 1, SCAN_THREADS, 0, s.stream, s.grid.dScanTmp, nb, out, n);
+  launch_chained(k_scan_add, nb, SCAN_THREADS, 0, s.stream, out, n, s.grid.dScanTmp);
   CK(cudaGetLastError());
 }
 
 __global__ void k_scatter(const int4* atomK, int N, const int* start, const int* inCell, int* orig) {
+  chain_wait();
   int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= N) return;
   orig[start[atomK[a].w] + inCell[a]] = a;
@@ -274,6 +281,7 @@ __global__ void k_scatter(const int4* atomK, int N, const int* start, const int*
 // along every stencil row), ties by ascending atom index.  Deterministic for
 // given coordinates.
 __global__ void k_sort_cells(const int* start, int nRanks, int* orig, const float4* __restrict__ pos0, float* key) {
+  chain_wait();
   int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= nRanks) return;
   int b = start[r], e = start[r + 1];
@@ -295,6 +303,7 @@ __global__ void k_sort_cells(const int* start, int nRanks, int* orig, const floa
 // number of atoms of the cell that precede it in (x key, atom index) order.
 // Cells of more than 32 atoms are sorted by lane 0 as above.
 __global__ void k_sort_cells_warp(const int* start, int nRanks, int* orig, const float4* __restrict__ pos0) {
+  chain_wait();
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= nRanks) return;
   const int b = start[r], n = start[r + 1] - b;
@@ -332,6 +341,7 @@ __global__ void k_sort_cells_warp(const int* start, int nRanks, int* orig, const
 // (pos0 of k_assign)
 __global__ void k_fill_slots(const int* orig, int N, const int4* atomK, const int* type, int4* K, uint8_t* type8,
                              int* slotOf, const float4* __restrict__ pos0, float4* pos4) {
+  chain_wait();
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= N) return;
   int a = orig[s];
@@ -377,6 +387,7 @@ __global__ void k_tile_info(const int* start, TileGeom g, int* info, int* maxOut
 // the charge, from the coordinates (after a change of the box since the build)
 __global__ void k_pack_mixed(const double* __restrict__ R, const double* __restrict__ charge, const int* orig,
                              const int4* K, int N, double scale, float4* pos4) {
+  chain_wait();
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= N) return;
   int a = orig[s];
@@ -398,6 +409,7 @@ __device__ __forceinline__ float4 pack_delta(float4 p0, double dx, double dy, do
 
 __global__ void k_pack_delta(const double* __restrict__ R, const double* __restrict__ R0, const int* orig,
                              const float4* __restrict__ pos0, int N, float scale, float4* pos4) {
+  chain_wait();
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= N) return;
   int a = orig[s];
@@ -408,6 +420,7 @@ __global__ void k_pack_delta(const double* __restrict__ R, const double* __restr
 // scaled FP64 coordinates Rs = R/L (src/EmDeeCode.f90:1228) in slot order, and their box
 // fractions (the FP64 mode has no FP32 positions between builds: they take that array)
 __global__ void k_pack_fp64(const double* __restrict__ R, const int* orig, int N, double L, double* Rs, int4* frac) {
+  chain_wait();
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= N) return;
   int a = orig[s];
@@ -423,11 +436,11 @@ void device_pack(System& s) {
   int N = s.natoms, th = 256, bl = (N + th - 1) / th;
   prof_begin(s, PK_PACK);
   if (s.precision == 1) {
-    k_pack_fp64<<<bl, th, 0, s.stream>>>(s.dR, g.dOrig, N, *s.Lbox, g.dRs64, (int4*)g.dPos4);
+    launch_chained(k_pack_fp64, bl, th, 0, s.stream, s.dR, g.dOrig, N, *s.Lbox, g.dRs64, (int4*)g.dPos4);
   } else if (*s.Lbox == s.builtL) {
-    k_pack_delta<<<bl, th, 0, s.stream>>>(s.dR, s.dR0, g.dOrig, g.dPos0, N, (float)((double)g.M / *s.Lbox), g.dPos4);
+    launch_chained(k_pack_delta, bl, th, 0, s.stream, s.dR, s.dR0, g.dOrig, g.dPos0, N, (float)((double)g.M / *s.Lbox), g.dPos4);
   } else {   // the box changed since the build: from the coordinates
-    k_pack_mixed<<<bl, th, 0, s.stream>>>(s.dR, s.dCharge, g.dOrig, g.dK, N, (double)g.M / *s.Lbox, g.dPos4);
+    launch_chained(k_pack_mixed, bl, th, 0, s.stream, s.dR, s.dCharge, g.dOrig, g.dK, N, (double)g.M / *s.Lbox, g.dPos4);
   }
   CK(cudaGetLastError());
   prof_end(s, PK_PACK);
@@ -527,6 +540,7 @@ __device__ __forceinline__ size_t nb_index(int t, int capC, int tileStride, int 
 #endif
 template <bool GENERAL, bool MINIMG, int MODE>
 __global__ void __maxnreg__(MODE == BUILD_ONE ? BUILD_MAXNREG : 64) k_build(BuildArgs A) {
+  chain_wait();
   constexpr bool SPLIT = MODE == BUILD_SPLIT;
   extern __shared__ __align__(16) unsigned char sraw[];
   __shared__ int ws[33];
@@ -1100,16 +1114,16 @@ static bool build_lists(System& s, bool reuse) {
     CK(cudaMemsetAsync(g.dCount, 0, sizeof(int) * (g.nRanks + 1), s.stream));
     s.prof.total += reuse ? 7 : 8;   // assign, 3 scan phases, scatter, sort, fill (, tile info)
     // the slot array holds each atom's place in its cell until k_fill_slots
-    k_assign<<<bl, th, 0, s.stream>>>(s.dR, s.dCharge, N, (double)M / L, geo, g.dAtomK, g.dCount, g.dSlotOf,
+    launch_chained(k_assign, bl, th, 0, s.stream, s.dR, s.dCharge, N, (double)M / L, geo, g.dAtomK, g.dCount, g.dSlotOf,
                                       g.dPos0, s.dR0);
     CK(cudaGetLastError());
     device_scan(s, g.dCount, g.dStart, g.nRanks);
-    k_scatter<<<bl, th, 0, s.stream>>>(g.dAtomK, N, g.dStart, g.dSlotOf, g.dOrig);
+    launch_chained(k_scatter, bl, th, 0, s.stream, g.dAtomK, N, g.dStart, g.dSlotOf, g.dOrig);
     if (perCell >= 8.0)   // dense cells: a warp per cell
-      k_sort_cells_warp<<<(g.nRanks + 7) / 8, 256, 0, s.stream>>>(g.dStart, g.nRanks, g.dOrig, g.dPos0);
+      launch_chained(k_sort_cells_warp, (g.nRanks + 7) / 8, 256, 0, s.stream, g.dStart, g.nRanks, g.dOrig, g.dPos0);
     else
-      k_sort_cells<<<(g.nRanks + 255) / 256, 256, 0, s.stream>>>(g.dStart, g.nRanks, g.dOrig, g.dPos0, g.dKeyX);
-    k_fill_slots<<<bl, th, 0, s.stream>>>(g.dOrig, N, g.dAtomK, s.dType, g.dK, g.dType8, g.dSlotOf, g.dPos0,
+      launch_chained(k_sort_cells, (g.nRanks + 255) / 256, 256, 0, s.stream, g.dStart, g.nRanks, g.dOrig, g.dPos0, g.dKeyX);
+    launch_chained(k_fill_slots, bl, th, 0, s.stream, g.dOrig, N, g.dAtomK, s.dType, g.dK, g.dType8, g.dSlotOf, g.dPos0,
                                           g.dPos4);
     int* dMax = g.dTileInfo + 2 * g.nTiles;
     CK(cudaMemsetAsync(dMax, 0, sizeof(int) * 4, s.stream));
@@ -1224,7 +1238,8 @@ static bool build_lists(System& s, bool reuse) {
     A.nb = nbList;
     A.cap = cap;
     CK(cudaMemsetAsync(A.maxCount, 0, sizeof(int), s.stream));
-    kb<<<g.nTiles, buildThreads, smem, s.stream>>>(A);
+    if (chain_fits(g.nTiles)) launch_chained(kb, g.nTiles, buildThreads, smem, s.stream, A);
+    else kb<<<g.nTiles, buildThreads, smem, s.stream>>>(A);
     s.prof.total++;
     CK(cudaGetLastError());
     int* mc = s.hFlags + 2;   // pinned: largest list, tile-size overflow
@@ -1640,6 +1655,7 @@ __global__ void __launch_bounds__(SKIN_THREADS) k_step_fused(double* __restrict_
                                                              float4* __restrict__ pos4, longlong2* partial,
                                                              unsigned int* ticket, double* result,
                                                              double* hostResult, double* __restrict__ s0) {
+  chain_wait();
   __shared__ MaxPrev wsum[SKIN_THREADS / 32];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1727,7 +1743,7 @@ void device_step_fused(System& s, double CP, bool vv, double* s0) {
   prof_begin(s, PK_MOVE);
 #define STEP_ARGS s.dR, s.dP, s.F(), s.dInvMass, s.dR0, N, chunks, s.pendCF[0], s.pendCF[1], CP, s.skinSq, g.dSlotOf, \
                   g.dPos0, scale, g.dPos4, (longlong2*)s.dPartials, s.dTicket, s.dResult, s.hResult, s0
-#define STEP_LAUNCH(NK, UM, PK, FM, VV) k_step_fused<NK, UM, PK, FM, VV><<<blocks, SKIN_THREADS, 0, s.stream>>>(STEP_ARGS)
+#define STEP_LAUNCH(NK, UM, PK, FM, VV) launch_chained(k_step_fused<NK, UM, PK, FM, VV>, blocks, SKIN_THREADS, 0, s.stream, STEP_ARGS)
 #define STEP_NK(UM, PK, FM)                            \
   if (vv) STEP_LAUNCH(1, UM, PK, FM, true);            \
   else if (s.npend == 0) STEP_LAUNCH(0, UM, PK, FM, false); \

@@ -11,6 +11,7 @@
 // Newton's-third-law half lists).
 #include <algorithm>
 
+#include "chain.cuh"
 #include "reduce.cuh"
 #include "system.hpp"
 #include "tile.cuh"
@@ -60,6 +61,7 @@ struct PairArgsD {
 // (FP64 lanes 52 -> 66 % in use; tiles of 62 atoms in warps of 32 leave the rest).
 template <bool COMPUTE, int MOD>
 __global__ void __launch_bounds__(PAIR64_THREADS) k_pair_fp64(PairArgsD A) {
+  chain_wait();
   extern __shared__ __align__(32) unsigned char sraw[];
   const TileGeom g = A.g;
   const int t = blockIdx.x, cells = g.TB * g.TB * g.TB;
@@ -143,7 +145,8 @@ __global__ void __launch_bounds__(PAIR64_THREADS) k_pair_fp64(PairArgsD A) {
 template <bool COMPUTE, int MOD>
 static void launch_fp64(System& s, const PairArgsD& A, size_t smem, int nTiles, int threads) {
   CK(cudaFuncSetAttribute(k_pair_fp64<COMPUTE, MOD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_pair_fp64<COMPUTE, MOD><<<nTiles, threads, smem, s.stream>>>(A);
+  if (chain_fits(nTiles)) launch_chained(k_pair_fp64<COMPUTE, MOD>, nTiles, threads, smem, s.stream, A);
+  else k_pair_fp64<COMPUTE, MOD><<<nTiles, threads, smem, s.stream>>>(A);
 }
 
 template <bool COMPUTE>

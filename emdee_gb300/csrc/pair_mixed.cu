@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cstdlib>
 
+#include "chain.cuh"
 #include "f32x2.cuh"
 #include "reduce.cuh"
 #include "system.hpp"
@@ -96,6 +97,7 @@ __device__ __noinline__ bool refilter_exact(const PairArgsF& A, const int* lay, 
 // wrap would bring the sentinel back).
 template <bool COMPUTE, int VAR, int MOD, bool MINIMG, bool COUNT, bool REFILTER>
 __global__ void PAIR_BOUNDS k_pair_mixed(PairArgsF A) {
+  chain_wait();
   // plain, shifted and force-shifted Lennard-Jones: two list entries per step of the
   // inner loop in packed FP32 arithmetic, which halves the issued instructions (force-
   // shifted, 100,003 atoms: 13.2 M warp instructions per launch one entry at a time,
@@ -299,7 +301,8 @@ static void launch(System& s, PairArgsF& A, size_t smem, int nTiles, int threads
 #endif
     configured = smem;
   }
-  kern<<<nTiles, threads, smem, s.stream>>>(A);
+  if (chain_fits(nTiles)) launch_chained(kern, nTiles, threads, smem, s.stream, A);
+  else kern<<<nTiles, threads, smem, s.stream>>>(A);
 }
 
 // Several atom types and charges in one branch-free evaluation: every type pair "none"
@@ -324,6 +327,7 @@ static const int PAIR_THREADS_TYPES = 512;
 
 template <bool COMPUTE, bool COUL, bool LSHIFT, bool CSHIFT, bool MINIMG>
 __global__ void __launch_bounds__(PAIR_THREADS_TYPES) k_pair_types(PairArgsF A) {
+  chain_wait();
   if (A.skip != nullptr && __double_as_longlong(*A.skip) != 0) return;
   extern __shared__ __align__(16) unsigned char sraw[];
   const TileGeom g = A.g;
@@ -451,7 +455,8 @@ template <bool COMPUTE, bool COUL, bool LSHIFT, bool CSHIFT, bool MINIMG>
 static void launch_types(System& s, PairArgsF& A, size_t smem, int nTiles, int threads) {
   auto kern = k_pair_types<COMPUTE, COUL, LSHIFT, CSHIFT, MINIMG>;
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<nTiles, threads, smem, s.stream>>>(A);
+  if (chain_fits(nTiles)) launch_chained(kern, nTiles, threads, smem, s.stream, A);
+  else kern<<<nTiles, threads, smem, s.stream>>>(A);
 }
 
 template <bool COMPUTE, bool MINIMG>

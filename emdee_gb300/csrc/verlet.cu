@@ -11,6 +11,7 @@
 // FP64, -fmad=false: every statement rounds like the oracle's.
 #include <algorithm>
 
+#include "chain.cuh"
 #include "bodies.cuh"
 #include "reduce.cuh"
 #include "system.hpp"
@@ -25,6 +26,7 @@ __global__ void __launch_bounds__(VV_THREADS) k_vv_pre_free(double* __restrict__
                                                             const double* __restrict__ F,
                                                             const double* __restrict__ invMass, const int* list,
                                                             int n, double dt, double dt_2, double* __restrict__ s0) {
+  chain_wait();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const int j = list ? list[q] : q;
@@ -48,6 +50,7 @@ __global__ void __launch_bounds__(VV_THREADS) k_vv_post_free(const double* __res
                                                              const double* __restrict__ s0, double* partials,
                                                              unsigned int* ticket, double* result, double* hostResult,
                                                              const double* skip) {
+  chain_wait();
   if (skip != nullptr && __double_as_longlong(*skip) != 0) return;   // a rebuild is due
   double v[5] = {0, 0, 0, 0, 0};
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
@@ -109,6 +112,7 @@ template <bool COMPUTE>
 __global__ void __launch_bounds__(VV_THREADS) k_vv_pre_body(BodyArgs A, const double* __restrict__ F,
                                                             double* __restrict__ R, double dt, double dt_2, int mode,
                                                             double* __restrict__ r0, double* __restrict__ q0) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= A.nb) return;
   BodyState b = A.b[i];
@@ -135,6 +139,7 @@ __global__ void __launch_bounds__(VV_THREADS) k_vv_post_body(BodyArgs A, const d
                                                              double dt_2, int mode, const double* __restrict__ r0,
                                                              const double* __restrict__ q0, double* partials,
                                                              unsigned int* ticket, double* result, double* hostResult) {
+  chain_wait();
   double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < A.nb) {
@@ -192,10 +197,10 @@ static void verlet_pre(System& s, double dt, bool compute, int mode) {
   } else if (nf > 0) {
     const int* list = s.dFree;
     if (compute)
-      k_vv_pre_free<true, FMA><<<vv_blocks(nf), VV_THREADS, 0, s.stream>>>(s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt,
+      launch_chained(k_vv_pre_free<true, FMA>, vv_blocks(nf), VV_THREADS, 0, s.stream, s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt,
                                                                       dt_2, w.s0);
     else
-      k_vv_pre_free<false, FMA><<<vv_blocks(nf), VV_THREADS, 0, s.stream>>>(s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt,
+      launch_chained(k_vv_pre_free<false, FMA>, vv_blocks(nf), VV_THREADS, 0, s.stream, s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt,
                                                                        dt_2, w.s0);
     CK(cudaGetLastError());
     s.prof.total++;
@@ -204,10 +209,10 @@ static void verlet_pre(System& s, double dt, bool compute, int mode) {
     ensure(w.r0, w.r0Cap, (size_t)3 * s.nbodies);
     ensure(w.q0, w.q0Cap, (size_t)4 * s.nbodies);
     if (compute)
-      k_vv_pre_body<true><<<vv_body_blocks(s.nbodies), VV_BODY_THREADS, 0, s.stream>>>(body_args(s), s.F(), s.dR, dt,
+      launch_chained(k_vv_pre_body<true>, vv_body_blocks(s.nbodies), VV_BODY_THREADS, 0, s.stream, body_args(s), s.F(), s.dR, dt,
                                                                                         dt_2, mode, w.r0, w.q0);
     else
-      k_vv_pre_body<false><<<vv_body_blocks(s.nbodies), VV_BODY_THREADS, 0, s.stream>>>(body_args(s), s.F(), s.dR, dt,
+      launch_chained(k_vv_pre_body<false>, vv_body_blocks(s.nbodies), VV_BODY_THREADS, 0, s.stream, body_args(s), s.F(), s.dR, dt,
                                                                                          dt_2, mode, w.r0, w.q0);
     CK(cudaGetLastError());
     s.prof.total++;
@@ -224,11 +229,11 @@ static void post_free(System& s, double dt, bool compute, const double* skip) {
   ensure(w.partF, w.partFCap, (size_t)5 * blocks);
   const int* list = all ? nullptr : s.dFree;
   if (compute)
-    k_vv_post_free<true, FMA><<<blocks, VV_THREADS, 0, s.stream>>>(s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt, dt_2,
+    launch_chained(k_vv_post_free<true, FMA>, blocks, VV_THREADS, 0, s.stream, s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt, dt_2,
                                                               w.s0, w.partF, s.dTicket + 6, s.dResult + 34,
                                                               s.hResult + 34, skip);
   else
-    k_vv_post_free<false, FMA><<<blocks, VV_THREADS, 0, s.stream>>>(s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt, dt_2,
+    launch_chained(k_vv_post_free<false, FMA>, blocks, VV_THREADS, 0, s.stream, s.dR, s.dP, s.F(), s.dInvMass, list, nf, dt, dt_2,
                                                                w.s0, nullptr, nullptr, nullptr, nullptr, skip);
   CK(cudaGetLastError());
   s.prof.total++;
@@ -251,11 +256,11 @@ static void verlet_post(System& s, double dt, bool compute, int mode, double* ou
     const int blocks = vv_body_blocks(s.nbodies);
     ensure(w.partB, w.partBCap, (size_t)9 * blocks);
     if (compute)
-      k_vv_post_body<true><<<blocks, VV_BODY_THREADS, 0, s.stream>>>(body_args(s), s.F(), dt, dt_2, mode, w.r0, w.q0,
+      launch_chained(k_vv_post_body<true>, blocks, VV_BODY_THREADS, 0, s.stream, body_args(s), s.F(), dt, dt_2, mode, w.r0, w.q0,
                                                                      w.partB, s.dTicket + 5, s.dResult + 24,
                                                                      s.hResult + 24);
     else
-      k_vv_post_body<false><<<blocks, VV_BODY_THREADS, 0, s.stream>>>(body_args(s), s.F(), dt, dt_2, mode, w.r0,
+      launch_chained(k_vv_post_body<false>, blocks, VV_BODY_THREADS, 0, s.stream, body_args(s), s.F(), dt, dt_2, mode, w.r0,
                                                                       w.q0, nullptr, nullptr, nullptr, nullptr);
     CK(cudaGetLastError());
     s.prof.total++;
