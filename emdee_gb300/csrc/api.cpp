@@ -307,8 +307,9 @@ static void compute_forces_impl(tEmDee* md) {
     // the skin decision (left by the fused step, or queued here) stays on the device with
     // the packed positions: the pair kernel and what follows it run unless a rebuild is
     // due, and one synchronisation returns both the decision and the sums
-    if (!s.skinReady) device_skin_launch(s);
-    if (!s.packReady) device_pack(s);
+    const bool both = !s.skinReady && !s.packReady && *s.Lbox == s.builtL;
+    if (!s.skinReady) device_skin_launch(s, both);
+    if (!s.packReady && !both) device_pack(s);
     s.packReady = true;
     forcesDone = device_pair_forces(s, compute, true);
     rebuild = !forcesDone;
@@ -365,7 +366,7 @@ static void compute_forces_impl(tEmDee* md) {
   md->Virial.Total = r[2] + r[3] + Wlong + bonded[1] + bonded[3];
   md->Virial.Body = 0.0;
   if (s.nbodies != 0) {   // src/EmDeeData.f90:926-953
-    md->Virial.Body = -r[6];
+    md->Virial.Body = -r[BODY_RESULT + 6];
     md->Virial.Total = md->Virial.Total + md->Virial.Body;
   }
   if (compute) {
@@ -535,6 +536,7 @@ tEmDee EmDee_system(int threads, int layers, double rc, double skin, int N, int*
   CK(cudaStreamCreateWithFlags(&s->sideStream, cudaStreamNonBlocking));
   CK(cudaEventCreateWithFlags(&s->forkEvent, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&s->joinEvent, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&s->doneEvent, cudaEventDisableTiming));
   size_t b3 = sizeof(double) * 3 * N;
   CK(cudaMalloc(&s->dR, b3));
   CK(cudaMalloc(&s->dP, b3));
@@ -567,12 +569,12 @@ tEmDee EmDee_system(int threads, int layers, double rc, double skin, int N, int*
     CK(cudaMalloc(&s->dFree, sizeof(int) * (s->nfree > 0 ? s->nfree : 1)));
     if (s->nfree > 0) CK(cudaMemcpy(s->dFree, s->freeList.data(), sizeof(int) * s->nfree, cudaMemcpyHostToDevice));
   }
-  CK(cudaMallocHost(&s->hResult, sizeof(double) * 64));
+  CK(cudaMallocHost(&s->hResult, sizeof(double) * 80));
   CK(cudaMallocHost(&s->hFlags, sizeof(int) * 16));
-  CK(cudaMalloc(&s->dResult, sizeof(double) * 64));
+  CK(cudaMalloc(&s->dResult, sizeof(double) * 80));
   CK(cudaMalloc(&s->dTicket, sizeof(unsigned int) * 16));
   CK(cudaMemset(s->dTicket, 0, sizeof(unsigned int) * 16));
-  memset(s->hResult, 0, sizeof(double) * 64);
+  memset(s->hResult, 0, sizeof(double) * 80);
 
   md.Builds = 0;
   md.DoF = 3 * (N - 1);
@@ -652,6 +654,7 @@ void EmDee_destroy(tEmDee* md) {
   if (s->ownsLbox) delete s->Lbox;
   cudaEventDestroy(s->forkEvent);
   cudaEventDestroy(s->joinEvent);
+  cudaEventDestroy(s->doneEvent);
   cudaStreamDestroy(s->sideStream);
   cudaStreamDestroy(s->stream);
   delete s;
@@ -1301,7 +1304,7 @@ void EmDee_boost(tEmDee* md, double lambda, double alpha, double dt) {
   s.boostQueued = false;
   if (lambda != 0.0 && !s.forcesUpToDate[s.layer - 1]) {
     s.boost = bb;
-    s.boostReq = s.nbodies > 0 && compute;   // queued behind the forces: one wait for both sums
+    s.boostReq = s.nbodies > 0;   // queued behind the forces
     compute_forces_impl(md);
     s.boostReq = false;
   }
@@ -1317,7 +1320,7 @@ void EmDee_boost(tEmDee* md, double lambda, double alpha, double dt) {
   flush_pending(s);
   if (s.nbodies > 0) {
     if (!s.boostQueued) {
-      bodies_boost_launch(s, bb, nullptr);
+      bodies_boost_launch(s, bb, nullptr, false);
       if (compute) CK(cudaStreamSynchronize(s.stream));
     }
     if (compute) bodies_boost_sums(s, bb);

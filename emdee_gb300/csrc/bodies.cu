@@ -58,16 +58,20 @@ __device__ __forceinline__ double body_Bt(const double* q, const double* p, int 
   return -qk * p[0] + q[0] * pk + qb * pa - qa * pb;
 }
 
-// force_and_torque, then pcm and pi updates; 2KE translational (bodies) and
-// rotational partial sums.  Lane c < 3 takes component c of the vectors.
+// force_and_torque, then pcm and pi updates; KIN: 2KE translational (bodies) and
+// rotational sums into result[0..5]; VIR: the sum over bodies and their atoms of F . delta
+// (the body virial is its negative) into result[6], which saves k_body_virial's pass where a
+// boost with sums follows the forces.  Lane c < 3 takes component c of the vectors.
+template <bool KIN, bool VIR>
 __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_boost(BodyArgs A, const double* __restrict__ F, double CP,
-                                                                   double CF, int translate, int rotate, int kinetic,
+                                                                   double CF, int translate, int rotate,
                                                                    double* partials, unsigned int* ticket,
                                                                    double* result, double* hostResult,
                                                                    const double* skip) {
   chain_wait();
   if (skip != nullptr && __double_as_longlong(*skip) != 0) return;   // a rebuild is due
-  double k6[6] = {0, 0, 0, 0, 0, 0};
+  constexpr int NQ = KIN ? (VIR ? 7 : 6) : 1;
+  double k6[NQ] = {};
   const BodyLane g = body_lane();
   if (g.i < A.nb) {
     BodyState& B = A.b[g.i];
@@ -78,6 +82,7 @@ __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_boost(BodyArgs A, c
       const double* Fj = &F[3 * A.atom[first + j]];
       const double* dj = &A.delta[3 * (first + j)];
       f += Fj[k];
+      if (VIR && c < 3) k6[NQ - 1] += Fj[k] * dj[k];
       tau += dj[k1] * Fj[k2] - dj[k2] * Fj[k1];
     }
     double pcm = B.pcm[k], omega = B.omega[k];
@@ -98,7 +103,7 @@ __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_boost(BodyArgs A, c
       B.pcm[c] = pcm;
       B.omega[c] = omega;
     }
-    if (kinetic) {
+    if constexpr (KIN) {
       const double kt = invMass * (pcm * pcm), kr = MoI * (omega * omega);
 #pragma unroll
       for (int d = 0; d < 3; d++) {
@@ -107,33 +112,51 @@ __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_boost(BodyArgs A, c
       }
     }
   }
-  if (kinetic) grid_reduce<6, BODY_GROUP_THREADS>(k6, partials, ticket, result, hostResult);
+  constexpr int off = KIN ? 0 : 6;
+  if (KIN || VIR)
+    grid_reduce<NQ, BODY_GROUP_THREADS>(k6, partials, ticket, result + off, hostResult + off);
 }
 
 // rb_series_step (rigid.cuh) on the four lanes of a body: lane c sums the coefficients
 // of quaternion component c and, for c < 3, of w_c; the others come by shuffles.
 // Components of w are held in the lane's cyclic order x0 = w_{r+1}, x1 = w_{r+2},
 // x2 = w_r (r = c, or 0 in lane 3), so that w_r' ~ x0 x1 in every lane.
+//
+// Order N: RB_SERIES_ORDER, or BODY_ORDER_WIDE in a warp with a body that turns by more
+// than RB_SERIES_STEP: steps of BODY_STEP_WIDE, where the same bound on the first
+// omitted term holds ((2 / pi 0.125)^11 = (2 / pi 0.184)^13 = 8e-13 of a first term that
+// is itself small).  The few fast bodies set the kernel's time, a warp per quarter of an
+// SM: one step of order 12 is 312 multiply-adds, two of order 10 are 440.  Signs are
+// flipped on the integer pipe.
+constexpr int BODY_ORDER_WIDE = 12;
+constexpr double BODY_STEP_WIDE = 0.184;
+
+__device__ __forceinline__ double flip(double x, long long mask) {
+  return __longlong_as_double(__double_as_longlong(x) ^ mask);
+}
+
+template <int N>
 __device__ __forceinline__ void body_series_step(const BodyLane& g, double kap, double (&w)[3], double (&q)[4]) {
-  constexpr int N = RB_SERIES_ORDER;
-  constexpr double inv[N + 1] = {0.0,       1.0,       1.0 / 2.0, 1.0 / 3.0, 1.0 / 4.0, 1.0 / 5.0,
-                                 1.0 / 6.0, 1.0 / 7.0, 1.0 / 8.0, 1.0 / 9.0, 1.0 / 10.0};
+  constexpr double inv[13] = {0.0,       1.0,       1.0 / 2.0, 1.0 / 3.0, 1.0 / 4.0,  1.0 / 5.0, 1.0 / 6.0,
+                              1.0 / 7.0, 1.0 / 8.0, 1.0 / 9.0, 1.0 / 10.0, 1.0 / 11.0, 1.0 / 12.0};
+  static_assert(N <= 12, "reciprocals up to 1 / 12");
   const int c = g.c, r = c < 3 ? c : 0, r1 = (r + 1) % 3, r2 = (r + 2) % 3;
   // component c of B(q) w = sum over k of sign * q_{c xor (k + 1)} w_k
   auto sgn = [&](int k) {   // rows of rb_B: (-,-,-), (+,-,+), (+,+,-), (-,+,+)
-    return c == 0 ? -1.0 : c == 1 ? (k == 1 ? -1.0 : 1.0) : c == 2 ? (k == 2 ? -1.0 : 1.0) : (k == 0 ? -1.0 : 1.0);
+    const bool minus = c == 0 || (c == 1 && k == 1) || (c == 2 && k == 2) || (c == 3 && k == 0);
+    return minus ? (long long)0x8000000000000000ull : 0ll;
   };
   const int p0 = c ^ (r1 + 1), p1 = c ^ (r2 + 1), p2 = c ^ (r + 1);
-  const double s0 = sgn(r1), s1 = sgn(r2), s2 = sgn(r);
+  const long long s0 = sgn(r1), s1 = sgn(r2), s2 = sgn(r);
   auto at3 = [](const double (&v)[3], int k) { return k == 0 ? v[0] : k == 1 ? v[1] : v[2]; };
   auto at4 = [](const double (&v)[4], int k) { return k == 0 ? v[0] : k == 1 ? v[1] : k == 2 ? v[2] : v[3]; };
   double X0[N + 1], X1[N + 1], X2[N + 1], B0[N + 1], B1[N + 1], B2[N + 1], Q[N + 1];
   X0[0] = at3(w, r1);
   X1[0] = at3(w, r2);
   X2[0] = at3(w, r);
-  B0[0] = s0 * at4(q, p0);
-  B1[0] = s1 * at4(q, p1);
-  B2[0] = s2 * at4(q, p2);
+  B0[0] = flip(at4(q, p0), s0);
+  B1[0] = flip(at4(q, p1), s1);
+  B2[0] = flip(at4(q, p2), s2);
   Q[0] = at4(q, c);
 #pragma unroll
   for (int n = 0; n < N; n++) {
@@ -149,9 +172,9 @@ __device__ __forceinline__ void body_series_step(const BodyLane& g, double kap, 
     X0[n + 1] = body_get(g, a, r1);
     X1[n + 1] = body_get(g, a, r2);
     X2[n + 1] = body_get(g, a, r);
-    B0[n + 1] = s0 * body_get(g, Q[n + 1], p0);
-    B1[n + 1] = s1 * body_get(g, Q[n + 1], p1);
-    B2[n + 1] = s2 * body_get(g, Q[n + 1], p2);
+    B0[n + 1] = flip(body_get(g, Q[n + 1], p0), s0);
+    B1[n + 1] = flip(body_get(g, Q[n + 1], p1), s1);
+    B2[n + 1] = flip(body_get(g, Q[n + 1], p2), s2);
   }
   double x = X2[N], y = Q[N];   // small terms first
 #pragma unroll
@@ -191,11 +214,11 @@ __global__ void __launch_bounds__(BODY_THREADS) k_body_move(BodyArgs A, double* 
 // The same with the exact rotation by the series (rb_rotate_series, operation by
 // operation) on BODY_LANES lanes per body.
 __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_move_series(BodyArgs A, double* __restrict__ R, double CR,
-                                                                         double CP, double dt, int translate) {
+                                                                         double CP, double dt, double invdt,
+                                                                         int translate) {
   chain_wait();
   const BodyLane g = body_lane();
-  if (g.i >= A.nb) return;
-  BodyState& B = A.b[g.i];
+  BodyState& B = A.b[min(g.i, A.nb - 1)];
   double MoI[3], omega[3], TwoKr = 0.0, Iw1 = 0.0, Iw2 = 0.0, invMoI[3];
   for (int k = 0; k < 3; k++) {
     MoI[k] = B.MoI[k];
@@ -207,19 +230,30 @@ __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_move_series(BodyArg
     TwoKr += Iw * omega[k];
   }
   int steps;
-  if (!rb_series_steps(TwoKr * invMoI[2] * (dt * dt), MoI[2], Iw1 * Iw1 + Iw2 * Iw2, steps)) {
+  const double theta2 = TwoKr * invMoI[2] * (dt * dt);
+  const bool series = rb_series_steps(theta2, MoI[2], Iw1 * Iw1 + Iw2 * Iw2, steps);
+  const bool wide = __any_sync(0xffffffffu, series && steps > 1);
+  if (g.i >= A.nb) return;
+  if (!series) {
     if (g.c == 0) body_move_one(A, g.i, R, CR, CP, dt, translate, 1, 0);
     return;
+  }
+  if (wide) {
+    steps = 1;
+    while (theta2 > (BODY_STEP_WIDE * steps) * (BODY_STEP_WIDE * steps)) steps++;
   }
   const int c = g.c, k = c < 3 ? c : 0, first = B.first, NP = B.NP;
   double q[4] = {B.q[0], B.q[1], B.q[2], B.q[3]};
   double rcm = B.rcm[k];
   if (translate) rcm = CR * rcm + CP * B.invMass * B.pcm[k];
-  const double h = steps == 1 ? dt : dt / steps, back = steps == 1 ? 1.0 / dt : steps / dt;
+  const double h = steps == 1 ? dt : dt / steps, back = steps == 1 ? invdt : steps * invdt;
   const double kap = k == 0 ? (MoI[1] - MoI[2]) * invMoI[0]
                             : k == 1 ? (MoI[2] - MoI[0]) * invMoI[1] : (MoI[0] - MoI[1]) * invMoI[2];
   double w[3] = {h * omega[0], h * omega[1], h * omega[2]};
-  for (int n = 0; n < steps; n++) body_series_step(g, kap, w, q);
+  if (wide)
+    for (int n = 0; n < steps; n++) body_series_step<BODY_ORDER_WIDE>(g, kap, w, q);
+  else
+    body_series_step<RB_SERIES_ORDER>(g, kap, w, q);
   const double n2 = q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3], f = 1.5 - 0.5 * n2;
   double v[3];
   for (int n = 0; n < 4; n++) q[n] *= f;
@@ -398,9 +432,9 @@ void bodies_update(System& s) {
 }
 
 // boost of free atoms (through the list) and bodies
-void bodies_boost_launch(System& s, const System::BodyBoost& b, const double* skip) {
+void bodies_boost_launch(System& s, const System::BodyBoost& b, const double* skip, bool virial) {
   int freeBlocks = std::min(body_blocks(s.nfree), 1184);
-  ensure_scratch(s, freeBlocks * 3 + body_group_blocks(s.nbodies) * 6, 1);
+  ensure_scratch(s, freeBlocks * 3 + body_group_blocks(s.nbodies) * 7, 1);
   if (b.translate && s.nfree > 0) {
     int blocks = freeBlocks;
     if (b.kinetic) {
@@ -414,15 +448,17 @@ void bodies_boost_launch(System& s, const System::BodyBoost& b, const double* sk
     CK(cudaGetLastError());
     s.prof.total++;
   }
-  launch_chained(k_body_boost, body_group_blocks(s.nbodies), BODY_GROUP_THREADS, 0, s.stream,
-      body_args(s), s.F(), b.CP, b.CF, b.translate, b.rotate, b.kinetic, s.dBodyScratch + freeBlocks * 3,
-      s.dTicket + 3, s.dResult + 16, s.hResult + 16, skip);
+  auto kern = b.kinetic ? (virial ? k_body_boost<true, true> : k_body_boost<true, false>)
+                        : (virial ? k_body_boost<false, true> : k_body_boost<false, false>);
+  launch_chained(kern, body_group_blocks(s.nbodies), BODY_GROUP_THREADS, 0, s.stream, body_args(s), s.F(), b.CP, b.CF,
+                 b.translate, b.rotate, s.dBodyScratch + freeBlocks * 3, s.dTicket + 3, s.dResult + BODY_RESULT,
+                 s.hResult + BODY_RESULT, skip);
   CK(cudaGetLastError());
   s.prof.total++;
 }
 
 void bodies_boost_sums(System& s, const System::BodyBoost& b) {
-  const double* k6 = s.hResult + 16;
+  const double* k6 = s.hResult + BODY_RESULT;
   for (int k = 0; k < 3; k++) {
     s.hResult[10 + k] = (b.translate && s.nfree > 0 ? s.hResult[10 + k] : 0.0) + k6[k];
     s.hResult[13 + k] = k6[3 + k];
@@ -438,7 +474,7 @@ void bodies_move(System& s, double CR, double CP, double dt, bool translate, boo
   }
   if (rotate && mode == 0)
     launch_chained(k_body_move_series, body_group_blocks(s.nbodies), BODY_GROUP_THREADS, 0, s.stream, body_args(s), s.dR, CR, CP,
-                                                                                          dt, translate);
+                   dt, 1.0 / dt, translate);
   else
     launch_chained(k_body_move, body_blocks(s.nbodies), BODY_THREADS, 0, s.stream, body_args(s), s.dR, CR, CP, dt, translate,
                                                                        rotate, mode);
@@ -450,7 +486,8 @@ void bodies_virial_launch(System& s, const double* skip) {
   int blocks = body_blocks(s.nbodies);
   ensure_scratch(s, blocks, 1);
   launch_chained(k_body_virial, blocks, BODY_THREADS, 0, s.stream, body_args(s), s.F(), s.dBodyScratch, s.dTicket + 3,
-                                                        s.dResult + 6, s.hResult + 6, skip);
+                                                        s.dResult + BODY_RESULT + 6, s.hResult + BODY_RESULT + 6,
+                 skip);
   CK(cudaGetLastError());
   s.prof.total++;
 }

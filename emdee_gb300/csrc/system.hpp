@@ -228,6 +228,7 @@ struct System {
   // beside the pair kernel, between two events on the system's stream
   cudaStream_t sideStream = nullptr;
   cudaEvent_t forkEvent = nullptr, joinEvent = nullptr;
+  cudaEvent_t doneEvent = nullptr;   // the sums of a force computation are in place
   double *dR = nullptr, *dP = nullptr, *dR0 = nullptr, *dLayerF = nullptr;
   bool ownsRP = true;
   double *dInvMass = nullptr, *dCharge = nullptr;
@@ -332,8 +333,9 @@ void prof_drop_last(System& s);
 // the lists must be rebuilt.  Synchronizes the stream.
 bool device_skin_check(System& s);
 // The same check queued only: the rebuild flag stays in dResult[9] (and hResult[9] after
-// the next synchronisation).
-void device_skin_launch(System& s);
+// the next synchronisation).  pack: with the FP32 positions of device_pack, for mixed
+// precision in the box of the last build.
+void device_skin_launch(System& s, bool pack);
 // Cell binning, tile sort and neighbor-list build (src/neighbor_lists.f90:63-300).
 // With two-level lists active it builds the outer lists (radius rc + skin + outer skin).
 void device_build_lists(System& s);
@@ -410,10 +412,12 @@ void device_pair_statistics(System& s, long* listed, long* within);
 void bodies_update(System& s);
 // boost of free atoms and bodies; after a synchronisation, bodies_boost_sums leaves 2KE in
 // hResult[10..12] (translational) and [13..15] (rotational)
-void bodies_boost_launch(System& s, const System::BodyBoost& b, const double* skip);
+// (virial: with the sum of bodies_virial_launch)
+void bodies_boost_launch(System& s, const System::BodyBoost& b, const double* skip, bool virial);
 void bodies_boost_sums(System& s, const System::BodyBoost& b);
 void bodies_move(System& s, double CR, double CP, double dt, bool translate, bool rotate, int mode);
-// result in hResult[6] (the virial is its negative) after a synchronisation
+// result in hResult[BODY_RESULT + 6] (the virial is its negative) after a synchronisation
+const int BODY_RESULT = 64;   // slots of the body kernels' sums: 2KE (6), virial
 void bodies_virial_launch(System& s, const double* skip);
 void bodies_assign(System& s, double* k6);
 void bodies_particle_momenta(System& s, double* dOut);
