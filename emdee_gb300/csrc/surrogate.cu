@@ -696,9 +696,12 @@ __global__ void __launch_bounds__(128) k_sg_mlp(TileArgs T, const float* __restr
 // The same computation as k_sg_mlp (BF16 operands rounded at the same points, FP32
 // accumulation) with tcgen05.mma: M = 128 atoms per tile (one species), operands in
 // shared memory in the canonical K-major layout without swizzle, accumulators in
-// tensor memory.  Persistent blocks of 128 threads hold the BF16 weights of both
-// species for their whole life and take 128-atom tiles in turn; thread t owns row t
-// of a tile, which is TMEM lane t (warp w reads lanes 32w..32w+31).  Thread 0
+// tensor memory.  Persistent blocks of 256 threads take 128-atom tiles in turn and load
+// the BF16 weights of a species at their first tile of it; threads r and r + 128 own row
+// r of a tile, TMEM lane r (warp w reads lanes 32 (w mod 4).. + 31), and half of its
+// columns each.  The kernel is bound by the latency of a tile's chain (loads, four GEMMs,
+// 64 columns of silu and its derivative per row in between): with one thread per row and
+// both species' weights loaded up front 8 x 8000 atoms took 67 us, so 37.  Thread 0
 // issues each GEMM (one tcgen05.mma per K = 16) and commits it to an mbarrier that
 // every thread waits on.  Per tile:
 //   Z1 = G W1          TMEM columns   0..63   (K = 32)
@@ -709,7 +712,7 @@ __global__ void __launch_bounds__(128) k_sg_mlp(TileArgs T, const float* __restr
 // Waits are bounded: a wait that runs out sets *err, the block stops taking tiles,
 // frees its tensor memory and returns (the host reports the error).
 
-constexpr int TC_M = 128, TC_COLS = 256;
+constexpr int TC_M = 128, TC_COLS = 256, TC_THREADS = 2 * TC_M;
 
 // byte offset of element (r, k) of a K-major operand with K columns: 8 x 16-byte core
 // matrices, consecutive along K (leading byte offset 128), row groups of 8 K/8 core
@@ -730,6 +733,7 @@ struct TcSmem {
   TcWeights w[NS];
   alignas(128) unsigned char G[TC_M * DIN * 2];   // A operand of Z1 (K 32)
   alignas(128) unsigned char X[TC_M * H * 2];     // A operand of the other GEMMs (K 64)
+  float epart[TC_M];   // energies of the upper columns
   alignas(8) unsigned long long bar;
   unsigned int taddr;
 };
@@ -787,17 +791,29 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// 16 consecutive FP32 columns of this thread's TMEM lane
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
+// 16 or 32 consecutive FP32 columns of this thread's TMEM lane; tc_ld_wait before their use
+__device__ __forceinline__ void tc_ld(uint32_t taddr, float (&v)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
+        "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
       : "r"(taddr));
+}
+__device__ __forceinline__ void tc_ld(uint32_t taddr, float (&v)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+      "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
+        "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]),
+        "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]),
+        "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+      : "r"(taddr));
+}
+template <int N>
+__device__ __forceinline__ void tc_ld_wait(float (&v)[N]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-  for (int q = 0; q < 16; q++) v[q] = __uint_as_float(r[q]);
+  for (int q = 0; q < N; q++) asm volatile("" : "+f"(v[q]));   // the values are read after the wait
 }
 
 // 8 BF16 values (from 8 floats) into one 16-byte chunk of a K-major operand
@@ -810,20 +826,33 @@ __device__ __forceinline__ void tc_st8(unsigned char* base, int r, int k, int K,
   *reinterpret_cast<uint4*>(base + tc_off(r, k, K)) = w;
 }
 
+// Called by all TC_THREADS threads; four consecutive n at a time, every load in flight
 __device__ void tc_load_weights(TcWeights& w, const float* p) {
-  for (int q = threadIdx.x; q < DIN * H; q += blockDim.x) {
-    const int k = q / H, n = q % H;   // W1[k][n]
-    const __nv_bfloat16 v = __float2bfloat16(p[OFF_W1 + q]);
-    *reinterpret_cast<__nv_bfloat16*>(w.B1 + tc_off(n, k, DIN)) = v;   // B1[n][k]
-    *reinterpret_cast<__nv_bfloat16*>(w.B4 + tc_off(k, n, H)) = v;     // B4[k][n] (rows: input index)
+  constexpr int L1 = DIN * H / 4 / TC_THREADS, L2 = H * H / 4 / TC_THREADS;
+  static_assert(DIN * H == 4 * TC_THREADS * L1 && H * H == 4 * TC_THREADS * L2, "whole rounds of loads");
+  float x[L1 + L2][4];
+#pragma unroll
+  for (int r = 0; r < L1 + L2; r++) {
+    const float* src = p + (r < L1 ? OFF_W1 + 4 * (r * TC_THREADS + threadIdx.x)
+                                   : OFF_W2 + 4 * ((r - L1) * TC_THREADS + threadIdx.x));
+#pragma unroll
+    for (int v = 0; v < 4; v++) x[r][v] = src[v];
   }
-  for (int q = threadIdx.x; q < H * H; q += blockDim.x) {
-    const int k = q / H, n = q % H;   // W2[k][n]
-    const __nv_bfloat16 v = __float2bfloat16(p[OFF_W2 + q]);
-    *reinterpret_cast<__nv_bfloat16*>(w.B2 + tc_off(n, k, H)) = v;   // B2[n][k]
-    *reinterpret_cast<__nv_bfloat16*>(w.B3 + tc_off(k, n, H)) = v;   // B3[k][n] (rows: a1 index)
+#pragma unroll
+  for (int r = 0; r < L1 + L2; r++) {
+    const bool first = r < L1;   // W1[k][n], else W2[k][n]
+    const int q = 4 * ((first ? r : r - L1) * TC_THREADS + (int)threadIdx.x), k = q / H, n = q % H;
+    const int K = first ? DIN : H;
+    unsigned char* Bt = first ? w.B1 : w.B2;   // Bt[n][k]
+    unsigned char* B = first ? w.B4 : w.B3;    // B[k][n] (rows: input or a1 index)
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+      const __nv_bfloat16 b = __float2bfloat16(x[r][v]);
+      *reinterpret_cast<__nv_bfloat16*>(Bt + tc_off(n + v, k, K)) = b;
+      *reinterpret_cast<__nv_bfloat16*>(B + tc_off(k, n + v, H)) = b;
+    }
   }
-  for (int q = threadIdx.x; q < H; q += blockDim.x) {
+  for (int q = threadIdx.x; q < H; q += TC_THREADS) {
     w.b1[q] = p[OFF_B1 + q];
     w.b2[q] = p[OFF_B2 + q];
     w.w3[q] = p[OFF_W3 + q];
@@ -831,13 +860,13 @@ __device__ void tc_load_weights(TcWeights& w, const float* p) {
   if (threadIdx.x == 0) w.b3 = p[OFF_B3];
 }
 
-__global__ void __launch_bounds__(128, 1) k_sg_mlp_tc(TileArgs T, const float* __restrict__ params,
-                                                      const float* __restrict__ Gin, float* __restrict__ Eatom,
-                                                      float* __restrict__ dEdG, int* __restrict__ err) {
+__global__ void __launch_bounds__(TC_THREADS, 2) k_sg_mlp_tc(TileArgs T, const float* __restrict__ params,
+                                                             const float* __restrict__ Gin,
+                                                             float* __restrict__ Eatom, float* __restrict__ dEdG,
+                                                             int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char raw[];
   TcSmem& S = *reinterpret_cast<TcSmem*>(raw);
-  const int t = threadIdx.x, warp = t >> 5;
-  for (int sp = 0; sp < NS; sp++) tc_load_weights(S.w[sp], params + sp * PER_SPECIES);
+  const int t = threadIdx.x, warp = t >> 5, row = t % TC_M, half = t / TC_M;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&S.taddr)),
                  "r"(TC_COLS)
@@ -853,7 +882,10 @@ __global__ void __launch_bounds__(128, 1) k_sg_mlp_tc(TileArgs T, const float* _
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = S.taddr, bar = smem_u32(&S.bar);
-  const uint32_t lane_base = (uint32_t)(32 * warp) << 16;   // this warp's TMEM lanes
+  const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;   // this warp's TMEM lanes
+  constexpr int HC = H / 2, GC = DIN / 2;   // columns of a thread
+  const int c0 = half * HC, g0 = half * GC;
+  unsigned loaded = 0;   // species whose weights are in place
   uint32_t phase = 0;
   bool ok = true;
   // one GEMM: operands written by all threads before, accumulator read by all after;
@@ -874,72 +906,70 @@ __global__ void __launch_bounds__(128, 1) k_sg_mlp_tc(TileArgs T, const float* _
   for (int ti = blockIdx.x; ti < T.ntiles; ti += gridDim.x) {
     const int3 tile = T.tiles[ti];
     const TcWeights& W = S.w[tile.z];
-    const bool have = t < tile.y;
-    const int atom = have ? T.atoms[tile.x + t] : 0;
+    if (!(loaded >> tile.z & 1u)) {   // read by the GEMMs after the fence and barrier of run
+      tc_load_weights(S.w[tile.z], params + tile.z * PER_SPECIES);
+      loaded |= 1u << tile.z;
+    }
+    const bool have = row < tile.y;
+    const int atom = have ? T.atoms[tile.x + row] : 0;
     {   // G row -> BF16 A operand
-      float g[DIN];
+      float g[GC];
 #pragma unroll
-      for (int k = 0; k < DIN; k += 4) {
-        const float4 v = have ? *reinterpret_cast<const float4*>(Gin + (size_t)atom * DIN + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int k = 0; k < GC; k += 4) {
+        const float4 v =
+            have ? *reinterpret_cast<const float4*>(Gin + (size_t)atom * DIN + g0 + k) : make_float4(0.f, 0.f, 0.f, 0.f);
         g[k] = v.x;
         g[k + 1] = v.y;
         g[k + 2] = v.z;
         g[k + 3] = v.w;
       }
 #pragma unroll
-      for (int k = 0; k < DIN; k += 8) tc_st8(S.G, t, k, DIN, g + k);
+      for (int k = 0; k < GC; k += 8) tc_st8(S.G, row, g0 + k, DIN, g + k);
     }
     run([&] { tc_gemm<DIN, H>(tm + 0, S.G, W.B1); });
     if (!ok) break;
+    float z[HC];
+    tc_ld(tm + lane_base + c0, z);   // A1 = silu(Z1 + b1)
+    tc_ld_wait(z);
 #pragma unroll
-    for (int c = 0; c < H; c += 16) {   // A1 = silu(Z1 + b1)
-      float z[16];
-      tc_ld16(tm + lane_base + c, z);
+    for (int q = 0; q < HC; q++) z[q] = silu(z[q] + W.b1[c0 + q]);
 #pragma unroll
-      for (int q = 0; q < 16; q++) z[q] = silu(z[q] + W.b1[c + q]);
-      tc_st8(S.X, t, c, H, z);
-      tc_st8(S.X, t, c + 8, H, z + 8);
-    }
+    for (int q = 0; q < HC; q += 8) tc_st8(S.X, row, c0 + q, H, z + q);
     run([&] { tc_gemm<H, H>(tm + 64, S.X, W.B2); });
     if (!ok) break;
     float e = 0.f;
+    tc_ld(tm + lane_base + 64 + c0, z);   // E and dE/dZ2
+    tc_ld_wait(z);
 #pragma unroll
-    for (int c = 0; c < H; c += 16) {   // E and dE/dZ2
-      float z[16];
-      tc_ld16(tm + lane_base + 64 + c, z);
-#pragma unroll
-      for (int q = 0; q < 16; q++) {
-        const float u = z[q] + W.b2[c + q];
-        e += W.w3[c + q] * silu(u);
-        z[q] = W.w3[c + q] * dsilu(u);
-      }
-      tc_st8(S.X, t, c, H, z);
-      tc_st8(S.X, t, c + 8, H, z + 8);
+    for (int q = 0; q < HC; q++) {
+      const float u = z[q] + W.b2[c0 + q];
+      e += W.w3[c0 + q] * silu(u);
+      z[q] = W.w3[c0 + q] * dsilu(u);
     }
-    if (have) Eatom[atom] = e + W.b3;
+#pragma unroll
+    for (int q = 0; q < HC; q += 8) tc_st8(S.X, row, c0 + q, H, z + q);
+    if (half == 1) S.epart[row] = e;
     run([&] { tc_gemm<H, H>(tm + 128, S.X, W.B3); });
     if (!ok) break;
+    if (half == 0 && have) Eatom[atom] = (e + S.epart[row]) + W.b3;
+    float d[HC];
+    tc_ld(tm + lane_base + 128 + c0, d);   // dE/dZ1 = dE/dA1 silu'(Z1 + b1)
+    tc_ld(tm + lane_base + c0, z);
+    tc_ld_wait(d);
+    tc_ld_wait(z);
 #pragma unroll
-    for (int c = 0; c < H; c += 16) {   // dE/dZ1 = dE/dA1 silu'(Z1 + b1)
-      float d[16], z[16];
-      tc_ld16(tm + lane_base + 128 + c, d);
-      tc_ld16(tm + lane_base + c, z);
+    for (int q = 0; q < HC; q++) d[q] *= dsilu(z[q] + W.b1[c0 + q]);
 #pragma unroll
-      for (int q = 0; q < 16; q++) d[q] *= dsilu(z[q] + W.b1[c + q]);
-      tc_st8(S.X, t, c, H, d);
-      tc_st8(S.X, t, c + 8, H, d + 8);
-    }
+    for (int q = 0; q < HC; q += 8) tc_st8(S.X, row, c0 + q, H, d + q);
     run([&] { tc_gemm<H, DIN>(tm + 192, S.X, W.B4); });
     if (!ok) break;
+    float o[GC];
+    tc_ld(tm + lane_base + 192 + g0, o);   // dE/dG
+    tc_ld_wait(o);
+    if (have)
 #pragma unroll
-    for (int c = 0; c < DIN; c += 16) {   // dE/dG
-      float d[16];
-      tc_ld16(tm + lane_base + 192 + c, d);
-      if (have)
-#pragma unroll
-        for (int q = 0; q < 16; q += 4)
-          *reinterpret_cast<float4*>(dEdG + (size_t)atom * DIN + c + q) = make_float4(d[q], d[q + 1], d[q + 2], d[q + 3]);
-    }
+      for (int q = 0; q < GC; q += 4)
+        *reinterpret_cast<float4*>(dEdG + (size_t)atom * DIN + g0 + q) = make_float4(o[q], o[q + 1], o[q + 2], o[q + 3]);
   }
   if (!ok && t == 0) {
     atomicExch(err, 1);
@@ -1282,7 +1312,7 @@ static void sg_network(Surrogate& S, const float* dParams, cudaStream_t st) {
   } else {
     TileArgs T{S.dAtoms, S.dTiles128, (int)S.tiles128.size()};
     const int blocks = std::min(T.ntiles, 2 * 152);
-    k_sg_mlp_tc<<<blocks, 128, tc_smem_bytes(), st>>>(T, dParams, S.dG, S.dEatom, S.dEdG, S.dTcError);
+    k_sg_mlp_tc<<<blocks, TC_THREADS, tc_smem_bytes(), st>>>(T, dParams, S.dG, S.dEatom, S.dEdG, S.dTcError);
   }
   CK(cudaGetLastError());
 }
