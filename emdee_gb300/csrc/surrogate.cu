@@ -281,11 +281,13 @@ __device__ __forceinline__ float nearest(float x) { return __fadd_rn(__fadd_rn(x
 
 // Verlet lists (global atom indices), entry e of atom q at list[q * cap + e], in the order
 // of the neighbor cells and of their atoms.  A block per cell stages the candidates of
-// its atoms (27 cells, or with M < 3 the whole chain) in shared memory; a warp per atom
-// goes through them side by side and places the accepted ones by ballots.  More than
-// LIST_CAND candidates are taken in several stages.  (One thread per atom, gathering
-// each candidate's index and position: 428 us at 8 x 8000 atoms; 142 us so.)
-constexpr int LIST_CAND = 2048, LIST_THREADS = 256;
+// its atoms (27 cells, or with M < 3 the whole chain) in shared memory; a warp goes
+// through them side by side for LIST_ATOMS atoms at a time and places the accepted ones
+// by ballots.  More than LIST_CAND candidates are taken in several stages.  Bound by
+// instruction issue: 36 instructions per 32 candidates of one atom before the load and
+// the loop were shared by LIST_ATOMS (8 x 8000 atoms: 142 -> 111 us; one thread per atom,
+// gathering each candidate's index and position: 428 us).
+constexpr int LIST_CAND = 2048, LIST_THREADS = 256, LIST_ATOMS = 2;
 __global__ void __launch_bounds__(LIST_THREADS) k_sg_list(const float4* __restrict__ pos, Geometry G,
                                                           const int* __restrict__ starts,
                                                           const int* __restrict__ sorted, int cap,
@@ -314,47 +316,74 @@ __global__ void __launch_bounds__(LIST_THREADS) k_sg_list(const float4* __restri
   __syncthreads();
   const int total = base[ncell];
   int longest = 0;
+  const unsigned below = (1u << lane) - 1u;
+  // this warp's share of the cell's atoms
+  const int o0 = own0 + (own1 - own0) * warp / (LIST_THREADS / 32),
+            o1 = own0 + (own1 - own0) * (warp + 1) / (LIST_THREADS / 32);
   for (int c0 = 0; c0 < total; c0 += LIST_CAND) {
     const int nc = min(LIST_CAND, total - c0);
     if (c0 > 0) __syncthreads();
-    for (int c = threadIdx.x; c < nc; c += LIST_THREADS) {
-      int k = 0;
-      while (base[k + 1] <= c0 + c) k++;
-      const int j = sorted[first[k] + (c0 + c - base[k])];
-      float4 p = pos[j];
+    // a warp per neighbor cell (the whole block where there is one)
+    const int width = ncell == 1 ? LIST_THREADS : 32;
+    for (int k = ncell == 1 ? 0 : warp; k < ncell; k += LIST_THREADS / 32) {
+      float sx = 0.f, sy = 0.f, sz = 0.f;
       if (M >= 3) {   // cells across the box's faces: the image on this side
         const int nx = x + k % 3 - 1, ny = y + k / 3 % 3 - 1, nz = z + k / 9 - 1;
-        p.x += nx < 0 ? -G.L : nx >= M ? G.L : 0.f;
-        p.y += ny < 0 ? -G.L : ny >= M ? G.L : 0.f;
-        p.z += nz < 0 ? -G.L : nz >= M ? G.L : 0.f;
+        sx = nx < 0 ? -G.L : nx >= M ? G.L : 0.f;
+        sy = ny < 0 ? -G.L : ny >= M ? G.L : 0.f;
+        sz = nz < 0 ? -G.L : nz >= M ? G.L : 0.f;
       }
-      p.w = __int_as_float(j);
-      cand[c] = p;
+      const int u0 = max(0, c0 - base[k]), u1 = min(base[k + 1] - base[k], c0 + nc - base[k]);
+      for (int u = u0 + (ncell == 1 ? (int)threadIdx.x : lane); u < u1; u += width) {
+        const int j = sorted[first[k] + u];
+        float4 p = pos[j];
+        p.x += sx;
+        p.y += sy;
+        p.z += sz;
+        p.w = __int_as_float(j);
+        cand[base[k] + u - c0] = p;
+      }
     }
     __syncthreads();
-    for (int o = own0 + warp; o < own1; o += LIST_THREADS / 32) {
-      const int q = sorted[o];
-      const float4 p = pos[q];
-      int* out = list + (size_t)q * cap;
-      int n = c0 > 0 ? count[q] : 0;
-      for (int c = lane; c - lane < nc; c += 32) {
-        const float4 pj = cand[min(c, nc - 1)];
-        const int j = __float_as_int(pj.w);
-        float ex = p.x - pj.x, ey = p.y - pj.y, ez = p.z - pj.z;
-        if (M < 4) {   // a neighbor cell may hold a nearer image
-          ex -= G.L * nearest(ex * G.invL);
-          ey -= G.L * nearest(ey * G.invL);
-          ez -= G.L * nearest(ez * G.invL);
-        }
-        const bool in = c < nc && j != q && ex * ex + ey * ey + ez * ez < G.rlist2;
-        const unsigned m = __ballot_sync(0xffffffffu, in);
-        const int at = n + __popc(m & ((1u << lane) - 1u));
-        if (in && at < cap) out[at] = j;
-        n += __popc(m);
+    for (int o = o0; o < o1; o += LIST_ATOMS) {
+      const int na = min(LIST_ATOMS, o1 - o);
+      int q[LIST_ATOMS], n[LIST_ATOMS];
+      float4 p[LIST_ATOMS];
+      int* out[LIST_ATOMS];
+#pragma unroll
+      for (int a = 0; a < LIST_ATOMS; a++) {
+        q[a] = sorted[min(o + a, o1 - 1)];
+        p[a] = pos[q[a]];
+        out[a] = list + (size_t)q[a] * cap;
+        n[a] = c0 > 0 ? count[q[a]] : 0;
       }
-      if (lane == 0) count[q] = n;
+      for (int c = lane; c - lane < nc; c += 32) {
+        const bool have = c < nc;
+        const float4 pj = cand[have ? c : 0];
+        const int j = __float_as_int(pj.w);
+#pragma unroll
+        for (int a = 0; a < LIST_ATOMS; a++) {
+          if (a >= na) break;
+          float ex = p[a].x - pj.x, ey = p[a].y - pj.y, ez = p[a].z - pj.z;
+          if (M < 4) {   // a neighbor cell may hold a nearer image
+            ex -= G.L * nearest(ex * G.invL);
+            ey -= G.L * nearest(ey * G.invL);
+            ez -= G.L * nearest(ez * G.invL);
+          }
+          const bool in = have && j != q[a] && ex * ex + ey * ey + ez * ez < G.rlist2;
+          const unsigned m = __ballot_sync(0xffffffffu, in);
+          const int at = n[a] + __popc(m & below);
+          if (in && at < cap) out[a][at] = j;
+          n[a] += __popc(m);
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < LIST_ATOMS; a++) {
+        if (a >= na) break;
+        if (lane == 0) count[q[a]] = n[a];
+        longest = max(longest, n[a]);
+      }
       __syncwarp();
-      longest = max(longest, n);
     }
   }
   if (lane == 0 && longest > cap) atomicMax(overflow, longest);
