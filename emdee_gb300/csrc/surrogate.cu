@@ -31,6 +31,7 @@
 
 #include <cuda_bf16.h>
 
+#include "chain.cuh"
 #include "reduce.cuh"
 #include "system.hpp"
 #include "tile.cuh"
@@ -175,14 +176,14 @@ __device__ void load_weights(WeightsSmem& w, const float* p) {
 
 // ---- geometry kernels ---------------------------------------------------------------
 
+__device__ __forceinline__ float wrapped(double x, double L) { return (float)(x - L * floor(x / L)); }
+
+// (the fourth component is not read)
 __global__ void k_sg_pack(const double* __restrict__ R, int total, double L, float4* __restrict__ pos) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= total) return;
   float p[3];
-  for (int d = 0; d < 3; d++) {
-    const double x = R[3 * q + d];
-    p[d] = (float)(x - L * floor(x / L));
-  }
+  for (int d = 0; d < 3; d++) p[d] = wrapped(R[3 * q + d], L);
   pos[q] = make_float4(p[0], p[1], p[2], 0.f);
 }
 
@@ -504,6 +505,7 @@ __global__ void __launch_bounds__(32 * WARP_ATOMS) k_sg_desc(const float4* __res
                                                              const int* __restrict__ count, int cap,
                                                              float* __restrict__ Gout, int* __restrict__ near,
                                                              int* __restrict__ nearCount) {
+  chain_wait();
   __shared__ NeighborBuffer nbuf[WARP_ATOMS];
   __shared__ float hbuf[WARP_ATOMS][32 * HROW];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * WARP_ATOMS + warp;
@@ -548,6 +550,7 @@ __global__ void __launch_bounds__(32 * WARP_ATOMS, 4) k_sg_force(const float4* _
                                                               const int* __restrict__ nearCount, int cap,
                                                               const float* __restrict__ dEdG,
                                                               double* __restrict__ F) {
+  chain_wait();
   // per neighbor: dh[16], r_hat[3], index
   __shared__ __align__(16) float dbuf[WARP_ATOMS][32 * DROW];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * WARP_ATOMS + warp;
@@ -596,6 +599,7 @@ __global__ void __launch_bounds__(32 * WARP_ATOMS, 4) k_sg_udesc(const float4* _
                                                               const int* __restrict__ near,
                                                               const int* __restrict__ nearCount, int cap,
                                                               const float4* __restrict__ v, float* __restrict__ U) {
+  chain_wait();
   __shared__ float hbuf[WARP_ATOMS][32 * HROW];
   __shared__ float wbuf[WARP_ATOMS][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * WARP_ATOMS + warp;
@@ -893,6 +897,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_sg_mlp_tc(TileArgs T, const f
                                                              const float* __restrict__ Gin,
                                                              float* __restrict__ Eatom, float* __restrict__ dEdG,
                                                              int* __restrict__ err) {
+  chain_wait();
   extern __shared__ __align__(1024) unsigned char raw[];
   TcSmem& S = *reinterpret_cast<TcSmem*>(raw);
   const int t = threadIdx.x, warp = t >> 5, row = t % TC_M, half = t / TC_M;
@@ -1059,6 +1064,7 @@ __device__ __forceinline__ void column_sums(float (&x)[8][2], float* out) {
 __global__ void __launch_bounds__(128) k_sg_train(TileArgs T, int nt0, int nb0, const float* __restrict__ params,
                                                   const float* __restrict__ Gin, const float* __restrict__ Uin,
                                                   const float* __restrict__ eAtom, float* __restrict__ part) {
+  chain_wait();
   extern __shared__ __align__(16) unsigned char raw[];
   TrainSmem& S = *reinterpret_cast<TrainSmem*>(raw);
   const int species = (int)blockIdx.x < nb0 ? 0 : 1;
@@ -1264,19 +1270,25 @@ __global__ void k_sg_chain_sum(const float* __restrict__ x, int N, double* __res
   }
 }
 
-// velocity Verlet pieces for the chains (FP64, unit masses)
-__global__ void k_sg_kick_drift(double* __restrict__ R, double* __restrict__ P, const double* __restrict__ F, int n3,
-                                double half, double dt) {
+// velocity Verlet pieces for the chains (FP64, unit masses): END ends a step with a kick of
+// half, BEGIN begins the next with a kick of half, the drift over dt and the FP32
+// positions of k_sg_pack.  One pass per step instead of three.
+template <bool END, bool BEGIN>
+__global__ void k_sg_advance(double* __restrict__ R, double* __restrict__ P, const double* __restrict__ F, int n3,
+                             double half, double dt, double L, float* __restrict__ pos) {
+  chain_wait();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n3) return;
-  const double p = P[q] + half * F[q];
+  const double f = half * F[q];
+  double p = P[q];
+  if (END) p = p + f;
+  if (BEGIN) p = p + f;
   P[q] = p;
-  R[q] = R[q] + dt * p;
-}
-__global__ void k_sg_kick(double* __restrict__ P, const double* __restrict__ F, int n3, double half) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n3) return;
-  P[q] = P[q] + half * F[q];
+  if (BEGIN) {
+    const double x = R[q] + dt * p;
+    R[q] = x;
+    pos[4 * (q / 3) + q % 3] = wrapped(x, L);
+  }
 }
 
 }  // namespace sg
@@ -1341,7 +1353,7 @@ static void sg_network(Surrogate& S, const float* dParams, cudaStream_t st) {
   } else {
     TileArgs T{S.dAtoms, S.dTiles128, (int)S.tiles128.size()};
     const int blocks = std::min(T.ntiles, 2 * 152);
-    k_sg_mlp_tc<<<blocks, TC_THREADS, tc_smem_bytes(), st>>>(T, dParams, S.dG, S.dEatom, S.dEdG, S.dTcError);
+    launch_chained(k_sg_mlp_tc, blocks, TC_THREADS, tc_smem_bytes(), st, T, dParams, S.dG, S.dEatom, S.dEdG, S.dTcError);
   }
   CK(cudaGetLastError());
 }
@@ -1481,32 +1493,42 @@ void EmDee_surrogate_get_params(void* h, float* params) {
   CK(cudaMemcpy(params, S.dParams, sizeof(float) * sg::NPARAM, cudaMemcpyDeviceToHost));
 }
 
+// lists (if wanted) or, unless they are in place, the FP32 positions; then the descriptors
+static void sg_descriptors(Surrogate& S, const double* dR, bool rebuild, bool packed, cudaStream_t st) {
+  using namespace sg;
+  if (rebuild) sg_build_lists(S, dR, st);
+  else if (!packed) k_sg_pack<<<sg_blocks(S.total), 256, 0, st>>>(dR, S.total, S.L, S.dPos);
+  launch_chained(k_sg_desc, sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st, S.dPos, S.G, S.dSpecies, S.dList, S.dCount,
+                 S.cap, S.dG, S.dNear, S.dNearCount);
+  CK(cudaGetLastError());
+}
+
+static void sg_forces(Surrogate& S, const double* dR, double* dF, double* dE, bool rebuild, bool packed,
+                      cudaStream_t st) {
+  using namespace sg;
+  sg_descriptors(S, dR, rebuild, packed, st);
+  sg_network(S, S.dParams, st);
+  launch_chained(k_sg_force, sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st, S.dPos, S.G, S.dSpecies, S.dNear,
+                 S.dNearCount, S.cap, S.dEdG, dF);
+  CK(cudaGetLastError());
+  if (dE) k_sg_chain_sum<<<S.G.chains, 1024, 0, st>>>(S.dEatom, S.G.N, dE);
+}
+
 // Rebuilds the Verlet lists (rebuild != 0) and computes descriptors: dGout (optional, device,
 // [chains * N][32] FP32)
 void EmDee_surrogate_descriptors(void* h, const double* dR, float* dGout, int rebuild, void* stream) {
-  using namespace sg;
   Surrogate& S = *(Surrogate*)h;
   cudaStream_t st = (cudaStream_t)stream;
-  if (rebuild) sg_build_lists(S, dR, st);
-  else k_sg_pack<<<sg_blocks(S.total), 256, 0, st>>>(dR, S.total, S.L, S.dPos);
-  k_sg_desc<<<sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dList, S.dCount, S.cap, S.dG,
-                                                                 S.dNear, S.dNearCount);
-  CK(cudaGetLastError());
-  if (dGout) CK(cudaMemcpyAsync(dGout, S.dG, sizeof(float) * S.total * DIN, cudaMemcpyDeviceToDevice, st));
+  sg_descriptors(S, dR, rebuild != 0, false, st);
+  if (dGout) CK(cudaMemcpyAsync(dGout, S.dG, sizeof(float) * S.total * sg::DIN, cudaMemcpyDeviceToDevice, st));
 }
 
 // Surrogate forces (device FP64 [chains * N][3]) and energies per chain (device FP64 [chains]);
 // lists rebuilt when rebuild != 0.  Returns the largest neighbor count seen (list capacity check).
 int EmDee_surrogate_forces(void* h, const double* dR, double* dF, double* dE, int rebuild, void* stream) {
-  using namespace sg;
   Surrogate& S = *(Surrogate*)h;
   cudaStream_t st = (cudaStream_t)stream;
-  EmDee_surrogate_descriptors(h, dR, nullptr, rebuild, stream);
-  sg_network(S, S.dParams, st);
-  k_sg_force<<<sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dNear, S.dNearCount, S.cap,
-                                                                  S.dEdG, dF);
-  CK(cudaGetLastError());
-  if (dE) k_sg_chain_sum<<<S.G.chains, 1024, 0, st>>>(S.dEatom, S.G.N, dE);
+  sg_forces(S, dR, dF, dE, rebuild != 0, false, st);
   int ov = 0;
   if (rebuild) {
     int flags[2];
@@ -1543,10 +1565,10 @@ void EmDee_surrogate_gradient(void* h, const double* dR, const double* dEtrue, c
   k_sg_residual<<<std::min(SG_RES_BLOCKS, sg_blocks(S.total)), RES_THREADS, 0, st>>>(
       S.dF, dFtrue, S.dE, dEtrue, C, N, wE, fscale, S.dV, S.dEres, S.dResPart, S.dTicket,
       S.dResPart + 2 * SG_RES_BLOCKS, S.hLoss);
-  k_sg_udesc<<<sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st>>>(S.dPos, S.G, S.dSpecies, S.dNear, S.dNearCount,
+  launch_chained(k_sg_udesc, sg_warp_blocks(S.total), 32 * WARP_ATOMS, 0, st, S.dPos, S.G, S.dSpecies, S.dNear, S.dNearCount,
                                                                   S.cap, S.dV, S.dU);
   TileArgs T{S.dAtoms, S.dTrainTiles, (int)S.tiles.size()};
-  k_sg_train<<<S.trainBlocks, 128, sizeof(TrainSmem), st>>>(T, S.tiles0, S.trainBlocks0, S.dParams, S.dG, S.dU,
+  launch_chained(k_sg_train, S.trainBlocks, 128, sizeof(TrainSmem), st, T, S.tiles0, S.trainBlocks0, S.dParams, S.dG, S.dU,
                                                             S.dEres, S.dPart);
   k_sg_reduce<<<dim3((PER_SPECIES + REDUCE_PARAMS - 1) / REDUCE_PARAMS, NS), REDUCE_PARAMS * REDUCE_SLICES, 0, st>>>(
       S.dPart, S.trainBlocks0, S.trainBlocks, dGrad);
@@ -1574,11 +1596,14 @@ void EmDee_surrogate_trajectory(void* h, double* dR, double* dP, double* dF, dou
   Surrogate& S = *(Surrogate*)h;
   cudaStream_t st = (cudaStream_t)stream;
   const int n3 = 3 * S.total;
+  auto advance = [&](void (*kernel)(double*, double*, const double*, int, double, double, double, float*)) {
+    launch_chained(kernel, sg_blocks(n3), 256, 0, st, dR, dP, dF, n3, 0.5 * dt, dt, S.L, (float*)S.dPos);
+  };
   for (int k = 0; k < n; k++) {
-    sg::k_sg_kick_drift<<<sg_blocks(n3), 256, 0, st>>>(dR, dP, dF, n3, 0.5 * dt, dt);
-    EmDee_surrogate_forces(h, dR, dF, k == n - 1 ? dE : nullptr, 0, stream);
-    sg::k_sg_kick<<<sg_blocks(n3), 256, 0, st>>>(dP, dF, n3, 0.5 * dt);
+    advance(k == 0 ? sg::k_sg_advance<false, true> : sg::k_sg_advance<true, true>);
+    sg_forces(S, dR, dF, k == n - 1 ? dE : nullptr, false, true, st);
   }
+  if (n > 0) advance(sg::k_sg_advance<true, false>);
   CK(cudaGetLastError());
 }
 
