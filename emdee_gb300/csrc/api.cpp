@@ -311,7 +311,7 @@ static void compute_forces_impl(tEmDee* md) {
     if (!s.skinReady) device_skin_launch(s, both);
     if (!s.packReady && !both) device_pack(s);
     s.packReady = true;
-    forcesDone = device_pair_forces(s, compute, true);
+    forcesDone = device_pair_forces(s, compute, AFTER_SKIN);
     rebuild = !forcesDone;
   } else if (!rebuild) {
     rebuild = s.skinReady ? device_skin_from_step(s) : device_skin_check(s);
@@ -323,6 +323,11 @@ static void compute_forces_impl(tEmDee* md) {
       // the filtering launch computes this step's forces as well
       device_rebuild_two_level(s, compute);
       forcesDone = true;
+    } else if (s.precision == 0 && s.pairs_exist[s.layer - 1] && !two_level_active(s)) {
+      // one synchronisation for the build and the forces on its lists
+      device_build_lists(s, true);
+      forcesDone = device_pair_forces(s, compute, AFTER_BUILD);
+      if (!forcesDone) device_build_lists(s);   // a list or a tile had outgrown its room
     } else {
       device_build_lists(s);
     }

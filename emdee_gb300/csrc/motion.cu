@@ -385,7 +385,7 @@ bool pair_lj_only(System& s) {
          !(s.P(0, 0, l).coulomb && s.coul[l].kind != MK_COUL_NONE);
 }
 
-bool device_pair_forces(System& s, bool compute, bool speculative) {
+bool device_pair_forces(System& s, bool compute, PairLaunch when) {
   const int l = s.layer - 1;
   const double L = *s.Lbox, invL2 = 1.0 / (L * L);
   const bool useInRc = s.useInRc[l] != 0;
@@ -405,18 +405,20 @@ bool device_pair_forces(System& s, bool compute, bool speculative) {
   // kernel on the side stream, and their forces are added after it.  Their FP64 chains
   // leave most issue slots of an SM to its FP32 loop: 10 steps of 512 flexible waters
   // 852 -> 709 us, 3 steps of 1000 rigid waters with Ewald sums 1123 -> 1085 us.
-  const double* skip = speculative ? s.dResult + 9 : nullptr;
+  const double* skip =
+      when == AFTER_SKIN ? s.dResult + 9 : when == AFTER_BUILD ? s.dResult + BUILD_FAILED : nullptr;
   const bool kspace = s.queueExtras && s.coul[l].requires_kspace, bonded = s.queueExtras && bonded_active(s);
   if (kspace || bonded) CK(cudaEventRecord(s.forkEvent, s.stream));
   prof_begin(s, PK_PAIR);
   if (s.precision == 1) {
     device_pair_forces_fp64(s, compute, useInRc, rc2);
   } else {
-    s.pairSkip = speculative ? s.dResult + 9 : nullptr;
+    s.pairSkip = skip;
     device_pair_forces_mixed(s, compute, useInRc, rc2, pair_lj_only(s) ? 0 : 1);
     s.pairSkip = nullptr;
   }
   prof_end(s, PK_PAIR);
+  if (when == AFTER_BUILD) build_flags(s);
   // A boost that waits for these forces (free atoms, no bond, angle or k-space forces
   // to be added to them) gets its kinetic sums from a pass queued right behind the
   // pair kernel, which skips it too when a rebuild is due
@@ -450,7 +452,7 @@ bool device_pair_forces(System& s, bool compute, bool speculative) {
   // returns all of them.
   if (early) CK(cudaEventSynchronize(s.doneEvent));
   else CK(cudaStreamSynchronize(s.stream));
-  if (speculative && s.hResult[9] != 0.0) {
+  if ((when == AFTER_SKIN && s.hResult[9] != 0.0) || (when == AFTER_BUILD && !build_settled(s))) {
     if (chain) prof_drop_last(s);   // the kinetic pass returned at once as well
     prof_drop_last(s);
     return false;

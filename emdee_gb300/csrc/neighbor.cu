@@ -201,9 +201,12 @@ __device__ __forceinline__ float charge_f32(double q) {
 // reference's int(M (R/L - floor(R/L))) by rounding at a cell boundary changes
 // only the order of candidates, not the pair set.
 __global__ void k_assign(const double* __restrict__ R, const double* __restrict__ charge, int N, double scale,
-                         TileGeom g, int4* atomK, int* count, int* inCell, float4* pos0, double* __restrict__ R0) {
+                         TileGeom g, int4* atomK, int* count, int* inCell, float4* pos0, double* __restrict__ R0,
+                         int* dMax, unsigned long long* fail) {
   chain_wait();
   int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a < 4) dMax[a] = 0;   // the maxima of this build and its failure flag
+  if (a == 4) *fail = 0ull;
   if (a >= N) return;
   int c[3], K[3];
   float u[3];
@@ -229,15 +232,20 @@ __global__ void k_assign(const double* __restrict__ R, const double* __restrict_
   inCell[a] = base + __popc(peers & ((1u << lane) - 1u));
 }
 
-// three-phase device-wide exclusive scan (counts -> starts), starts[n] = total
+// device-wide exclusive scan (counts -> starts) in two phases, starts[n] = total: tiles,
+// then every block adds the tiles before its own.  The counts are left zero for the next
+// build.  (Launches and memsets are what a rebuild of a small system costs.)
 static const int SCAN_THREADS = 256, SCAN_ITEMS = 8, SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
-__global__ void k_scan_local(const int* in, int* out, int n, int* blockSums) {
+__global__ void k_scan_local(int* in, int* out, int n, int* blockSums) {
   chain_wait();
   __shared__ int buf[SCAN_TILE];
   __shared__ int ws[33];
   int base = blockIdx.x * SCAN_TILE;
-  for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS) buf[k] = base + k < n ? in[base + k] : 0;
+  for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS) {
+    buf[k] = base + k < n ? in[base + k] : 0;
+    if (base + k < n) in[base + k] = 0;
+  }
   __syncthreads();
   int total = block_exclusive_scan<SCAN_ITEMS>(buf, SCAN_TILE, ws);
   for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS)
@@ -245,37 +253,25 @@ __global__ void k_scan_local(const int* in, int* out, int n, int* blockSums) {
   if (threadIdx.x == 0) blockSums[blockIdx.x] = total;
 }
 
-__global__ void k_scan_sums(int* blockSums, int nb, int* out, int n) {
-  chain_wait();
-  __shared__ int ws[33];
-  __shared__ int carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int base = 0; base < nb; base += SCAN_TILE) {
-    __shared__ int buf[SCAN_TILE];
-    for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS) buf[k] = base + k < nb ? blockSums[base + k] : 0;
-    __syncthreads();
-    int total = block_exclusive_scan<SCAN_ITEMS>(buf, SCAN_TILE, ws);
-    for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS)
-      if (base + k < nb) blockSums[base + k] = buf[k] + carry;
-    __syncthreads();
-    if (threadIdx.x == 0) carry += total;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[n] = carry;
-}
-
 __global__ void k_scan_add(int* out, int n, const int* blockSums) {
   chain_wait();
-  int base = blockIdx.x * SCAN_TILE, add = blockSums[blockIdx.x];
+  __shared__ int ws[SCAN_THREADS / 32];
+  int before = 0;
+  for (int b = threadIdx.x; b < (int)blockIdx.x; b += SCAN_THREADS) before += blockSums[b];
+  before = __reduce_add_sync(0xffffffffu, before);
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = before;
+  __syncthreads();
+  int add = 0;
+  for (int w = 0; w < SCAN_THREADS / 32; w++) add += ws[w];
+  const int base = blockIdx.x * SCAN_TILE;
   for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS)
     if (base + k < n) out[base + k] += add;
+  if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) out[n] = add + blockSums[blockIdx.x];
 }
 
-static void device_scan(System& s, const int* in, int* out, int n) {
+static void device_scan(System& s, int* in, int* out, int n) {
   int nb = (n + SCAN_TILE - 1) / SCAN_TILE;
   launch_chained(k_scan_local, nb, SCAN_THREADS, 0, s.stream, in, out, n, s.grid.dScanTmp);
-  launch_chained(k_scan_sums, 1, SCAN_THREADS, 0, s.stream, s.grid.dScanTmp, nb, out, n);
   launch_chained(k_scan_add, nb, SCAN_THREADS, 0, s.stream, out, n, s.grid.dScanTmp);
   CK(cudaGetLastError());
 }
@@ -464,6 +460,7 @@ void device_pack(System& s) {
 
 struct BuildArgs {
   TileGeom g;
+  unsigned long long* fail;   // set if a list or a tile outgrew its room: the force kernels queued behind skip
   const int2* tab;
   const float4* pos4;
   const int* start;
@@ -588,7 +585,10 @@ __global__ void __maxnreg__(MODE == BUILD_ONE ? BUILD_MAXNREG : 64) k_build(Buil
     // reported (the host re-sizes and builds again) before anything is staged
     const int tileCount = A.start[(t + 1) * g.TB * g.TB * g.TB] - A.start[t * g.TB * g.TB * g.TB];
     if (tileCount > A.tileStride || haloCount > A.haloCap) {
-      if (threadIdx.x == 0) atomicOr(A.maxCount + 1, 1);
+      if (threadIdx.x == 0) {
+        atomicOr(A.maxCount + 1, 1);
+        *A.fail = 1ull;
+      }
       return;
     }
   }
@@ -841,7 +841,10 @@ __global__ void __maxnreg__(MODE == BUILD_ONE ? BUILD_MAXNREG : 64) k_build(Buil
     longest = max(longest, n);
   }
   longest = __reduce_max_sync(0xffffffffu, longest);
-  if ((threadIdx.x & 31) == 0 && longest > 0) atomicMax(A.maxCount, longest);
+  if ((threadIdx.x & 31) == 0 && longest > 0) {
+    atomicMax(A.maxCount, longest);
+    if (longest > A.cap) *A.fail = 1ull;
+  }
 }
 
 template <typename T>
@@ -1058,10 +1061,16 @@ void device_tune_tile(System& s, bool ljOnly, void (*pair)(System&)) {
   g_tileTuned.push_back({key, choice});
 }
 
+void build_flags(System& s) {
+  CK(cudaMemcpyAsync(s.hFlags + 2, s.grid.dTileInfo + 2 * s.grid.nTiles + 2, 2 * sizeof(int), cudaMemcpyDeviceToHost,
+                     s.stream));
+}
+
 // src/neighbor_lists.f90:175-195 (build part) and 199-300.  reuse: keep the tile
 // sizes of the previous build when the cell geometry is unchanged (no per-tile
 // count pass and no synchronisation for it); returns false if a tile outgrew them.
-static bool build_lists(System& s, bool reuse) {
+// defer: returns without waiting for the build (build_settled).
+static bool build_lists(System& s, bool reuse, bool defer) {
   Grid& g = s.grid;
   GridCaps& c = g.caps;
   const int N = s.natoms;
@@ -1087,7 +1096,10 @@ static bool build_lists(System& s, bool reuse) {
     g.nTiles = geo.nT * geo.nT * geo.nT;
     g.nRanks = g.nTiles * TB * TB * TB;
     g.haloCells = geo.haloCells;
-    grow(g.dCount, c.ranks, (size_t)g.nRanks + 1);
+    if (c.ranks < (size_t)g.nRanks + 1) {   // zero between builds (k_scan_local)
+      grow(g.dCount, c.ranks, (size_t)g.nRanks + 1);
+      CK(cudaMemsetAsync(g.dCount, 0, sizeof(int) * c.ranks, s.stream));
+    }
     if (!g.dStart || c.scan < (size_t)g.nRanks + 1) {
       CK(cudaFree(g.dStart));
       CK(cudaFree(g.dScanTmp));
@@ -1122,11 +1134,11 @@ static bool build_lists(System& s, bool reuse) {
       c.tiles = g.nTiles;
     }
     int th = 256, bl = (N + th - 1) / th;
-    CK(cudaMemsetAsync(g.dCount, 0, sizeof(int) * (g.nRanks + 1), s.stream));
-    s.prof.total += reuse ? 7 : 8;   // assign, 3 scan phases, scatter, sort, fill (, tile info)
+    int* dMax = g.dTileInfo + 2 * g.nTiles;
+    s.prof.total += reuse ? 6 : 7;   // assign, 2 scan phases, scatter, sort, fill (, tile info)
     // the slot array holds each atom's place in its cell until k_fill_slots
     launch_chained(k_assign, bl, th, 0, s.stream, s.dR, s.dCharge, N, (double)M / L, geo, g.dAtomK, g.dCount, g.dSlotOf,
-                                      g.dPos0, s.dR0);
+                                      g.dPos0, s.dR0, dMax, (unsigned long long*)(s.dResult + BUILD_FAILED));
     CK(cudaGetLastError());
     device_scan(s, g.dCount, g.dStart, g.nRanks);
     launch_chained(k_scatter, bl, th, 0, s.stream, g.dAtomK, N, g.dStart, g.dSlotOf, g.dOrig);
@@ -1136,8 +1148,6 @@ static bool build_lists(System& s, bool reuse) {
       launch_chained(k_sort_cells, (g.nRanks + 255) / 256, 256, 0, s.stream, g.dStart, g.nRanks, g.dOrig, g.dPos0, g.dKeyX);
     launch_chained(k_fill_slots, bl, th, 0, s.stream, g.dOrig, N, g.dAtomK, s.dType, g.dK, g.dType8, g.dSlotOf, g.dPos0,
                                           g.dPos4);
-    int* dMax = g.dTileInfo + 2 * g.nTiles;
-    CK(cudaMemsetAsync(dMax, 0, sizeof(int) * 4, s.stream));
     if (reuse) break;
     k_tile_info<<<g.nTiles, 128, 0, s.stream>>>(g.dStart, geo, g.dTileInfo, dMax);
     CK(cudaGetLastError());
@@ -1219,6 +1229,7 @@ static bool build_lists(System& s, bool reuse) {
   A.selfIdx = g.dSelf;
   A.tileStride = g.tileStride;
   A.maxCount = g.dTileInfo + 2 * g.nTiles + 2;
+  A.fail = (unsigned long long*)(s.dResult + BUILD_FAILED);
   grow(g.dLayout, g.layoutCap, (size_t)g.nTiles * (2 * g.haloCells + 1));
   A.layout = g.dLayout;
   const bool general = build_general(s);
@@ -1248,13 +1259,17 @@ static bool build_lists(System& s, bool reuse) {
     grow(nbList, nbCap, need);
     A.nb = nbList;
     A.cap = cap;
-    CK(cudaMemsetAsync(A.maxCount, 0, sizeof(int), s.stream));
+    if (attempt > 0) {   // k_assign zeroed them for the first
+      CK(cudaMemsetAsync(A.maxCount, 0, sizeof(int), s.stream));
+      CK(cudaMemsetAsync(A.fail, 0, sizeof(*A.fail), s.stream));
+    }
     if (chain_fits(g.nTiles)) launch_chained(kb, g.nTiles, buildThreads, smem, s.stream, A);
     else kb<<<g.nTiles, buildThreads, smem, s.stream>>>(A);
     s.prof.total++;
     CK(cudaGetLastError());
-    int* mc = s.hFlags + 2;   // pinned: largest list, tile-size overflow
-    CK(cudaMemcpyAsync(mc, A.maxCount, 2 * sizeof(int), cudaMemcpyDeviceToHost, s.stream));
+    if (defer) break;
+    const int* mc = s.hFlags + 2;   // pinned: largest list, tile-size overflow
+    build_flags(s);
     CK(cudaStreamSynchronize(s.stream));
     if (mc[1]) return false;
     if (mc[0] <= cap) break;
@@ -1272,11 +1287,13 @@ static bool build_lists(System& s, bool reuse) {
   return true;
 }
 
-void device_build_lists(System& s) {
+void device_build_lists(System& s, bool defer) {
   prof_begin(s, PK_BUILD);
-  if (!build_lists(s, true)) build_lists(s, false);
+  if (!build_lists(s, true, defer)) build_lists(s, false, false);
   prof_end(s, PK_BUILD);
 }
+
+bool build_settled(const System& s) { return !s.hFlags[3] && s.hFlags[2] <= s.grid.cap; }
 
 // ---------------------------------------------------------------------------------
 // two-level lists

@@ -338,7 +338,13 @@ bool device_skin_check(System& s);
 void device_skin_launch(System& s, bool pack);
 // Cell binning, tile sort and neighbor-list build (src/neighbor_lists.f90:63-300).
 // With two-level lists active it builds the outer lists (radius rc + skin + outer skin).
-void device_build_lists(System& s);
+// defer (single-level lists): the build is queued only; after build_flags (a copy, queued)
+// and a synchronisation build_settled tells whether its lists and tiles had room, otherwise it is to be repeated
+// without defer.  Until then dResult[BUILD_FAILED] is a nonzero word if they had not.
+void device_build_lists(System& s, bool defer = false);
+void build_flags(System& s);
+bool build_settled(const System& s);
+const int BUILD_FAILED = 72;
 // Tile edge and block sizes tuned by timing builds and pair launches on the system
 // (first build, mixed precision); pair(s) computes the forces once on the current lists.
 void device_tune_tile(System& s, bool ljOnly, void (*pair)(System&));
@@ -370,10 +376,12 @@ void device_pair_refilter(System& s, bool compute, const double* skip);
 void device_pack(System& s);
 // Pair forces, energies and virials of the current layer into s.F();
 // leaves Epair, Ecoul, Wpair, Wcoul in hResult after synchronizing.
-// Forces of the current layer; energies and virials in hResult[0..3].  speculative
-// (mixed precision, after a fused step): the kernel runs only if the step's skin
-// check found no rebuild due; returns false if it did not run.
-bool device_pair_forces(System& s, bool compute, bool speculative = false);
+// Forces of the current layer; energies and virials in hResult[0..3].  AFTER_SKIN,
+// AFTER_BUILD (mixed precision): what the launches depend on is still on the device (the
+// rebuild flag, or whether the build queued before them had room); they return at once if
+// it is set, and the call, after its synchronisation, returns false.
+enum PairLaunch { PAIR_NOW, AFTER_SKIN, AFTER_BUILD };
+bool device_pair_forces(System& s, bool compute, PairLaunch when = PAIR_NOW);
 // P <- CP P + CF F (free atoms); optional 2KE per dimension into hResult[10..12].
 void device_boost(System& s, double CP, double CF, bool kinetic);
 // 2KE per dimension (hResult[10..12]) of the momenta after the pending kicks and one
