@@ -242,11 +242,12 @@ __global__ void k_scan_local(int* in, int* out, int n, int* blockSums) {
   __shared__ int buf[SCAN_TILE];
   __shared__ int ws[33];
   int base = blockIdx.x * SCAN_TILE;
-  for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS) {
-    buf[k] = base + k < n ? in[base + k] : 0;
-    if (base + k < n) in[base + k] = 0;
-  }
+  for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS) buf[k] = base + k < n ? in[base + k] : 0;
   __syncthreads();
+  // (after the loads: a store between them keeps each waiting for the one before, 34 us
+  // against 7 for the 438,976 cells of 1,048,576 atoms)
+  for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS)
+    if (base + k < n) in[base + k] = 0;
   int total = block_exclusive_scan<SCAN_ITEMS>(buf, SCAN_TILE, ws);
   for (int k = threadIdx.x; k < SCAN_TILE; k += SCAN_THREADS)
     if (base + k < n) out[base + k] = buf[k];
