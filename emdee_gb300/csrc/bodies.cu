@@ -1,8 +1,8 @@
 // bodies.cu -- rigid bodies on the device: per-body force and torque, momentum
 // and position updates, exact or NO_SQUISH rotation, kinetic energies, the
 // rigid-body virial, and momentum assignment (src/EmDeeData.f90:157-189,
-// 420-439, 823-953; src/ArBee.f90).  One thread per body, FP64, compiled with
-// -fmad=false.  Free atoms of a system with bodies go through index-list
+// 420-439, 823-953; src/ArBee.f90).  FP64, compiled with -fmad=false; four lanes
+// per body in the boost and the exact rotation, one thread elsewhere.  Free atoms of a system with bodies go through index-list
 // variants of the boost and move kernels.
 #include <vector>
 

@@ -12,9 +12,10 @@
 //   k_sg_list      Verlet lists within rc + skin from a cell list (per chain), a block
 //                  per cell
 //   k_sg_desc      descriptors, a warp per atom, Gaussians by the two-term product recurrence
-//   k_sg_mlp       per-species tiles of 64 atoms: forward and backward through the
-//                  network on the tensor cores (mma.sync m16n8k16, BF16 operands,
-//                  FP32 accumulation): E_i and dE/dG_i
+//   k_sg_mlp_tc    per-species tiles of 128 atoms: forward and backward through the
+//                  network on the tensor cores (tcgen05, BF16 operands, FP32
+//                  accumulation): E_i and dE/dG_i; k_sg_mlp, tiles of 64 atoms by
+//                  mma.sync m16n8k16, is kept for comparison
 //   k_sg_force     the adjoint: F_i = -sum_j (dE/dG_i[s_j] + dE/dG_j[s_i]) . dh/dr r_hat
 //   k_sg_udesc     training: u_i[c, k] = sum_j h'_k(r_ij) (v_i - v_j) . r_hat_ij, the
 //                  force residual v pulled back to descriptor space
@@ -23,6 +24,7 @@
 //                  gradient is the gradient of the energy + force loss; weight
 //                  gradients as tensor-core GEMMs over 64-atom tiles, per-block
 //                  partials reduced in block order
+//   k_sg_advance   trajectories: everything between two force evaluations
 //   k_sg_adam      Adam update of the FP32 master parameters
 #include <algorithm>
 #include <cmath>

@@ -262,7 +262,8 @@ int EmDee_tile_edge(tEmDee md);
 
 /* Threads per block of the thread-per-atom list build (kernel 0) and of the
    single-type Lennard-Jones force kernel (kernel 1) on the current tiles: tuned with
-   the tile edge (every thread takes the same number of a tile's atoms). */
+   the tile edge (every thread takes the same number of a tile's atoms; systems too
+   small to fill the GPU split an atom's list over 2 to 32 threads of the block). */
 int EmDee_tile_threads(tEmDee md, int kernel);
 
 /* No counterpart in the reference.  EmDee_boost's momentum update and
