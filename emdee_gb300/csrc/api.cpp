@@ -576,6 +576,9 @@ tEmDee EmDee_system(int threads, int layers, double rc, double skin, int N, int*
   }
   CK(cudaMallocHost(&s->hResult, sizeof(double) * 80));
   CK(cudaMallocHost(&s->hFlags, sizeof(int) * 16));
+  CK(cudaMallocHost(&s->hSkinDone, 2 * sizeof(unsigned long long)));
+  s->hSkinDone[0] = s->hSkinDone[1] = 0;
+  s->hPairDone = (unsigned int*)(s->hSkinDone + 1);
   CK(cudaMalloc(&s->dResult, sizeof(double) * 80));
   CK(cudaMalloc(&s->dTicket, sizeof(unsigned int) * 16));
   CK(cudaMemset(s->dTicket, 0, sizeof(unsigned int) * 16));
@@ -655,6 +658,7 @@ void EmDee_destroy(tEmDee* md) {
   cudaFree(s->dResult);
   cudaFreeHost(s->hResult);
   cudaFreeHost(s->hFlags);
+  cudaFreeHost(s->hSkinDone);
   cudaFreeHost(s->hMirrorR); cudaFreeHost(s->hMirrorP); cudaFreeHost(s->hMirrorF); cudaFreeHost(s->hMirrorLayerF);
   if (s->ownsLbox) delete s->Lbox;
   cudaEventDestroy(s->forkEvent);

@@ -10,6 +10,7 @@
 #include "ffkick.cuh"
 #include "fpconv.h"
 #include "reduce.cuh"
+#include <chrono>
 #include <vector>
 
 #include "system.hpp"
@@ -385,6 +386,25 @@ bool pair_lj_only(System& s) {
          !(s.P(0, 0, l).coulomb && s.coul[l].kind != MK_COUL_NONE);
 }
 
+// A step whose last kernel is the pair kernel: its sums, or the skin check's decision for a
+// rebuild, are read as soon as they are written, a few microseconds before the stream
+// reports the drained grid (800 atoms, 20 steps: 658 -> 609 us; 100,003 atoms, 10 steps:
+// 777 -> 753).  Every block's forces are visible device-wide by then (a block is counted
+// after them).  Bounded: after 20 ms the caller waits for the stream, which reports
+// errors as well.
+static bool poll_results(System& s) {
+  const auto t0 = std::chrono::steady_clock::now();
+  auto wait = [&](auto&& ready) {
+    for (int k = 1; !ready(); k++)
+      if ((k & 255) == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(20)) return false;
+    return true;
+  };
+  unsigned long long skin = 0;
+  if (!wait([&] { return (skin = __atomic_load_n(s.hSkinDone, __ATOMIC_ACQUIRE)) >> 1 == s.skinStamp; })) return false;
+  s.hResult[9] = skin & 1 ? 1.0 : 0.0;
+  return (skin & 1) || wait([&] { return __atomic_load_n(s.hPairDone, __ATOMIC_ACQUIRE) == s.pairStamp; });
+}
+
 bool device_pair_forces(System& s, bool compute, PairLaunch when) {
   const int l = s.layer - 1;
   const double L = *s.Lbox, invL2 = 1.0 / (L * L);
@@ -408,23 +428,28 @@ bool device_pair_forces(System& s, bool compute, PairLaunch when) {
   const double* skip =
       when == AFTER_SKIN ? s.dResult + 9 : when == AFTER_BUILD ? s.dResult + BUILD_FAILED : nullptr;
   const bool kspace = s.queueExtras && s.coul[l].requires_kspace, bonded = s.queueExtras && bonded_active(s);
-  if (kspace || bonded) CK(cudaEventRecord(s.forkEvent, s.stream));
-  prof_begin(s, PK_PAIR);
-  if (s.precision == 1) {
-    device_pair_forces_fp64(s, compute, useInRc, rc2);
-  } else {
-    s.pairSkip = skip;
-    device_pair_forces_mixed(s, compute, useInRc, rc2, pair_lj_only(s) ? 0 : 1);
-    s.pairSkip = nullptr;
-  }
-  prof_end(s, PK_PAIR);
-  if (when == AFTER_BUILD) build_flags(s);
   // A boost that waits for these forces (free atoms, no bond, angle or k-space forces
   // to be added to them) gets its kinetic sums from a pass queued right behind the
   // pair kernel, which skips it too when a rebuild is due
   const int l2 = s.layer - 1;
   const bool chain = s.keChainReq && s.precision == 0 && s.nbodies == 0 && s.bondedTerms.bonds.empty() &&
                      s.bondedTerms.angles.empty() && !s.coul[l2].requires_kspace;
+  const bool poll = when == AFTER_SKIN && s.precision == 0 && !chain && !kspace && !bonded && s.nbodies == 0 &&
+                    !s.vvReq && !s.prof.on;
+  if (kspace || bonded) CK(cudaEventRecord(s.forkEvent, s.stream));
+  prof_begin(s, PK_PAIR);
+  if (s.precision == 1) {
+    device_pair_forces_fp64(s, compute, useInRc, rc2);
+  } else {
+    s.pairSkip = skip;
+    s.pairStamp++;
+    s.pairDone = poll ? s.hPairDone : nullptr;
+    device_pair_forces_mixed(s, compute, useInRc, rc2, pair_lj_only(s) ? 0 : 1);
+    s.pairSkip = nullptr;
+    s.pairDone = nullptr;
+  }
+  prof_end(s, PK_PAIR);
+  if (when == AFTER_BUILD) build_flags(s);
   if (chain) launch_kinetic_two(s, s.keChainCF, skip);
   bool early = false;
   if (s.queueExtras) {
@@ -451,7 +476,8 @@ bool device_pair_forces(System& s, bool compute, PairLaunch when) {
   // and rebuild flag ([8], [9]), straight into the pinned hResult, so one synchronisation
   // returns all of them.
   if (early) CK(cudaEventSynchronize(s.doneEvent));
-  else CK(cudaStreamSynchronize(s.stream));
+  else if (!(poll && poll_results(s)))
+    CK(cudaStreamSynchronize(s.stream));
   if ((when == AFTER_SKIN && s.hResult[9] != 0.0) || (when == AFTER_BUILD && !build_settled(s))) {
     if (chain) prof_drop_last(s);   // the kinetic pass returned at once as well
     prof_drop_last(s);

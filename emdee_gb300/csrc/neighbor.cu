@@ -82,7 +82,8 @@ __global__ void __launch_bounds__(SKIN_THREADS) k_skin(const double* __restrict_
                                                        unsigned int* ticket, double* result, double* hostResult,
                                                        const int* __restrict__ slotOf,
                                                        const float4* __restrict__ pos0, float scale,
-                                                       float4* __restrict__ pos4) {
+                                                       float4* __restrict__ pos4, unsigned long long* done,
+                                                       unsigned int stamp) {
   chain_wait();
   __shared__ MaxPrev wsum[SKIN_THREADS / 32];
   __shared__ bool last;
@@ -134,6 +135,7 @@ __global__ void __launch_bounds__(SKIN_THREADS) k_skin(const double* __restrict_
     result[8] = hostResult[8] = value;   // pinned host memory: read after the synchronisation
     result[9] = hostResult[9] = value > skinSq ? 1.0 : 0.0;
     *ticket = 0;
+    *(volatile unsigned long long*)done = 2ull * stamp + (value > skinSq ? 1 : 0);   // pinned, one store
   }
 }
 
@@ -153,7 +155,7 @@ void device_skin_launch(System& s, bool pack) {
   prof_begin(s, PK_SKIN);
   launch_chained(pack ? k_skin<true> : k_skin<false>, blocks, SKIN_THREADS, 0, s.stream, s.dR, s.dR0, N, chunks,
                  s.skinSq, (longlong2*)s.dPartials, s.dTicket, s.dResult, s.hResult, g.dSlotOf, g.dPos0,
-                 (float)((double)g.M / *s.Lbox), g.dPos4);
+                 (float)((double)g.M / *s.Lbox), g.dPos4, s.hSkinDone, ++s.skinStamp);
   CK(cudaGetLastError());
   prof_end(s, PK_SKIN);
 }
@@ -1683,7 +1685,8 @@ __global__ void __launch_bounds__(SKIN_THREADS) k_step_fused(double* __restrict_
                                                              const float4* __restrict__ pos0, float scale,
                                                              float4* __restrict__ pos4, longlong2* partial,
                                                              unsigned int* ticket, double* result,
-                                                             double* hostResult, double* __restrict__ s0) {
+                                                             double* hostResult, double* __restrict__ s0,
+                                                             unsigned long long* done, unsigned int stamp) {
   chain_wait();
   __shared__ MaxPrev wsum[SKIN_THREADS / 32];
   __shared__ bool last;
@@ -1755,6 +1758,7 @@ __global__ void __launch_bounds__(SKIN_THREADS) k_step_fused(double* __restrict_
     hostResult[8] = value;   // pinned host memory: read after the next synchronisation
     hostResult[9] = result[9];
     *ticket = 0;
+    *(volatile unsigned long long*)done = 2ull * stamp + (value > skinSq ? 1 : 0);
   }
 }
 
@@ -1769,9 +1773,10 @@ void device_step_fused(System& s, double CP, bool vv, double* s0) {
     s.pendCF[0] = 0.5 * CP;
     s.npend = 1;
   }
+  s.skinStamp++;
   prof_begin(s, PK_MOVE);
 #define STEP_ARGS s.dR, s.dP, s.F(), s.dInvMass, s.dR0, N, chunks, s.pendCF[0], s.pendCF[1], CP, s.skinSq, g.dSlotOf, \
-                  g.dPos0, scale, g.dPos4, (longlong2*)s.dPartials, s.dTicket, s.dResult, s.hResult, s0
+                  g.dPos0, scale, g.dPos4, (longlong2*)s.dPartials, s.dTicket, s.dResult, s.hResult, s0, s.hSkinDone, s.skinStamp
 #define STEP_LAUNCH(NK, UM, PK, FM, VV) launch_chained(k_step_fused<NK, UM, PK, FM, VV>, blocks, SKIN_THREADS, 0, s.stream, STEP_ARGS)
 #define STEP_NK(UM, PK, FM)                            \
   if (vv) STEP_LAUNCH(1, UM, PK, FM, true);            \

@@ -67,6 +67,8 @@ struct PairArgsF {
   unsigned int* ticket;
   double* result;
   double* hostResult;   // pinned host copy of the sums, written by the last block
+  unsigned int* done;   // pinned: gets stamp after them
+  unsigned int stamp;
   // filtering launches (nb, count and cap above describe the outer lists): every
   // entry within rc + skin (FP32 distance, FP64 test of the reference inside the
   // band lo2In..hi2In) goes to the lists written here, in the outer lists' order
@@ -287,7 +289,7 @@ __global__ void PAIR_BOUNDS k_pair_mixed(PairArgsF A) {
   const float v[5] = {0.5f * Ep, 0.5f * Ec, 0.5f * Wp, 0.5f * Wc, 0.5f * within};
   constexpr unsigned MASK = (COMPUTE ? (VAR == 1 ? 3u : 1u) : 0u) | (VAR == 1 ? 12u : 4u) | (COUNT ? 16u : 0u);
   grid_reduce_ff<5, PAIR_MAX_THREADS, MASK>(v, reinterpret_cast<float2*>(A.partials), A.ticket, A.result,
-                                            A.hostResult);
+                                            A.hostResult, A.done, A.stamp);
 }
 
 template <bool COMPUTE, int VAR, int MOD, bool MINIMG, bool COUNT, bool REFILTER = false>
@@ -448,7 +450,7 @@ __global__ void __launch_bounds__(PAIR_THREADS_TYPES) k_pair_types(PairArgsF A) 
   const float v[5] = {0.5f * Ep, 0.5f * Ec, 0.5f * Wp, 0.5f * Wc, 0.f};
   constexpr unsigned MASK = (COMPUTE ? (COUL ? 3u : 1u) : 0u) | (COUL ? 12u : 4u);
   grid_reduce_ff<5, PAIR_THREADS_TYPES, MASK>(v, reinterpret_cast<float2*>(A.partials), A.ticket, A.result,
-                                              A.hostResult);
+                                              A.hostResult, A.done, A.stamp);
 }
 
 template <bool COMPUTE, bool COUL, bool LSHIFT, bool CSHIFT, bool MINIMG>
@@ -540,6 +542,8 @@ static size_t pair_args(System& s, bool useInRc, double rc2scaled, bool general,
   A.ticket = s.dTicket;
   A.result = s.dResult;
   A.hostResult = s.hResult;
+  A.done = s.pairDone;
+  A.stamp = s.pairStamp;
   A.nbIn = nullptr;
   A.countIn = nullptr;
   A.capIn = 0;

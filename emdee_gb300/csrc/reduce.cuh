@@ -181,10 +181,12 @@ __device__ __forceinline__ void grid_reduce_ff2(const float (&vh)[NQ], const flo
 // Per-thread FP32 values -> result[q] (FP64), also into result2 if set.  partials holds
 // NQ float2 per block.
 // The last block (ticket) sums the partials in block order; the result does not
-// depend on block scheduling.
+// depend on block scheduling.  done (pinned host memory), if set, gets the value stamp
+// once result2 is in place: the host can read it there before the grid has drained.
 template <int NQ, int THREADS, unsigned MASK = ~0u>
 __device__ __forceinline__ void grid_reduce_ff(const float (&v)[NQ], float2* partials, unsigned int* ticket,
-                                               double* result, double* result2 = nullptr) {
+                                               double* result, double* result2 = nullptr,
+                                               unsigned int* done = nullptr, unsigned int stamp = 0) {
   __shared__ float2 red[NQ][THREADS / 32];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
@@ -248,8 +250,13 @@ __device__ __forceinline__ void grid_reduce_ff(const float (&v)[NQ], float2* par
       for (int w = 0; w < nw; w++) ff_add(h, l, red[q][w].x, red[q][w].y);
     result[q] = (double)h + (double)l;
     if (result2) result2[q] = (double)h + (double)l;   // e.g. pinned host memory: no copy back
+    if (done) __threadfence_system();
   }
-  if (threadIdx.x == 0) *ticket = 0;
+  __syncwarp();
+  if (threadIdx.x == 0) {
+    *ticket = 0;
+    if (done) *(volatile unsigned int*)done = stamp;
+  }
 }
 
 }  // namespace emdee

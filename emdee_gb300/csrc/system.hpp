@@ -281,6 +281,12 @@ struct System {
   } boost = {};
   bool boostReq = false, boostQueued = false;
   bool phaseShared = false;   // R/P aliased with another system (no deferral then)
+  // pinned: twice the stamp of the last finished skin check, plus its rebuild flag; and the
+  // stamp of the last pair launch whose sums are in hResult.  pairDone: set for a launch
+  // that is to leave its stamp
+  unsigned long long* hSkinDone = nullptr;
+  unsigned int *hPairDone = nullptr, *pairDone = nullptr;
+  unsigned int skinStamp = 0, pairStamp = 0;
   const double* pairSkip = nullptr;   // device rebuild flag the mixed pair kernel checks first
   double builtL = 0;           // box length at the last build
   // two-level neighbor lists (EmDee_set_outer_skin): outerSkin < 0 not set, 0 off
