@@ -63,7 +63,7 @@ __device__ __forceinline__ double body_Bt(const double* q, const double* p, int 
 // (the body virial is its negative) into result[6], which saves k_body_virial's pass where a
 // boost with sums follows the forces.  Lane c < 3 takes component c of the vectors.
 template <bool KIN, bool VIR>
-__global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_boost(BodyArgs A, const double* __restrict__ F, double CP,
+__global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_boost(BodyArgs A, const double* F, double CP,
                                                                    double CF, int translate, int rotate,
                                                                    double* partials, unsigned int* ticket,
                                                                    double* result, double* hostResult,
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_move_series(BodyArg
 }
 
 // W = sum over bodies and their atoms of F . delta (the body virial is -W)
-__global__ void __launch_bounds__(BODY_THREADS) k_body_virial(BodyArgs A, const double* __restrict__ F,
+__global__ void __launch_bounds__(BODY_THREADS) k_body_virial(BodyArgs A, const double* F,
                                                               double* partials, unsigned int* ticket, double* result,
                                                               double* hostResult, const double* skip) {
   chain_wait();
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(BODY_THREADS) k_body_particle_momenta(BodyArgs
 
 // free atoms only: boost and move through the free-atom list
 template <bool KIN>
-__global__ void __launch_bounds__(BODY_THREADS) k_boost_free(double* __restrict__ P, const double* __restrict__ F,
+__global__ void __launch_bounds__(BODY_THREADS) k_boost_free(double* __restrict__ P, const double* F,
                                                              const double* __restrict__ invMass, const int* freeList,
                                                              int nfree, double CP, double CF, double* partials,
                                                              unsigned int* ticket, double* result, double* hostResult,
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(BODY_THREADS) k_boost_free(double* __restrict_
   if (KIN) grid_reduce<3, BODY_THREADS>(k2, partials, ticket, result, hostResult);
 }
 
-__global__ void __launch_bounds__(BODY_THREADS) k_move_free(double* __restrict__ R, const double* __restrict__ P,
+__global__ void __launch_bounds__(BODY_THREADS) k_move_free(double* __restrict__ R, const double* P,
                                                             const double* __restrict__ invMass, const int* freeList,
                                                             int nfree, double CR, double CP) {
   chain_wait();

@@ -10,6 +10,12 @@
 // that the pair kernel on the main stream needs (1000 waters with Ewald sums 1074 -> 1114
 // us with its sums chained, 1033 without).  Kernels launched the ordinary way are ordered as
 // always, whatever is before or behind them, and chain_wait returns at once in them.
+//
+// A kernel that is launched so starts while the one before it still writes.  What any kernel
+// writes is therefore not declared `const T* __restrict__` there, nor read by __ldg: both
+// promise memory that nobody writes while the kernel runs, and such a load may be moved
+// in front of the wait or served from a line read before it.  Only arrays that the host set up
+// (masses, charges, species) are.
 #pragma once
 #include <utility>
 

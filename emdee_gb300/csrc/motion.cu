@@ -28,7 +28,7 @@ static const int MOTION_THREADS = 256;
 // fused multiply-add, which halves the work on GB300's narrow FP64 pipe; FP64
 // mode keeps the reference's separately rounded statements.
 template <bool KIN, bool UNITCP, bool UNITM, bool FMA>
-__global__ void __launch_bounds__(MOTION_THREADS) k_boost(double* __restrict__ P, const double* __restrict__ F,
+__global__ void __launch_bounds__(MOTION_THREADS) k_boost(double* __restrict__ P, const double* F,
                                                           const double* __restrict__ invMass, int N, double CP,
                                                           double CF, double* partials, unsigned int* ticket,
                                                           double* twoKE, double* hostKE) {
@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(MOTION_THREADS) k_boost(double* __restrict__ P
 }
 
 template <bool UNITCR, bool UNITM, bool FMA>
-__global__ void __launch_bounds__(MOTION_THREADS) k_move(double* __restrict__ R, const double* __restrict__ P,
+__global__ void __launch_bounds__(MOTION_THREADS) k_move(double* __restrict__ R, const double* P,
                                                          const double* __restrict__ invMass, int N, double CR,
                                                          double CP) {
   chain_wait();
@@ -224,8 +224,8 @@ bool device_kinetic(System& s, double* twoKE, const double* src, const double* s
 // applied in order with the fused multiply-adds of k_step_fused) without writing P:
 // the kicks stay deferred.  Flat walk over P[3N] as in k_kinetic.
 template <int NK, bool UNITM>
-__global__ void __launch_bounds__(MOTION_THREADS) k_kinetic_pending(const double* __restrict__ P,
-                                                                    const double* __restrict__ F,
+__global__ void __launch_bounds__(MOTION_THREADS) k_kinetic_pending(const double* P,
+                                                                    const double* F,
                                                                     const double* __restrict__ invMass, int N,
                                                                     double cf0, double cf1, double cf2,
                                                                     double* partials, unsigned int* ticket,
@@ -274,8 +274,8 @@ void device_kinetic_pending(System& s, double CF) {
 // 2KE per dimension of P + CF F and of P + CF F + CF F (two kicks in sequence, as
 // k_step_fused applies them), P unchanged: 4 fused multiply-adds per component.
 template <bool UNITM>
-__global__ void __launch_bounds__(MOTION_THREADS) k_kinetic_two(const double* __restrict__ P,
-                                                                const double* __restrict__ F,
+__global__ void __launch_bounds__(MOTION_THREADS) k_kinetic_two(const double* P,
+                                                                const double* F,
                                                                 const double* __restrict__ invMass, int N, double cf,
                                                                 double* partials, unsigned int* ticket, double* result,
                                                                 double* hostResult, const double* skip) {
@@ -305,8 +305,8 @@ __global__ void __launch_bounds__(MOTION_THREADS) k_kinetic_two(const double* __
 // exact FP32 values (the mixed-precision pair forces), in float-float arithmetic
 // (ffkick.cuh); the sums agree with the FP64 ones to ~1e-14 (relative).
 constexpr int KE_FF_LOADS = 4;
-__global__ void __launch_bounds__(MOTION_THREADS) k_kinetic_two_ff(const double* __restrict__ P,
-                                                                   const double* __restrict__ F, int N, float cfh,
+__global__ void __launch_bounds__(MOTION_THREADS) k_kinetic_two_ff(const double* P,
+                                                                   const double* F, int N, float cfh,
                                                                    float cfl, float2* partials, unsigned int* ticket,
                                                                    double* result, double* hostResult,
                                                                    const double* skip) {

@@ -77,11 +77,11 @@ __device__ __forceinline__ float4 pack_delta(float4 p0, double dx, double dy, do
 // PACK: also the FP32 positions of k_pack_delta, from the displacements at hand (one pass
 // over R and R0 less: 4096 rigid waters, 5 steps, 783 -> 779 us).
 template <bool PACK>
-__global__ void __launch_bounds__(SKIN_THREADS) k_skin(const double* __restrict__ R, const double* __restrict__ R0,
+__global__ void __launch_bounds__(SKIN_THREADS) k_skin(const double* R, const double* R0,
                                                        int N, int chunks, double skinSq, longlong2* partial,
                                                        unsigned int* ticket, double* result, double* hostResult,
-                                                       const int* __restrict__ slotOf,
-                                                       const float4* __restrict__ pos0, float scale,
+                                                       const int* slotOf,
+                                                       const float4* pos0, float scale,
                                                        float4* __restrict__ pos4, unsigned long long* done,
                                                        unsigned int stamp) {
   chain_wait();
@@ -202,7 +202,7 @@ __device__ __forceinline__ float charge_f32(double q) {
 // build reads u instead of recomputing it.  A cell index that differs from the
 // reference's int(M (R/L - floor(R/L))) by rounding at a cell boundary changes
 // only the order of candidates, not the pair set.
-__global__ void k_assign(const double* __restrict__ R, const double* __restrict__ charge, int N, double scale,
+__global__ void k_assign(const double* R, const double* __restrict__ charge, int N, double scale,
                          TileGeom g, int4* atomK, int* count, int* inCell, float4* pos0, double* __restrict__ R0,
                          int* dMax, unsigned long long* fail) {
   chain_wait();
@@ -290,7 +290,7 @@ __global__ void k_scatter(const int4* atomK, int N, const int* start, const int*
 // so the build's staged positions are sorted along x within every cell and hence
 // along every stencil row), ties by ascending atom index.  Deterministic for
 // given coordinates.
-__global__ void k_sort_cells(const int* start, int nRanks, int* orig, const float4* __restrict__ pos0, float* key) {
+__global__ void k_sort_cells(const int* start, int nRanks, int* orig, const float4* pos0, float* key) {
   chain_wait();
   int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= nRanks) return;
@@ -312,7 +312,7 @@ __global__ void k_sort_cells(const int* start, int nRanks, int* orig, const floa
 // The same order for dense cells: one warp per cell; each atom's place is the
 // number of atoms of the cell that precede it in (x key, atom index) order.
 // Cells of more than 32 atoms are sorted by lane 0 as above.
-__global__ void k_sort_cells_warp(const int* start, int nRanks, int* orig, const float4* __restrict__ pos0) {
+__global__ void k_sort_cells_warp(const int* start, int nRanks, int* orig, const float4* pos0) {
   chain_wait();
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= nRanks) return;
@@ -350,7 +350,7 @@ __global__ void k_sort_cells_warp(const int* start, int nRanks, int* orig, const
 // per slot: image cell, type, slot of the atom, and the FP32 position and charge
 // (pos0 of k_assign)
 __global__ void k_fill_slots(const int* orig, int N, const int4* atomK, const int* type, int4* K, uint8_t* type8,
-                             int* slotOf, const float4* __restrict__ pos0, float4* pos4) {
+                             int* slotOf, const float4* pos0, float4* pos4) {
   chain_wait();
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= N) return;
@@ -395,7 +395,7 @@ __global__ void k_tile_info(const int* start, TileGeom g, int* info, int* maxOut
 
 // cell-local position of each slot in units of the cell edge, u = M R/L - K, and
 // the charge, from the coordinates (after a change of the box since the build)
-__global__ void k_pack_mixed(const double* __restrict__ R, const double* __restrict__ charge, const int* orig,
+__global__ void k_pack_mixed(const double* R, const double* __restrict__ charge, const int* orig,
                              const int4* K, int N, double scale, float4* pos4) {
   chain_wait();
   int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -417,8 +417,8 @@ __device__ __forceinline__ float4 pack_delta(float4 p0, double dx, double dy, do
   return make_float4(fmaf(d2f(dx), scale, p0.x), fmaf(d2f(dy), scale, p0.y), fmaf(d2f(dz), scale, p0.z), p0.w);
 }
 
-__global__ void k_pack_delta(const double* __restrict__ R, const double* __restrict__ R0, const int* orig,
-                             const float4* __restrict__ pos0, int N, float scale, float4* pos4) {
+__global__ void k_pack_delta(const double* R, const double* R0, const int* orig,
+                             const float4* pos0, int N, float scale, float4* pos4) {
   chain_wait();
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= N) return;
@@ -429,7 +429,7 @@ __global__ void k_pack_delta(const double* __restrict__ R, const double* __restr
 
 // scaled FP64 coordinates Rs = R/L (src/EmDeeCode.f90:1228) in slot order, and their box
 // fractions (the FP64 mode has no FP32 positions between builds: they take that array)
-__global__ void k_pack_fp64(const double* __restrict__ R, const int* orig, int N, double L, double* Rs, int4* frac) {
+__global__ void k_pack_fp64(const double* R, const int* orig, int N, double L, double* Rs, int4* frac) {
   chain_wait();
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= N) return;
@@ -1677,12 +1677,12 @@ static const int STEP_CHUNKS = 2;   // at most 64 consecutive atoms per warp (sk
 // start values in s0 if it is set; each statement as in k_vv_pre_free.
 template <int NK, bool UNITM, bool PACK, bool FMA, bool VV>
 __global__ void __launch_bounds__(SKIN_THREADS) k_step_fused(double* __restrict__ R, double* __restrict__ P,
-                                                             const double* __restrict__ F,
+                                                             const double* F,
                                                              const double* __restrict__ invMass,
-                                                             const double* __restrict__ R0, int N, int chunks, double cf0,
+                                                             const double* R0, int N, int chunks, double cf0,
                                                              double cf1, double CP, double skinSq,
-                                                             const int* __restrict__ slotOf,
-                                                             const float4* __restrict__ pos0, float scale,
+                                                             const int* slotOf,
+                                                             const float4* pos0, float scale,
                                                              float4* __restrict__ pos4, longlong2* partial,
                                                              unsigned int* ticket, double* result,
                                                              double* hostResult, double* __restrict__ s0,

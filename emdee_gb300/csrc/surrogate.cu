@@ -430,7 +430,7 @@ struct NeighborBuffer {
 };
 
 template <class F>
-__device__ __forceinline__ void for_neighbors(const float4* __restrict__ pos, const Geometry& G, int q, const int* list,
+__device__ __forceinline__ void for_neighbors(const float4* pos, const Geometry& G, int q, const int* list,
                                               int n, NeighborBuffer& B, F&& batch) {
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -475,7 +475,7 @@ __device__ __forceinline__ void for_neighbors(const float4* __restrict__ pos, co
 
 // batch(n, d, j) over the neighbors k_sg_desc left in `near`, 32 at a time
 template <class F>
-__device__ __forceinline__ void each_neighbor(const float4* __restrict__ pos, const Geometry& G, int q, const int* near,
+__device__ __forceinline__ void each_neighbor(const float4* pos, const Geometry& G, int q, const int* near,
                                               int n, F&& batch) {
   const int lane = threadIdx.x & 31;
   const float4 pi = pos[q];
@@ -501,10 +501,10 @@ __device__ __forceinline__ PairGeom unit_vector(const float4& d) {
 constexpr int HROW = NG + 1;
 
 // 8 x 8000 atoms: 195 us with one thread per atom, 92 us so.
-__global__ void __launch_bounds__(32 * WARP_ATOMS) k_sg_desc(const float4* __restrict__ pos, Geometry G,
+__global__ void __launch_bounds__(32 * WARP_ATOMS) k_sg_desc(const float4* pos, Geometry G,
                                                              const uint8_t* __restrict__ species,
-                                                             const int* __restrict__ list,
-                                                             const int* __restrict__ count, int cap,
+                                                             const int* list,
+                                                             const int* count, int cap,
                                                              float* __restrict__ Gout, int* __restrict__ near,
                                                              int* __restrict__ nearCount) {
   chain_wait();
@@ -546,11 +546,11 @@ __global__ void __launch_bounds__(32 * WARP_ATOMS) k_sg_desc(const float4* __res
 // lines per load instead of 32), and three of them add one force component each.
 // 8 x 8000 atoms: 293 us with one thread per atom, 116 us so.
 constexpr int DROW = NG + 4;   // rows of 16 + 4 floats: 16-byte aligned, in different banks
-__global__ void __launch_bounds__(32 * WARP_ATOMS, 4) k_sg_force(const float4* __restrict__ pos, Geometry G,
+__global__ void __launch_bounds__(32 * WARP_ATOMS, 4) k_sg_force(const float4* pos, Geometry G,
                                                               const uint8_t* __restrict__ species,
-                                                              const int* __restrict__ near,
-                                                              const int* __restrict__ nearCount, int cap,
-                                                              const float* __restrict__ dEdG,
+                                                              const int* near,
+                                                              const int* nearCount, int cap,
+                                                              const float* dEdG,
                                                               double* __restrict__ F) {
   chain_wait();
   // per neighbor: dh[16], r_hat[3], index
@@ -562,7 +562,7 @@ __global__ void __launch_bounds__(32 * WARP_ATOMS, 4) k_sg_force(const float4* _
   const int part = lane & 3, comp = part < 3 ? part : 0;
   float* D = dbuf[warp];
   const float4* own = reinterpret_cast<const float4*>(dEdG + (size_t)q * DIN) + part;
-  const float4 own0 = __ldg(&own[0]), own1 = __ldg(&own[NG / 4]);   // this lane's Gaussians of both species
+  const float4 own0 = own[0], own1 = own[NG / 4];   // this lane's Gaussians of both species
   float f = 0.f;
   each_neighbor(pos, G, q, near + (size_t)q * cap, nearCount[q], [&](int n, float4 d, int j) {
     {
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(32 * WARP_ATOMS, 4) k_sg_force(const float4* _
       const float* row = D + nb * DROW;
       const int code = __float_as_int(row[NG + 3]), jj = code & 0x7FFFFFFF;
       const float4 x = code < 0 ? own1 : own0, dh = *reinterpret_cast<const float4*>(row + 4 * part);
-      const float4 y = __ldg(reinterpret_cast<const float4*>(dEdG + (size_t)jj * DIN + si * NG) + part);
+      const float4 y = reinterpret_cast<const float4*>(dEdG + (size_t)jj * DIN + si * NG)[part];
       float s = (x.x + y.x) * dh.x + (x.y + y.y) * dh.y + (x.z + y.z) * dh.z + (x.w + y.w) * dh.w;
       s += __shfl_xor_sync(0xffffffffu, s, 1);
       s += __shfl_xor_sync(0xffffffffu, s, 2);
@@ -596,11 +596,11 @@ __global__ void __launch_bounds__(32 * WARP_ATOMS, 4) k_sg_force(const float4* _
 
 // u_i[s_j, k] = sum_j dh_k(r_ij) (v_i - v_j) . r_hat_ij (force residual in descriptor space).
 // 8 x 8000 atoms: 248 us with one thread per atom, 93 us so.
-__global__ void __launch_bounds__(32 * WARP_ATOMS, 4) k_sg_udesc(const float4* __restrict__ pos, Geometry G,
+__global__ void __launch_bounds__(32 * WARP_ATOMS, 4) k_sg_udesc(const float4* pos, Geometry G,
                                                               const uint8_t* __restrict__ species,
-                                                              const int* __restrict__ near,
-                                                              const int* __restrict__ nearCount, int cap,
-                                                              const float4* __restrict__ v, float* __restrict__ U) {
+                                                              const int* near,
+                                                              const int* nearCount, int cap,
+                                                              const float4* v, float* __restrict__ U) {
   chain_wait();
   __shared__ float hbuf[WARP_ATOMS][32 * HROW];
   __shared__ float wbuf[WARP_ATOMS][32];
@@ -895,8 +895,8 @@ __device__ void tc_load_weights(TcWeights& w, const float* p) {
   if (threadIdx.x == 0) w.b3 = p[OFF_B3];
 }
 
-__global__ void __launch_bounds__(TC_THREADS, 2) k_sg_mlp_tc(TileArgs T, const float* __restrict__ params,
-                                                             const float* __restrict__ Gin,
+__global__ void __launch_bounds__(TC_THREADS, 2) k_sg_mlp_tc(TileArgs T, const float* params,
+                                                             const float* Gin,
                                                              float* __restrict__ Eatom, float* __restrict__ dEdG,
                                                              int* __restrict__ err) {
   chain_wait();
@@ -1063,9 +1063,9 @@ __device__ __forceinline__ void column_sums(float (&x)[8][2], float* out) {
 // shuffles per warp (shared-memory atomics, eight lanes to an address, were most of
 // 2 x 419 us at 8 x 8000 atoms; 173 us so); the weight GEMMs take their operands
 // transposed by ldmatrix, so that two blocks fit an SM (91 us).
-__global__ void __launch_bounds__(128) k_sg_train(TileArgs T, int nt0, int nb0, const float* __restrict__ params,
-                                                  const float* __restrict__ Gin, const float* __restrict__ Uin,
-                                                  const float* __restrict__ eAtom, float* __restrict__ part) {
+__global__ void __launch_bounds__(128) k_sg_train(TileArgs T, int nt0, int nb0, const float* params,
+                                                  const float* Gin, const float* Uin,
+                                                  const float* eAtom, float* __restrict__ part) {
   chain_wait();
   extern __shared__ __align__(16) unsigned char raw[];
   TrainSmem& S = *reinterpret_cast<TrainSmem*>(raw);
@@ -1276,7 +1276,7 @@ __global__ void k_sg_chain_sum(const float* __restrict__ x, int N, double* __res
 // half, BEGIN begins the next with a kick of half, the drift over dt and the FP32
 // positions of k_sg_pack.  One pass per step instead of three.
 template <bool END, bool BEGIN>
-__global__ void k_sg_advance(double* __restrict__ R, double* __restrict__ P, const double* __restrict__ F, int n3,
+__global__ void k_sg_advance(double* __restrict__ R, double* __restrict__ P, const double* F, int n3,
                              double half, double dt, double L, float* __restrict__ pos) {
   chain_wait();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;

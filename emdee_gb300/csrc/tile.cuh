@@ -102,7 +102,7 @@ inline float box_limit(double r2) { return (float)(r2 * 18446744073709551616.0 *
 // entries differ in place but hardly in number, run f together.  lp: the atom's first
 // chunk, chunk c at lp[c * stride].
 template <class Keep, class F>
-__device__ __forceinline__ void masked_entries(const uint4* __restrict__ lp, int stride, int n, Keep&& keep, F&& f) {
+__device__ __forceinline__ void masked_entries(const uint4* lp, int stride, int n, Keep&& keep, F&& f) {
   for (int k0 = 0; k0 < n; k0 += 128) {
     unsigned m[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
@@ -277,7 +277,7 @@ __device__ __forceinline__ void stage_marked(const TileGeom& g, int n, const flo
 // Stages the halo of tile t from the layout saved by the list build (global
 // memory: off[0..haloCells], then cst[0..haloCells-1]); returns the halo size.
 // Ends without a barrier.
-__device__ __forceinline__ int stage_frame_saved(const TileGeom& g, const int* __restrict__ lay, const float4* pos4,
+__device__ __forceinline__ int stage_frame_saved(const TileGeom& g, const int* lay, const float4* pos4,
                                                  float4* hpos, uint8_t* htype, const uint8_t* type8) {
   for (int h = threadIdx.x; h < g.haloCells; h += blockDim.x)
     mark_halo_cell(hpos, h, lay[h], lay[h + 1], lay[g.haloCells + 1 + h]);
@@ -289,7 +289,7 @@ __device__ __forceinline__ int stage_frame_saved(const TileGeom& g, const int* _
 
 // Slot of halo index q of the tile whose saved layout is lay: its halo cell is the
 // last one that starts at or before q.
-__device__ __forceinline__ int saved_slot(const TileGeom& g, const int* __restrict__ lay, int q) {
+__device__ __forceinline__ int saved_slot(const TileGeom& g, const int* lay, int q) {
   int lo = 0, hi = g.haloCells - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;

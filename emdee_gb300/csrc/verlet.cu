@@ -23,7 +23,7 @@ static const int VV_THREADS = 128;
 // list == nullptr: atoms 0..n-1; otherwise the atoms list[0..n-1]
 template <bool COMPUTE, bool FMA>
 __global__ void __launch_bounds__(VV_THREADS) k_vv_pre_free(double* __restrict__ R, double* __restrict__ P,
-                                                            const double* __restrict__ F,
+                                                            const double* F,
                                                             const double* __restrict__ invMass, const int* list,
                                                             int n, double dt, double dt_2, double* __restrict__ s0) {
   chain_wait();
@@ -43,11 +43,11 @@ __global__ void __launch_bounds__(VV_THREADS) k_vv_pre_free(double* __restrict__
 
 // v[0..2] 2KE_t per dimension, v[3] Ks_t, v[4] Us
 template <bool COMPUTE, bool FMA>
-__global__ void __launch_bounds__(VV_THREADS) k_vv_post_free(const double* __restrict__ R, double* __restrict__ P,
-                                                             const double* __restrict__ F,
+__global__ void __launch_bounds__(VV_THREADS) k_vv_post_free(const double* R, double* __restrict__ P,
+                                                             const double* F,
                                                              const double* __restrict__ invMass, const int* list,
                                                              int n, double dt, double dt_2,
-                                                             const double* __restrict__ s0, double* partials,
+                                                             const double* s0, double* partials,
                                                              unsigned int* ticket, double* result, double* hostResult,
                                                              const double* skip) {
   chain_wait();
@@ -109,7 +109,7 @@ __device__ __forceinline__ void vv_virtual_rotation(const BodyState& b, double d
 }
 
 template <bool COMPUTE>
-__global__ void __launch_bounds__(VV_THREADS) k_vv_pre_body(BodyArgs A, const double* __restrict__ F,
+__global__ void __launch_bounds__(VV_THREADS) k_vv_pre_body(BodyArgs A, const double* F,
                                                             double* __restrict__ R, double dt, double dt_2, int mode,
                                                             double* __restrict__ r0, double* __restrict__ q0) {
   chain_wait();
@@ -135,9 +135,9 @@ __global__ void __launch_bounds__(VV_THREADS) k_vv_pre_body(BodyArgs A, const do
 
 // v[0..2] 2KE_t, v[3..5] 2KE_r, v[6] Ks_t, v[7] Ks_r, v[8] Us
 template <bool COMPUTE>
-__global__ void __launch_bounds__(VV_THREADS) k_vv_post_body(BodyArgs A, const double* __restrict__ F, double dt,
-                                                             double dt_2, int mode, const double* __restrict__ r0,
-                                                             const double* __restrict__ q0, double* partials,
+__global__ void __launch_bounds__(VV_THREADS) k_vv_post_body(BodyArgs A, const double* F, double dt,
+                                                             double dt_2, int mode, const double* r0,
+                                                             const double* q0, double* partials,
                                                              unsigned int* ticket, double* result, double* hostResult) {
   chain_wait();
   double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
