@@ -454,8 +454,10 @@ __global__ void __launch_bounds__(THREADS) k_replicas(const RepDesc* __restrict_
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = THREADS / 32;
   int done = (int)D.out[7];
   // Lists as the system's were built, from the positions of the last build (R0): those of
-  // an earlier run serve if they were made from the same positions, bit for bit.
+  // an earlier run serve if they were made from the same positions, bit for bit, and had
+  // room (lists that outgrew it are built again, which reports them in this launch's out).
   bool same = true;
+  for (int i = threadIdx.x; i < D.N; i += THREADS) same = same && D.count[i] <= D.cap;
   for (int q = threadIdx.x; q < 3 * D.N; q += THREADS)
     same = same && __double_as_longlong(D.Rb[q]) == __double_as_longlong(D.R0[q]);
   if (!__syncthreads_and(same)) rep_build<THREADS>(S, D.R0, (float4*)pos, cellStart, cursor, false);
