@@ -292,9 +292,9 @@ __device__ __forceinline__ void rep_pairs(const RepDesc& D, const int4* pos, con
   const float rc2 = D.rc2, unit2 = D.unit2, unit = D.unit;
   const float sigc = mdl.sigsq * unit2, eps48 = 2.0f * mdl.eps24;
   const int cap = D.cap;
-  const uint4* __restrict__ list = D.list;
-  const int* __restrict__ count = D.count;
-  const int* __restrict__ orig = D.orig;
+  const uint4* list = D.list;   // rebuilt by this kernel: plain loads
+  const int* count = D.count;
+  const int* orig = D.orig;
   double* __restrict__ F = D.F;
   const int sub = TPA == 1 ? 0 : (int)(threadIdx.x & (TPA - 1));
   const unsigned pmask = TPA == 1 ? 0xffffffffu : (3u << ((threadIdx.x & 31) & ~1u));
@@ -305,9 +305,9 @@ __device__ __forceinline__ void rep_pairs(const RepDesc& D, const int4* pos, con
     float fx = 0.f, fy = 0.f, fz = 0.f;
     const int nch = (n + 7) >> 3;
     // 8 entries per 16-byte load, the next chunk requested before this one is used
-    uint4 cur = sub < nch ? __ldg(&list[(size_t)sub * N + i]) : make_uint4(0u, 0u, 0u, 0u);
+    uint4 cur = sub < nch ? list[(size_t)sub * N + i] : make_uint4(0u, 0u, 0u, 0u);
     for (int c = sub; c < nch; c += TPA) {
-      const uint4 nxt = c + TPA < nch ? __ldg(&list[(size_t)(c + TPA) * N + i]) : cur;
+      const uint4 nxt = c + TPA < nch ? list[(size_t)(c + TPA) * N + i] : cur;
       const unsigned words[4] = {cur.x, cur.y, cur.z, cur.w};
       const int left = n - 8 * c;   // entries of this chunk, if fewer than 8
 #pragma unroll

@@ -35,3 +35,8 @@ def test_inputs_are_plain(file, name, params, body):
     readonly = set(re.findall(r"const \w+\* __restrict__ (\w+)", params)) - CONSTANT
     assert not readonly, (file, name, readonly)
     assert "__ldg" not in body, (file, name)
+
+
+def test_replica_lists_are_plain():
+    """k_replicas rebuilds its lists between its own reads of them"""
+    assert "__ldg" not in open(os.path.join(CSRC, "replicas.cu")).read()
