@@ -239,20 +239,21 @@ __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_move_series(BodyArg
     return;
   }
   if (wide) {
-    steps = 1;
+    steps = 0;
     while (theta2 > (BODY_STEP_WIDE * steps) * (BODY_STEP_WIDE * steps)) steps++;
   }
   const int c = g.c, k = c < 3 ? c : 0, first = B.first, NP = B.NP;
   double q[4] = {B.q[0], B.q[1], B.q[2], B.q[3]};
   double rcm = B.rcm[k];
   if (translate) rcm = CR * rcm + CP * B.invMass * B.pcm[k];
-  const double h = steps == 1 ? dt : dt / steps, back = steps == 1 ? invdt : steps * invdt;
+  const double h = steps == 0 ? 1.0 : steps == 1 ? dt : dt / steps,
+               back = steps == 0 ? 1.0 : steps == 1 ? invdt : steps * invdt;
   const double kap = k == 0 ? (MoI[1] - MoI[2]) * invMoI[0]
                             : k == 1 ? (MoI[2] - MoI[0]) * invMoI[1] : (MoI[0] - MoI[1]) * invMoI[2];
   double w[3] = {h * omega[0], h * omega[1], h * omega[2]};
   if (wide)
     for (int n = 0; n < steps; n++) body_series_step<BODY_ORDER_WIDE>(g, kap, w, q);
-  else
+  else if (steps > 0)
     body_series_step<RB_SERIES_ORDER>(g, kap, w, q);
   const double n2 = q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3], f = 1.5 - 0.5 * n2;
   double v[3];

@@ -287,14 +287,15 @@ RB_HD void rb_series_step(const double (&kap)[3], double (&w)[3], double (&q)[4]
   }
 }
 
-// Steps of the series for theta2 = 2K dt^2 / I3; false for more than RB_SERIES_MAX, for
-// degenerate moments and for bodies that turn about their first axis only (perp: the
-// square of the other components of I w), which the closed form handles apart.
+// Steps of the series for theta2 = 2K dt^2 / I3, none for no turn (dt = 0: q and w stay, and
+// there is no dt to divide w dt by); false for more than RB_SERIES_MAX, for degenerate
+// moments and for bodies that turn about their first axis only (perp: the square of the
+// other components of I w), which the closed form handles apart.
 RB_HD bool rb_series_steps(double theta2, double I3, double perp, int& steps) {
   const double most = RB_SERIES_STEP * RB_SERIES_MAX;
   if (!(theta2 <= most * most) || !(I3 > 0.0)) return false;   // NaN: the closed form
   if (perp < 2.220446049250313e-16) return false;
-  steps = 1;
+  steps = 0;
   while (steps < RB_SERIES_MAX && theta2 > (RB_SERIES_STEP * steps) * (RB_SERIES_STEP * steps)) steps++;
   return true;
 }
@@ -308,7 +309,8 @@ RB_HD bool rb_rotate_series(BodyState& b, double dt, const double* d, double* de
   }
   int steps;
   if (!rb_series_steps(TwoKr * b.invMoI[2] * (dt * dt), b.MoI[2], Iw[1] * Iw[1] + Iw[2] * Iw[2], steps)) return false;
-  const double h = steps == 1 ? dt : dt / steps, back = steps == 1 ? 1.0 / dt : steps / dt;
+  const double h = steps == 0 ? 1.0 : steps == 1 ? dt : dt / steps,
+               back = steps == 0 ? 1.0 : steps == 1 ? 1.0 / dt : steps / dt;
   const double kap[3] = {(b.MoI[1] - b.MoI[2]) * b.invMoI[0], (b.MoI[2] - b.MoI[0]) * b.invMoI[1],
                          (b.MoI[0] - b.MoI[1]) * b.invMoI[2]};
   double w[3] = {h * b.omega[0], h * b.omega[1], h * b.omega[2]};
