@@ -19,6 +19,7 @@
 namespace emdee {
 
 static const int PAIR64_THREADS = 128;
+static const int PAIR64_STATIC = 512;   // the kernel's static shared memory at most (the sums of grid_reduce)
 
 struct __align__(32) D4 {
   double x, y, z, w;
@@ -59,7 +60,11 @@ struct PairArgsD {
 // fractions now picks those that can lie within it (masked_entries).  32,003 atoms,
 // force-shifted: 650 -> 450 us
 // (FP64 lanes 52 -> 66 % in use; tiles of 62 atoms in warps of 32 leave the rest).
-template <bool COMPUTE, int MOD>
+// STAGED: the fractions are staged beside the coordinates.  A halo that does not fit so in
+// shared memory (beyond 4732 atoms) goes without them: every entry gets the FP64 distance
+// (9000 atoms, 5300 in a halo, one type: 6.52 ms, masked by fractions made from the staged
+// coordinates on the way 8.49; 5500 in one halo 3.38 and 4.46 ms).
+template <bool COMPUTE, int MOD, bool STAGED>
 __global__ void __launch_bounds__(PAIR64_THREADS) k_pair_fp64(PairArgsD A) {
   chain_wait();
   extern __shared__ __align__(32) unsigned char sraw[];
@@ -67,7 +72,7 @@ __global__ void __launch_bounds__(PAIR64_THREADS) k_pair_fp64(PairArgsD A) {
   const int t = blockIdx.x, cells = g.TB * g.TB * g.TB;
   D4* hpos = (D4*)sraw;   // Rs.xyz, charge
   int4* hfrac = (int4*)(hpos + A.haloCap + 1);
-  uint8_t* htype = (uint8_t*)(hfrac + A.haloCap + 1);
+  uint8_t* htype = (uint8_t*)(hfrac + (STAGED ? A.haloCap + 1 : 0));
   // from the layout saved by the list build: every halo index's slot first (in the
   // position it will hold), then the atoms, one thread each
   const int* lay = A.layout + (size_t)t * (2 * g.haloCells + 1);
@@ -81,7 +86,7 @@ __global__ void __launch_bounds__(PAIR64_THREADS) k_pair_fp64(PairArgsD A) {
   for (int q = threadIdx.x; q < halo; q += blockDim.x) {
     const int sj = mark[q * (sizeof(D4) / sizeof(int))];
     hpos[q] = D4{A.Rs[3 * sj], A.Rs[3 * sj + 1], A.Rs[3 * sj + 2], MOD < 0 ? A.charge[A.orig[sj]] : 0.0};
-    hfrac[q] = A.frac[sj];
+    if (STAGED) hfrac[q] = A.frac[sj];
     if (MOD < 0) htype[q] = A.type8[sj];
   }
   __syncthreads();
@@ -104,37 +109,41 @@ __global__ void __launch_bounds__(PAIR64_THREADS) k_pair_fp64(PairArgsD A) {
     const int n = min(A.count[si], A.cap);
     const uint4* lp = reinterpret_cast<const uint4*>(A.nb) + ((size_t)t * capC * A.tileStride + li);
     double Fi[3] = {0.0, 0.0, 0.0};
-    const int4 fi = hfrac[qi];
-    masked_entries(
-        lp, A.tileStride, n, [&](int qj) { return box_dist2(fi, hfrac[qj]) < A.limit; },
-        [&](int qj) {
-          const D4 pj = hpos[qj];
-          const double Rij[3] = {wrap_half(pi.x - pj.x), wrap_half(pi.y - pj.y), wrap_half(pi.z - pj.z)};
-          const double r2 = Rij[0] * Rij[0] + Rij[1] * Rij[1] + Rij[2] * Rij[2];
-          if (!(r2 < A.Rc2)) return;
-          within++;
-          const double invR2 = A.invL2 / r2;
-          const double invR = sqrt(invR2);   // dropped where the models do not use it
-          double Wsum;
-          if (MOD >= 0) {
-            double E = 0.0;
-            if (COMPUTE) {
-              nb_compute(lj, E, Wsum, invR, invR2);
-              modifier_compute(lj, E, Wsum, invR, invR2);
-              Ep += E;
-            } else {
-              Wsum = nb_virial(lj, invR, invR2);
-              modifier_virial(lj, Wsum, invR, invR2);
-            }
-            Wp += Wsum;
-          } else {
-            const PairEntry<double>& pe = A.table[ti * A.ntypes + htype[qj]];
-            const bool ijch = ich && fabs(pj.w) > 2.220446049250313e-16;
-            Wsum = pair_eval<double, COMPUTE>(pe, coul, ijch, pi.w, pj.w, invR, invR2, Ep, Ec, Wp, Wc);
-          }
-          const double s = Wsum * invR2;
-          for (int d = 0; d < 3; d++) Fi[d] += s * Rij[d];
-        });
+    auto pair = [&](int qj) {
+      const D4 pj = hpos[qj];
+      const double Rij[3] = {wrap_half(pi.x - pj.x), wrap_half(pi.y - pj.y), wrap_half(pi.z - pj.z)};
+      const double r2 = Rij[0] * Rij[0] + Rij[1] * Rij[1] + Rij[2] * Rij[2];
+      if (!(r2 < A.Rc2)) return;
+      within++;
+      const double invR2 = A.invL2 / r2;
+      const double invR = sqrt(invR2);   // dropped where the models do not use it
+      double Wsum;
+      if (MOD >= 0) {
+        double E = 0.0;
+        if (COMPUTE) {
+          nb_compute(lj, E, Wsum, invR, invR2);
+          modifier_compute(lj, E, Wsum, invR, invR2);
+          Ep += E;
+        } else {
+          Wsum = nb_virial(lj, invR, invR2);
+          modifier_virial(lj, Wsum, invR, invR2);
+        }
+        Wp += Wsum;
+      } else {
+        const PairEntry<double>& pe = A.table[ti * A.ntypes + htype[qj]];
+        const bool ijch = ich && fabs(pj.w) > 2.220446049250313e-16;
+        Wsum = pair_eval<double, COMPUTE>(pe, coul, ijch, pi.w, pj.w, invR, invR2, Ep, Ec, Wp, Wc);
+      }
+      const double s = Wsum * invR2;
+      for (int d = 0; d < 3; d++) Fi[d] += s * Rij[d];
+    };
+    if (STAGED) {
+      const int4 fi = hfrac[qi];
+      masked_entries(lp, A.tileStride, n, [&](int qj) { return box_dist2(fi, hfrac[qj]) < A.limit; }, pair);
+    } else {
+      const uint16_t* entry = reinterpret_cast<const uint16_t*>(lp);
+      for (int k = 0; k < n; k++) pair(entry[(size_t)(k >> 3) * A.tileStride * 8 + (k & 7)]);
+    }
     double* Fa = A.F + 3 * (size_t)A.orig[si];
     for (int d = 0; d < 3; d++) Fa[d] = A.L * Fi[d];
   }
@@ -142,24 +151,25 @@ __global__ void __launch_bounds__(PAIR64_THREADS) k_pair_fp64(PairArgsD A) {
   grid_reduce<5, PAIR64_THREADS>(v, A.partials, A.ticket, A.result, A.hostResult);
 }
 
-template <bool COMPUTE, int MOD>
+template <bool COMPUTE, bool STAGED, int MOD>
 static void launch_fp64(System& s, const PairArgsD& A, size_t smem, int nTiles, int threads) {
-  CK(cudaFuncSetAttribute(k_pair_fp64<COMPUTE, MOD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  if (chain_fits(nTiles)) launch_chained(k_pair_fp64<COMPUTE, MOD>, nTiles, threads, smem, s.stream, A);
-  else k_pair_fp64<COMPUTE, MOD><<<nTiles, threads, smem, s.stream>>>(A);
+  auto kern = k_pair_fp64<COMPUTE, MOD, STAGED>;
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (chain_fits(nTiles)) launch_chained(kern, nTiles, threads, smem, s.stream, A);
+  else kern<<<nTiles, threads, smem, s.stream>>>(A);
 }
 
-template <bool COMPUTE>
+template <bool COMPUTE, bool STAGED>
 static void launch_fp64_mod(System& s, const PairArgsD& A, size_t smem, int nt, int th, int mod) {
   switch (mod) {
-    case NONE: launch_fp64<COMPUTE, NONE>(s, A, smem, nt, th); break;
-    case SHIFTED: launch_fp64<COMPUTE, SHIFTED>(s, A, smem, nt, th); break;
-    case SHIFTED_FORCE: launch_fp64<COMPUTE, SHIFTED_FORCE>(s, A, smem, nt, th); break;
-    case SMOOTHED: launch_fp64<COMPUTE, SMOOTHED>(s, A, smem, nt, th); break;
-    case SHIFTED_SMOOTHED: launch_fp64<COMPUTE, SHIFTED_SMOOTHED>(s, A, smem, nt, th); break;
-    case SQUARE_SMOOTHED: launch_fp64<COMPUTE, SQUARE_SMOOTHED>(s, A, smem, nt, th); break;
-    case SHIFTED_SQUARE_SMOOTHED: launch_fp64<COMPUTE, SHIFTED_SQUARE_SMOOTHED>(s, A, smem, nt, th); break;
-    default: launch_fp64<COMPUTE, -1>(s, A, smem, nt, th); break;
+    case NONE: launch_fp64<COMPUTE, STAGED, NONE>(s, A, smem, nt, th); break;
+    case SHIFTED: launch_fp64<COMPUTE, STAGED, SHIFTED>(s, A, smem, nt, th); break;
+    case SHIFTED_FORCE: launch_fp64<COMPUTE, STAGED, SHIFTED_FORCE>(s, A, smem, nt, th); break;
+    case SMOOTHED: launch_fp64<COMPUTE, STAGED, SMOOTHED>(s, A, smem, nt, th); break;
+    case SHIFTED_SMOOTHED: launch_fp64<COMPUTE, STAGED, SHIFTED_SMOOTHED>(s, A, smem, nt, th); break;
+    case SQUARE_SMOOTHED: launch_fp64<COMPUTE, STAGED, SQUARE_SMOOTHED>(s, A, smem, nt, th); break;
+    case SHIFTED_SQUARE_SMOOTHED: launch_fp64<COMPUTE, STAGED, SHIFTED_SQUARE_SMOOTHED>(s, A, smem, nt, th); break;
+    default: launch_fp64<COMPUTE, STAGED, -1>(s, A, smem, nt, th); break;
   }
 }
 
@@ -194,12 +204,16 @@ void device_pair_forces_fp64(System& s, bool compute, bool useInRc, double rc2sc
   A.layout = g.dLayout;
   A.frac = (const int4*)g.dPos4;
   A.limit = box_limit(A.Rc2);
-  const size_t smem = (size_t)(g.maxHalo + 1) * (sizeof(D4) + sizeof(int4) + 1) + 16;
+  const size_t atom = sizeof(D4) + 1, halo = g.maxHalo + 1, limit = 227 * 1024 - PAIR64_STATIC;
+  const bool staged = halo * (atom + sizeof(int4)) + 16 <= limit;
+  const size_t smem = halo * (staged ? atom + sizeof(int4) : atom) + 16;
+  if (smem > limit) fatal("pair forces", "too many atoms around a cell for FP64 arithmetic");
   const int mod = pair_lj_only(s) ? s.P(0, 0, s.layer - 1).model.p.modifier : -1;
   // as many threads as the largest tile has atoms, in whole warps, up to PAIR64_THREADS
   const int th = std::min(PAIR64_THREADS, (g.tileAtoms + 31) / 32 * 32);
-  if (compute) launch_fp64_mod<true>(s, A, smem, g.nTiles, th, mod);
-  else launch_fp64_mod<false>(s, A, smem, g.nTiles, th, mod);
+  auto run = staged ? (compute ? launch_fp64_mod<true, true> : launch_fp64_mod<false, true>)
+                    : (compute ? launch_fp64_mod<true, false> : launch_fp64_mod<false, false>);
+  run(s, A, smem, g.nTiles, th, mod);
   CK(cudaGetLastError());
 }
 
