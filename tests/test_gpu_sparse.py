@@ -1,0 +1,55 @@
+"""Two droplets in boxes far larger than they are, where nearly all of up to 24 million cells
+are empty: grids of tens to hundreds of thousands of tiles and cell blocks.  Against the CPU oracle
+in the smallest box (the drops are out of each other's reach in all of them).  Coordinates
+uploaded with and without a rebuild, then ordinary steps.  Bounds as in test_gpu_tiles."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from emdee_gb300.emdee import MIXED
+from mdrun import fcc_lattice, velocity_verlet
+from test_gpu_tiles import gpu, oracle  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def droplet(lib, L, precision=None):
+    N, rng = 400, np.random.default_rng(5)
+    md = lib.system(1, 1, 2.5, 0.3, N)
+    if precision is not None:
+        lib.EmDee_set_precision(md, precision)
+    lib.EmDee_set_pair_model(md, 1, 1, lib.EmDee_shifted_force(lib.EmDee_pair_lj_cut(1.0, 1.0)), 0.0)
+    R = fcc_lattice(N, 8.0, 0.05, 1) - 4.0   # the first drop lies across the box's corner
+    R[N // 2:] += 0.47 * L
+    lib.upload(md, "box", np.array([L]))
+    lib.upload(md, "coordinates", R)
+    lib.upload(md, "momenta", rng.standard_normal((N, 3)))
+    return md, R
+
+
+def check(gpu, oracle, md, ref, N):  # noqa: F811
+    assert md.Builds == ref.Builds
+    assert np.array_equal(gpu.neighbor_pairs(md), oracle.neighbor_pairs(ref))
+    F, G = gpu.download(md, "forces", (N, 3)), oracle.download(ref, "forces", (N, 3))
+    assert np.sqrt(((F - G) ** 2).sum()) <= 1e-5 * np.sqrt((G ** 2).sum())
+    scale = abs(ref.Energy.Potential) + abs(ref.Virial.Total)
+    assert abs(md.Energy.Potential - ref.Energy.Potential) <= 1e-5 * scale
+    assert abs(md.Virial.Total - ref.Virial.Total) <= 1e-5 * scale
+
+
+@pytest.mark.parametrize("L", [60.0, 130.0, 400.0])
+def test_droplets(gpu, oracle, monkeypatch, L):  # noqa: F811
+    monkeypatch.setenv("EMDEE_AUTOTUNE", "0")
+    (md, R), (ref, R0) = droplet(gpu, L, MIXED), droplet(oracle, 60.0)
+    N = len(R)
+    check(gpu, oracle, md, ref, N)
+    for shift in (0.01, 1.5, -0.7):   # within the skin, then two rebuilds
+        for lib, m, r in ((gpu, md, R), (oracle, ref, R0)):
+            lib.upload(m, "coordinates", r + shift)
+            lib.EmDee_compute_forces(C.byref(m))
+        check(gpu, oracle, md, ref, N)
+    for lib, m in ((gpu, md), (oracle, ref)):
+        velocity_verlet(lib, m, 0.004, 12, 4)
+    check(gpu, oracle, md, ref, N)
+    gpu.EmDee_destroy(C.byref(md))
