@@ -289,6 +289,10 @@ static void initialize_system(tEmDee* md) {   // src/EmDeeCode.f90:916-923 and s
   }
 }
 
+// A pair launch that only finds its skip flag set takes 0.52 ns a tile (244,000 tiles: 127 us),
+// a decision brought to the host first one more synchronisation, 5 to 10 us.
+static const int QUEUED_TILES = 16384;
+
 // src/EmDeeCode.f90:1215-1277
 static void compute_forces_impl(tEmDee* md) {
   System& s = *sys_of(*md);
@@ -303,7 +307,10 @@ static void compute_forces_impl(tEmDee* md) {
   bool rebuild = !s.r0Valid, forcesDone = false;
   s.queueExtras = true;
   s.extrasQueued = false;
-  if (!rebuild && s.precision == 0 && s.pairs_exist[s.layer - 1]) {
+  // (positions that no fused step has checked: not with so many tiles that a pair launch
+  // which finds a rebuild due costs more than the synchronisation it saves)
+  const bool queued = (s.skinReady && s.packReady) || s.grid.nTiles <= QUEUED_TILES;
+  if (!rebuild && s.precision == 0 && s.pairs_exist[s.layer - 1] && queued) {
     // the skin decision (left by the fused step, or queued here) stays on the device with
     // the packed positions: the pair kernel and what follows it run unless a rebuild is
     // due, and one synchronisation returns both the decision and the sums
