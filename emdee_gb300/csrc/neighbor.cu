@@ -617,19 +617,18 @@ __global__ void __maxnreg__(MODE == BUILD_ONE ? BUILD_MAXNREG : 64) k_build(Buil
     __syncthreads();
   }
   const int haloCount = off[g.haloCells];
-  {
-    // sizes taken from the previous build: a tile or halo that outgrew them is
-    // reported (the host re-sizes and builds again) before anything is staged
-    const int tileCount = A.start[(t + 1) * g.TB * g.TB * g.TB] - A.start[t * g.TB * g.TB * g.TB];
-    if (tileCount > A.tileStride || haloCount > A.haloCap) {
-      if (threadIdx.x == 0) {
-        atomicOr(A.maxCount + 1, 1);
-        *A.fail = 1ull;
-      }
-      return;
+  const int tb = A.start[t * cells], te = A.start[(t + 1) * cells];
+  // sizes taken from the previous build: a tile or halo that outgrew them is
+  // reported (the host re-sizes and builds again) before anything is staged
+  if (te - tb > A.tileStride || haloCount > A.haloCap) {
+    if (threadIdx.x == 0) {
+      atomicOr(A.maxCount + 1, 1);
+      *A.fail = 1ull;
     }
+    return;
   }
   for (int h = threadIdx.x; h <= g.haloCells; h += blockDim.x) lay[h] = off[h];
+  if (te == tb) return;   // no lists, but the force kernels stage the tile's halo
   // every thread reads back only the first slots it wrote itself
   for (int h = threadIdx.x; h < g.haloCells; h += blockDim.x)
     mark_halo_cell(hpos, h, off[h], off[h + 1], lay[g.haloCells + 1 + h]);
@@ -655,7 +654,6 @@ __global__ void __maxnreg__(MODE == BUILD_ONE ? BUILD_MAXNREG : 64) k_build(Buil
   };
   const bool none = A.ntypes == 1 && !sinter[0];   // the only type pair does not interact: empty lists
   const bool layered = GENERAL && A.layered;
-  const int tb = A.start[t * cells], te = A.start[(t + 1) * cells];
   const int HW = g.HW, capC = A.cap >> 3, chunkStride = A.tileStride * 8;
   const int loBits = __float_as_int(A.lo2);
   const unsigned band = (unsigned)(__float_as_int(A.hi2) - loBits);
