@@ -123,15 +123,18 @@ RB_HD void rb_rotate_no_squish(BodyState& b, double delta_t, int n, const double
 }
 
 // Carlson's duplication algorithms for RF, RC and RJ (relative tolerance 1e-3
-// on the deviations, as in src/math.f90:505-638)
+// on the deviations, as in src/math.f90:505-638).  The deviations shrink by 4 per pass; the
+// loops end on NaN (a body of no extent, a state that has blown up) and after RB_PASSES.
+static const int RB_PASSES = 1100;   // from any ratio of the arguments: log4 of 2^2098, and a few
+
 RB_HDN inline double rb_RF(double x, double y, double z) {
   double xn = x, yn = y, zn = z, mu, xd, yd, zd;
-  for (;;) {
+  for (int pass = 0; pass < RB_PASSES; pass++) {
     mu = (xn + yn + zn) / 3.0;
     xd = 2.0 - (mu + xn) / mu;
     yd = 2.0 - (mu + yn) / mu;
     zd = 2.0 - (mu + zn) / mu;
-    if (fmax(fabs(xd), fmax(fabs(yd), fabs(zd))) < 0.001) break;
+    if (!(fmax(fabs(xd), fmax(fabs(yd), fabs(zd))) >= 0.001)) break;
     double xr = sqrt(xn), yr = sqrt(yn), zr = sqrt(zn), lam = xr * (yr + zr) + yr * zr;
     xn = (xn + lam) * 0.25;
     yn = (yn + lam) * 0.25;
@@ -144,10 +147,10 @@ RB_HDN inline double rb_RF(double x, double y, double z) {
 
 RB_HDN inline double rb_RC(double x, double y) {
   double xn = x, yn = y, mu, sn;
-  for (;;) {
+  for (int pass = 0; pass < RB_PASSES; pass++) {
     mu = (xn + yn + yn) / 3.0;
     sn = (yn + mu) / mu - 2.0;
-    if (fabs(sn) < 0.001) break;
+    if (!(fabs(sn) >= 0.001)) break;
     double lam = 2.0 * sqrt(xn) * sqrt(yn) + yn;
     xn = (xn + lam) * 0.25;
     yn = (yn + lam) * 0.25;
@@ -158,13 +161,13 @@ RB_HDN inline double rb_RC(double x, double y) {
 
 RB_HDN inline double rb_RJ(double x, double y, double z, double p) {
   double xn = x, yn = y, zn = z, pn = p, sigma = 0.0, power4 = 1.0, mu, xd, yd, zd, pd;
-  for (;;) {
+  for (int pass = 0; pass < RB_PASSES; pass++) {
     mu = (xn + yn + zn + pn + pn) * 0.2;
     xd = (mu - xn) / mu;
     yd = (mu - yn) / mu;
     zd = (mu - zn) / mu;
     pd = (mu - pn) / mu;
-    if (fmax(fmax(fabs(xd), fabs(yd)), fmax(fabs(zd), fabs(pd))) < 0.001) break;
+    if (!(fmax(fmax(fabs(xd), fabs(yd)), fmax(fabs(zd), fabs(pd))) >= 0.001)) break;
     double xr = sqrt(xn), yr = sqrt(yn), zr = sqrt(zn), lam = xr * (yr + zr) + yr * zr;
     double al = pn * (xr + yr + zr) + xr * yr * zr;
     al = al * al;
