@@ -237,45 +237,49 @@ __global__ void k_sg_scatter(const int* __restrict__ cellOf, Geometry G, const i
 // Deterministic order inside a cell (ascending atom index): a warp per cell, each atom's
 // place is the number of atoms of the cell with a smaller index.  Cells of more than
 // 32 * SORT_REGS atoms are sorted by lane 0.  (8 x 8000 atoms in cells of 64: one thread
-// per cell took 343 us, 8 us so.)
+// per cell took 343 us, 8 us so.)  Where most cells hold no or one atom a warp looks at
+// `per` of them, up to 32, for those that hold more.
 constexpr int SORT_REGS = 8;
-__global__ void k_sg_sort(const int* __restrict__ starts, int n, int* __restrict__ sorted) {
-  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (r >= n) return;
-  const int b = starts[r], m = starts[r + 1] - b;
-  if (m <= 1) return;
-  if (m > 32 * SORT_REGS) {
-    if (lane == 0)
-      for (int i = b + 1; i < b + m; i++) {
-        const int v = sorted[i];
-        int j = i - 1;
-        while (j >= b && sorted[j] > v) {
-          sorted[j + 1] = sorted[j];
-          j--;
+__global__ void k_sg_sort(const int* __restrict__ starts, int n, int per, int* __restrict__ sorted) {
+  const int lane = threadIdx.x & 31, r0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per;
+  const int mine = r0 + lane;
+  unsigned todo = __ballot_sync(0xffffffffu, lane < per && mine < n && starts[mine + 1] - starts[mine] > 1);
+  for (; todo != 0; todo &= todo - 1) {
+    const int r = r0 + __ffs(todo) - 1;
+    const int b = starts[r], m = starts[r + 1] - b;
+    if (m > 32 * SORT_REGS) {
+      if (lane == 0)
+        for (int i = b + 1; i < b + m; i++) {
+          const int v = sorted[i];
+          int j = i - 1;
+          while (j >= b && sorted[j] > v) {
+            sorted[j + 1] = sorted[j];
+            j--;
+          }
+          sorted[j + 1] = v;
         }
-        sorted[j + 1] = v;
-      }
-    return;
-  }
-  int v[SORT_REGS], place[SORT_REGS];
-#pragma unroll
-  for (int u = 0; u < SORT_REGS; u++) {
-    v[u] = 32 * u + lane < m ? sorted[b + 32 * u + lane] : 0;
-    place[u] = 0;
-  }
-#pragma unroll
-  for (int w = 0; w < SORT_REGS; w++) {
-    if (32 * w >= m) break;
-    for (int k = 0; k < min(32, m - 32 * w); k++) {
-      const int x = __shfl_sync(0xffffffffu, v[w], k);
-#pragma unroll
-      for (int u = 0; u < SORT_REGS; u++) place[u] += x < v[u] ? 1 : 0;
+      continue;
     }
-  }
-  __syncwarp();
+    int v[SORT_REGS], place[SORT_REGS];
 #pragma unroll
-  for (int u = 0; u < SORT_REGS; u++)
-    if (32 * u + lane < m) sorted[b + place[u]] = v[u];
+    for (int u = 0; u < SORT_REGS; u++) {
+      v[u] = 32 * u + lane < m ? sorted[b + 32 * u + lane] : 0;
+      place[u] = 0;
+    }
+#pragma unroll
+    for (int w = 0; w < SORT_REGS; w++) {
+      if (32 * w >= m) break;
+      for (int k = 0; k < min(32, m - 32 * w); k++) {
+        const int x = __shfl_sync(0xffffffffu, v[w], k);
+#pragma unroll
+        for (int u = 0; u < SORT_REGS; u++) place[u] += x < v[u] ? 1 : 0;
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < SORT_REGS; u++)
+      if (32 * u + lane < m) sorted[b + place[u]] = v[u];
+  }
 }
 
 // rintf for |x| < 2^22 on the FP32 adders (the conversion unit runs at a quarter of
@@ -290,18 +294,29 @@ __device__ __forceinline__ float nearest(float x) { return __fadd_rn(__fadd_rn(x
 // instruction issue: 36 instructions per 32 candidates of one atom before the load and
 // the loop were shared by LIST_ATOMS (8 x 8000 atoms: 142 -> 111 us; one thread per atom,
 // gathering each candidate's index and position: 428 us).
+// Where the chains have more cells than atoms the blocks are those of the atoms' cells
+// instead: block b takes the cell of the b-th atom in cell order, if that is its first
+// (cellOf set; forces with new lists of 2000 atoms in 54,872 cells: 206 -> 167 us).
 constexpr int LIST_CAND = 2048, LIST_THREADS = 256, LIST_ATOMS = 2;
 __global__ void __launch_bounds__(LIST_THREADS) k_sg_list(const float4* __restrict__ pos, Geometry G,
                                                           const int* __restrict__ starts,
-                                                          const int* __restrict__ sorted, int cap,
+                                                          const int* __restrict__ sorted,
+                                                          const int* __restrict__ cellOf, int cap,
                                                           int* __restrict__ list, int* __restrict__ count,
                                                           int* __restrict__ overflow) {
   __shared__ float4 cand[LIST_CAND];   // position (M >= 3: the image next to the cell) and index
   __shared__ int first[28], base[28];   // candidates of the neighbor cells: first slot, running count
-  const int M = G.M, cells = M * M * M, chain = blockIdx.x / cells, cell = blockIdx.x % cells;
+  const int M = G.M, cells = M * M * M;
+  int id = blockIdx.x;
+  if (cellOf != nullptr) {
+    const int q = sorted[blockIdx.x];
+    id = q / G.N * cells + cellOf[q];
+    if (starts[id] != (int)blockIdx.x) return;
+  }
+  const int chain = id / cells, cell = id % cells;
   const int x = cell % M, y = (cell / M) % M, z = cell / (M * M);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int own0 = starts[blockIdx.x], own1 = starts[blockIdx.x + 1];
+  const int own0 = starts[id], own1 = starts[id + 1];
   if (own0 == own1) return;
   const int ncell = M >= 3 ? 27 : 1;   // M < 3: every cell of the chain once
   if (threadIdx.x < ncell) {
@@ -1335,8 +1350,11 @@ static void sg_build_lists(Surrogate& S, const double* dR, cudaStream_t st) {
   k_sg_count<<<sg_blocks(S.total), 256, 0, st>>>(S.dPos, S.G, S.dCellOf, S.dCounts);
   k_sg_scan<<<1, 256, 0, st>>>(S.dCounts, cells, S.dStarts);
   k_sg_scatter<<<sg_blocks(S.total), 256, 0, st>>>(S.dCellOf, S.G, S.dStarts, S.dCursor, S.dSorted);
-  k_sg_sort<<<(cells + 7) / 8, 256, 0, st>>>(S.dStarts, cells, S.dSorted);
-  k_sg_list<<<cells, LIST_THREADS, 0, st>>>(S.dPos, S.G, S.dStarts, S.dSorted, S.cap, S.dList, S.dCount, S.dOverflow);
+  const int per = cells > S.total ? 32 : 1;
+  k_sg_sort<<<(cells + 8 * per - 1) / (8 * per), 256, 0, st>>>(S.dStarts, cells, per, S.dSorted);
+  k_sg_list<<<std::min(cells, S.total), LIST_THREADS, 0, st>>>(S.dPos, S.G, S.dStarts, S.dSorted,
+                                                               cells > S.total ? S.dCellOf : nullptr, S.cap, S.dList,
+                                                               S.dCount, S.dOverflow);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(S.dR0, dR, sizeof(double) * 3 * S.total, cudaMemcpyDeviceToDevice, st));
 }
