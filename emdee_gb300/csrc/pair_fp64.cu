@@ -18,7 +18,7 @@
 
 namespace emdee {
 
-static const int PAIR64_THREADS = 128;
+static const int PAIR64_THREADS = 128, PAIR64_MANY = 8192;
 static const int PAIR64_STATIC = 512;   // the kernel's static shared memory at most (the sums of grid_reduce)
 
 struct __align__(32) D4 {
@@ -73,23 +73,26 @@ __global__ void __launch_bounds__(PAIR64_THREADS) k_pair_fp64(PairArgsD A) {
   D4* hpos = (D4*)sraw;   // Rs.xyz, charge
   int4* hfrac = (int4*)(hpos + A.haloCap + 1);
   uint8_t* htype = (uint8_t*)(hfrac + (STAGED ? A.haloCap + 1 : 0));
-  // from the layout saved by the list build: every halo index's slot first (in the
-  // position it will hold), then the atoms, one thread each
-  const int* lay = A.layout + (size_t)t * (2 * g.haloCells + 1);
-  int* mark = (int*)sraw;
-  for (int h = threadIdx.x; h < g.haloCells; h += blockDim.x) {
-    const int b = lay[h], e = lay[h + 1], s0 = lay[g.haloCells + 1 + h];
-    for (int q = b; q < e; q++) mark[q * (sizeof(D4) / sizeof(int))] = s0 + q - b;
+  const int tb = A.start[t * cells], te = A.start[(t + 1) * cells];
+  if (te > tb) {   // (a nearly empty box has hundreds of thousands of tiles without atoms)
+    // from the layout saved by the list build: every halo index's slot first (in the
+    // position it will hold), then the atoms, one thread each
+    const int* lay = A.layout + (size_t)t * (2 * g.haloCells + 1);
+    int* mark = (int*)sraw;
+    for (int h = threadIdx.x; h < g.haloCells; h += blockDim.x) {
+      const int b = lay[h], e = lay[h + 1], s0 = lay[g.haloCells + 1 + h];
+      for (int q = b; q < e; q++) mark[q * (sizeof(D4) / sizeof(int))] = s0 + q - b;
+    }
+    __syncthreads();
+    const int halo = lay[g.haloCells];
+    for (int q = threadIdx.x; q < halo; q += blockDim.x) {
+      const int sj = mark[q * (sizeof(D4) / sizeof(int))];
+      hpos[q] = D4{A.Rs[3 * sj], A.Rs[3 * sj + 1], A.Rs[3 * sj + 2], MOD < 0 ? A.charge[A.orig[sj]] : 0.0};
+      if (STAGED) hfrac[q] = A.frac[sj];
+      if (MOD < 0) htype[q] = A.type8[sj];
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  const int halo = lay[g.haloCells];
-  for (int q = threadIdx.x; q < halo; q += blockDim.x) {
-    const int sj = mark[q * (sizeof(D4) / sizeof(int))];
-    hpos[q] = D4{A.Rs[3 * sj], A.Rs[3 * sj + 1], A.Rs[3 * sj + 2], MOD < 0 ? A.charge[A.orig[sj]] : 0.0};
-    if (STAGED) hfrac[q] = A.frac[sj];
-    if (MOD < 0) htype[q] = A.type8[sj];
-  }
-  __syncthreads();
   NBParams<double> coul;
   if (MOD < 0) coul = *A.coul;
   NBParams<double> lj = A.table[0].model;
@@ -97,7 +100,6 @@ __global__ void __launch_bounds__(PAIR64_THREADS) k_pair_fp64(PairArgsD A) {
     lj.kind = MK_LJ_CUT;
     lj.modifier = MOD;
   }
-  const int tb = A.start[t * cells], te = A.start[(t + 1) * cells];
   const int capC = A.cap >> 3;
   double Ep = 0.0, Ec = 0.0, Wp = 0.0, Wc = 0.0;
   int within = 0;
@@ -209,8 +211,12 @@ void device_pair_forces_fp64(System& s, bool compute, bool useInRc, double rc2sc
   const size_t smem = halo * (staged ? atom + sizeof(int4) : atom) + 16;
   if (smem > limit) fatal("pair forces", "too many atoms around a cell for FP64 arithmetic");
   const int mod = pair_lj_only(s) ? s.P(0, 0, s.layer - 1).model.p.modifier : -1;
-  // as many threads as the largest tile has atoms, in whole warps, up to PAIR64_THREADS
-  const int th = std::min(PAIR64_THREADS, (g.tileAtoms + 31) / 32 * 32);
+  // As many threads as the largest tile has atoms, in whole warps, up to PAIR64_THREADS, and
+  // enough for the halo's cells; all of them where the last block has very many tiles' sums to
+  // add.  2000 atoms in a box of 60 (1331 tiles), 10 steps: 1155 us with 32 threads, 889 with
+  // 64; in a box of 150 (19,683 tiles) 6.27 ms with 64, 4.98 with 128
+  const int fit = std::max(halo_min_threads(A.g), (g.tileAtoms + 31) / 32 * 32);
+  const int th = g.nTiles >= PAIR64_MANY ? PAIR64_THREADS : std::min(PAIR64_THREADS, fit);
   auto run = staged ? (compute ? launch_fp64_mod<true, true> : launch_fp64_mod<false, true>)
                     : (compute ? launch_fp64_mod<true, false> : launch_fp64_mod<false, false>);
   run(s, A, smem, g.nTiles, th, mod);

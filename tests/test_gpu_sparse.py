@@ -7,7 +7,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from emdee_gb300.emdee import MIXED
+from emdee_gb300.emdee import FP64, MIXED
 from mdrun import fcc_lattice, velocity_verlet
 from test_gpu_tiles import gpu, oracle  # noqa: F401
 
@@ -52,4 +52,15 @@ def test_droplets(gpu, oracle, monkeypatch, L):  # noqa: F811
     for lib, m in ((gpu, md), (oracle, ref)):
         velocity_verlet(lib, m, 0.004, 12, 4)
     check(gpu, oracle, md, ref, N)
+    gpu.EmDee_destroy(C.byref(md))
+
+
+@pytest.mark.parametrize("L", [60.0, 130.0])
+def test_fp64(gpu, oracle, L):  # noqa: F811
+    """FP64 forces with many empty tiles, in blocks of every size: FP64 rounding, 1e-12"""
+    (md, R), (ref, _) = droplet(gpu, L, FP64), droplet(oracle, 60.0)
+    N = len(R)
+    F, G = gpu.download(md, "forces", (N, 3)), oracle.download(ref, "forces", (N, 3))
+    assert np.sqrt(((F - G) ** 2).sum()) <= 1e-12 * np.sqrt((G ** 2).sum())
+    assert abs(md.Energy.Potential - ref.Energy.Potential) <= 1e-12 * abs(ref.Energy.Potential)
     gpu.EmDee_destroy(C.byref(md))
