@@ -341,21 +341,24 @@ __global__ void __launch_bounds__(PAIR_THREADS_TYPES) k_pair_types(PairArgsF A) 
   float* kq = (float*)(tbl + ntab);
   uint8_t* htype = (uint8_t*)(kq + ntab);
   const float w = 1.0f / A.invw;
-  for (int k = threadIdx.x; k < ntab; k += blockDim.x) {
-    const PairEntry<float>& pe = A.table[k];
-    const bool lj = pe.model.kind == MK_LJ_CUT;
-    tbl[k] = TypePair{lj ? pe.model.sigsq * A.invw2 : 0.f, lj ? pe.model.eps4 : 0.f,
-                      lj && pe.model.modifier == SHIFTED_FORCE ? pe.model.fshift * w : 0.f,
-                      lj && pe.model.modifier != NONE ? pe.model.eshift : 0.f};
-    kq[k] = pe.coulomb ? pe.kCoul : 0.f;
+  const int tb = A.start[t * cells], te = A.start[(t + 1) * cells];
+  if (te > tb) {   // (nothing for the tiles without atoms of a nearly empty box)
+    for (int k = threadIdx.x; k < ntab; k += blockDim.x) {
+      const PairEntry<float>& pe = A.table[k];
+      const bool lj = pe.model.kind == MK_LJ_CUT;
+      tbl[k] = TypePair{lj ? pe.model.sigsq * A.invw2 : 0.f, lj ? pe.model.eps4 : 0.f,
+                        lj && pe.model.modifier == SHIFTED_FORCE ? pe.model.fshift * w : 0.f,
+                        lj && pe.model.modifier != NONE ? pe.model.eshift : 0.f};
+      kq[k] = pe.coulomb ? pe.kCoul : 0.f;
+    }
+    if (threadIdx.x == 0) {
+      hpos[A.haloCap] = make_float4(1e9f, 1e9f, 1e9f, 0.f);
+      htype[A.haloCap] = 0;
+    }
+    const int* lay = A.layout + (size_t)t * (2 * g.haloCells + 1);
+    stage_frame_saved(g, lay, A.pos4, hpos, htype, A.type8);
+    __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    hpos[A.haloCap] = make_float4(1e9f, 1e9f, 1e9f, 0.f);
-    htype[A.haloCap] = 0;
-  }
-  const int* lay = A.layout + (size_t)t * (2 * g.haloCells + 1);
-  stage_frame_saved(g, lay, A.pos4, hpos, htype, A.type8);
-  __syncthreads();
   float alpha = 0.f, beta = 0.f, cfsh = 0.f, cesh = 0.f;
   if (COUL) {
     alpha = A.coul->alpha * w;
@@ -363,7 +366,6 @@ __global__ void __launch_bounds__(PAIR_THREADS_TYPES) k_pair_types(PairArgsF A) 
     cfsh = A.coul->fshift * w;
     cesh = A.coul->eshift;
   }
-  const int tb = A.start[t * cells], te = A.start[(t + 1) * cells];
   const int capC = A.cap >> 3;
   float Ep = 0.f, Ec = 0.f, Wp = 0.f, Wc = 0.f;
   const int tpa = A.tpa, sub = threadIdx.x & (tpa - 1);

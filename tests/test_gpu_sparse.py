@@ -64,3 +64,26 @@ def test_fp64(gpu, oracle, L):  # noqa: F811
     assert np.sqrt(((F - G) ** 2).sum()) <= 1e-12 * np.sqrt((G ** 2).sum())
     assert abs(md.Energy.Potential - ref.Energy.Potential) <= 1e-12 * abs(ref.Energy.Potential)
     gpu.EmDee_destroy(C.byref(md))
+
+
+def test_types_and_charges(gpu, oracle):  # noqa: F811
+    """Two types with damped charges, where most tiles have no atoms; bounds of test_gpu_tiles"""
+    N, L, rng = 300, 80.0, np.random.default_rng(3)
+    R = fcc_lattice(N, 7.5, 0.05, 2) - 3.0
+    R[::2] += 0.4 * L * (np.arange(N // 2) % 2)[:, None]
+    q, out = rng.uniform(-1, 1, N), []
+    for lib, precision in ((gpu, MIXED), (oracle, None)):
+        md = lib.system(1, 1, 2.5, 0.3, N, np.arange(N) % 2 + 1, [1.0, 2.0])
+        if precision is not None:
+            lib.EmDee_set_precision(md, precision)
+        for t in (1, 2):
+            lib.EmDee_set_pair_model(md, t, t, lib.EmDee_pair_lj_cut(0.5 * t, 1.0), 0.9)
+        lib.EmDee_set_coul_model(md, lib.EmDee_shifted_force(lib.EmDee_coul_damped(0.6)))
+        lib.upload(md, "charges", q)
+        lib.upload(md, "box", np.array([L]))
+        lib.upload(md, "coordinates", R)
+        out.append((lib.download(md, "forces", (N, 3)), md.Energy.Potential, md.Energy.Coulomb, md.Virial.Total))
+    (F, E, Q, W), (G, E0, Q0, W0) = out
+    assert np.sqrt(((F - G) ** 2).sum()) <= 3e-5 * np.sqrt((G ** 2).sum())
+    scale = abs(E0) + abs(Q0) + abs(W0)
+    assert max(abs(E - E0), abs(Q - Q0), abs(W - W0)) <= 1e-5 * scale
