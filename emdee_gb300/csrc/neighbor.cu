@@ -955,13 +955,14 @@ static int choose_tile(System& s, int M, double perCell) {
 
 // Tile edge, threads per atom and block sizes tuned on the system itself at its first
 // build (mixed precision, EMDEE_TILE unset).  For each edge from min(rule - 1, 3)
-// (from 1 in small systems, where few large tiles leave most SMs idle) to 6 cells (the
-// rule's edge always among them) a first build sizes the tiles; then the list build
-// and the pair kernel are timed with CUDA events (the faster of two launches, after a
-// warm-up launch of the pair kernel), each after a pass that moves the memory traffic
-// of an integration step, at the rule's shape, at block sizes from 64 to 512 threads
-// (threads loop over the tile's atoms in rounds; the best size balances the rounds of
-// typical tiles against residency) and at 2 to 32 threads per atom.  The cost of an
+// (from the least that gives a tile an atom in small systems, where few large tiles leave
+// most SMs idle) to 6 cells (the rule's edge always among them) a first build sizes the
+// tiles; then the list build and the pair kernel are timed with CUDA events (the faster of two
+// launches, after a warm-up launch of the pair kernel), each after a pass that moves the
+// memory traffic of an integration step, at the rule's shape and, on the edges whose cost so
+// is within 1.5 of the least, at block sizes from 64 to 512 threads (threads loop over the
+// tile's atoms in rounds; the best size balances the rounds of typical tiles against
+// residency) and at 2 to 32 threads per atom.  The cost of an
 // edge is its fastest pair launch plus a seventh of its fastest build (a rebuild
 // every ~7 steps, typical of a liquid with the reference's skin).  The rule's edge
 // and block sizes stay unless another choice is more than 5 % cheaper.  The choice
@@ -1030,55 +1031,86 @@ void device_tune_tile(System& s, bool ljOnly, void (*pair)(System&)) {
     return best;
   };
   const bool log = getenv("EMDEE_TUNE_LOG") != nullptr;
-  double best = 1e30, ruleCost = 1e30;
-  TileChoice choice = {rule, 0, 0, 0, 0};
+  auto timed_build = [&] {
+    const double ms = timed([&] { device_build_lists(s); });
+    if (log)
+      fprintf(stderr, "  edge %d build, %d per atom, %d threads: %.1f us\n", s.tileOverride, s.buildTpa,
+              build_block_threads(s), 1e3 * ms);
+    return ms;
+  };
+  auto timed_pair = [&] {
+    pair(s);   // warm-up
+    const double ms = timed([&] { pair(s); });
+    if (log)
+      fprintf(stderr, "  edge %d pair, %d per atom, %d threads: %.1f us\n", s.tileOverride, s.pairTpa,
+              pair_block_threads(s), 1e3 * ms);
+    return ms;
+  };
+  // the rule's shape on every edge
+  struct Edge {
+    int tb;
+    double build, pair;
+    double cost() const { return pair + build / 7.0; }
+  };
+  std::vector<Edge> edges;
+  double bestRule = 1e30;
   const bool small = s.natoms < 152 * 1024;   // fewer atoms than half the GPU's threads
-  for (int tb = small ? 1 : std::max(1, std::min(rule - 1, 3)); tb <= std::min(6, M); tb++) {
+  int lowest = std::max(1, std::min(rule - 1, 3));
+  if (small) {   // the least edge that gives a tile an atom
+    int tb = 1;
+    while (tb < lowest && perCell * (tb * tb * tb) < 1.0) tb++;
+    lowest = tb;
+  }
+  for (int tb = lowest; tb <= std::min(6, M); tb++) {
     use_choice(s, TileChoice{tb, 0, 0, 0, 0});
     device_build_lists(s);   // sizes the tiles of this edge
     if (s.grid.TB != tb) continue;   // did not fit (halo or shared memory): the build shrank the edge
-    // (threads per atom, threads per block): the rule's (0, 0), then with one thread per
-    // atom 64 to 256 threads in steps of 32 and 320 to 512 in steps of 64, from the least the
-    // halo scans need up to the largest tile, and the splits that the GPU has threads for
-    const int thMin = halo_min_threads(make_geom(s.grid.M, tb)), thMax = (s.grid.tileAtoms + 31) / 32 * 32;
-    std::vector<std::pair<int, int>> shapes = {{0, 0}};
-    for (int th = 64; th <= 512; th += th < 256 ? 32 : 64)
-      if (th >= thMin && th <= std::max(thMax, 64)) shapes.push_back({1, th});
-    for (int tpa = 2; tpa <= 32; tpa *= 2)
-      if ((double)s.natoms * tpa <= 152.0 * 2048 * 2) shapes.push_back({tpa, 0});
-    double msBuild = 1e30, msPair = 1e30, ruleBuild = 0.0, rulePair = 0.0;
+    edges.push_back(Edge{tb, timed_build(), timed_pair()});
+    bestRule = std::min(bestRule, edges.back().cost());
+  }
+  double best = 1e30, ruleCost = 1e30;
+  TileChoice choice = {rule, 0, 0, 0, 0};
+  for (const Edge& e : edges) {
+    const int tb = e.tb;
+    if (tb == rule) ruleCost = e.cost();
+    double msBuild = e.build, msPair = e.pair;
     TileChoice here = {tb, 0, 0, 0, 0};
-    for (const auto& sh : shapes) {
-      s.buildTpa = sh.first;
-      s.buildThreads = sh.second;
-      const double ms = timed([&] { device_build_lists(s); });
-      if (log)
-        fprintf(stderr, "  edge %d build, %d per atom, %d threads: %.1f us\n", tb, sh.first, build_block_threads(s),
-                1e3 * ms);
-      if (sh.first == 0) ruleBuild = ms;
-      if (ms < msBuild) {
-        msBuild = ms;
-        here.buildTpa = sh.first;
-        here.buildThreads = sh.second;
+    // other shapes have gained up to 1.3 times on the rule's
+    if (e.cost() <= 1.5 * bestRule) {
+      use_choice(s, here);
+      device_build_lists(s);
+      // (threads per atom, threads per block): with one thread per atom 64 to 256 threads
+      // in steps of 32 and 320 to 512 in steps of 64, from the least the halo scans need up to the
+      // largest tile, and the splits that the GPU has threads and the lists entries for
+      const int thMin = halo_min_threads(make_geom(s.grid.M, tb)), thMax = (s.grid.tileAtoms + 31) / 32 * 32;
+      const double entries = expected_entries(s);
+      std::vector<std::pair<int, int>> shapes;
+      for (int th = 64; th <= 512; th += th < 256 ? 32 : 64)
+        if (th >= thMin && (th <= thMax || (th == 64 && entries >= 2.0))) shapes.push_back({1, th});
+      for (int tpa = 2; tpa <= 32; tpa *= 2)
+        if ((double)s.natoms * tpa <= 152.0 * 2048 * 2 && entries >= tpa) shapes.push_back({tpa, 0});
+      for (const auto& sh : shapes) {
+        s.buildTpa = sh.first;
+        s.buildThreads = sh.second;
+        const double ms = timed_build();
+        if (ms < msBuild) {
+          msBuild = ms;
+          here.buildTpa = sh.first;
+          here.buildThreads = sh.second;
+        }
       }
-    }
-    for (const auto& sh : shapes) {
-      s.pairTpa = sh.first;
-      s.pairThreads = sh.second;
-      pair(s);   // warm-up
-      const double ms = timed([&] { pair(s); });
-      if (log)
-        fprintf(stderr, "  edge %d pair, %d per atom, %d threads: %.1f us\n", tb, sh.first, pair_block_threads(s),
-                1e3 * ms);
-      if (sh.first == 0) rulePair = ms;
-      if (ms < msPair) {
-        msPair = ms;
-        here.pairTpa = sh.first;
-        here.pairThreads = sh.second;
+      for (const auto& sh : shapes) {
+        s.pairTpa = sh.first;
+        s.pairThreads = sh.second;
+        const double ms = timed_pair();
+        if (ms < msPair) {
+          msPair = ms;
+          here.pairTpa = sh.first;
+          here.pairThreads = sh.second;
+        }
       }
     }
     const double cost = msPair + msBuild / 7.0;
-    if (tb == rule) ruleCost = rulePair + ruleBuild / 7.0;
     if (log)
       fprintf(stderr, "tile edge %d (at most %d atoms per tile): cost %.1f us, build %d x %d, pair %d x %d\n", tb,
               s.grid.tileAtoms, 1e3 * cost, here.buildTpa, here.buildThreads, here.pairTpa, here.pairThreads);

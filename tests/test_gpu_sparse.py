@@ -87,3 +87,18 @@ def test_types_and_charges(gpu, oracle):  # noqa: F811
     assert np.sqrt(((F - G) ** 2).sum()) <= 3e-5 * np.sqrt((G ** 2).sum())
     scale = abs(E0) + abs(Q0) + abs(W0)
     assert max(abs(E - E0), abs(Q - Q0), abs(W - W0)) <= 1e-5 * scale
+
+
+def test_tuned(gpu, oracle):  # noqa: F811
+    """The first forces time tile edges: none so small that 11 million cells get a tile each,
+    which would take 41 GB (2 KB of halo layout and 1.7 KB of lists a tile); edge 3, the least
+    they should try, has 405,000 tiles with 5.5 and 13 KB, 7.5 GB"""
+    import torch
+    free = torch.cuda.mem_get_info()[0]
+    md, _ = droplet(gpu, 311.0, MIXED)
+    used = free - torch.cuda.mem_get_info()[0]
+    assert gpu.EmDee_tile_edge(md) >= 3 and used < 16 << 30, (gpu.EmDee_tile_edge(md), used)
+    ref, _ = droplet(oracle, 60.0)
+    F, G = gpu.download(md, "forces", (400, 3)), oracle.download(ref, "forces", (400, 3))
+    assert np.sqrt(((F - G) ** 2).sum()) <= 1e-5 * np.sqrt((G ** 2).sum())
+    gpu.EmDee_destroy(C.byref(md))
