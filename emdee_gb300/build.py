@@ -36,7 +36,8 @@ UNITS = {
     "bonded.cu": ["-fmad=false"],
     "surrogate.cu": [],
 }
-HEADERS = ["system.hpp", "pairmath.cuh", "tile.cuh", "f32x2.cuh", "ffkick.cuh", "fpconv.h", "reduce.cuh", "rigid.cuh", "bodies.cuh", os.path.join("..", "..", "include", "emdee.h")]
+HEADERS = sorted(f for f in os.listdir(CSRC) if f.endswith((".h", ".hpp", ".cuh")))   # rebuild on any of them
+HEADERS.append(os.path.join("..", "..", "include", "emdee.h"))
 
 
 def _stale(target, deps):
