@@ -30,5 +30,12 @@ EMD_HD_INLINE bool d2f_normal(unsigned long long b) {
   return e >= 1 && e <= 253;
 }
 
+// a - b of two box fractions in units of 2^-32 (modulo 1), as a signed 32-bit number:
+// subtracted as unsigned, because the difference of two ints may overflow, which C++ leaves
+// undefined (and refuses in the constant expressions below)
+EMD_HD_INLINE constexpr int box_delta(int a, int b) { return (int)((unsigned int)a - (unsigned int)b); }
+static_assert(box_delta(-2147483647 - 1, 2147483647) == 1 && box_delta(2147483647, -2147483647 - 1) == -1 &&
+                  box_delta(1500000000, -1500000000) == -1294967296 && box_delta(3, 5) == -2,
+              "differences of box fractions wrap around");
 
 }  // namespace emdee

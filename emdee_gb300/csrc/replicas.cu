@@ -313,7 +313,7 @@ __device__ __forceinline__ void rep_pairs(const RepDesc& D, const int4* pos, con
 #pragma unroll
       for (int u = 0; u < 8; u++) {
         const int4 pj = pos[(words[u >> 1] >> ((u & 1) * 16)) & 0xFFFF];
-        const float dx = (float)(pi.x - pj.x), dy = (float)(pi.y - pj.y), dz = (float)(pi.z - pj.z);
+        const float dx = (float)box_delta(pi.x, pj.x), dy = (float)box_delta(pi.y, pj.y), dz = (float)box_delta(pi.z, pj.z);
         const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
         const bool in = r2 < rc2 && u < left;
         const float inv2 = in ? Ops<float>::rcp(r2) : 0.f;   // zeroes every term of the others

@@ -83,15 +83,15 @@ __device__ __forceinline__ double wrap_half(double x) {
 }
 
 // Fraction of the box of a scaled coordinate, in units of 2^-32, modulo 1: the low word
-// of x 2^32 + 1.5 2^52.  Differences of two such numbers are minimum images as they
-// stand (32-bit wrap-around).
+// of x 2^32 + 1.5 2^52.  Differences of two such numbers (box_delta) are minimum images as
+// they stand.
 __device__ __forceinline__ int box_fraction(double x) {
   if ((__double2hiint(x) & 0x7FFFFFFF) >= 0x41200000) x = __dsub_rn(x, floor(x));   // 2^19 boxes away
   return __double2loint(fma(x, 4294967296.0, 6755399441055744.0));
 }
 // squared distance of two atoms in those units, FP32 (relative error ~3e-7)
 __device__ __forceinline__ float box_dist2(int4 a, int4 b) {
-  const float dx = (float)(a.x - b.x), dy = (float)(a.y - b.y), dz = (float)(a.z - b.z);
+  const float dx = (float)box_delta(a.x, b.x), dy = (float)box_delta(a.y, b.y), dz = (float)box_delta(a.z, b.z);
   return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
 }
 // Limit below which box_dist2 may belong to a pair with r^2 < r2 (scaled FP64 units)
