@@ -1154,7 +1154,8 @@ static bool build_lists(System& s, bool reuse, bool defer) {
   double perCell = (double)N / ((double)M * M * M);
   int TB = choose_tile(s, M, perCell);
   reuse = reuse && g.M == M && g.TB == TB && g.maxHalo > 0 && g.tileStride > 0 && c.atoms >= (size_t)N;
-  size_t smemLimit = 200 * 1024;
+  // the entries past the halo (BUILD_PAD, one of them a sentinel) come on top
+  size_t smemLimit = 200 * 1024 + (BUILD_PAD - 1) * (sizeof(float4) + sizeof(int) + 1);
   for (;;) {
     TileGeom geo = make_geom(M, TB);
     g.M = M;

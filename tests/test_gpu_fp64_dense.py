@@ -35,3 +35,18 @@ def test_refused():
                       "system(emdee_gb300.load(), N=7500, rho=0.85, rc=7.2, skin=0.5, precision=FP64)"])
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert r.returncode == 1 and "too many atoms around a cell" in r.stderr, r.stderr
+
+
+@pytest.mark.parametrize("N,fits", [(12766, True), (12768, False)])
+def test_largest_halo(N, fits):
+    """The list build takes 12,766 atoms of one type in a halo (all atoms of a box of five cells
+    per edge), no more: 200 KB of positions, offsets and a sentinel"""
+    code = "\n".join(["import sys; sys.path[:0] = [%r, %r]" % (ROOT, os.path.join(ROOT, "tests")),
+                      "import emdee_gb300", "from emdee_gb300.emdee import MIXED", "from test_gpu_tiles import system",
+                      "md = system(emdee_gb300.load(), N=%d, rho=0.85, rc=9.0, skin=0.5, pair='sf', precision=MIXED)" % N,
+                      "print(md.Energy.Potential)"])
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    if fits:
+        assert r.returncode == 0 and np.isfinite(float(r.stdout)), r.stderr
+    else:
+        assert r.returncode == 1 and "too many atoms around a cell" in r.stderr, r.stderr
