@@ -70,7 +70,8 @@ __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_boost(BodyArgs A, c
                                                                    const double* skip) {
   chain_wait();
   if (skip != nullptr && __double_as_longlong(*skip) != 0) return;   // a rebuild is due
-  constexpr int NQ = KIN ? (VIR ? 7 : 6) : 1;
+  static_assert(KIN || !VIR, "the virial comes with the kinetic sums");
+  constexpr int NQ = VIR ? 7 : KIN ? 6 : 1;
   double k6[NQ] = {};
   const BodyLane g = body_lane();
   if (g.i < A.nb) {
@@ -112,9 +113,7 @@ __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_boost(BodyArgs A, c
       }
     }
   }
-  constexpr int off = KIN ? 0 : 6;
-  if (KIN || VIR)
-    grid_reduce<NQ, BODY_GROUP_THREADS>(k6, partials, ticket, result + off, hostResult + off);
+  if (KIN) grid_reduce<NQ, BODY_GROUP_THREADS>(k6, partials, ticket, result, hostResult);
 }
 
 // rb_series_step (rigid.cuh) on the four lanes of a body: lane c sums the coefficients
@@ -449,8 +448,7 @@ void bodies_boost_launch(System& s, const System::BodyBoost& b, const double* sk
     CK(cudaGetLastError());
     s.prof.total++;
   }
-  auto kern = b.kinetic ? (virial ? k_body_boost<true, true> : k_body_boost<true, false>)
-                        : (virial ? k_body_boost<false, true> : k_body_boost<false, false>);
+  auto kern = !b.kinetic ? k_body_boost<false, false> : virial ? k_body_boost<true, true> : k_body_boost<true, false>;
   launch_chained(kern, body_group_blocks(s.nbodies), BODY_GROUP_THREADS, 0, s.stream, body_args(s), s.F(), b.CP, b.CF,
                  b.translate, b.rotate, s.dBodyScratch + freeBlocks * 3, s.dTicket + 3, s.dResult + BODY_RESULT,
                  s.hResult + BODY_RESULT, skip);

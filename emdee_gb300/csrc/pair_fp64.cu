@@ -27,7 +27,6 @@ struct __align__(32) D4 {
 
 struct PairArgsD {
   TileGeom g;
-  const int2* tab;
   const double* Rs;        // slot order, double[N][3]
   const double* charge;    // API order
   const uint8_t* type8;
@@ -180,7 +179,6 @@ void device_pair_forces_fp64(System& s, bool compute, bool useInRc, double rc2sc
   const double L = *s.Lbox;
   PairArgsD A;
   A.g = make_geom(g.M, g.TB);
-  A.tab = g.dHaloTab;
   A.Rs = g.dRs64;
   A.charge = s.dCharge;
   A.type8 = g.dType8;

@@ -43,7 +43,6 @@ static const int PAIR_THREADS_GENERAL = 1024;
 
 struct PairArgsF {
   TileGeom g;
-  const int2* tab;
   const int* layout;   // halo layout saved by the list build
   const float4* pos4;
   const uint8_t* type8;
@@ -519,7 +518,6 @@ static size_t pair_args(System& s, bool useInRc, double rc2scaled, bool general,
   Grid& g = s.grid;
   const double L = *s.Lbox, w = L / g.M;
   A.g = make_geom(g.M, g.TB);
-  A.tab = g.dHaloTab;
   A.layout = g.dLayout;
   A.pos4 = g.dPos4;
   A.type8 = g.dType8;

@@ -191,19 +191,6 @@ __host__ __device__ __forceinline__ int tile_threads(int stride, int rounds, int
   return th < 32 ? 32 : th > cap ? cap : th;
 }
 
-// off[h] = first halo index of halo cell h of tile t; off[haloCells] = halo size.
-__device__ __forceinline__ int halo_offsets(const TileGeom& g, int t, const int* start, int* off, int* ws) {
-  for (int h = threadIdx.x; h < g.haloCells; h += blockDim.x) {
-    int hx, hy, hz, r = halo_rank(g, t, h, hx, hy, hz);
-    off[h] = start[r + 1] - start[r];
-  }
-  __syncthreads();
-  int total = block_exclusive_scan<8>(off, g.haloCells, ws);
-  if (threadIdx.x == 0) off[g.haloCells] = total;
-  __syncthreads();
-  return total;
-}
-
 // Per-tile halo table, written once per list build: for halo cell h of tile t,
 // tab[t * haloCells + h] = (rank of the cell, hx | hy << 8 | hz << 16).
 __device__ __forceinline__ int2 halo_entry(const TileGeom& g, int t, int h) {

@@ -20,7 +20,7 @@ namespace emdee {
 
 static const int VV_THREADS = 128;
 
-// list == nullptr: atoms 0..n-1; otherwise the atoms list[0..n-1]
+// free atoms list[0..n-1] of a system with bodies (others: k_step_fused)
 template <bool COMPUTE, bool FMA>
 __global__ void __launch_bounds__(VV_THREADS) k_vv_pre_free(double* __restrict__ R, double* __restrict__ P,
                                                             const double* F,
@@ -29,15 +29,14 @@ __global__ void __launch_bounds__(VV_THREADS) k_vv_pre_free(double* __restrict__
   chain_wait();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
-  const int j = list ? list[q] : q;
+  const int j = list[q];
   const double im = invMass[j];
   for (int d = 0; d < 3; d++) {
     const double p = P[3 * j + d], f = F[3 * j + d];
     if (COMPUTE) s0[3 * q + d] = 2.5 * R[3 * j + d] + dt_2 * im * (p - dt_2 * f);
     const double pn = FMA ? fma(dt_2, f, p) : 1.0 * p + dt_2 * f;
     P[3 * j + d] = pn;
-    R[3 * j + d] = FMA ? (list == nullptr && im == 1.0 ? fma(dt, pn, R[3 * j + d]) : fma(dt * pn, im, R[3 * j + d]))
-                       : 1.0 * R[3 * j + d] + dt * pn * im;
+    R[3 * j + d] = FMA ? fma(dt * pn, im, R[3 * j + d]) : 1.0 * R[3 * j + d] + dt * pn * im;
   }
 }
 
