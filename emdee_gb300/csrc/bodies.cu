@@ -217,6 +217,8 @@ __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_move_series(BodyArg
                                                                          int translate) {
   chain_wait();
   const BodyLane g = body_lane();
+  // warps past the last body would read one that another warp writes
+  if ((int)(blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / BODY_LANES >= A.nb) return;
   BodyState& B = A.b[min(g.i, A.nb - 1)];
   double MoI[3], omega[3], TwoKr = 0.0, Iw1 = 0.0, Iw2 = 0.0, invMoI[3];
   for (int k = 0; k < 3; k++) {
