@@ -35,11 +35,16 @@ __device__ __forceinline__ void chain_wait() {
   if (gridDim.x <= CHAIN_BLOCKS) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Whether a grid of this many long blocks is launched chained: its blocks take their
-// places while the grid before them still holds some, so with one to a few blocks per SM
-// the SMs that were free first end up with two while others have none (a pair kernel of
-// 180 tiles: 10 steps of 50,021 atoms of two types 902 -> 935 us).  Up to one block per SM,
-// or several waves of blocks, even out.
+// Whether a grid of this many long blocks (the list build, the pair kernels) is launched
+// chained.  Its blocks take their places while the grid before them still holds some, so with
+// one to a few blocks per SM the SMs that were free first end up with two while others have
+// none.  In the steps themselves the overlap outweighs that: at a fixed tile edge, 10 steps
+// are 4 to 6 % faster chained at 216 and 343 tiles, 3 to 4 % at 512 and 729, 2 to 3 % at 1000 to
+// 1728, 7 to 10 % at 27 to 125.  But the tuner times launches one at a time behind a pass over memory,
+// where it sees only the uneven placement (50,021 atoms of two types on 180 tiles of 3 cells:
+// 54 us chained, 50.5 not, 50 on the few tiles of 5 cells), and would leave the edge that is better
+// in the steps (800 us for 10) for the other (880).  So grids between one block per SM
+// and four are launched the ordinary way.
 inline bool chain_fits(int blocks) { return blocks <= 152 || blocks >= 4 * 152; }
 
 template <class... P, class... A>
