@@ -237,48 +237,58 @@ __global__ void k_sg_scatter(const int* __restrict__ cellOf, Geometry G, const i
 // Deterministic order inside a cell (ascending atom index): a warp per cell, each atom's
 // place is the number of atoms of the cell with a smaller index.  Cells of more than
 // 32 * SORT_REGS atoms are sorted by lane 0.  (8 x 8000 atoms in cells of 64: one thread
-// per cell took 343 us, 8 us so.)  Where most cells hold no or one atom a warp looks at
-// `per` of them, up to 32, for those that hold more.
+// per cell took 343 us, 8 us so.)  SPARSE: a warp looks at 32 cells, of which most hold no or
+// one atom, for those that hold more.
 constexpr int SORT_REGS = 8;
-__global__ void k_sg_sort(const int* __restrict__ starts, int n, int per, int* __restrict__ sorted) {
-  const int lane = threadIdx.x & 31, r0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per;
-  const int mine = r0 + lane;
-  unsigned todo = __ballot_sync(0xffffffffu, lane < per && mine < n && starts[mine + 1] - starts[mine] > 1);
-  for (; todo != 0; todo &= todo - 1) {
-    const int r = r0 + __ffs(todo) - 1;
-    const int b = starts[r], m = starts[r + 1] - b;
-    if (m > 32 * SORT_REGS) {
-      if (lane == 0)
-        for (int i = b + 1; i < b + m; i++) {
-          const int v = sorted[i];
-          int j = i - 1;
-          while (j >= b && sorted[j] > v) {
-            sorted[j + 1] = sorted[j];
-            j--;
-          }
-          sorted[j + 1] = v;
+__device__ __forceinline__ void sort_cell(int b, int m, int* __restrict__ sorted) {
+  const int lane = threadIdx.x & 31;
+  if (m > 32 * SORT_REGS) {
+    if (lane == 0)
+      for (int i = b + 1; i < b + m; i++) {
+        const int v = sorted[i];
+        int j = i - 1;
+        while (j >= b && sorted[j] > v) {
+          sorted[j + 1] = sorted[j];
+          j--;
         }
-      continue;
-    }
-    int v[SORT_REGS], place[SORT_REGS];
-#pragma unroll
-    for (int u = 0; u < SORT_REGS; u++) {
-      v[u] = 32 * u + lane < m ? sorted[b + 32 * u + lane] : 0;
-      place[u] = 0;
-    }
-#pragma unroll
-    for (int w = 0; w < SORT_REGS; w++) {
-      if (32 * w >= m) break;
-      for (int k = 0; k < min(32, m - 32 * w); k++) {
-        const int x = __shfl_sync(0xffffffffu, v[w], k);
-#pragma unroll
-        for (int u = 0; u < SORT_REGS; u++) place[u] += x < v[u] ? 1 : 0;
+        sorted[j + 1] = v;
       }
-    }
-    __syncwarp();
+    return;
+  }
+  int v[SORT_REGS], place[SORT_REGS];
 #pragma unroll
-    for (int u = 0; u < SORT_REGS; u++)
-      if (32 * u + lane < m) sorted[b + place[u]] = v[u];
+  for (int u = 0; u < SORT_REGS; u++) {
+    v[u] = 32 * u + lane < m ? sorted[b + 32 * u + lane] : 0;
+    place[u] = 0;
+  }
+#pragma unroll
+  for (int w = 0; w < SORT_REGS; w++) {
+    if (32 * w >= m) break;
+    for (int k = 0; k < min(32, m - 32 * w); k++) {
+      const int x = __shfl_sync(0xffffffffu, v[w], k);
+#pragma unroll
+      for (int u = 0; u < SORT_REGS; u++) place[u] += x < v[u] ? 1 : 0;
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < SORT_REGS; u++)
+    if (32 * u + lane < m) sorted[b + place[u]] = v[u];
+}
+
+template <bool SPARSE>
+__global__ void k_sg_sort(const int* __restrict__ starts, int n, int* __restrict__ sorted) {
+  const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (SPARSE) {
+    const int r = 32 * warp + lane;
+    unsigned todo = __ballot_sync(0xffffffffu, r < n && starts[r + 1] - starts[r] > 1);
+    for (; todo != 0; todo &= todo - 1) {
+      const int c = 32 * warp + __ffs(todo) - 1;
+      sort_cell(starts[c], starts[c + 1] - starts[c], sorted);
+    }
+  } else if (warp < n) {
+    const int b = starts[warp], m = starts[warp + 1] - b;
+    if (m > 1) sort_cell(b, m, sorted);
   }
 }
 
@@ -296,8 +306,9 @@ __device__ __forceinline__ float nearest(float x) { return __fadd_rn(__fadd_rn(x
 // gathering each candidate's index and position: 428 us).
 // Where the chains have more cells than atoms the blocks are those of the atoms' cells
 // instead: block b takes the cell of the b-th atom in cell order, if that is its first
-// (cellOf set; forces with new lists of 2000 atoms in 54,872 cells: 206 -> 167 us).
+// (BY_ATOM; forces with new lists of 2000 atoms in 54,872 cells: 206 -> 167 us).
 constexpr int LIST_CAND = 2048, LIST_THREADS = 256, LIST_ATOMS = 2;
+template <bool BY_ATOM>
 __global__ void __launch_bounds__(LIST_THREADS) k_sg_list(const float4* __restrict__ pos, Geometry G,
                                                           const int* __restrict__ starts,
                                                           const int* __restrict__ sorted,
@@ -308,7 +319,7 @@ __global__ void __launch_bounds__(LIST_THREADS) k_sg_list(const float4* __restri
   __shared__ int first[28], base[28];   // candidates of the neighbor cells: first slot, running count
   const int M = G.M, cells = M * M * M;
   int id = blockIdx.x;
-  if (cellOf != nullptr) {
+  if (BY_ATOM) {
     const int q = sorted[blockIdx.x];
     id = q / G.N * cells + cellOf[q];
     if (starts[id] != (int)blockIdx.x) return;
@@ -1350,11 +1361,11 @@ static void sg_build_lists(Surrogate& S, const double* dR, cudaStream_t st) {
   k_sg_count<<<sg_blocks(S.total), 256, 0, st>>>(S.dPos, S.G, S.dCellOf, S.dCounts);
   k_sg_scan<<<1, 256, 0, st>>>(S.dCounts, cells, S.dStarts);
   k_sg_scatter<<<sg_blocks(S.total), 256, 0, st>>>(S.dCellOf, S.G, S.dStarts, S.dCursor, S.dSorted);
-  const int per = cells > S.total ? 32 : 1;
-  k_sg_sort<<<(cells + 8 * per - 1) / (8 * per), 256, 0, st>>>(S.dStarts, cells, per, S.dSorted);
-  k_sg_list<<<std::min(cells, S.total), LIST_THREADS, 0, st>>>(S.dPos, S.G, S.dStarts, S.dSorted,
-                                                               cells > S.total ? S.dCellOf : nullptr, S.cap, S.dList,
-                                                               S.dCount, S.dOverflow);
+  const bool sparse = cells > S.total;
+  const int per = sparse ? 256 : 8;   // cells per block
+  (sparse ? k_sg_sort<true> : k_sg_sort<false>)<<<(cells + per - 1) / per, 256, 0, st>>>(S.dStarts, cells, S.dSorted);
+  (sparse ? k_sg_list<true> : k_sg_list<false>)<<<std::min(cells, S.total), LIST_THREADS, 0, st>>>(
+      S.dPos, S.G, S.dStarts, S.dSorted, S.dCellOf, S.cap, S.dList, S.dCount, S.dOverflow);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(S.dR0, dR, sizeof(double) * 3 * S.total, cudaMemcpyDeviceToDevice, st));
 }
