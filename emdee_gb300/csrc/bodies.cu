@@ -2,8 +2,8 @@
 // and position updates, exact or NO_SQUISH rotation, kinetic energies, the
 // rigid-body virial, and momentum assignment (src/EmDeeData.f90:157-189,
 // 420-439, 823-953; src/ArBee.f90).  FP64, compiled with -fmad=false; four lanes
-// per body in the boost and the exact rotation, one thread elsewhere.  Free atoms of a system with bodies go through index-list
-// variants of the boost and move kernels.
+// per body in the boost and the exact rotation, one thread elsewhere.  Free atoms of a
+// system with bodies go through index-list variants of the boost and move kernels.
 #include <vector>
 
 #include "chain.cuh"
@@ -210,8 +210,10 @@ __global__ void __launch_bounds__(BODY_THREADS) k_body_move(BodyArgs A, double* 
   if (i < A.nb) body_move_one(A, i, R, CR, CP, dt, translate, rotate, mode);
 }
 
-// The same with the exact rotation by the series (rb_rotate_series, operation by
-// operation) on BODY_LANES lanes per body.
+// The same with the exact rotation by the series (that of rb_rotate_series, summed in the order
+// of the lanes) on BODY_LANES lanes per body.  Order and steps are those of the warp, so
+// that its 8 bodies take them together: within the bound above (8e-13 of a small first term)
+// a body's result depends on whether one of the others turns fast.
 __global__ void __launch_bounds__(BODY_GROUP_THREADS) k_body_move_series(BodyArgs A, double* __restrict__ R, double CR,
                                                                          double CP, double dt, double invdt,
                                                                          int translate) {

@@ -1620,8 +1620,9 @@ void EmDee_surrogate_adam(void* h, const float* dGrad, double lr, int step, void
 }
 
 // n velocity-Verlet steps of the chains (device FP64 R, P [chains * N][3]) on the surrogate
-// forces; F holds the forces of the current R on entry and on return.  The lists are rebuilt at
-// the start.  Returns the surrogate energies of the final positions in dE (device, [chains]).
+// forces; F holds the forces of the current R on entry and on return.  The lists are those of
+// the last call that rebuilt them (EmDee_surrogate_forces).  Returns the surrogate energies of the
+// final positions in dE (device, [chains]).
 void EmDee_surrogate_trajectory(void* h, double* dR, double* dP, double* dF, double* dE, int n, double dt,
                                 void* stream) {
   Surrogate& S = *(Surrogate*)h;
