@@ -546,7 +546,7 @@ __device__ __forceinline__ bool excluded(const BuildArgs& A, int a, int b) {
 static const int BUILD_THREADS = 512;
 static const int BUILD_THREADS_RULE = 256;
 static const int BUILD_THREADS_SPLIT = 1024;  // split build: several threads per tile atom
-enum BuildMode : int { BUILD_ONE = 0, BUILD_SPLIT, BUILD_WARP };
+enum BuildMode : int { BUILD_ONE = 0, BUILD_SPLIT, BUILD_WARP, BUILD_SPARSE };
 static const int BUILD_PAD = 4;               // halo entries past the last one, far away
 
 // List layout: for tile t, chunk c (8 entries) and tile-local atom li, the
@@ -576,12 +576,13 @@ __device__ __forceinline__ size_t nb_index(int t, int capC, int tileStride, int 
 // fill the lanes (4096 water molecules, 17 atoms per cell: 262
 // us with 8 threads per atom, 130 us so).
 // GENERAL: several atom types, bodies, exclusions or layered lists; MINIMG: M = 5.
-// Register budget: thread-per-atom variants BUILD_MAXNREG (a nearly empty box is bound by
-// its blocks of 64 threads in flight, 14 per SM and 12 with 80 registers: 1000 atoms in
-// 244,000 tiles 2575 -> 2418 us a rebuild; dense boxes the same within 0.4 %), the split one, in
-// blocks of up to 1024 threads, 64.
+// BUILD_SPARSE: BUILD_ONE for boxes with more tiles than atoms, which are bound by their
+// blocks of 64 threads in flight: 64 registers (1000 atoms in 244,000 tiles, a rebuild 2475 us
+// with 80, 2223 so).
+// Register budget: BUILD_ONE BUILD_MAXNREG (1,048,576 atoms: 565 us with 80, 569 with 72, and
+// the 72 led the tuner astray more often), the others 64, in blocks of up to 1024 threads.
 #ifndef BUILD_MAXNREG
-#define BUILD_MAXNREG 72
+#define BUILD_MAXNREG 80
 #endif
 template <bool GENERAL, bool MINIMG, int MODE>
 __global__ void __maxnreg__(MODE == BUILD_ONE ? BUILD_MAXNREG : 64) k_build(BuildArgs A) {
@@ -797,7 +798,7 @@ __global__ void __maxnreg__(MODE == BUILD_ONE ? BUILD_MAXNREG : 64) k_build(Buil
       // sentinel padding of the last chunk
       if ((n & 7) && lane < 8 - (n & 7) && n + lane < A.cap)
         myList[((n + lane) >> 3) * chunkStride + ((n + lane) & 7)] = (uint16_t)A.haloCap;
-    } else if (MODE == BUILD_ONE) {
+    } else if (MODE == BUILD_ONE || MODE == BUILD_SPARSE) {
       // rows in the order dz = -2..2 (outer), dy = -2..2 (inner); layered lists take the
       // inner entries in a first sweep and the outer ones in a second.  The last 8 entries
       // sit in four registers until they are complete.
@@ -1313,7 +1314,8 @@ static bool build_lists(System& s, bool reuse, bool defer) {
 #define BUILD_KERNEL(MODE)                                                             \
   kb = general ? (A.minimg ? k_build<true, true, MODE> : k_build<true, false, MODE>)   \
                : (A.minimg ? k_build<false, true, MODE> : k_build<false, false, MODE>)
-  if (A.tpa == 1) BUILD_KERNEL(BUILD_ONE);
+  if (A.tpa == 1 && g.nTiles > N) BUILD_KERNEL(BUILD_SPARSE);
+  else if (A.tpa == 1) BUILD_KERNEL(BUILD_ONE);
   else if (A.tpa < 32) BUILD_KERNEL(BUILD_SPLIT);
   else BUILD_KERNEL(BUILD_WARP);
 #undef BUILD_KERNEL
