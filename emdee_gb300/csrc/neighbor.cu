@@ -956,8 +956,8 @@ static int choose_tile(System& s, int M, double perCell) {
 
 // Tile edge, threads per atom and block sizes tuned on the system itself at its first
 // build (mixed precision, EMDEE_TILE unset).  For each edge from min(rule - 1, 3)
-// (from the least that gives a tile an atom in small systems, where few large tiles leave
-// most SMs idle) to 6 cells (the rule's edge always among them) a first build sizes the
+// (in small systems, where few large tiles leave most SMs idle, from the least that gives a
+// tile an atom and no SM more than 64 tiles) to 6 cells (the rule's edge always among them) a first build sizes the
 // tiles; then the list build and the pair kernel are timed with CUDA events (the faster of two
 // launches, after a warm-up launch of the pair kernel), each after a pass that moves the
 // memory traffic of an integration step, at the rule's shape and, on the edges whose cost so
@@ -1057,9 +1057,10 @@ void device_tune_tile(System& s, bool ljOnly, void (*pair)(System&)) {
   double bestRule = 1e30;
   const bool small = s.natoms < 152 * 1024;   // fewer atoms than half the GPU's threads
   int lowest = std::max(1, std::min(rule - 1, 3));
-  if (small) {   // the least edge that gives a tile an atom
+  if (small) {   // the least edge that gives a tile an atom, and no SM more than 64 tiles
     int tb = 1;
-    while (tb < lowest && perCell * (tb * tb * tb) < 1.0) tb++;
+    auto tiles = [&](int e) { return std::pow((M + e - 1) / e, 3.0); };
+    while (tb < lowest && (perCell * (tb * tb * tb) < 1.0 || tiles(tb) > 64 * 152)) tb++;
     lowest = tb;
   }
   for (int tb = lowest; tb <= std::min(6, M); tb++) {
