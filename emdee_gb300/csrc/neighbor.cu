@@ -1049,7 +1049,7 @@ void device_tune_tile(System& s, bool ljOnly, void (*pair)(System&)) {
   };
   // the rule's shape on every edge
   struct Edge {
-    int tb;
+    int tb, tileAtoms;
     double build, pair;
     double cost() const { return pair + build / 7.0; }
   };
@@ -1067,7 +1067,7 @@ void device_tune_tile(System& s, bool ljOnly, void (*pair)(System&)) {
     use_choice(s, TileChoice{tb, 0, 0, 0, 0});
     device_build_lists(s);   // sizes the tiles of this edge
     if (s.grid.TB != tb) continue;   // did not fit (halo or shared memory): the build shrank the edge
-    edges.push_back(Edge{tb, timed_build(), timed_pair()});
+    edges.push_back(Edge{tb, s.grid.tileAtoms, timed_build(), timed_pair()});
     bestRule = std::min(bestRule, edges.back().cost());
   }
   double best = 1e30, ruleCost = 1e30;
@@ -1115,7 +1115,7 @@ void device_tune_tile(System& s, bool ljOnly, void (*pair)(System&)) {
     const double cost = msPair + msBuild / 7.0;
     if (log)
       fprintf(stderr, "tile edge %d (at most %d atoms per tile): cost %.1f us, build %d x %d, pair %d x %d\n", tb,
-              s.grid.tileAtoms, 1e3 * cost, here.buildTpa, here.buildThreads, here.pairTpa, here.pairThreads);
+              e.tileAtoms, 1e3 * cost, here.buildTpa, here.buildThreads, here.pairTpa, here.pairThreads);
     if (cost < best) {
       best = cost;
       choice = here;
